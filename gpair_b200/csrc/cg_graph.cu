@@ -645,12 +645,15 @@ static int stage_table(BatchGraph *B, gpair_ctx **ctx, int n, int stage, double 
                        int prep_passes)
 {
     const bool tc = stage == GS_PREP_IMAGE || stage == GS_PREP_TRIALS || stage == GS_BUILD_W;
+    // instances on the uv grid skip the direct adjoint's stages and the others the grid's (no blocks)
     const size_t sz = tc ? gp_tc_stage_args_size(stage) : gp_stage_args_size(stage);
     std::vector<unsigned char> h(sz * (size_t)n);
     std::vector<int> start((size_t)n + 1, 0);
     int op0 = -1;
     for (int k = 0; k < n; k++) {
         int nb = 0, op = -1, rc;
+        start[k + 1] = start[k];
+        if (ctx[k]->ug ? gp_stage_direct_only(stage) : gp_stage_grid_only(stage)) continue;
         if (tc) {
             rc = gp_tc_stage_args(ctx[k], stage, h.data() + sz * k, &nb, &op, prep_passes);
             if (!rc && op0 >= 0 && op != op0) rc = GPAIR_ERR_STATE;  // one operand element type per launch
@@ -696,10 +699,12 @@ static int build_lockstep_staged(gpair_ctx **ctx_in, int n, BatchGraph *B, int w
     const int ngrp = (int)cls_begin.size() - 1;
     // adjoint classes: the same without the forward operand kind (key >> 3), contiguous in key order
     std::vector<int> acls_begin;
-    for (int k = 0; k < n; k++)
-        if (acls_begin.empty() || (key[order[k]] >> 3) != (key[order[k - 1]] >> 3) || k - acls_begin.back() == 256)
-            acls_begin.push_back(k);
-    acls_begin.push_back(n);
+    int ndirect = 0;  // instances on the uv grid come last and have no adjoint contraction
+    for (; ndirect < n && !ctx[ndirect]->ug; ndirect++)
+        if (acls_begin.empty() || (key[order[ndirect]] >> 3) != (key[order[ndirect - 1]] >> 3) ||
+            ndirect - acls_begin.back() == 256)
+            acls_begin.push_back(ndirect);
+    acls_begin.push_back(ndirect);
     const int nadj = (int)acls_begin.size() - 1;
     // every instance's tensor state and batch buffers (no allocation inside a capture)
     for (int k = 0; k < n; k++) {
@@ -727,7 +732,7 @@ static int build_lockstep_staged(gpair_ctx **ctx_in, int n, BatchGraph *B, int w
     B->ngrp = ngrp;
     B->grps = (void **)calloc((size_t)ngrp, sizeof(void *));
     B->grps_img = (void **)calloc((size_t)ngrp, sizeof(void *));
-    B->grps_adj = (void **)calloc((size_t)nadj, sizeof(void *));
+    B->grps_adj = (void **)calloc((size_t)nadj + 1, sizeof(void *));
     if (!B->grps || !B->grps_img || !B->grps_adj) return GPAIR_ERR_ALLOC;
     B->nadj = nadj;
     int rc = GPAIR_OK;
@@ -758,6 +763,7 @@ static int build_lockstep_staged(gpair_ctx **ctx_in, int n, BatchGraph *B, int w
 
     auto stage = [&](int st, const int *gate) {
         const bool tc = st == GS_PREP_IMAGE || st == GS_PREP_TRIALS || st == GS_BUILD_W;
+        if (!B->stg_total[st]) return (int)GPAIR_OK;  // no instance takes part
         return tc ? gp_tc_stage_group_launch(c0, st, op_prep, B->stg_args[st], B->stg_start[st], n, B->stg_total[st],
                                              gate)
                   : gp_stage_group_launch(c0, st, B->stg_args[st], B->stg_start[st], n, B->stg_total[st], gate);
@@ -807,12 +813,16 @@ static int build_lockstep_staged(gpair_ctx **ctx_in, int n, BatchGraph *B, int w
         [&]() {
             int r;
             if ((r = stamp(0)) || (r = stage(GS_PREP_IMAGE, act)) || (r = stamp(1))) return r;
-            if ((r = gemms(B->grps_img, cls_begin)) || (r = stamp(2))) return r;
+            if ((r = gemms(B->grps_img, cls_begin)) || (r = stage(GS_UG_ROWS, act)) || (r = stage(GS_UG_INTERP, act)) ||
+                (r = stamp(2)))
+                return r;
             if ((r = stage(GS_VIS_DATA, act)) || (r = stamp(3))) return r;
             if ((r = stage(GS_ADJ_WEIGHTS, act)) || (r = stamp(4))) return r;
-            if ((r = stage(GS_BUILD_W, act)) || (r = stamp(5))) return r;
-            if ((r = gemms(B->grps_adj, acls_begin)) || (r = stamp(6))) return r;
-            if ((r = stage(GS_GRAD_FINALIZE, act)) || (r = stamp(7))) return r;
+            if ((r = stage(GS_BUILD_W, act)) || (r = stage(GS_UG_SPREAD, act)) || (r = stamp(5))) return r;
+            if ((r = gemms(B->grps_adj, acls_begin)) || (r = stage(GS_UG_GATHER, act)) || (r = stage(GS_UG_COLS, act)) ||
+                (r = stamp(6)))
+                return r;
+            if ((r = stage(GS_GRAD_FINALIZE, act)) || (r = stage(GS_UG_GRAD, act)) || (r = stamp(7))) return r;
             if ((r = stage(GS_DESCENT, act)) || (r = stamp(8))) return r;
             if ((r = route(GR_LS0S, h_ls))) return r;
             return stamp(9);
@@ -839,7 +849,9 @@ static int build_lockstep_staged(gpair_ctx **ctx_in, int n, BatchGraph *B, int w
         [&]() {
             int r;
             if ((r = stamp(10)) || (r = stage(GS_PREP_TRIALS, lsg)) || (r = stamp(11))) return r;
-            if ((r = gemms(B->grps, cls_begin)) || (r = stamp(12))) return r;
+            if ((r = gemms(B->grps, cls_begin)) || (r = stage(GS_UG_ROWS_T, lsg)) || (r = stage(GS_UG_INTERP_T, lsg)) ||
+                (r = stamp(12)))
+                return r;
             if ((r = stage(GS_CHI2_BATCH, lsg)) || (r = stamp(13))) return r;
             if ((r = route(GR_LSN, h_ls))) return r;
             return stamp(14);

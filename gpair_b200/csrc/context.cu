@@ -59,6 +59,7 @@ static void free_problem(gpair_ctx *c)
     FREE_DEV(c->trib); FREE_DEV(c->cw); FREE_DEV(c->inc_off); FREE_DEV(c->inc_idx); FREE_DEV(c->gpart);
     gp_batch_free(c);
     gp_tc_free(c);
+    gp_ug_free(c);
     c->have_problem = 0;
 }
 
@@ -189,6 +190,22 @@ int gp_build_incidence(gpair_ctx *c, const int64_t *uvpnt)
     return GPAIR_OK;
 }
 
+// What the direct contractions need: tables, partial visibility entries (the
+// CUDA-core forward's row tiles or the tensor forward's entries) and split-K
+// partial images. A problem on the uv grid has none until a precision mode
+// that takes the direct contractions is set.
+int gp_direct_prepare(gpair_ctx *c)
+{
+    if (c->fx) return GPAIR_OK;
+    const size_t nk = c->nuv ? c->nuv : 1;
+    const int mt = gp_cdiv(c->N, 64), mt_cap = mt > gp_tc_forward_entries(c->N) ? mt : gp_tc_forward_entries(c->N);
+    if (!c->vpart) GP_CUDA(c, cudaMalloc(&c->vpart, (size_t)mt_cap * nk * sizeof(float2)));
+    if (!c->gpart) GP_CUDA(c, cudaMalloc(&c->gpart, (size_t)c->gpart_cap * c->npix * sizeof(float)));
+    if (!c->fy) GP_CUDA(c, cudaMalloc(&c->fy, nk * c->N * sizeof(float2)));
+    GP_CUDA(c, cudaMalloc(&c->fx, nk * c->N * sizeof(float2)));  // last: its presence says that all exist
+    return c->have_uv ? gp_gen_twiddles(c) : GPAIR_OK;
+}
+
 // Problem upload. uv may be NULL when the twiddles are supplied as tables
 // afterwards (reference boundary path, gpu_copy_dft).
 int gp_set_problem_core(gpair_ctx *c, int N, float pix, int nuv, const gpair_uv *uv, int npow, int nbis,
@@ -225,18 +242,12 @@ int gp_set_problem_core(gpair_ctx *c, int N, float pix, int nuv, const gpair_uv 
     GP_CUDA(c, cudaMalloc(&c->tri, nt * sizeof(int4)));
     GP_CUDA(c, cudaMalloc(&c->phasor, nt * sizeof(float2)));
     GP_CUDA(c, cudaMalloc(&c->uvc, nk * sizeof(float2)));
-    GP_CUDA(c, cudaMalloc(&c->fx, nk * N * sizeof(float2)));
-    GP_CUDA(c, cudaMalloc(&c->fy, nk * N * sizeof(float2)));
-    // partial visibility entries: the CUDA-core forward's row tiles or the tensor forward's entries
-    const int mt_cap = c->mt > gp_tc_forward_entries(N) ? c->mt : gp_tc_forward_entries(N);
-    GP_CUDA(c, cudaMalloc(&c->vpart, (size_t)mt_cap * nk * sizeof(float2)));
     GP_CUDA(c, cudaMalloc(&c->visd, nk * sizeof(double2)));
     GP_CUDA(c, cudaMalloc(&c->visi, nk * sizeof(float2)));
     GP_CUDA(c, cudaMalloc(&c->cw, nk * sizeof(float2)));
     GP_CUDA(c, cudaMalloc(&c->trib, 3 * nt * sizeof(float2)));
     // room for twice the default split count: the autotuner may shorten the split-K tiles
     c->gpart_cap = 2 * max_splits;
-    GP_CUDA(c, cudaMalloc(&c->gpart, (size_t)c->gpart_cap * c->npix * sizeof(float)));
     GP_CUDA(c, cudaMemsetAsync(c->mock, 0, nd * sizeof(float), c->stream));
     GP_CUDA(c, cudaMemsetAsync(c->visd, 0, nk * sizeof(double2), c->stream));
     GP_CUDA(c, cudaMemsetAsync(c->visi, 0, nk * sizeof(float2), c->stream));
@@ -267,9 +278,10 @@ int gp_set_problem_core(gpair_ctx *c, int N, float pix, int nuv, const gpair_uv 
         std::vector<float2> uvc(nuv);
         for (int k = 0; k < nuv; k++) uvc[k] = make_float2(uv[k].u, uv[k].v);
         GP_CUDA(c, cudaMemcpyAsync(c->uvc, uvc.data(), nuv * sizeof(float2), cudaMemcpyHostToDevice, c->stream));
-        rc = gp_gen_twiddles(c);
-        if (rc) return rc;
+        if ((rc = gp_ug_plan(c, uv))) return rc;
     }
+    gp_ug_choose(c);
+    if (!c->ug && (rc = gp_direct_prepare(c))) return rc;
     rc = gp_build_incidence(c, uvpnt);
     if (rc) return rc;
     c->have_problem = 1;
@@ -295,10 +307,13 @@ extern "C" int gpair_set_precision(gpair_ctx *c, int mode)
     if (!c || mode < GPAIR_PREC_FP32 || mode > GPAIR_PREC_SPLIT16F8) return GPAIR_ERR_INVALID;
     int old = c->precision;
     c->precision = mode;
-    if (mode != GPAIR_PREC_FP32 && c->have_problem) {
-        int rc = gp_tc_prepare(c);
+    if (c->have_problem) {
+        gp_ug_choose(c);
+        int rc = c->ug ? GPAIR_OK : gp_direct_prepare(c);
+        if (!rc && mode != GPAIR_PREC_FP32) rc = gp_tc_prepare(c);
         if (rc) {
             c->precision = old;
+            gp_ug_choose(c);
             return rc;
         }
     }
@@ -1116,9 +1131,10 @@ extern "C" int gpair_time_stages(gpair_ctx *c, int reps, double *ms, int max_sta
         if ((rc = gp_vis_data(c))) break;
         cudaEventRecord(E[3], c->stream);
         if ((rc = gp_adj_weights_only(c))) break;
-        if (tc && (rc = gp_tc_build_w(c))) break;
+        const bool direct_tc = tc && !c->ug;
+        if (direct_tc && (rc = gp_tc_build_w(c))) break;
         cudaEventRecord(E[4], c->stream);
-        if ((rc = tc ? gp_tc_adjoint_gemm(c) : gp_adjoint_contraction(c, GPAIR_IMG_CURR))) break;
+        if ((rc = direct_tc ? gp_tc_adjoint_gemm(c) : gp_adjoint_contraction(c, GPAIR_IMG_CURR))) break;
         cudaEventRecord(E[5], c->stream);
         if ((rc = gp_grad_finalize(c, GPAIR_IMG_CURR, GRAD_FUSED, 1e-3f))) break;
         cudaEventRecord(E[6], c->stream);

@@ -254,6 +254,9 @@ struct gpair_ctx {
 
     // tensor-core operand buffers (GPAIR_PREC_SPLIT16 / TF32), see umma path
     void *tc_state;
+    // the DFT and its adjoint through a grid of the uv plane (uvgrid.cu): the problem's plan (UgState), or
+    // null; ug is the plan where the precision mode takes it, null: the direct contractions
+    void *ug_plan, *ug;
 
     // handles for layer 1
     gpair_buf h_image, h_image_temp, h_fgn, h_fg, h_dd, h_tg, h_eg, h_dg, h_model;
@@ -480,8 +483,19 @@ enum {
     GS_CHI2_BATCH = 7,   // chi2 of every trial, then CTRL_AFTER_BATCH
     GS_UPDATE = 8,       // image update with the accepted step, gradient backup
     GS_CTRL_END = 9,     // end of the iteration (trace row)
-    GS_COUNT = 10
+    // instances that take the uv grid (uvgrid.cu), in place of GS_BUILD_W and GS_GRAD_FINALIZE
+    GS_UG_ROWS = 10,     // grid values of the current image
+    GS_UG_INTERP = 11,   // its visibilities
+    GS_UG_SPREAD = 12,   // adjoint: per-cell patches, then the grid, then its columns
+    GS_UG_GATHER = 13,
+    GS_UG_COLS = 14,
+    GS_UG_GRAD = 15,     // gradient of the current image, then CTRL_BEGIN
+    GS_UG_ROWS_T = 16,   // the batched trials' grid values and visibilities
+    GS_UG_INTERP_T = 17,
+    GS_COUNT = 18
 };
+static inline bool gp_stage_grid_only(int st) { return st >= GS_UG_ROWS; }
+static inline bool gp_stage_direct_only(int st) { return st == GS_BUILD_W || st == GS_GRAD_FINALIZE; }
 size_t gp_stage_args_size(int stage);
 int gp_stage_args(gpair_ctx *c, int stage, double *trace, void *out, int *nblocks);
 int gp_stage_group_launch(gpair_ctx *c, int stage, const void *d_args, const int *d_start, int n, int total,
@@ -494,6 +508,25 @@ int gp_tc_stage_args(gpair_ctx *c, int stage, void *out, int *nblocks, int *op, 
 int gp_tc_prep_trials_passes(gpair_ctx *const *ctx, int n, int op);
 int gp_tc_stage_group_launch(gpair_ctx *c, int stage, int op, const void *d_args, const int *d_start, int n,
                              int total, const int *gate);
+// tables and partial-sum buffers of the direct contractions (no-op when they exist)
+int gp_direct_prepare(gpair_ctx *c);
+// uv grid (uvgrid.cu): plan of a problem (none where no mode would take it), the choice for the
+// context's precision mode (sets c->ug), x contraction on the CUDA cores, visibilities from T
+// (1 or GP_NTR images), adjoint up to S
+int gp_ug_plan(gpair_ctx *c, const gpair_uv *uv);
+void gp_ug_choose(gpair_ctx *c);
+void gp_ug_free(gpair_ctx *c);
+int gp_ug_batch_alloc(gpair_ctx *c);
+int gp_tc_stack_rows(int N);  // rows per image of the batched trials' operand stack
+int gp_ug_x(gpair_ctx *c, const float *img, int images);
+int gp_ug_vis(gpair_ctx *c, int images);
+int gp_ug_adjoint(gpair_ctx *c);
+size_t gp_ug_stage_args_size(int stage);
+int gp_ug_stage_args(gpair_ctx *c, int stage, void *out, int *nblocks);
+int gp_ug_stage_group_launch(gpair_ctx *c, int stage, const void *d_args, const int *d_start, int n, int total,
+                             const int *gate);
+// the tensor path's T: row scales, rows per image and partial sums (1 or GP_NTR images)
+int gp_tc_ug_rows(gpair_ctx *c, int images, const float **rsc, int *lrows, int *splits);
 int gp_tc_build_w(gpair_ctx *c);
 int gp_tc_adjoint_gemm(gpair_ctx *c);
 int gp_tc_prep_split_trial(gpair_ctx *c);

@@ -36,6 +36,7 @@
 #include "group.cuh"
 #include "reduce.cuh"
 #include "umma.cuh"
+#include "uvgrid.cuh"
 
 __device__ void cg_control(DevScalars *__restrict__ sc, int what);
 __device__ void cg_set_handles(DevScalars *__restrict__ sc, int what, cudaGraphConditionalHandle h_iter,
@@ -279,6 +280,10 @@ int gp_forward(gpair_ctx *c, int which)
         return GPAIR_ERR_STATE; // tensor path requested but unavailable: fail loudly
     }
     const float *img = (which == GPAIR_IMG_TEMP) ? c->image_temp : c->image;
+    if (c->ug) {
+        int rc = gp_ug_x(c, img, 1);
+        return rc ? rc : gp_ug_vis(c, 1);
+    }
     c->mt = gp_cdiv(c->N, FB_M);
     dim3 grid(gp_cdiv(c->nuv, FB_K), c->mt);
     k_fwd_simt<<<grid, 256, 0, c->stream>>>(img, c->fx, c->fy, c->N, c->nuv, c->vpart, nullptr);
@@ -458,6 +463,7 @@ __global__ void __launch_bounds__(GP_THREADS) k_vis_sum(const float2 *__restrict
 
 static int vis_data_launch(gpair_ctx *c, int direct)
 {
+    if (c->ug) direct = 1;  // the grid's forward leaves V in visd
     if (!direct && c->mt > VIS_PRESUM_ENTRIES && c->nuv > 0) {
         int nb = gp_cdiv(c->nuv, GP_THREADS);
         if (nb > 4 * 148) nb = 4 * 148;
@@ -699,6 +705,7 @@ int gp_adjoint(gpair_ctx *c, int which)
 
 int gp_adjoint_contraction(gpair_ctx *c, int which)
 {
+    if (c->ug) return gp_ug_adjoint(c);
     if (c->precision != GPAIR_PREC_FP32) return gp_tc_adjoint(c, which);
     int S = c->splits_simt;
     int kchunk = gp_cdiv(c->nuv, S);
@@ -900,8 +907,190 @@ static GradFinalizeArgs grad_finalize_args(gpair_ctx *c, int which, int mode, fl
     return a;
 }
 
+// --------------------------- adjoint x contraction and gradient assembly
+//
+// Pixels (y, h) and (y, N-1-h): even = sum_jx Re S cos, odd = sum_jx Im S sin,
+// g = even -+ odd. FP32 FMAs, K = nbx; then the data gradient, the entropy and
+// full gradients and the CG dot products as in k_grad_finalize. A block makes
+// 16 m image rows x 16 m folded columns, m x m of them per thread.
+struct UgGradArgs {
+    const float2 *S, *ftab;
+    int N, H, gw, m, mode;
+    const float *img, *model;
+    float alpha;
+    int alpha_from_state;
+    float *data_grad, *entropy_grad, *out;
+    const float *g_old, *d;
+    int dot_slot;
+    double *partials;
+    DevScalars *sc;
+    FusedCtrl fc;
+    GP_VGRID_FIELDS;
+};
+
+template <int M>
+__device__ __forceinline__ void ug_grad_body(const UgGradArgs &A, const GpVGrid &vg)
+{
+    constexpr int T = 16 * M, K = 64 / M;
+    __shared__ float2 Ss[K][T + 1];  // [jx][y]
+    __shared__ float2 Fs[K][T + 1];  // [jx][h]
+    __shared__ double smem[4 * 32];
+    const int N = A.N, H = A.H, mode = A.mode;
+    DevScalars *__restrict__ sc = A.sc;
+    const int ht = (H + T - 1) / T;
+    const int y0 = (vg.bx / ht) * T, h0 = (vg.bx % ht) * T;
+    const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
+    double even[M][M], odd[M][M];
+#pragma unroll
+    for (int i = 0; i < M; i++)
+#pragma unroll
+        for (int j = 0; j < M; j++) even[i][j] = odd[i][j] = 0.0;
+    for (int k0 = 0; k0 < A.gw; k0 += K) {
+        const int nk = min(K, A.gw - k0);
+#pragma unroll
+        for (int e0 = 0; e0 < K * T; e0 += 256) {
+            const int e = e0 + threadIdx.x;
+            const int ks = e % K, y = y0 + e / K;  // rows of S are contiguous in jx
+            Ss[ks][e / K] = (y < N && ks < nk) ? __ldg(&A.S[(size_t)y * A.gw + k0 + ks]) : make_float2(0.f, 0.f);
+            const int k = e / T, r = e % T, h = h0 + r;
+            Fs[k][r] = (h < H && k < nk) ? __ldg(&A.ftab[(size_t)(k0 + k) * H + h]) : make_float2(0.f, 0.f);
+        }
+        __syncthreads();
+        for (int k1 = 0; k1 < nk; k1 += 16) {  // FP32 over 16 columns (zeros past nk), FP64 over the sixteens
+            float2 acc[M][M];
+#pragma unroll
+            for (int i = 0; i < M; i++)
+#pragma unroll
+                for (int j = 0; j < M; j++) acc[i][j] = make_float2(0.f, 0.f);
+#pragma unroll
+            for (int k = 0; k < 16; k++) {
+                float2 s[M], f[M];
+#pragma unroll
+                for (int i = 0; i < M; i++) {
+                    s[i] = Ss[k1 + k][ty + 16 * i];
+                    f[i] = Fs[k1 + k][tx + 16 * i];
+                }
+#pragma unroll
+                for (int i = 0; i < M; i++)
+#pragma unroll
+                    for (int j = 0; j < M; j++) {
+                        acc[i][j].x = fmaf(s[i].x, f[j].x, acc[i][j].x);
+                        acc[i][j].y = fmaf(s[i].y, f[j].y, acc[i][j].y);
+                    }
+            }
+#pragma unroll
+            for (int i = 0; i < M; i++)
+#pragma unroll
+                for (int j = 0; j < M; j++) {
+                    even[i][j] += (double)acc[i][j].x;
+                    odd[i][j] += (double)acc[i][j].y;
+                }
+        }
+        __syncthreads();
+    }
+    const double C = sc->adj_c;
+    const int reg_kind = sc->reg_kind;
+    const float alpha = A.alpha_from_state ? (float)sc->cg.alpha : A.alpha;
+    double dots[4] = {0.0, 0.0, 0.0, 0.0};
+    const float *__restrict__ img = A.img, *__restrict__ model = A.model, *__restrict__ g_old = A.g_old;
+    const float *__restrict__ dir = A.d;
+#pragma unroll
+    for (int i = 0; i < M; i++) {
+        // the 2 M pixels of one image row at a time: every load before the first use
+        const int y = y0 + ty + 16 * i;
+        int p[2 * M];
+        float I[2 * M], m[2 * M], e[2 * M], go[2 * M], d[2 * M];
+#pragma unroll
+        for (int j = 0; j < M; j++) {
+            const int h = h0 + tx + 16 * j;
+            const bool ok = y < N && h < H;
+            p[2 * j] = ok ? y * N + (N - 1 - h) : -1;
+            p[2 * j + 1] = ok && N - 1 - h != h ? y * N + h : -1;
+        }
+#pragma unroll
+        for (int q = 0; q < 2 * M; q++)
+            if (mode == GRAD_FUSED && p[q] >= 0) {
+                I[q] = img[p[q]];
+                m[q] = model[p[q]];
+                e[q] = A.entropy_grad[p[q]];
+                go[q] = g_old[p[q]];
+                d[q] = dir[p[q]];
+            }
+#pragma unroll
+        for (int q = 0; q < 2 * M; q++) {
+            if (p[q] < 0) continue;
+            const double g = (q & 1) ? even[i][q / 2] + odd[i][q / 2] : even[i][q / 2] - odd[i][q / 2];
+            const float gd = (float)(g - C);
+            A.data_grad[p[q]] = gd;
+            if (mode == GRAD_FUSED) {
+                const float eg = reg_grad(I[q], m[q], e[q], reg_kind);
+                A.entropy_grad[p[q]] = eg;
+                const float fg = gd - alpha * eg;
+                A.out[p[q]] = fg;
+                const double fgd = fg;
+                dots[0] += fgd * fgd;
+                dots[1] += fgd * (double)go[q];
+                dots[2] += fgd * (double)d[q];
+                dots[3] += (double)d[q] * (double)go[q];
+            }
+        }
+    }
+    if (mode != GRAD_FUSED) return;
+    block_sum<4>(dots, smem);
+    if (threadIdx.x == 0)
+        for (int i = 0; i < 4; i++) A.partials[4 * vg.bx + i] = dots[i];
+    if (last_block_of(&sc->counter[RED_GRAD], vg.nbx)) {
+        double o[4];
+        finish_sum<4>(A.partials, vg.nbx, o, smem);
+        if (threadIdx.x == 0) {
+            for (int i = 0; i < 4; i++) sc->grad_dots[A.dot_slot][i] = o[i];
+            if (!isfinite(o[0])) sc->nonfinite |= 4u;
+            sc->counter[RED_GRAD] = 0;
+            run_fused_ctrl(sc, A.fc);
+        }
+    }
+}
+
+template <int M>
+__global__ void __launch_bounds__(256) k_ug_grad(const UgGradArgs a)
+{
+    gp_pdl_enter();
+    ug_grad_body<M>(a, gp_vgrid_hw());
+}
+
+struct UgGradOp {
+    using Args = UgGradArgs;
+    static __device__ __forceinline__ void run(const Args &a, const GpVGrid &v)
+    {
+        if (a.m == 4) ug_grad_body<4>(a, v);
+        else ug_grad_body<2>(a, v);
+    }
+};
+
+// Pixels per thread and side: two where the tiles' partial sums fit, else four. The pixels' FP64
+// logarithms want warps more than the contraction wants register tiles: at 1024^2 four a side (128
+// blocks) took 62 us, two (512 blocks) 20.
+static int ug_grad_m(int N) { return gp_cdiv(N, 32) * gp_cdiv((N + 1) / 2, 32) <= GP_MAX_PARTIALS ? 2 : 4; }
+
+static UgGradArgs ug_grad_args(gpair_ctx *c, int which, int mode, float alpha, FusedCtrl fc)
+{
+    const UgState *g = (const UgState *)c->ug;
+    const int m = ug_grad_m(g->N), T = 16 * m;
+    UgGradArgs a = {g->S, g->ftab, g->N, g->H, g->nbx, m, mode, which == GPAIR_IMG_TEMP ? c->image_temp : c->image,
+                    c->model, alpha, alpha < 0.f, c->data_grad, c->entropy_grad,
+                    which == GPAIR_IMG_TEMP ? c->grad_temp : c->full_grad_new, c->full_grad, c->descent_dir,
+                    which == GPAIR_IMG_TEMP ? 1 : 0, slot_partials(c, RED_GRAD), c->sc, fc,
+                    gp_cdiv(g->N, T) * gp_cdiv(g->H, T), 1};
+    return a;
+}
+
 int gp_grad_finalize(gpair_ctx *c, int which, int mode, float alpha)
 {
+    if (c->ug) {
+        const UgGradArgs a = ug_grad_args(c, which, mode, alpha, take_fused_ctrl(c));
+        GP_LAUNCH(c, gp_launch(c, ug_grad_m(c->N) == 4 ? k_ug_grad<4> : k_ug_grad<2>, dim3(a.nbx), dim3(256), 0, a));
+        return GPAIR_OK;
+    }
     const GradFinalizeArgs a = grad_finalize_args(c, which, mode, alpha, take_fused_ctrl(c));
     GP_LAUNCH(c, gp_launch(c, k_grad_finalize, dim3(a.nbx), dim3(GP_THREADS), 0, a));
     return GPAIR_OK;
@@ -1518,14 +1707,19 @@ int gp_batch_alloc(gpair_ctx *c)
         int rc = gp_tc_batch_prepare(c, &epp_tc);
         if (rc) return rc;
     }
-    if (c->image_trials) return GPAIR_OK;
+    if (c->ug) {
+        int rc = gp_ug_batch_alloc(c);
+        if (rc) return rc;
+    }
+    // the partial entries of any precision mode's direct forward (tensor: one per TC_EPI_COLS rows)
+    const size_t nk = (size_t)GP_NTR * (c->nuv ? c->nuv : 1);
     const int mt_simt = gp_cdiv(c->N, FB_M);
     const int epp_max = mt_simt > epp_tc ? mt_simt : epp_tc;
+    if (!c->ug && !c->vpart_b) GP_CUDA(c, cudaMalloc(&c->vpart_b, sizeof(float2) * epp_max * nk));
+    if (!c->visb && (c->ug || epp_max > VIS_PRESUM_ENTRIES)) GP_CUDA(c, cudaMalloc(&c->visb, sizeof(double2) * nk));
+    if (c->image_trials) return GPAIR_OK;
     GP_CUDA(c, cudaMalloc(&c->image_trials, sizeof(float) * (size_t)GP_NTR * c->npix));
-    GP_CUDA(c, cudaMalloc(&c->vpart_b, sizeof(float2) * (size_t)GP_NTR * epp_max * (c->nuv ? c->nuv : 1)));
     GP_CUDA(c, cudaMalloc(&c->partials_b, sizeof(double) * (size_t)GP_NTR * 1024 * 2));
-    if (epp_max > VIS_PRESUM_ENTRIES)
-        GP_CUDA(c, cudaMalloc(&c->visb, sizeof(double2) * (size_t)GP_NTR * (c->nuv ? c->nuv : 1)));
     int nsm = 148;
     GP_CUDA(c, cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, c->device));
     c->batch_wave[0] = batch_wave_blocks((const void *)k_trials_prep, nsm);
@@ -1535,7 +1729,7 @@ int gp_batch_alloc(gpair_ctx *c)
 
 void gp_batch_free(gpair_ctx *c)
 {
-    if (c->image_trials) c->buf_gen++;
+    if (c->image_trials || c->vpart_b || c->visb) c->buf_gen++;
     if (c->image_trials) cudaFree(c->image_trials);
     if (c->vpart_b) cudaFree(c->vpart_b);
     if (c->partials_b) cudaFree(c->partials_b);
@@ -1565,7 +1759,7 @@ static VisChi2BatchArgs batch_chi2_args(gpair_ctx *c, int epp, FusedCtrl fc, con
     if (nb > c->batch_wave[1]) nb = c->batch_wave[1];  // one wave over the batch
     if (nb > 1024) nb = 1024;
     if (nb < 1) nb = 1;
-    const double2 *vb = (presum && epp > VIS_PRESUM_ENTRIES && c->visb) ? c->visb : nullptr;
+    const double2 *vb = (c->ug || (presum && epp > VIS_PRESUM_ENTRIES && c->visb)) ? c->visb : nullptr;
     VisChi2BatchArgs a = {c->vpart_b, epp, c->nuv, c->npow, c->nbis, c->data, c->data_err, c->tri, c->phasor,
                           c->partials_b, c->sc, fc, gate, vb, nb, GP_NTR};
     return a;
@@ -1574,7 +1768,7 @@ static VisChi2BatchArgs batch_chi2_args(gpair_ctx *c, int epp, FusedCtrl fc, con
 static int batch_chi2(gpair_ctx *c, int epp)
 {
     const VisChi2BatchArgs a = batch_chi2_args(c, epp, take_fused_ctrl(c), c->gate, 1);
-    if (a.visb) {
+    if (a.visb && !c->ug) {  // the grid's forward leaves the trials' V there
         int nb = gp_cdiv(c->nuv, GP_THREADS);
         if (nb > 148) nb = 148;  // 8 trials: about eight blocks per SM
         GP_LAUNCH(c, gp_launch(c, k_vis_sum_batch, dim3(nb, GP_NTR), dim3(GP_THREADS), 0, (const float2 *)c->vpart_b,
@@ -1607,9 +1801,13 @@ static int eval_batch(gpair_ctx *c, cudaEvent_t *ev)
         if (ev) cudaEventRecord(ev[1], c->stream);
         gp_stage_begin(c, 1);
         epp = gp_cdiv(c->N, FB_M);
-        dim3 grid(gp_cdiv(c->nuv, FB_K), epp, GP_NTR);
-        k_fwd_simt<<<grid, 256, 0, c->stream>>>(c->image_trials, c->fx, c->fy, c->N, c->nuv, c->vpart_b, c->gate);
-        GP_LAUNCH_CHECK(c);
+        if (c->ug) {
+            if ((rc = gp_ug_x(c, c->image_trials, GP_NTR)) || (rc = gp_ug_vis(c, GP_NTR))) return rc;
+        } else {
+            dim3 grid(gp_cdiv(c->nuv, FB_K), epp, GP_NTR);
+            k_fwd_simt<<<grid, 256, 0, c->stream>>>(c->image_trials, c->fx, c->fy, c->N, c->nuv, c->vpart_b, c->gate);
+            GP_LAUNCH_CHECK(c);
+        }
     }
     gp_stage_end(c);
     if (ev) cudaEventRecord(ev[2], c->stream);
@@ -1630,6 +1828,7 @@ int gp_eval_batch_part(gpair_ctx *c, int part)
     if (c->precision == GPAIR_PREC_FP32) return GPAIR_ERR_STATE;
     if (part == 1) return gp_tc_trials_prep_split(c, c->partials_b);
     if ((rc = gp_tc_batch_prepare(c, nullptr))) return rc;
+    if (c->ug && (rc = gp_ug_vis(c, GP_NTR))) return rc;
     return batch_chi2(c, c->epp);
 }
 
@@ -1673,12 +1872,34 @@ __global__ void k_update_pixel_vis(const float2 *__restrict__ fx, const float2 *
     visd[k] = make_double2((F * V.x + d * er) * inv, (F * V.y + d * ei) * inv);
 }
 
+// The same where the problem keeps no tables: Fx[k][x] and Fy[k][y] as k_gen_twiddles forms them
+__global__ void k_update_pixel_vis_uv(const float2 *__restrict__ uvc, float pix, int nuv, int x, int y,
+                                      double2 *__restrict__ visd, const DevScalars *__restrict__ sc)
+{
+    const int k = blockIdx.x * blockDim.x + threadIdx.x;
+    if (k >= nuv) return;
+    const float2 uv = uvc[k];
+    double tu = RPMAS_D * (double)pix * (double)uv.x * (double)x, tv = RPMAS_D * (double)pix * (double)uv.y * (double)y;
+    tu -= rint(tu);
+    tv -= rint(tv);
+    double su, cu, sv, cv;
+    sincospi(2.0 * tu, &su, &cu);
+    sincospi(2.0 * tv, &sv, &cv);
+    const double er = cu * cv + su * sv, ei = su * cv - cu * sv;
+    const double F = sc->upd_flux_old, d = sc->upd_delta, inv = sc->invflux;
+    const double2 V = visd[k];
+    visd[k] = make_double2((F * V.x + d * er) * inv, (F * V.y + d * ei) * inv);
+}
+
 int gp_update_pixel(gpair_ctx *c, int x, int y, float value)
 {
     const int p = x + y * c->N;
     k_update_pixel_scalar<<<1, 32, 0, c->stream>>>(c->image, c->model, p, value, c->sc);
     GP_LAUNCH_CHECK(c);
-    if (c->nuv) {
+    if (c->ug) {
+        k_update_pixel_vis_uv<<<gp_cdiv(c->nuv, 256), 256, 0, c->stream>>>(c->uvc, c->pix, c->nuv, x, y, c->visd, c->sc);
+        GP_LAUNCH_CHECK(c);
+    } else if (c->nuv) {
         k_update_pixel_vis<<<gp_cdiv(c->nuv, 256), 256, 0, c->stream>>>(c->fx, c->fy, c->N, c->nuv, x, y, c->visd,
                                                                        c->sc);
         GP_LAUNCH_CHECK(c);
@@ -2237,7 +2458,8 @@ size_t gp_stage_args_size(int stage)
     case GS_CHI2_BATCH: return sizeof(VisChi2BatchArgs);
     case GS_UPDATE: return sizeof(UpdateImageArgs);
     case GS_CTRL_END: return sizeof(CtrlArgs);
-    default: return gp_tc_stage_args_size(stage);
+    case GS_UG_GRAD: return sizeof(UgGradArgs);
+    default: return gp_stage_grid_only(stage) ? gp_ug_stage_args_size(stage) : gp_tc_stage_args_size(stage);
     }
 }
 
@@ -2252,7 +2474,7 @@ static int put_args(const A &a, void *out, int *nblocks)
 int gp_stage_args(gpair_ctx *c, int stage, double *trace, void *out, int *nblocks)
 {
     switch (stage) {
-    case GS_VIS_DATA: return put_args(vis_data_args(c, 0, ctrl_only(-1)), out, nblocks);
+    case GS_VIS_DATA: return put_args(vis_data_args(c, c->ug ? 1 : 0, ctrl_only(-1)), out, nblocks);
     case GS_ADJ_WEIGHTS: return put_args(adj_weights_args(c), out, nblocks);
     case GS_GRAD_FINALIZE:
         return put_args(grad_finalize_args(c, GPAIR_IMG_CURR, GRAD_FUSED, -1.f, ctrl_only(CTRL_BEGIN)), out, nblocks);
@@ -2264,7 +2486,9 @@ int gp_stage_args(gpair_ctx *c, int stage, double *trace, void *out, int *nblock
         const CtrlArgs a = {c->sc, CTRL_END, 0, 0, 0, trace, 1, 1, 1};
         return put_args(a, out, nblocks);
     }
-    default: return GPAIR_ERR_INVALID;
+    case GS_UG_GRAD:
+        return put_args(ug_grad_args(c, GPAIR_IMG_CURR, GRAD_FUSED, -1.f, ctrl_only(CTRL_BEGIN)), out, nblocks);
+    default: return gp_stage_grid_only(stage) ? gp_ug_stage_args(c, stage, out, nblocks) : GPAIR_ERR_INVALID;
     }
 }
 
@@ -2288,6 +2512,9 @@ int gp_stage_group_launch(gpair_ctx *c, int stage, const void *d_args, const int
     case GS_CHI2_BATCH: return group_launch<VisChi2BatchOp, GP_THREADS>(c, d_args, d_start, n, total, gate);
     case GS_UPDATE: return group_launch<UpdateImageOp, 256>(c, d_args, d_start, n, total, gate);
     case GS_CTRL_END: return group_launch<CtrlOp, 32>(c, d_args, d_start, n, total, gate);
-    default: return GPAIR_ERR_INVALID;
+    case GS_UG_GRAD: return group_launch<UgGradOp, 256>(c, d_args, d_start, n, total, gate);
+    default:
+        return gp_stage_grid_only(stage) ? gp_ug_stage_group_launch(c, stage, d_args, d_start, n, total, gate)
+                                         : GPAIR_ERR_INVALID;
     }
 }

@@ -45,6 +45,7 @@
 #include "group.cuh"
 #include "reduce.cuh"
 #include "umma.cuh"
+#include "uvgrid.cuh"
 
 #define TC_BM 128
 #define TC_BN 256
@@ -114,6 +115,8 @@ __device__ __forceinline__ void split_f8(float v, float s_hi, float s_lo, __half
 // products per K step: 3 = hi*hi + hi*lo + lo*hi of split operands, 1 = hi*hi
 // At most TC_SPLIT_PRODUCTS products per adjoint split-K partial (FP32 accumulation)
 #define TC_SPLIT_PRODUCTS 4096
+// and per partial sum of the uv grid's x contraction
+#define TC_GRID_PRODUCTS 128
 
 template <typename OT> struct OpSplit;
 template <> struct OpSplit<__half> {
@@ -217,6 +220,11 @@ struct TcState {
     // CTA pairs (cta_group::2): B maps with 128-row boxes, A row counts padded
     // to 256; npairs = clusters of two that are resident at once
     int pair, npairs;
+    // grid: the context takes the uv grid (uvgrid.cu). fx_* then hold the grid's column
+    // twiddles [2 columns -> 128][N -> bk], the forward is the x contraction with the
+    // store epilogue (single CTAs, gkb K-blocks per partial sum), and the adjoint's
+    // operands do not exist
+    int grid, gkb, gsplits;
 };
 
 static inline int round_up(long long a, long long b) { return (int)(((a + b - 1) / b) * b); }
@@ -1384,13 +1392,19 @@ static int tc_make_map(gpair_ctx *c, CUtensorMap *m, const void *base, long long
     return GPAIR_OK;
 }
 
-// operand kind and product count of a precision mode, and the forward's operand kind
-static void tc_mode(int precision, int *op, int *nprod, int *fop = nullptr)
+// operand kind and product count of a context's precision mode, and the forward's operand
+// kind (on the uv grid the x contraction is too small for E4M3 cross terms to save time:
+// three f16 products)
+static void tc_mode(const gpair_ctx *c, int *op, int *nprod, int *fop)
 {
+    const int precision = c->precision;
     *op = (precision == GPAIR_PREC_TF32 || precision == GPAIR_PREC_TF32X3) ? OP_TF32 : OP_F16;
     *nprod = precision == GPAIR_PREC_TF32 ? 1 : 3;
-    if (fop) *fop = precision == GPAIR_PREC_SPLIT16F8 ? OP_F16F8 : *op;
+    *fop = precision == GPAIR_PREC_SPLIT16F8 && !c->ug ? OP_F16F8 : *op;
 }
+
+// tile layout of a context's contractions (the uv grid's x contraction fills half of a pair's rows: single CTAs)
+static int tc_pair_of(const gpair_ctx *c) { return c->tc_pair && !c->ug ? 1 : 0; }
 
 // 2-D tensor [rows][cols] of bytes (E4M3), boxes of 64 bytes x box_rows, 64 B swizzle
 static int tc_make_map8(gpair_ctx *c, CUtensorMap *m, const void *base, long long rows, long long cols, int box_rows)
@@ -1464,6 +1478,24 @@ void gp_tc_free(gpair_ctx *c)
     c->tc_state = nullptr;
 }
 
+// Column twiddles of the uv grid as the x contraction's A operand: row 2j + c =
+// (cos, sin)(2 pi j x'/M) / phi(x') of every pixel x, scaled by 2^10
+template <typename OT>
+__global__ void k_tc_grid_ops(const float2 *__restrict__ ftab, int nbx, int N, int H, int Kx_pad, int rows_pad,
+                              OT *__restrict__ hi, OT *__restrict__ lo)
+{
+    const long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (idx >= (long long)rows_pad * Kx_pad) return;
+    const int r = (int)(idx / Kx_pad), x = (int)(idx % Kx_pad), j = r >> 1;
+    float v = 0.f;
+    if (j < nbx && x < N) {
+        const int h = min(x, N - 1 - x);  // pixels h and N - 1 - h lie at -+x'
+        const float2 f = ftab[(size_t)j * H + h];
+        v = ((r & 1) ? (x == h && x != N - 1 - x ? -f.y : f.y) : f.x) * (float)(1 << TC_TW_LOG2);
+    }
+    split_store(hi, lo, (size_t)idx, v);
+}
+
 template <typename OT>
 static void launch_twiddle_ops(gpair_ctx *c, TcState *t, long long n_all)
 {
@@ -1492,10 +1524,13 @@ int gp_tc_prepare(gpair_ctx *c)
 {
     if (!c->have_problem) return GPAIR_OK;  // prepared when the problem is loaded
     int op, nprod, fop;
-    tc_mode(c->precision, &op, &nprod, &fop);
-    const int pair = c->tc_pair ? 1 : 0;
+    tc_mode(c, &op, &nprod, &fop);
+    const int pair = tc_pair_of(c);
+    const UgState *ug = (const UgState *)c->ug;
     TcState *old = (TcState *)c->tc_state;
-    if (old && old->op == op && old->nprod == nprod && old->fop == fop && old->pair == pair) return GPAIR_OK;
+    if (old && old->op == op && old->nprod == nprod && old->fop == fop && old->pair == pair &&
+        old->grid == (ug != nullptr))
+        return GPAIR_OK;
     if (old) {
         // another operand kind: rebuild every operand buffer for this mode
         GP_CUDA(c, cudaStreamSynchronize(c->stream));
@@ -1516,13 +1551,14 @@ int gp_tc_prepare(gpair_ctx *c)
     t->Kx_pad = round_up(N, t->bk);
     t->M_pad = round_up(N, TC_BN);
     const int tm = pair ? 256 : TC_BM;  // A rows per tile
-    t->rows_pad = round_up(2LL * nuv, tm);
+    t->rows_pad = round_up(2LL * (ug ? ug->nbx : nuv), tm);
+    t->grid = ug != nullptr;
     t->K2_pad = round_up(2LL * nuv, t->bk);
     t->xrows_pad = round_up(N, tm);
     GP_CUDA(c, cudaDeviceGetAttribute(&t->nsm, cudaDevAttrMultiProcessorCount, c->device));
     t->splits = gp_tc_splits(N, nuv, t->nsm, t->bk, pair, &t->kb_per);
     size_t img = (size_t)t->M_pad * t->Kx_pad, fxs = (size_t)t->rows_pad * t->Kx_pad;
-    size_t fxts = (size_t)t->xrows_pad * t->K2_pad, ws = (size_t)t->M_pad * t->K2_pad;
+    size_t fxts = ug ? 0 : (size_t)t->xrows_pad * t->K2_pad, ws = ug ? 0 : (size_t)t->M_pad * t->K2_pad;
     const bool f8 = fop == OP_F16F8;
     // f8: the forward's lo operands are E4M3 pairs (1 byte per element each)
     struct { void **p; size_t n; bool lo; int esz; } al[] = {
@@ -1539,24 +1575,45 @@ int gp_tc_prepare(gpair_ctx *c)
     }
     GP_CUDA(c, cudaMalloc(&t->rsc, sizeof(float) * (size_t)t->M_pad));
     GP_CUDA(c, cudaMemsetAsync(t->rsc, 0, sizeof(float) * (size_t)t->M_pad, c->stream));
+    if (ug) {
+        // partial sums of TC_GRID_PRODUCTS products: short FP32 chains, and more units than one per tile
+        t->gkb = TC_GRID_PRODUCTS / t->bk;
+        const int kb_total = t->Kx_pad / t->bk;
+        if (gp_cdiv(kb_total, t->gkb) > UG_MAX_SPLITS) t->gkb = gp_cdiv(kb_total, UG_MAX_SPLITS);
+        t->gsplits = gp_cdiv(kb_total, t->gkb);
+    }
     t->nanc = (N + 15) / 16;
-    GP_CUDA(c, cudaMalloc(&t->fya, sizeof(float2) * (size_t)nuv * t->nanc));
-    GP_CUDA(c, cudaMalloc(&t->fyr, sizeof(float2) * (size_t)nuv));
-    if (c->nuv) {
+    if (!ug) {
+        GP_CUDA(c, cudaMalloc(&t->fya, sizeof(float2) * (size_t)nuv * t->nanc));
+        GP_CUDA(c, cudaMalloc(&t->fyr, sizeof(float2) * (size_t)nuv));
+    }
+    if (c->nuv && !ug) {
         k_tc_fy_anchors<<<gp_cdiv((long long)c->nuv * t->nanc, 256), 256, 0, c->stream>>>(c->fy, c->nuv, N, t->nanc,
                                                                                          t->fya, t->fyr);
         GP_LAUNCH_CHECK(c);
     }
-    long long n_all = (long long)fxs + (long long)fxts;
-    if (op == OP_F16) launch_twiddle_ops<__half>(c, t, n_all);
-    else launch_twiddle_ops<float>(c, t, n_all);
+    if (ug) {
+        const unsigned int nb = gp_cdiv((long long)fxs, 256);
+        if (op == OP_F16)
+            k_tc_grid_ops<__half><<<nb, 256, 0, c->stream>>>(ug->ftab, ug->nbx, N, ug->H, t->Kx_pad, t->rows_pad,
+                                                             (__half *)t->fx_hi, (__half *)t->fx_lo);
+        else
+            k_tc_grid_ops<float><<<nb, 256, 0, c->stream>>>(ug->ftab, ug->nbx, N, ug->H, t->Kx_pad, t->rows_pad,
+                                                            (float *)t->fx_hi, (float *)t->fx_lo);
+    } else {
+        const long long n_all = (long long)fxs + (long long)fxts;
+        if (op == OP_F16) launch_twiddle_ops<__half>(c, t, n_all);
+        else launch_twiddle_ops<float>(c, t, n_all);
+    }
     GP_LAUNCH_CHECK(c);
     const int e = t->esz;
     const int bbox = pair ? 128 : TC_BN;  // B rows one CTA stages
     if ((rc = tc_make_map(c, &t->m_img_hi, t->img_hi, t->M_pad, t->Kx_pad, bbox, e))) return rc;
     if ((rc = tc_make_map(c, &t->m_fx_hi, t->fx_hi, t->rows_pad, t->Kx_pad, TC_BM, e))) return rc;
-    if ((rc = tc_make_map(c, &t->m_w_hi, t->w_hi, t->M_pad, t->K2_pad, bbox, e))) return rc;
-    if ((rc = tc_make_map(c, &t->m_fxt_hi, t->fxt_hi, t->xrows_pad, t->K2_pad, TC_BM, e))) return rc;
+    if (!ug) {
+        if ((rc = tc_make_map(c, &t->m_w_hi, t->w_hi, t->M_pad, t->K2_pad, bbox, e))) return rc;
+        if ((rc = tc_make_map(c, &t->m_fxt_hi, t->fxt_hi, t->xrows_pad, t->K2_pad, TC_BM, e))) return rc;
+    }
     if (nprod == 3) {
         if (f8) {
             if ((rc = tc_make_map8(c, &t->m_img8h, t->img8h, t->M_pad, t->Kx_pad, bbox))) return rc;
@@ -1569,8 +1626,10 @@ int gp_tc_prepare(gpair_ctx *c)
             if ((rc = tc_make_map(c, &t->m_img_lo, t->img_lo, t->M_pad, t->Kx_pad, bbox, e))) return rc;
             if ((rc = tc_make_map(c, &t->m_fx_lo, t->fx_lo, t->rows_pad, t->Kx_pad, TC_BM, e))) return rc;
         }
-        if ((rc = tc_make_map(c, &t->m_w_lo, t->w_lo, t->M_pad, t->K2_pad, bbox, e))) return rc;
-        if ((rc = tc_make_map(c, &t->m_fxt_lo, t->fxt_lo, t->xrows_pad, t->K2_pad, TC_BM, e))) return rc;
+        if (!ug) {
+            if ((rc = tc_make_map(c, &t->m_w_lo, t->w_lo, t->M_pad, t->K2_pad, bbox, e))) return rc;
+            if ((rc = tc_make_map(c, &t->m_fxt_lo, t->fxt_lo, t->xrows_pad, t->K2_pad, TC_BM, e))) return rc;
+        }
     } else {
         // the kernel never loads the lo maps in one-product mode; pass valid maps anyway
         t->m_img_lo = t->m_img_hi;
@@ -1665,6 +1724,7 @@ int gp_tc_shared_splits(gpair_ctx **ctx, int n)
         int rc;
         TcState *t = tc_state_ready(ctx[i], &rc);
         if (rc) return rc;
+        if (t->grid) continue;  // no split-K adjoint
         const int tiles = (t->xrows_pad / (t->pair ? 256 : TC_BM)) * (t->M_pad / TC_BN);
         total += (double)tiles * (double)(t->K2_pad / t->bk);
         if (!slots) slots = t->pair ? t->npairs : t->nsm;
@@ -1680,6 +1740,7 @@ int gp_tc_shared_splits(gpair_ctx **ctx, int n)
         gpair_ctx *c = ctx[i];
         if (c->precision == GPAIR_PREC_FP32) continue;
         TcState *t = (TcState *)c->tc_state;
+        if (t->grid) continue;
         const int kb_total = t->K2_pad / t->bk;
         int want = (int)(target * (double)kb_total / total + 0.5);  // splits of this context
         if (want < 1) want = 1;
@@ -1848,6 +1909,37 @@ static int tc_prep_rows_launch(gpair_ctx *c, TcState *t, int mode, int reduce, d
     return GPAIR_OK;
 }
 
+// Sizes of the uv grid's x contraction over the image rows of `images` images (the store
+// epilogue writes T[partial sum][image row][2 columns])
+static TcArgs tc_grid_args(gpair_ctx *c, TcState *t, int images)
+{
+    const UgState *g = (const UgState *)c->ug;
+    TcArgs a;
+    memset(&a, 0, sizeof(a));
+    a.m_tiles = t->rows_pad / TC_BM;
+    a.n_tiles = images > 1 ? images * t->Lb / TC_BN : t->M_pad / TC_BN;
+    a.kb_total = t->Kx_pad / t->bk;
+    a.kb_per_split = t->gkb;
+    a.units = a.m_tiles * a.n_tiles * t->gsplits;
+    a.gpart = images > 1 ? g->Tb : g->T;
+    a.out_ld = g->ldT;
+    a.out_rows = images > 1 ? images * t->Lb : c->N;
+    a.out_cols = 2 * g->nbx;
+    return a;
+}
+
+int gp_tc_ug_rows(gpair_ctx *c, int images, const float **rsc, int *lrows, int *splits)
+{
+    int rc;
+    TcState *t = tc_state_ready(c, &rc);
+    if (rc) return rc;
+    if (!t->grid) return GPAIR_ERR_STATE;
+    *rsc = images > 1 ? t->rscb : t->rsc;
+    *lrows = images > 1 ? t->Lb : c->N;
+    *splits = t->gsplits;
+    return GPAIR_OK;
+}
+
 // forward contraction on the already split image operand
 int gp_tc_forward_gemm(gpair_ctx *c)
 {
@@ -1855,6 +1947,11 @@ int gp_tc_forward_gemm(gpair_ctx *c)
     TcState *t = tc_state_ready(c, &rc);
     if (rc) return rc;
     TcArgs a;
+    if (t->grid) {
+        a = tc_grid_args(c, t, 1);
+        if ((rc = tc_launch<EPI_STORE>(c, t, tc_fwd_maps(t, false), a))) return rc;
+        return gp_ug_vis(c, 1);
+    }
     memset(&a, 0, sizeof(a));
     a.m_tiles = t->rows_pad / (t->pair ? 256 : TC_BM);  // twiddle-row tiles
     a.n_tiles = t->M_pad / TC_BN;     // image-row tiles
@@ -1878,6 +1975,8 @@ int gp_tc_forward_gemm(gpair_ctx *c)
 // Operand stack of the batched line-search trials: GP_NTR images of Lb rows
 // (Lb = 32, 64 or 128 for small images so that 256-row tiles hold several
 // whole images, else N rounded up to 256); partial entries of min(Lb, 256) rows.
+int gp_tc_stack_rows(int N) { return N <= 32 ? 32 : N <= 64 ? 64 : N <= 128 ? 128 : round_up(N, TC_BN); }
+
 int gp_tc_batch_prepare(gpair_ctx *c, int *epp)
 {
     int rc;
@@ -1885,7 +1984,7 @@ int gp_tc_batch_prepare(gpair_ctx *c, int *epp)
     if (rc) return rc;
     if (!t->imgb_hi) {
         const int N = c->N;
-        t->Lb = N <= 32 ? 32 : N <= 64 ? 64 : N <= 128 ? 128 : round_up(N, TC_BN);
+        t->Lb = gp_tc_stack_rows(N);
         const int erows = t->Lb < TC_EPI_COLS ? t->Lb : TC_EPI_COLS;
         t->epp_b = t->Lb / erows;
         const size_t rows = (size_t)GP_NTR * t->Lb, n = rows * t->Kx_pad;
@@ -1912,6 +2011,7 @@ int gp_tc_batch_prepare(gpair_ctx *c, int *epp)
             t->m_imgb_lo = t->m_imgb_hi;
         }
     }
+    if (t->grid && (rc = gp_ug_batch_alloc(c))) return rc;
     c->epp = t->epp_b;
     if (epp) *epp = t->epp_b;
     return GPAIR_OK;
@@ -1936,6 +2036,11 @@ int gp_tc_forward_batch_gemm(gpair_ctx *c)
     if (rc) return rc;
     if ((rc = gp_tc_batch_prepare(c, nullptr))) return rc;
     TcArgs a;
+    if (t->grid) {
+        a = tc_grid_args(c, t, GP_NTR);
+        if ((rc = tc_launch<EPI_STORE>(c, t, tc_fwd_maps(t, true), a))) return rc;
+        return gp_ug_vis(c, GP_NTR);
+    }
     memset(&a, 0, sizeof(a));
     a.m_tiles = t->rows_pad / (t->pair ? 256 : TC_BM);
     a.n_tiles = (GP_NTR * t->Lb) / TC_BN;
@@ -2017,6 +2122,7 @@ int gp_tc_build_w(gpair_ctx *c)
     int rc;
     TcState *t = tc_state_ready(c, &rc);
     if (rc) return rc;
+    if (t->grid) return GPAIR_ERR_STATE;  // no adjoint operands
     GP_LAUNCH(c, t->op == OP_F16 ? launch_build_w<__half>(c, t) : launch_build_w<float>(c, t));
     return GPAIR_OK;
 }
@@ -2027,6 +2133,7 @@ int gp_tc_adjoint_gemm(gpair_ctx *c)
     int rc;
     TcState *t = tc_state_ready(c, &rc);
     if (rc) return rc;
+    if (t->grid) return GPAIR_ERR_STATE;
     TcArgs a;
     memset(&a, 0, sizeof(a));
     a.m_tiles = t->xrows_pad / (t->pair ? 256 : TC_BM);  // image-column tiles (twiddle side)
@@ -2078,13 +2185,14 @@ void gp_tc_group_free(void *grp)
 // the tile layout, operand kind, product count and forward operand kind of a
 // context's tensor path (instances with equal keys can share a grouped forward;
 // with equal key >> 3 -- all but the forward operand kind -- a grouped adjoint),
-// or -1 on the CUDA cores. Sorting by key keeps both kinds of class contiguous.
+// or -1 on the CUDA cores. Sorting by key keeps both kinds of class contiguous;
+// contexts on the uv grid (no adjoint contraction) come last.
 int gp_tc_group_key(gpair_ctx *c)
 {
     if (c->precision == GPAIR_PREC_FP32) return -1;
     int op, nprod, fop;
-    tc_mode(c->precision, &op, &nprod, &fop);
-    return (((c->tc_pair ? 1 : 0) * 8 + op) * 4 + nprod) * 8 + fop;
+    tc_mode(c, &op, &nprod, &fop);
+    return ((((c->ug ? 2 : 0) + tc_pair_of(c)) * 8 + op) * 4 + nprod) * 8 + fop;
 }
 
 // one instance's entry of a grouped contraction of kind GP_TCG_*
@@ -2110,6 +2218,18 @@ static void tc_group_inst(gpair_ctx *c, TcState *t, int kind, TcGroupInst &g)
         return;
     }
     const bool batch = kind == GP_TCG_TRIALS;
+    if (t->grid) {
+        const TcArgs a = tc_grid_args(c, t, batch ? GP_NTR : 1);
+        g.m_tiles = a.m_tiles;
+        g.n_tiles = a.n_tiles;
+        g.kb_total = a.kb_total;
+        g.kb_per_split = a.kb_per_split;
+        g.units = a.units;
+        g.gpart = a.gpart;
+        g.out_ld = a.out_ld;
+        g.out_rows = a.out_rows;
+        g.out_cols = a.out_cols;
+    }
     const TcMaps fm = tc_fwd_maps(t, batch);
     g.A_hi = *fm.a_hi;
     g.A_lo = *fm.a_lo;
@@ -2117,6 +2237,7 @@ static void tc_group_inst(gpair_ctx *c, TcState *t, int kind, TcGroupInst &g)
     g.B_hi = *fm.b_hi;
     g.B_lo = *fm.b_lo;
     g.B_x = *fm.b_x;
+    if (t->grid) return;
     g.m_tiles = t->rows_pad / mt;
     g.n_tiles = batch ? (GP_NTR * t->Lb) / TC_BN : t->M_pad / TC_BN;
     g.kb_total = t->Kx_pad / t->bk;
@@ -2163,8 +2284,12 @@ int gp_tc_group_build_kind(gpair_ctx **ctx, int n, int kind, const int *gate, un
         if (rc) break;
         if (kind == GP_TCG_TRIALS && (rc = gp_batch_alloc(c))) break;
         // the adjoint is the same contraction for both forward operand kinds of an op
+        if (t->grid && kind == GP_TCG_ADJOINT) {
+            rc = GPAIR_ERR_STATE;
+            break;
+        }
         if (t0 && ((kind == GP_TCG_ADJOINT ? t->op != t0->op : t->fop != t0->fop) || t->nprod != t0->nprod ||
-                   t->pair != t0->pair)) {
+                   t->pair != t0->pair || t->grid != t0->grid)) {
             rc = GPAIR_ERR_STATE;
             break;
         }
@@ -2178,7 +2303,7 @@ int gp_tc_group_build_kind(gpair_ctx **ctx, int n, int kind, const int *gate, un
     }
     if (!rc) {
         G->n = n;
-        G->epi = kind == GP_TCG_ADJOINT ? EPI_STORE : EPI_FWD;
+        G->epi = kind == GP_TCG_ADJOINT || t0->grid ? EPI_STORE : EPI_FWD;
         G->op = kind == GP_TCG_ADJOINT ? t0->op : t0->fop;
         G->nprod = t0->nprod;
         G->pair = t0->pair;
@@ -2315,7 +2440,7 @@ int gp_tc_stage_args(gpair_ctx *c, int stage, void *out, int *nblocks, int *op, 
         return GPAIR_OK;
     }
     if (stage == GS_BUILD_W) {
-        if (!c->have_uv) return GPAIR_ERR_STATE;  // the table-only path reads Fy from its table
+        if (!c->have_uv || t->grid) return GPAIR_ERR_STATE;  // the table-only path reads Fy from its table
         const BuildWArgs a = tc_build_w_args(c, t);
         memcpy(out, &a, sizeof(a));
         *nblocks = a.nbx * a.nby;

@@ -1,0 +1,929 @@
+// uvgrid.cu -- the DFT to the uv points and its adjoint through a regular grid
+// of the uv plane.
+//
+// The image covers N pixels a side, so its transform E(a, b) = sum_yx I[y][x]
+// e^{2 pi i (a x' - b y')} (a, b in cycles per pixel, x' = x - (N-1)/2) is a
+// band-limited function of (a, b): it is known everywhere from its values on a
+// grid of spacing 1/M, M = 2 N, and a Kaiser-Bessel window of UG_W = 8 grid
+// points a side interpolates it (a nonuniform Fourier transform of type 2;
+// Dutt and Rokhlin 1993, Fessler and Sutton 2003). Dividing the image by the
+// window's transform phi is folded into the grid's own twiddles. A data set
+// has many more uv points than grid points inside its uv coverage (1024^2
+// workload: 194,560 uv points, 60 x 119 grid points), so two small
+// contractions onto the grid and 64 window products per uv point take the
+// place of the N^2 nuv contraction:
+//   forward   T[y][jx] = sum_x I[y][x] e^{2 pi i jx x'/M} / phi(x')          (tcgen05, or k_ug_x)
+//             G[jy][jx] = sum_y T[y][jx] e^{-2 pi i jy y'/M} / phi(y')       (k_ug_rows)
+//             V_k = sum over 8 x 8 grid points of G, window weights          (k_ug_interp)
+//   adjoint   C[jy][jx] = sum_k c_k at the 8 x 8 grid points around k        (k_ug_spread, k_ug_gather)
+//             S[y][jx] = sum_jy C[jy][jx] e^{-2 pi i jy y'/M} / phi(y')      (k_ug_cols)
+//             g[y][x] = Re sum_jx S[y][jx] e^{2 pi i jx x'/M} / phi(x')      (k_ug_grad, with the gradient assembly)
+// Conjugating uv points with a < 0 leaves jx >= -3, half of the plane.
+//
+// Accuracy. The window's own error is at most 4e-8 of the flux (FP64 model over
+// the workloads' uv points and flat, random and compact images). V measures
+// 7e-8 to 9e-8 relative on FP32 contexts (the direct FP32 sums 1e-7 to 4e-7),
+// the gradient 3e-8 to 2e-7 (as the direct sums) from 96 pixels up; on the
+// tensor paths the gradient measures 2e-6 to 4e-6 where the direct
+// contractions measure 2e-6 to 2e-5 (their accumulation truncates; the x
+// contraction's partial sums here are 128 products long).
+// Measured on a B200, one objective with its gradient (events around the
+// stages): 1024^2 and 194,560 uv points 3,240 -> 205 us on the tensor path,
+// 57,000 -> 205 us in FP32; 256^2 and 21,120 uv points 120 -> 99 us and 495 -> 86 us.
+//
+// Everything is summed in a fixed order: uv points are sorted by their grid
+// cell, and the adjoint adds per-cell patches, so there are no atomics.
+#include <math.h>
+#include <stdlib.h>
+#include <string.h>
+
+#include <vector>
+
+#include "gpair_internal.cuh"
+#include "group.cuh"
+#include "reduce.cuh"
+#include "uvgrid.cuh"
+
+#define UG_PI 3.14159265358979323846
+#define UG_RPMAS ((3.14159265358979323 / 180.0) / 3600000.0)  // radians per milliarcsecond, as k_gen_twiddles
+
+// ------------------------------------------------------------------ plan
+
+// I0 by its series (x <= pi UG_W)
+__device__ __forceinline__ double ug_bessel_i0(double x)
+{
+    const double t = 0.25 * x * x;
+    double term = 1.0, sum = 1.0;
+    for (int n = 1; n < 200; n++) {
+        term *= t / ((double)n * (double)n);
+        sum += term;
+        if (term < 1e-17 * sum) break;
+    }
+    return sum;
+}
+
+// Window weights and centre phase of every sorted uv point, from (u, v) in FP64
+__global__ void k_ug_points(const float2 *__restrict__ uvc, const int *__restrict__ src, const int *__restrict__ base,
+                            int nuv, double pix, int N, double M, int jxf, int J, int nbx, double beta,
+                            float *__restrict__ wts, float2 *__restrict__ phase)
+{
+    const int p = blockIdx.x * blockDim.x + threadIdx.x;
+    if (p >= nuv) return;
+    const int k = src[p] & 0x7fffffff;
+    const bool flip = src[p] < 0;
+    const float2 uv = uvc[k];
+    double a = UG_RPMAS * pix * (double)uv.x, b = UG_RPMAS * pix * (double)uv.y;
+    a -= rint(a);
+    b -= rint(b);
+    if (flip) {
+        a = -a;
+        b = -b;
+    }
+    const double gx = a * M - (double)(base[p] % nbx + jxf), gy = b * M - (double)(base[p] / nbx - J);
+    const double inv0 = 1.0 / ug_bessel_i0(beta);
+    for (int i = 0; i < UG_W; i++) {
+        const double tx = (gx - i) * (2.0 / UG_W), ty = (gy - i) * (2.0 / UG_W);
+        wts[(size_t)p * (2 * UG_W) + i] = (float)(ug_bessel_i0(beta * sqrt(fmax(0.0, 1.0 - tx * tx))) * inv0);
+        wts[(size_t)p * (2 * UG_W) + UG_W + i] = (float)(ug_bessel_i0(beta * sqrt(fmax(0.0, 1.0 - ty * ty))) * inv0);
+    }
+    double t = (a - b) * (0.5 * (double)(N - 1));
+    t -= rint(t);
+    double sn, cn;
+    sincospi(2.0 * t, &sn, &cn);
+    phase[p] = make_float2((float)cn, (float)sn);
+}
+
+// Grid twiddles over the folded image coordinate h (pixels h and N-1-h, at
+// -+x'_h, x'_h = (N-1)/2 - h): (cos, sin)(2 pi j x'_h / M) / phi(x'_h), FP64 phase.
+// ftab[j][h] for the columns j = jxf .. jxf + nbx - 1, ctab[h][j] for the rows j = 0 .. J
+__global__ void k_ug_tables(const double *__restrict__ invphi, int N, int H, double M, int jxf, int nbx, int J,
+                            float2 *__restrict__ ftab, float2 *__restrict__ ctab)
+{
+    long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    const long long nf = (long long)nbx * H;
+    int h, j;
+    if (i < nf) {
+        j = (int)(i / H) + jxf;
+        h = (int)(i % H);
+    } else {
+        i -= nf;
+        if (i >= (long long)H * (J + 1)) return;
+        h = (int)(i / (J + 1));
+        j = (int)(i % (J + 1));
+    }
+    double t = (double)j * (0.5 * (double)(N - 1) - (double)h) / M;
+    t -= rint(t);
+    double sn, cn;
+    sincospi(2.0 * t, &sn, &cn);
+    const double f = invphi[h];
+    const float2 v = make_float2((float)(cn * f), (float)(sn * f));
+    if ((long long)blockIdx.x * blockDim.x + threadIdx.x < nf) ftab[i] = v;
+    else ctab[i] = v;
+}
+
+// First window points of the uv points (host) and the grid's extent: columns
+// jxf .. jxf + nbx - 1, rows -J .. J. False when a coordinate is not finite.
+static bool ug_extent(const gpair_uv *uv, int nuv, float pix, double M, std::vector<int> &jx0, std::vector<int> &jy0,
+                      std::vector<unsigned char> &flip, int *jxf, int *nbx, int *J)
+{
+    int xmin = 1 << 30, xmax = -(1 << 30), ymax = 0;
+    for (int k = 0; k < nuv; k++) {
+        double a = UG_RPMAS * (double)pix * (double)uv[k].u, b = UG_RPMAS * (double)pix * (double)uv[k].v;
+        if (!isfinite(a) || !isfinite(b)) return false;
+        a -= rint(a);
+        b -= rint(b);
+        flip[k] = a < 0.0;
+        if (flip[k]) {
+            a = -a;
+            b = -b;
+        }
+        jx0[k] = (int)floor(a * M) - (UG_W / 2 - 1);
+        jy0[k] = (int)floor(b * M) - (UG_W / 2 - 1);
+        if (jx0[k] < xmin) xmin = jx0[k];
+        if (jx0[k] > xmax) xmax = jx0[k];
+        const int lo = -jy0[k], hi = jy0[k] + UG_W - 1;
+        if (lo > ymax) ymax = lo;
+        if (hi > ymax) ymax = hi;
+    }
+    *jxf = xmin;
+    *nbx = xmax - xmin + UG_W;
+    *J = ymax;
+    return true;
+}
+
+// Whether the grid's contractions are small beside the direct ones (UG_GRID_RATIO), with one partial sum
+// of the gradient's dot products per 64 x 64 tile
+static bool ug_small(int N, int nuv, int nbx, int J)
+{
+    const double direct = 2.0 * (double)N * N * (double)nuv;
+    const double grid = (double)nbx * (2.0 * N + 2.0 * J + 1.0) * (double)N;
+    return (long long)gp_cdiv(N, 64) * gp_cdiv((N + 1) / 2, 64) <= GP_MAX_PARTIALS && UG_GRID_RATIO * grid <= direct;
+}
+
+// The precision mode's least direct work 2 N^2 nuv for the grid (uvgrid.cuh)
+static double ug_min_work(int precision)
+{
+    if (precision == GPAIR_PREC_FP32) return UG_MIN_WORK_FP32;
+    return precision == GPAIR_PREC_SPLIT16F8 ? UG_MIN_WORK_F8 : UG_MIN_WORK_TC;
+}
+
+void gp_ug_choose(gpair_ctx *c)
+{
+    c->ug = c->ug_plan && 2.0 * (double)c->N * c->N * (double)c->nuv >= ug_min_work(c->precision) ? c->ug_plan : nullptr;
+}
+
+void gp_ug_free(gpair_ctx *c)
+{
+    UgState *g = (UgState *)c->ug_plan;
+    if (!g) return;
+    void *bufs[] = {g->src, g->base, g->wts, g->phase, g->chunk, g->cst, g->ftab, g->ctab, g->invphi,
+                    g->T, g->grid, g->patch, g->cgrid, g->S, g->Tb, g->gridb};
+    for (void *b : bufs)
+        if (b) cudaFree(b);
+    free(g);
+    c->ug_plan = nullptr;
+    c->ug = nullptr;
+}
+
+// Builds the plan of a problem given by (u, v) when some precision mode would
+// take it. The sizes of the context are set.
+int gp_ug_plan(gpair_ctx *c, const gpair_uv *uv)
+{
+    gp_ug_free(c);
+    const int N = c->N, nuv = c->nuv;
+    if (!uv || N < UG_MIN_WIDTH || 2.0 * (double)N * N * (double)nuv < UG_MIN_WORK_FP32) return GPAIR_OK;
+    const double M = UG_OVERSAMPLING * N;
+    std::vector<int> jx0(nuv), jy0(nuv);
+    std::vector<unsigned char> flip(nuv);
+    int jxf, nbx, J;
+    if (!ug_extent(uv, nuv, c->pix, M, jx0, jy0, flip, &jxf, &nbx, &J)) return GPAIR_OK;
+    if (!ug_small(N, nuv, nbx, J)) return GPAIR_OK;
+    const int cells = nbx * (2 * J + 1);
+    // counting sort by cell (stable), then runs of at most 32 points of one cell
+    std::vector<int> off((size_t)cells + 1, 0), src(nuv), base(nuv), cst((size_t)cells + 1, 0);
+    std::vector<int2> chunk;
+    for (int k = 0; k < nuv; k++) off[(size_t)(jy0[k] + J) * nbx + (jx0[k] - jxf) + 1]++;
+    for (int q = 0; q < cells; q++) {
+        cst[q] = (int)chunk.size();
+        for (int s = 0; s < off[q + 1]; s += 32) {
+            const int left = off[q + 1] - s;
+            chunk.push_back(make_int2(off[q] + s, left < 32 ? left : 32));
+        }
+        off[q + 1] += off[q];
+    }
+    cst[cells] = (int)chunk.size();
+    std::vector<int> pos(off.begin(), off.end() - 1);
+    for (int k = 0; k < nuv; k++) {
+        const int cell = (jy0[k] + J) * nbx + (jx0[k] - jxf);
+        const int p = pos[cell]++;
+        src[p] = k | (flip[k] ? (int)0x80000000 : 0);
+        base[p] = cell;
+    }
+    // 1 / phi over the folded coordinate: phi(x') = w sinh(z) / z / I0(beta), z^2 = beta^2 - (pi w x'/M)^2
+    const int H = (N + 1) / 2;
+    const double beta = UG_PI * UG_W * (1.0 - (double)N / (2.0 * M));
+    double i0 = 1.0, term = 1.0;
+    for (int n = 1; n < 200; n++) {
+        term *= 0.25 * beta * beta / ((double)n * n);
+        i0 += term;
+    }
+    std::vector<double> invphi(H);
+    for (int h = 0; h < H; h++) {
+        const double xi = UG_PI * UG_W * (0.5 * (N - 1) - h) / M;
+        const double z = sqrt(beta * beta - xi * xi);
+        invphi[h] = i0 * z / (UG_W * sinh(z));
+    }
+    UgState *g = (UgState *)calloc(1, sizeof(UgState));
+    if (!g) return GPAIR_ERR_ALLOC;
+    c->ug_plan = g;
+    g->N = N;
+    g->H = H;
+    g->jxf = jxf;
+    g->nbx = nbx;
+    g->J = J;
+    g->cells = cells;
+    g->nchunk = (int)chunk.size();
+    g->ldT = (2 * nbx + 3) & ~3;
+    cudaStream_t st = c->stream;
+    GP_CUDA(c, cudaMalloc(&g->src, sizeof(int) * nuv));
+    GP_CUDA(c, cudaMalloc(&g->base, sizeof(int) * nuv));
+    GP_CUDA(c, cudaMalloc(&g->wts, sizeof(float) * 2 * UG_W * (size_t)nuv));
+    GP_CUDA(c, cudaMalloc(&g->phase, sizeof(float2) * nuv));
+    GP_CUDA(c, cudaMalloc(&g->chunk, sizeof(int2) * g->nchunk));
+    GP_CUDA(c, cudaMalloc(&g->cst, sizeof(int) * ((size_t)cells + 1)));
+    GP_CUDA(c, cudaMalloc(&g->ftab, sizeof(float2) * (size_t)nbx * H));
+    GP_CUDA(c, cudaMalloc(&g->ctab, sizeof(float2) * (size_t)H * (J + 1)));
+    GP_CUDA(c, cudaMalloc(&g->invphi, sizeof(double) * H));
+    GP_CUDA(c, cudaMalloc(&g->grid, sizeof(float2) * (size_t)cells));
+    GP_CUDA(c, cudaMalloc(&g->patch, sizeof(float2) * UG_W * UG_W * (size_t)g->nchunk));
+    GP_CUDA(c, cudaMalloc(&g->cgrid, sizeof(float2) * (size_t)cells));
+    GP_CUDA(c, cudaMalloc(&g->S, sizeof(float2) * (size_t)N * nbx));
+    GP_CUDA(c, cudaMalloc(&g->T, sizeof(float) * (size_t)UG_MAX_SPLITS * N * g->ldT));
+    GP_CUDA(c, cudaMemcpyAsync(g->src, src.data(), sizeof(int) * nuv, cudaMemcpyHostToDevice, st));
+    GP_CUDA(c, cudaMemcpyAsync(g->base, base.data(), sizeof(int) * nuv, cudaMemcpyHostToDevice, st));
+    GP_CUDA(c, cudaMemcpyAsync(g->chunk, chunk.data(), sizeof(int2) * g->nchunk, cudaMemcpyHostToDevice, st));
+    GP_CUDA(c, cudaMemcpyAsync(g->cst, cst.data(), sizeof(int) * ((size_t)cells + 1), cudaMemcpyHostToDevice, st));
+    GP_CUDA(c, cudaMemcpyAsync(g->invphi, invphi.data(), sizeof(double) * H, cudaMemcpyHostToDevice, st));
+    k_ug_points<<<gp_cdiv(nuv, 128), 128, 0, st>>>(c->uvc, g->src, g->base, nuv, (double)c->pix, N, M, jxf, J, nbx,
+                                                   beta, g->wts, g->phase);
+    GP_LAUNCH_CHECK(c);
+    const long long nt = (long long)nbx * H + (long long)H * (J + 1);
+    k_ug_tables<<<gp_cdiv(nt, 256), 256, 0, st>>>(g->invphi, N, H, M, jxf, nbx, J, g->ftab, g->ctab);
+    GP_LAUNCH_CHECK(c);
+    GP_CUDA(c, cudaStreamSynchronize(st));  // the host arrays go out of scope
+    return GPAIR_OK;
+}
+
+// ----------------------------------------- x contraction on the CUDA cores
+//
+// T[y][2j + c] of one image (FP32 contexts), folded over x' -> -x': the cosine
+// row meets I[N-1-h] + I[h], the sine row I[N-1-h] - I[h]. A block makes 32
+// image rows x 32 columns over a slice of h; the slices are partial sums that
+// k_ug_rows adds.
+#define UGX_T 32
+struct UgXArgs {
+    const float *img;  // image b at img + b npix
+    const float2 *ftab;
+    float *T;  // [split][image row][ldT]
+    int N, H, nbx, ldT, splits, hper, images;
+    const int *gate;
+};
+
+__global__ void __launch_bounds__(256) k_ug_x(const UgXArgs a)
+{
+    gp_pdl_enter();
+    if (a.gate && !*a.gate) return;
+    __shared__ float2 Is[UGX_T][UGX_T + 1];  // [h][y] (even, odd)
+    __shared__ float2 Fs[UGX_T][UGX_T + 1];  // [h][j]
+    const int N = a.N, H = a.H;
+    const int y0 = blockIdx.x * UGX_T, j0 = blockIdx.y * UGX_T;
+    const int split = blockIdx.z % a.splits, image = blockIdx.z / a.splits;
+    const float *img = a.img + (size_t)image * N * N;
+    const int hb = split * a.hper, he = min(H, hb + a.hper);
+    const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    float2 acc[2][2];
+#pragma unroll
+    for (int i = 0; i < 2; i++)
+#pragma unroll
+        for (int j = 0; j < 2; j++) acc[i][j] = make_float2(0.f, 0.f);
+    for (int h0 = hb; h0 < he; h0 += UGX_T) {
+        const int h = h0 + lane;
+#pragma unroll
+        for (int r = 0; r < 4; r++) {
+            const int yy = warp + 8 * r, y = y0 + yy, j = j0 + yy;
+            float2 v = make_float2(0.f, 0.f), f = make_float2(0.f, 0.f);
+            if (h < he && y < N) {
+                const float p = __ldg(&img[(size_t)y * N + (N - 1 - h)]);
+                const float m = (N - 1 - h) != h ? __ldg(&img[(size_t)y * N + h]) : 0.f;
+                v = make_float2(p + m, p - m);
+            }
+            if (h < he && j < a.nbx) f = __ldg(&a.ftab[(size_t)j * H + h]);
+            Is[lane][yy] = v;
+            Fs[lane][yy] = f;
+        }
+        __syncthreads();
+#pragma unroll 8
+        for (int q = 0; q < UGX_T; q++) {
+            const float2 i0 = Is[q][ty], i1 = Is[q][ty + 16], f0 = Fs[q][tx], f1 = Fs[q][tx + 16];
+            acc[0][0].x = fmaf(i0.x, f0.x, acc[0][0].x);
+            acc[0][0].y = fmaf(i0.y, f0.y, acc[0][0].y);
+            acc[0][1].x = fmaf(i0.x, f1.x, acc[0][1].x);
+            acc[0][1].y = fmaf(i0.y, f1.y, acc[0][1].y);
+            acc[1][0].x = fmaf(i1.x, f0.x, acc[1][0].x);
+            acc[1][0].y = fmaf(i1.y, f0.y, acc[1][0].y);
+            acc[1][1].x = fmaf(i1.x, f1.x, acc[1][1].x);
+            acc[1][1].y = fmaf(i1.y, f1.y, acc[1][1].y);
+        }
+        __syncthreads();
+    }
+    float *T = a.T + ((size_t)split * a.images + image) * N * a.ldT;
+#pragma unroll
+    for (int i = 0; i < 2; i++)
+#pragma unroll
+        for (int j = 0; j < 2; j++) {
+            const int y = y0 + ty + 16 * i, jj = j0 + tx + 16 * j;
+            if (y < N && jj < a.nbx) *reinterpret_cast<float2 *>(&T[(size_t)y * a.ldT + 2 * jj]) = acc[i][j];
+        }
+}
+
+// ------------------------------------------------------ y contraction
+//
+// G[+-j][jx] of UGR_C columns jx and 32 rows j per block: lane = j, the eight
+// warps take every eighth folded image row h (pixels h and N-1-h), whose
+// folded T values (sum and difference of the two rows, partial sums added,
+// row scales removed) wait in shared memory. cos and sin serve +j and -j.
+// Bound by the L2 reads of the row twiddles (H x 32 x 8 B per block).
+#define UGR_H 256  // folded rows staged at once
+struct UgRowsArgs {
+    const float *T;  // image b: rows b lrows .. b lrows + N - 1
+    const float *rsc;  // power-of-two factor of every row (tensor path), or null
+    const float2 *ctab;
+    float2 *grid;  // image b at grid + b cells
+    int N, H, gw, J, ldT, cells, splits, lrows;  // gw: grid columns
+    size_t split_stride;
+    const int *gate;
+    GP_VGRID_FIELDS;
+};
+
+template <int C>
+__device__ __forceinline__ void ug_rows_body(const UgRowsArgs &A, const GpVGrid &vg)
+{
+    __shared__ __align__(16) float4 Ts[UGR_H * C];
+    __shared__ double red[8][32][C][4];
+    if (A.gate && !*A.gate) return;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int ctiles = (A.gw + C - 1) / C;
+    const int c0 = (vg.bx % ctiles) * C, j = (vg.bx / ctiles) * 32 + lane;
+    const int image = vg.by;
+    const int N = A.N, H = A.H, J1 = A.J + 1;
+    const size_t row0 = (size_t)image * A.lrows;
+    double acc[C][4];
+#pragma unroll
+    for (int q = 0; q < C; q++)
+#pragma unroll
+        for (int i = 0; i < 4; i++) acc[q][i] = 0.0;
+    for (int hb = 0; hb < H; hb += UGR_H) {
+        const int nh = min(UGR_H, H - hb);
+        for (int e = threadIdx.x; e < nh * C; e += blockDim.x) {
+            const int h = hb + e / C, col = c0 + e % C;
+            float2 p = make_float2(0.f, 0.f), m = make_float2(0.f, 0.f);
+            if (col < A.gw) {
+                const size_t rp = row0 + (N - 1 - h), rm = row0 + h;
+                const bool two = rp != rm;
+                for (int s = 0; s < A.splits; s++) {
+                    const float *T = A.T + s * A.split_stride;
+                    const float2 a = __ldg(reinterpret_cast<const float2 *>(T + rp * A.ldT + 2 * col));
+                    p.x += a.x;
+                    p.y += a.y;
+                    if (two) {
+                        const float2 b = __ldg(reinterpret_cast<const float2 *>(T + rm * A.ldT + 2 * col));
+                        m.x += b.x;
+                        m.y += b.y;
+                    }
+                }
+                if (A.rsc) {
+                    const float sp = __ldg(&A.rsc[rp]), sm = __ldg(&A.rsc[rm]);
+                    p.x *= sp;
+                    p.y *= sp;
+                    m.x *= sm;
+                    m.y *= sm;
+                }
+            }
+            Ts[e] = make_float4(p.x + m.x, p.y + m.y, p.x - m.x, p.y - m.y);
+        }
+        __syncthreads();
+        if (j < J1) {
+            const float2 *ct = A.ctab + (size_t)hb * J1 + j;
+#pragma unroll 8
+            for (int h = warp; h < nh; h += 8) {
+                const float2 wf = __ldg(&ct[(size_t)h * J1]);
+                const double wc = wf.x, ws = wf.y;
+#pragma unroll
+                for (int q = 0; q < C; q++) {
+                    const float4 t = Ts[h * C + q];
+                    acc[q][0] = fma(wc, (double)t.x, acc[q][0]);
+                    acc[q][1] = fma(wc, (double)t.y, acc[q][1]);
+                    acc[q][2] = fma(ws, (double)t.z, acc[q][2]);
+                    acc[q][3] = fma(ws, (double)t.w, acc[q][3]);
+                }
+            }
+        }
+        __syncthreads();
+    }
+#pragma unroll
+    for (int q = 0; q < C; q++)
+#pragma unroll
+        for (int i = 0; i < 4; i++) red[warp][lane][q][i] = acc[q][i];
+    __syncthreads();
+    for (int e = threadIdx.x; e < 32 * C; e += blockDim.x) {
+        const int l = e / C, q = e % C, jj = (vg.bx / ctiles) * 32 + l, col = c0 + q;
+        if (jj >= J1 || col >= A.gw) continue;
+        double t[4];
+#pragma unroll
+        for (int i = 0; i < 4; i++) {
+            t[i] = red[0][l][q][i];
+#pragma unroll
+            for (int w = 1; w < 8; w++) t[i] += red[w][l][q][i];
+        }
+        // sum T e^{-+i theta} = (even . cos) -+ i (odd . sin)
+        float2 *g = A.grid + (size_t)image * A.cells + col;
+        g[(size_t)(A.J + jj) * A.gw] = make_float2((float)(t[0] + t[3]), (float)(t[1] - t[2]));
+        g[(size_t)(A.J - jj) * A.gw] = make_float2((float)(t[0] - t[3]), (float)(t[1] + t[2]));
+    }
+}
+
+template <int C>
+__global__ void __launch_bounds__(256) k_ug_rows(const UgRowsArgs a)
+{
+    gp_pdl_enter();
+    ug_rows_body<C>(a, gp_vgrid_hw());
+}
+
+template <int C> struct UgRowsOp {
+    using Args = UgRowsArgs;
+    static __device__ __forceinline__ void run(const Args &a, const GpVGrid &v) { ug_rows_body<C>(a, v); }
+};
+
+// ------------------------------------------------------- interpolation
+//
+// V_k / F of one sorted uv point per thread. The points of a warp share a grid
+// cell or lie in neighbouring ones, so the 64 grid loads are served by one or
+// two sectors each; the window weights stream (64 B per point).
+#define UGI_THREADS 128
+struct UgInterpArgs {
+    const float2 *grid;
+    const int *src, *base;
+    const float *wts;
+    const float2 *phase;
+    const DevScalars *sc;
+    double2 *out;  // [nuv], or [GP_NTR][nuv] (trials)
+    int nuv, gw, cells, trials;
+    const int *gate;
+    GP_VGRID_FIELDS;
+};
+
+__device__ __forceinline__ void ug_interp_body(const UgInterpArgs &A, const GpVGrid &vg)
+{
+    if (A.gate && !*A.gate) return;
+    const int p = vg.bx * blockDim.x + threadIdx.x, image = vg.by;
+    if (p >= A.nuv) return;
+    const float4 *w4 = reinterpret_cast<const float4 *>(A.wts + (size_t)p * (2 * UG_W));
+    float w[2 * UG_W];
+#pragma unroll
+    for (int i = 0; i < 4; i++) *reinterpret_cast<float4 *>(&w[4 * i]) = __ldg(&w4[i]);
+    const float2 *g = A.grid + (size_t)image * A.cells + __ldg(&A.base[p]);
+    float re = 0.f, im = 0.f;
+#pragma unroll
+    for (int i = 0; i < UG_W; i++) {
+        float rr = 0.f, ri = 0.f;
+#pragma unroll
+        for (int j = 0; j < UG_W; j++) {
+            const float2 v = __ldg(&g[j]);
+            rr = fmaf(w[j], v.x, rr);
+            ri = fmaf(w[j], v.y, ri);
+        }
+        g += A.gw;
+        re = fmaf(w[UG_W + i], rr, re);
+        im = fmaf(w[UG_W + i], ri, im);
+    }
+    const float2 ph = __ldg(&A.phase[p]);
+    const int s = __ldg(&A.src[p]);
+    const double invF = A.trials ? A.sc->t_invflux[image] : A.sc->invflux;
+    const double vr = (double)re * ph.x - (double)im * ph.y;
+    const double vi = (double)re * ph.y + (double)im * ph.x;
+    A.out[(size_t)image * A.nuv + (s & 0x7fffffff)] = make_double2(vr * invF, (s < 0 ? -vi : vi) * invF);
+}
+
+__global__ void __launch_bounds__(UGI_THREADS) k_ug_interp(const UgInterpArgs a)
+{
+    gp_pdl_enter();
+    ug_interp_body(a, gp_vgrid_hw());
+}
+
+struct UgInterpOp {
+    using Args = UgInterpArgs;
+    static __device__ __forceinline__ void run(const Args &a, const GpVGrid &v) { ug_interp_body(a, v); }
+};
+
+// ------------------------------------------------------------ spreading
+//
+// One warp per run of at most 32 uv points of one grid cell: their 8 x 8 patch
+// sum_k c_k wx wy, two patch points per lane, in point order.
+struct UgSpreadArgs {
+    const float2 *cw;
+    const int *src;
+    const int2 *chunk;
+    const float *wts;
+    const float2 *phase;
+    float2 *patch;
+    int nchunk;
+    GP_VGRID_FIELDS;
+};
+
+__device__ __forceinline__ void ug_spread_body(const UgSpreadArgs &A, const GpVGrid &vg)
+{
+    const int lane = threadIdx.x & 31;
+    const int ch = vg.bx * (int)(blockDim.x >> 5) + (int)(threadIdx.x >> 5);
+    if (ch >= A.nchunk) return;  // warp-uniform
+    const int2 q = __ldg(&A.chunk[ch]);
+    float2 cv = make_float2(0.f, 0.f);
+    if (lane < q.y) {
+        // c_k e^{2 pi i (a - b)(N-1)/2}; a conjugated point contributes conj(c_k) (only the real part of the image is kept)
+        const int s = __ldg(&A.src[q.x + lane]);
+        float2 c = __ldg(&A.cw[s & 0x7fffffff]);
+        if (s < 0) c.y = -c.y;
+        const float2 ph = __ldg(&A.phase[q.x + lane]);
+        cv = make_float2(c.x * ph.x - c.y * ph.y, c.x * ph.y + c.y * ph.x);
+    }
+    const float *w = A.wts + (size_t)q.x * (2 * UG_W);
+    const int i = lane >> 3, j = lane & 7;
+    float2 a0 = make_float2(0.f, 0.f), a1 = make_float2(0.f, 0.f);
+#pragma unroll 4
+    for (int n = 0; n < q.y; n++) {
+        const float cx = __shfl_sync(0xffffffffu, cv.x, n), cy = __shfl_sync(0xffffffffu, cv.y, n);
+        const float wx = __ldg(&w[j]);
+        const float f0 = wx * __ldg(&w[UG_W + i]), f1 = wx * __ldg(&w[UG_W + 4 + i]);
+        a0.x = fmaf(f0, cx, a0.x);
+        a0.y = fmaf(f0, cy, a0.y);
+        a1.x = fmaf(f1, cx, a1.x);
+        a1.y = fmaf(f1, cy, a1.y);
+        w += 2 * UG_W;
+    }
+    float2 *out = A.patch + (size_t)ch * (UG_W * UG_W);
+    out[lane] = a0;
+    out[32 + lane] = a1;
+}
+
+__global__ void __launch_bounds__(256) k_ug_spread(const UgSpreadArgs a)
+{
+    gp_pdl_enter();
+    ug_spread_body(a, gp_vgrid_hw());
+}
+
+struct UgSpreadOp {
+    using Args = UgSpreadArgs;
+    static __device__ __forceinline__ void run(const Args &a, const GpVGrid &v) { ug_spread_body(a, v); }
+};
+
+// Grid point (jy, jx) = the patches of the cells (jy - i, jx - j) at (i, j): eight
+// threads per grid point (one per i), FP64, cells and runs in order.
+struct UgGatherArgs {
+    const int *cst;
+    const float2 *patch;
+    float2 *cgrid;
+    int gw, cells;
+    GP_VGRID_FIELDS;
+};
+
+__device__ __forceinline__ void ug_gather_body(const UgGatherArgs &A, const GpVGrid &vg)
+{
+    const int t = vg.bx * (int)blockDim.x + (int)threadIdx.x;
+    const int q = t >> 3, i = t & 7;
+    double re = 0.0, im = 0.0;
+    if (q < A.cells) {
+        const int jy = q / A.gw - i, jx = q % A.gw;
+        if (jy >= 0) {
+#pragma unroll
+            for (int j = 0; j < UG_W; j++) {
+                if (jx - j >= 0) {
+                    const int cell = jy * A.gw + jx - j;
+                    const int e = __ldg(&A.cst[cell + 1]);
+                    for (int s = __ldg(&A.cst[cell]); s < e; s++) {
+                        const float2 v = __ldg(&A.patch[(size_t)s * (UG_W * UG_W) + i * UG_W + j]);
+                        re += v.x;
+                        im += v.y;
+                    }
+                }
+            }
+        }
+    }
+#pragma unroll
+    for (int o = 4; o > 0; o >>= 1) {
+        re += __shfl_down_sync(0xffffffffu, re, o, 8);
+        im += __shfl_down_sync(0xffffffffu, im, o, 8);
+    }
+    if (i == 0 && q < A.cells) A.cgrid[q] = make_float2((float)re, (float)im);
+}
+
+__global__ void __launch_bounds__(256) k_ug_gather(const UgGatherArgs a)
+{
+    gp_pdl_enter();
+    ug_gather_body(a, gp_vgrid_hw());
+}
+
+struct UgGatherOp {
+    using Args = UgGatherArgs;
+    static __device__ __forceinline__ void run(const Args &a, const GpVGrid &v) { ug_gather_body(a, v); }
+};
+
+// ------------------------------------------------- adjoint y contraction
+//
+// S[y][jx] for 32 columns (lane = jx) and 8 UGC_H folded image rows per block
+// (a warp takes UGC_H of them, image rows h and N-1-h). The sums and
+// differences of the grid rows +-j wait in shared memory.
+#define UGC_H 2
+#define UGC_J 64
+struct UgColsArgs {
+    const float2 *cgrid, *ctab;
+    float2 *S;
+    int N, H, gw, J;
+    GP_VGRID_FIELDS;
+};
+
+__device__ __forceinline__ void ug_cols_body(const UgColsArgs &A, const GpVGrid &vg)
+{
+    __shared__ __align__(16) float4 Cs[UGC_J][32];  // (sum, difference)
+    __shared__ float2 Ws[8 * UGC_H][UGC_J];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int xt = (A.gw + 31) / 32;
+    const int jx = (vg.bx % xt) * 32 + lane, hb = (vg.bx / xt) * 8 * UGC_H;
+    const int J1 = A.J + 1;
+    double acc[UGC_H][4];  // even (re, im), odd (re, im)
+#pragma unroll
+    for (int r = 0; r < UGC_H; r++)
+#pragma unroll
+        for (int i = 0; i < 4; i++) acc[r][i] = 0.0;
+    for (int jb = 0; jb < J1; jb += UGC_J) {
+        const int nj = min(UGC_J, J1 - jb);
+        for (int jj = warp; jj < nj; jj += 8) {
+            const int j = jb + jj;
+            float2 p = make_float2(0.f, 0.f), m = make_float2(0.f, 0.f);
+            if (jx < A.gw) {
+                p = __ldg(&A.cgrid[(size_t)(A.J + j) * A.gw + jx]);
+                if (j) m = __ldg(&A.cgrid[(size_t)(A.J - j) * A.gw + jx]);
+            }
+            Cs[jj][lane] = make_float4(p.x + m.x, p.y + m.y, p.x - m.x, p.y - m.y);
+        }
+        for (int e = threadIdx.x; e < 8 * UGC_H * UGC_J; e += blockDim.x) {
+            const int r = e / UGC_J, jj = e % UGC_J, h = hb + r;
+            if (jj < nj) Ws[r][jj] = h < A.H ? __ldg(&A.ctab[(size_t)h * J1 + jb + jj]) : make_float2(0.f, 0.f);
+        }
+        __syncthreads();
+#pragma unroll 4
+        for (int jj = 0; jj < nj; jj++) {
+            const float4 v = Cs[jj][lane];
+#pragma unroll
+            for (int r = 0; r < UGC_H; r++) {
+                const float2 w = Ws[warp * UGC_H + r][jj];
+                acc[r][0] = fma((double)w.x, (double)v.x, acc[r][0]);
+                acc[r][1] = fma((double)w.x, (double)v.y, acc[r][1]);
+                acc[r][2] = fma((double)w.y, (double)v.z, acc[r][2]);
+                acc[r][3] = fma((double)w.y, (double)v.w, acc[r][3]);
+            }
+        }
+        __syncthreads();
+    }
+    if (jx >= A.gw) return;
+#pragma unroll
+    for (int r = 0; r < UGC_H; r++) {
+        const int h = hb + warp * UGC_H + r;
+        if (h >= A.H) continue;
+        // C[j] e^{-i theta} + C[-j] e^{i theta} = sum . cos - i difference . sin, theta -> -theta at row h
+        A.S[(size_t)(A.N - 1 - h) * A.gw + jx] = 
+            make_float2((float)(acc[r][0] + acc[r][3]), (float)(acc[r][1] - acc[r][2]));
+        if (h != A.N - 1 - h)
+            A.S[(size_t)h * A.gw + jx] =
+                make_float2((float)(acc[r][0] - acc[r][3]), (float)(acc[r][1] + acc[r][2]));
+    }
+}
+
+__global__ void __launch_bounds__(256) k_ug_cols(const UgColsArgs a)
+{
+    gp_pdl_enter();
+    ug_cols_body(a, gp_vgrid_hw());
+}
+
+struct UgColsOp {
+    using Args = UgColsArgs;
+    static __device__ __forceinline__ void run(const Args &a, const GpVGrid &v) { ug_cols_body(a, v); }
+};
+
+// ------------------------------------------------------------ host side
+
+// Buffers of the batched trials: rows for the tensor path's operand stack, which has at
+// least as many per image as the CUDA cores (N)
+int gp_ug_batch_alloc(gpair_ctx *c)
+{
+    UgState *g = (UgState *)c->ug;
+    if (g->gridb) return GPAIR_OK;
+    const size_t rows = (size_t)GP_NTR * gp_tc_stack_rows(c->N);
+    GP_CUDA(c, cudaMalloc(&g->Tb, sizeof(float) * UG_MAX_SPLITS * rows * g->ldT));
+    GP_CUDA(c, cudaMalloc(&g->gridb, sizeof(float2) * GP_NTR * (size_t)g->cells));
+    return GPAIR_OK;
+}
+
+// x contraction on the CUDA cores: the current or trial image, or the batch's trial images
+int gp_ug_x(gpair_ctx *c, const float *img, int images)
+{
+    UgState *g = (UgState *)c->ug;
+    UgXArgs a;
+    a.img = img;
+    a.ftab = g->ftab;
+    a.T = images > 1 ? g->Tb : g->T;
+    a.N = g->N;
+    a.H = g->H;
+    a.nbx = g->nbx;
+    a.ldT = g->ldT;
+    a.images = images;
+    const int bx = gp_cdiv(g->N, UGX_T), by = gp_cdiv(g->nbx, UGX_T);
+    // slices of h (whole tiles) until the blocks fill two waves of 148 SMs
+    int s = 1;
+    while (s < UG_MAX_SPLITS && 2 * s * UGX_T <= g->H && bx * by * images * s < 2 * 148) s *= 2;
+    a.hper = gp_cdiv(gp_cdiv(g->H, s), UGX_T) * UGX_T;
+    a.splits = gp_cdiv(g->H, a.hper);
+    a.gate = images > 1 ? c->gate : nullptr;
+    GP_LAUNCH(c, gp_launch(c, k_ug_x, dim3(bx, by, a.splits * images), dim3(256), 0, a));
+    (images > 1 ? g->splitsb : g->splits) = a.splits;
+    return GPAIR_OK;
+}
+
+// columns per block of the y contraction: one for a single image (enough blocks), four for a batch
+#define UGR_COLS_BATCH 4
+
+// rsc, lrows: row scales and rows per image of the tensor path's operand (null and N on the CUDA cores)
+static UgRowsArgs ug_rows_args(gpair_ctx *c, int images, int splits, const float *rsc, int lrows, const int *gate)
+{
+    UgState *g = (UgState *)c->ug;
+    UgRowsArgs a;
+    memset(&a, 0, sizeof(a));
+    a.T = images > 1 ? g->Tb : g->T;
+    a.rsc = rsc;
+    a.ctab = g->ctab;
+    a.grid = images > 1 ? g->gridb : g->grid;
+    a.N = g->N;
+    a.H = g->H;
+    a.gw = g->nbx;
+    a.J = g->J;
+    a.ldT = g->ldT;
+    a.cells = g->cells;
+    a.splits = splits;
+    a.lrows = lrows;
+    a.split_stride = (size_t)(images > 1 ? images * lrows : g->N) * g->ldT;
+    a.gate = gate;
+    a.nbx = gp_cdiv(g->nbx, images > 1 ? UGR_COLS_BATCH : 1) * gp_cdiv(g->J + 1, 32);
+    a.nby = images;
+    return a;
+}
+
+static UgInterpArgs ug_interp_args(gpair_ctx *c, int images, const int *gate)
+{
+    UgState *g = (UgState *)c->ug;
+    UgInterpArgs a;
+    memset(&a, 0, sizeof(a));
+    a.grid = images > 1 ? g->gridb : g->grid;
+    a.src = g->src;
+    a.base = g->base;
+    a.wts = g->wts;
+    a.phase = g->phase;
+    a.sc = c->sc;
+    a.out = images > 1 ? c->visb : c->visd;
+    a.nuv = c->nuv;
+    a.gw = g->nbx;
+    a.cells = g->cells;
+    a.trials = images > 1;
+    a.gate = gate;
+    a.nbx = gp_cdiv(c->nuv, UGI_THREADS);
+    a.nby = images;
+    return a;
+}
+
+static UgSpreadArgs ug_spread_args(gpair_ctx *c)
+{
+    UgState *g = (UgState *)c->ug;
+    UgSpreadArgs a = {c->cw, g->src, g->chunk, g->wts, g->phase, g->patch, g->nchunk, gp_cdiv(g->nchunk, 8), 1};
+    return a;
+}
+
+static UgGatherArgs ug_gather_args(gpair_ctx *c)
+{
+    UgState *g = (UgState *)c->ug;
+    UgGatherArgs a = {g->cst, g->patch, g->cgrid, g->nbx, g->cells, gp_cdiv(8LL * g->cells, 256), 1};
+    return a;
+}
+
+static UgColsArgs ug_cols_args(gpair_ctx *c)
+{
+    UgState *g = (UgState *)c->ug;
+    UgColsArgs a = {g->cgrid, g->ctab, g->S, g->N, g->H, g->nbx, g->J,
+                    gp_cdiv(g->nbx, 32) * gp_cdiv(g->H, 8 * UGC_H), 1};
+    return a;
+}
+
+// From T to the visibilities: V_k / F into visd (images = 1), or of every trial into visb
+int gp_ug_vis(gpair_ctx *c, int images)
+{
+    UgState *g = (UgState *)c->ug;
+    const float *rsc = nullptr;
+    int lrows = g->N, splits = images > 1 ? g->splitsb : g->splits;
+    if (c->precision != GPAIR_PREC_FP32) {
+        int rc = gp_tc_ug_rows(c, images, &rsc, &lrows, &splits);
+        if (rc) return rc;
+    }
+    const int *gate = images > 1 ? c->gate : nullptr;
+    const UgRowsArgs r = ug_rows_args(c, images, splits, rsc, lrows, gate);
+    GP_LAUNCH(c, gp_launch(c, images > 1 ? k_ug_rows<UGR_COLS_BATCH> : k_ug_rows<1>, dim3(r.nbx, r.nby), dim3(256), 0,
+                           r));
+    const UgInterpArgs t = ug_interp_args(c, images, gate);
+    GP_LAUNCH(c, gp_launch(c, k_ug_interp, dim3(t.nbx, t.nby), dim3(UGI_THREADS), 0, t));
+    return GPAIR_OK;
+}
+
+// From the uv weights c_k to S[y][jx], the x contraction's operand (gp_grad_finalize finishes the gradient)
+int gp_ug_adjoint(gpair_ctx *c)
+{
+    const UgSpreadArgs s = ug_spread_args(c);
+    GP_LAUNCH(c, gp_launch(c, k_ug_spread, dim3(s.nbx), dim3(256), 0, s));
+    const UgGatherArgs t = ug_gather_args(c);
+    GP_LAUNCH(c, gp_launch(c, k_ug_gather, dim3(t.nbx), dim3(256), 0, t));
+    const UgColsArgs q = ug_cols_args(c);
+    GP_LAUNCH(c, gp_launch(c, k_ug_cols, dim3(q.nbx), dim3(256), 0, q));
+    return GPAIR_OK;
+}
+
+// ------------------------------------------------- grouped stage launches
+
+size_t gp_ug_stage_args_size(int stage)
+{
+    switch (stage) {
+    case GS_UG_ROWS:
+    case GS_UG_ROWS_T: return sizeof(UgRowsArgs);
+    case GS_UG_INTERP:
+    case GS_UG_INTERP_T: return sizeof(UgInterpArgs);
+    case GS_UG_SPREAD: return sizeof(UgSpreadArgs);
+    case GS_UG_GATHER: return sizeof(UgGatherArgs);
+    case GS_UG_COLS: return sizeof(UgColsArgs);
+    default: return 0;
+    }
+}
+
+template <class A>
+static int put_args(const A &a, void *out, int *nblocks)
+{
+    memcpy(out, &a, sizeof(A));
+    *nblocks = a.nbx * a.nby;
+    return GPAIR_OK;
+}
+
+int gp_ug_stage_args(gpair_ctx *c, int stage, void *out, int *nblocks)
+{
+    const int images = (stage == GS_UG_ROWS_T || stage == GS_UG_INTERP_T) ? GP_NTR : 1;
+    switch (stage) {
+    case GS_UG_ROWS:
+    case GS_UG_ROWS_T: {
+        const float *rsc;
+        int lrows, splits, rc;
+        if ((rc = gp_tc_ug_rows(c, images, &rsc, &lrows, &splits))) return rc;
+        return put_args(ug_rows_args(c, images, splits, rsc, lrows, nullptr), out, nblocks);
+    }
+    case GS_UG_INTERP:
+    case GS_UG_INTERP_T: return put_args(ug_interp_args(c, images, nullptr), out, nblocks);
+    case GS_UG_SPREAD: return put_args(ug_spread_args(c), out, nblocks);
+    case GS_UG_GATHER: return put_args(ug_gather_args(c), out, nblocks);
+    case GS_UG_COLS: return put_args(ug_cols_args(c), out, nblocks);
+    default: return GPAIR_ERR_INVALID;
+    }
+}
+
+template <class Op, int THREADS>
+static int group_launch(gpair_ctx *c, const void *d_args, const int *d_start, int n, int total, const int *gate)
+{
+    GP_LAUNCH(c, gp_launch(c, k_grouped<Op, THREADS>, dim3(total), dim3(THREADS), 0,
+                           (const typename Op::Args *)d_args, d_start, n, gate));
+    return GPAIR_OK;
+}
+
+int gp_ug_stage_group_launch(gpair_ctx *c, int stage, const void *d_args, const int *d_start, int n, int total,
+                             const int *gate)
+{
+    if (total < 1 || n < 1) return GPAIR_ERR_INVALID;
+    switch (stage) {
+    case GS_UG_ROWS: return group_launch<UgRowsOp<1>, 256>(c, d_args, d_start, n, total, gate);
+    case GS_UG_ROWS_T: return group_launch<UgRowsOp<UGR_COLS_BATCH>, 256>(c, d_args, d_start, n, total, gate);
+    case GS_UG_INTERP:
+    case GS_UG_INTERP_T: return group_launch<UgInterpOp, UGI_THREADS>(c, d_args, d_start, n, total, gate);
+    case GS_UG_SPREAD: return group_launch<UgSpreadOp, 256>(c, d_args, d_start, n, total, gate);
+    case GS_UG_GATHER: return group_launch<UgGatherOp, 256>(c, d_args, d_start, n, total, gate);
+    case GS_UG_COLS: return group_launch<UgColsOp, 256>(c, d_args, d_start, n, total, gate);
+    default: return GPAIR_ERR_INVALID;
+    }
+}

@@ -1,0 +1,49 @@
+// uvgrid.cuh -- the uv-grid plan of a context (uvgrid.cu).
+#pragma once
+
+#include "gpair_internal.cuh"
+
+#define UG_W 8  // window width in grid points
+#define UG_OVERSAMPLING 2.0  // grid points per cycle and image width (2.5 and 3 measured no more accurate: FP32 rounding remains)
+#define UG_MAX_SPLITS 8  // partial sums of the x contraction
+
+// A problem takes the grid when the image is at least UG_MIN_WIDTH wide, its direct work 2 N^2 nuv is at
+// least UG_MIN_WORK_* of the precision mode and UG_GRID_RATIO times the grid's own contractions.
+// UG_MIN_WIDTH: on narrower images hundreds of uv points share a grid point, and its FP32 rounding no
+// longer averages out of the gradient (2e-7 to 4e-7 at 55 to 67 pixels, the direct sums 1e-7).
+// UG_MIN_WORK_FP32: where the CUDA-core contractions start to cost more than the grid's fixed launches
+// (147^2 x 1,904 uv: forward 22 against 17 us; 128^2 x 960: 16 against 15).
+// UG_MIN_WORK_TC, _F8: the tensor contractions are within a few us of the grid up to there (256^2 x 960
+// uv: 85 against 91 us for an objective with its gradient; 256^2 x 21,120: 120 against 99). Below it they also keep
+// what long runs reproduce: their rounding, 1e-6 to 1e-5 of the gradient and largest with E4M3 cross
+// terms, is a hundred times the grid's, and a CG run a few iterations on differs by up to 5e-5 with it.
+#define UG_MIN_WIDTH 96
+#define UG_MIN_WORK_FP32 4e7
+#define UG_MIN_WORK_TC 1.2e9
+#define UG_MIN_WORK_F8 4e9
+#define UG_GRID_RATIO 4.0
+
+struct UgState {
+    int N, H;            // image width, folded width (N + 1) / 2
+    int jxf, nbx, J;     // grid columns jxf .. jxf + nbx - 1, rows -J .. J
+    int cells, nchunk;   // nbx (2 J + 1); runs of at most 32 uv points of one cell
+    int ldT;             // floats per row of T
+    // uv points sorted by the cell of their first window point
+    int *src;            // [nuv] uv index, bit 31: conjugated
+    int *base;           // [nuv] cell
+    float *wts;          // [nuv][2 UG_W] window weights along x, then y
+    float2 *phase;       // [nuv] e^{2 pi i (a - b)(N-1)/2}
+    int2 *chunk;         // [nchunk] (first point, points)
+    int *cst;            // [cells + 1] first run of every cell
+    float2 *ftab, *ctab; // grid twiddles [nbx][H], [H][J + 1] (k_ug_tables)
+    double *invphi;      // [H] 1 / window transform
+    float *T;            // [splits][N][ldT] x contraction of one image
+    float2 *grid;        // [cells] G
+    float2 *patch;       // [nchunk][64]
+    float2 *cgrid;       // [cells] C
+    float2 *S;           // [N][nbx]
+    // batched trials
+    float *Tb;           // [splits][GP_NTR rows per image][ldT]
+    float2 *gridb;       // [GP_NTR][cells]
+    int splits, splitsb; // partial sums of the last CUDA-core x contraction
+};
