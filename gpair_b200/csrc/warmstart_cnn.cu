@@ -31,7 +31,6 @@
 #define CV_T 16    // output tile edge (pixels)
 #define CV_CO 16   // output channels per block
 #define CV_CI 8    // input channels per shared-memory chunk
-#define WG_CI 8    // input channels per weight-gradient block
 #define NTAP 9
 
 __device__ __forceinline__ float bf(const __nv_bfloat16 *w, size_t i) { return __bfloat162float(w[i]); }
@@ -102,55 +101,105 @@ __global__ void __launch_bounds__(CV_T *CV_T) k_conv3(const float *__restrict__ 
     }
 }
 
-// Weight and bias gradient partials: block (co, ci-chunk, slice) sums over the
-// images [slice*bps, (slice+1)*bps) and all pixels; part[slice][co][ci][tap],
-// bpart[slice][co] (bias, from the ci-chunk 0 blocks).
-__global__ void __launch_bounds__(256) k_conv3_wgrad(const float *__restrict__ in, const float *__restrict__ g,
-                                                     float *__restrict__ part, float *__restrict__ bpart, int B,
-                                                     int Cin, int Cout, int H, int W, int bps)
+// Weight and bias gradient partials: block (CO output channels, input channel,
+// slice) sums over the images [slice*bps, (slice+1)*bps) and all pixels;
+// part[slice][co][ci][tap], bpart[slice][co] (bias, from the blocks of the first
+// input channel). Thread t sums the pixels p = t mod 256 in order, image by
+// image; the threads' sums go through a shuffle tree and then over the warps
+// in order. Bound by instruction issue: 9 predicated input loads and CO of g for
+// 9 CO FMAs, the pixel's coordinates advanced without a division, and U pixels
+// loaded before the first is used. (One output and 8 input channels per block
+// made 32 blocks of a 16 -> 16 layer, each waiting for one pixel's loads at a
+// time: 16 images of 64^2 took 765 us, now 66; 128 -> 128 at 8^2 318, now 41.)
+#define WG_THREADS 256
+template <int CO, int U>
+__global__ void __launch_bounds__(WG_THREADS) k_conv3_wgrad(const float *__restrict__ in, const float *__restrict__ g,
+                                                            float *__restrict__ part, float *__restrict__ bpart, int B,
+                                                            int Cin, int Cout, int H, int W, int bps)
 {
-    __shared__ float red[8][WG_CI * NTAP + 1];
-    const int co = blockIdx.x, ci0 = blockIdx.y * WG_CI, slice = blockIdx.z;
+    constexpr int NV = CO * NTAP + CO;
+    __shared__ float red[WG_THREADS / 32][NV];
+    const int co0 = blockIdx.x * CO, ci = blockIdx.y, slice = blockIdx.z;
     const int b0 = slice * bps, b1 = min(B, b0 + bps);
-    float acc[WG_CI * NTAP + 1];
+    float acc[NV];  // [co][tap], then the bias sums
 #pragma unroll
-    for (int i = 0; i < WG_CI * NTAP + 1; i++) acc[i] = 0.f;
+    for (int i = 0; i < NV; i++) acc[i] = 0.f;
     const int HW = H * W;
-    for (int b = b0; b < b1; b++) {
-        const float *gb = g + ((size_t)b * Cout + co) * HW;
-        const float *ib = in + (size_t)b * Cin * HW;
-        for (int p = threadIdx.x; p < HW; p += blockDim.x) {
-            const float gv = gb[p];
-            acc[WG_CI * NTAP] += gv;
-            if (gv == 0.f) continue;
-            const int y = p / W, x = p - y * W;
+    // this thread's pixels of an image (a block smaller than 256 threads has one per thread), over the slice's images
+    const int per = (int)threadIdx.x < HW ? (HW - (int)threadIdx.x + WG_THREADS - 1) / WG_THREADS : 0;
+    const int steps = per * (b1 - b0);
+    const int dy = WG_THREADS / W, dx = WG_THREADS - dy * W, yt = (int)threadIdx.x / W, xt = (int)threadIdx.x - yt * W;
+    const float *gp = g + ((size_t)b0 * Cout + co0) * HW + threadIdx.x;
+    const float *ip = in + ((size_t)b0 * Cin + ci) * HW + threadIdx.x;
+    const int no = min(CO, Cout - co0);
+    int left = per, y = yt, x = xt;
+    for (int s = 0; s < steps; s += U) {
+        float gv[U][CO], v[U][NTAP];
 #pragma unroll
-            for (int k = 0; k < NTAP; k++) {
-                const int yy = y + k / 3 - 1, xx = x + k % 3 - 1;
-                if (yy < 0 || yy >= H || xx < 0 || xx >= W) continue;
+        for (int u = 0; u < U; u++) {
+            const bool live = s + u < steps;
+            const bool r0 = live && y > 0, r2 = live && y + 1 < H, c0 = x > 0, c2 = x + 1 < W;
 #pragma unroll
-                for (int c = 0; c < WG_CI; c++)
-                    if (ci0 + c < Cin) acc[c * NTAP + k] = fmaf(gv, ib[(size_t)(ci0 + c) * HW + yy * W + xx], acc[c * NTAP + k]);
+            for (int o = 0; o < CO; o++) gv[u][o] = live && o < no ? __ldg(gp + (size_t)o * HW) : 0.f;
+            const float *u0 = ip - W, *u2 = ip + W;
+            v[u][0] = r0 && c0 ? __ldg(u0 - 1) : 0.f;
+            v[u][1] = r0 ? __ldg(u0) : 0.f;
+            v[u][2] = r0 && c2 ? __ldg(u0 + 1) : 0.f;
+            v[u][3] = live && c0 ? __ldg(ip - 1) : 0.f;
+            v[u][4] = live ? __ldg(ip) : 0.f;
+            v[u][5] = live && c2 ? __ldg(ip + 1) : 0.f;
+            v[u][6] = r2 && c0 ? __ldg(u2 - 1) : 0.f;
+            v[u][7] = r2 ? __ldg(u2) : 0.f;
+            v[u][8] = r2 && c2 ? __ldg(u2 + 1) : 0.f;
+            if (--left > 0) {
+                gp += WG_THREADS;
+                ip += WG_THREADS;
+                y += dy;
+                x += dx;
+                if (x >= W) {
+                    x -= W;
+                    y++;
+                }
+            } else {  // the next image
+                const int back = (per - 1) * WG_THREADS;
+                gp += (ptrdiff_t)Cout * HW - back;
+                ip += (ptrdiff_t)Cin * HW - back;
+                y = yt;
+                x = xt;
+                left = per;
             }
         }
+#pragma unroll
+        for (int u = 0; u < U; u++)
+#pragma unroll
+            for (int o = 0; o < CO; o++) {
+                acc[CO * NTAP + o] += gv[u][o];
+                if (gv[u][o] != 0.f) {  // masked pixels add nothing
+#pragma unroll
+                    for (int k = 0; k < NTAP; k++) acc[o * NTAP + k] = fmaf(gv[u][o], v[u][k], acc[o * NTAP + k]);
+                }
+            }
     }
-    // fixed-order block reduction: warp shuffles, then one pass over the 8 warps
+    // fixed-order block reduction: warp shuffles, then one pass over the warps
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
 #pragma unroll
-    for (int i = 0; i < WG_CI * NTAP + 1; i++) {
+    for (int i = 0; i < NV; i++) {
         float v = acc[i];
+#pragma unroll
         for (int off = 16; off > 0; off >>= 1) v += __shfl_down_sync(0xffffffffu, v, off);
         if (lane == 0) red[warp][i] = v;
     }
     __syncthreads();
-    for (int i = threadIdx.x; i < WG_CI * NTAP + 1; i += blockDim.x) {
+    const int nw = (int)(blockDim.x >> 5);
+    for (int i = threadIdx.x; i < NV; i += blockDim.x) {
         float v = 0.f;
-        for (int w8 = 0; w8 < (int)(blockDim.x >> 5); w8++) v += red[w8][i];
-        if (i < WG_CI * NTAP) {
-            const int c = i / NTAP, k = i % NTAP;
-            if (ci0 + c < Cin) part[(((size_t)slice * Cout + co) * Cin + ci0 + c) * NTAP + k] = v;
+        for (int w = 0; w < nw; w++) v += red[w][i];
+        if (i < CO * NTAP) {
+            const int co = co0 + i / NTAP, k = i % NTAP;
+            if (co < Cout) part[(((size_t)slice * Cout + co) * Cin + ci) * NTAP + k] = v;
         } else if (blockIdx.y == 0) {
-            bpart[(size_t)slice * Cout + co] = v;
+            const int co = co0 + i - CO * NTAP;
+            if (co < Cout) bpart[(size_t)slice * Cout + co] = v;
         }
     }
 }
@@ -163,6 +212,20 @@ __global__ void k_reduce_slices(const float *__restrict__ part, int n, int slice
     float s = 0.f;
     for (int k = 0; k < slices; k++) s += part[(size_t)k * n + i];
     out[i] = s;
+}
+
+// The same for a weight gradient (nw values) and its bias gradient (nb) in one launch
+__global__ void k_reduce_wgrad(const float *__restrict__ part, int nw, const float *__restrict__ bpart, int nb,
+                               int slices, float *__restrict__ dw, float *__restrict__ db)
+{
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= nw + nb) return;
+    const float *p = i < nw ? part + i : bpart + (i - nw);
+    const size_t ld = i < nw ? nw : nb;
+    float s = 0.f;
+    for (int k = 0; k < slices; k++) s += __ldg(p + (size_t)k * ld);
+    if (i < nw) dw[i] = s;
+    else db[i - nw] = s;
 }
 
 __global__ void k_relu_mask(const float *__restrict__ y, float *__restrict__ g, long long n)
@@ -378,10 +441,18 @@ extern "C" int gpair_cnn_conv3x3_bwd_weight(const float *in, const float *gpre, 
     const long long nw = (long long)Cout * Cin * NTAP;
     if ((long long)slices * (nw + Cout) > scratch_floats) return GPAIR_ERR_INVALID;
     float *part = scratch, *bpart = scratch + (size_t)slices * nw;
-    dim3 g(Cout, cdiv_ll(Cin, WG_CI), slices);
-    k_conv3_wgrad<<<g, 256, 0, CNN_STREAM(stream)>>>(in, gpre, part, bpart, B, Cin, Cout, H, W, bps);
-    k_reduce_slices<<<cdiv_ll(nw, 256), 256, 0, CNN_STREAM(stream)>>>(part, (int)nw, slices, dw);
-    k_reduce_slices<<<cdiv_ll(Cout, 256), 256, 0, CNN_STREAM(stream)>>>(bpart, Cout, slices, db);
+    // a thread per pixel of an image, up to 256: the warps past them would add zeros
+    const int threads = H * W >= WG_THREADS ? WG_THREADS : (H * W + 31) / 32 * 32;
+    // four output channels a block (9 input loads for 36 FMAs) where that still makes two blocks per SM
+    const cudaStream_t st = CNN_STREAM(stream);
+    auto go = [&](auto kernel, int co) {
+        kernel<<<dim3(cdiv_ll(Cout, co), Cin, slices), threads, 0, st>>>(in, gpre, part, bpart, B, Cin, Cout, H, W, bps);
+    };
+    const long long blocks = (long long)Cout * Cin * slices;
+    if (blocks >= 4 * 2 * 148) go(k_conv3_wgrad<4, 2>, 4);
+    else if (blocks >= 2 * 2 * 148) go(k_conv3_wgrad<2, 4>, 2);
+    else go(k_conv3_wgrad<1, 4>, 1);
+    k_reduce_wgrad<<<cdiv_ll(nw + Cout, 256), 256, 0, st>>>(part, (int)nw, bpart, Cout, slices, dw, db);
     return cnn_status();
 }
 
