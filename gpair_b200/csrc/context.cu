@@ -83,6 +83,11 @@ static void set_handle(gpair_buf *h, float *p, size_t n, int id)
     h->id = id;
 }
 
+// Host arrays up to this size (a 256 x 256 image) pass through the context's pinned staging buffer: one memcpy
+// and an asynchronous copy. Above it the memcpy dominates and the driver's own path for pageable memory is taken.
+// 24 uploads of 64^2 to 256^2 images: 870 us with a wait each, 440 staged.
+#define GP_STAGE_BYTES ((size_t)256 << 10)
+
 // (Re)allocate the image-sized buffers for width N; contents are zeroed.
 int gp_alloc_images(gpair_ctx *c, int N)
 {
@@ -138,7 +143,20 @@ extern "C" int gpair_create(gpair_ctx **out, int device)
         if (cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking) != cudaSuccess) { rc = GPAIR_ERR_CUDA; break; }
         if (cudaMalloc(&c->sc, sizeof(DevScalars)) != cudaSuccess) { rc = GPAIR_ERR_ALLOC; break; }
         if (cudaMemset(c->sc, 0, sizeof(DevScalars)) != cudaSuccess) { rc = GPAIR_ERR_CUDA; break; }
-        if (cudaMallocHost(&c->sc_host, sizeof(DevScalars)) != cudaSuccess) { rc = GPAIR_ERR_ALLOC; break; }
+        // one pinned block: the scalars' mirror, the results of blocking calls, the staging of small host arrays
+        const size_t at_res = (sizeof(DevScalars) + 63) / 64 * 64, at_stage = at_res + 64;
+        static_assert(sizeof(GpHostResult) <= 64, "layout of the pinned block");
+        if (cudaMallocHost(&c->sc_host, at_stage + GP_STAGE_BYTES) != cudaSuccess) {
+            rc = GPAIR_ERR_ALLOC;
+            break;
+        }
+        c->hres = reinterpret_cast<GpHostResult *>(reinterpret_cast<char *>(c->sc_host) + at_res);
+        c->stage = reinterpret_cast<char *>(c->sc_host) + at_stage;
+        if (cudaEventCreateWithFlags(&c->stage_ev, cudaEventDisableTiming) != cudaSuccess ||
+            cudaEventCreate(&c->run_e0) != cudaSuccess || cudaEventCreate(&c->run_e1) != cudaSuccess) {
+            rc = GPAIR_ERR_CUDA;
+            break;
+        }
         size_t pbytes = sizeof(double) * RED_NSLOTS * GP_MAX_PARTIALS * 4;
         if (cudaMalloc(&c->partials, pbytes) != cudaSuccess) { rc = GPAIR_ERR_ALLOC; break; }
     } while (0);
@@ -160,6 +178,9 @@ extern "C" int gpair_destroy(gpair_ctx *c)
     FREE_DEV(c->sc);
     FREE_DEV(c->partials);
     if (c->sc_host) cudaFreeHost(c->sc_host);
+    if (c->stage_ev) cudaEventDestroy(c->stage_ev);
+    if (c->run_e0) cudaEventDestroy(c->run_e0);
+    if (c->run_e1) cudaEventDestroy(c->run_e1);
     if (c->st_ev) {
         for (int i = 0; i < 2 * GP_MAX_STAGE_REC; i++)
             if (c->st_ev[i]) cudaEventDestroy(c->st_ev[i]);
@@ -326,14 +347,32 @@ extern "C" int gpair_set_image(gpair_ctx *c, int which, const float *image)
 {
     if (!c || !image || !c->image) return GPAIR_ERR_STATE;
     float *dst = which == GPAIR_IMG_TEMP ? c->image_temp : c->image;
-    GP_CUDA(c, cudaMemcpyAsync(dst, image, c->npix * sizeof(float), cudaMemcpyHostToDevice, c->stream));
-    GP_CUDA(c, cudaStreamSynchronize(c->stream));
+    const size_t bytes = c->npix * sizeof(float);
+    if (bytes <= GP_STAGE_BYTES) {
+        // the caller's array is free as soon as it is staged; the copy runs in stream order
+        if (c->stage_busy) GP_CUDA(c, cudaEventSynchronize(c->stage_ev));
+        c->stage_busy = 0;
+        memcpy(c->stage, image, bytes);
+        GP_CUDA(c, cudaMemcpyAsync(dst, c->stage, bytes, cudaMemcpyHostToDevice, c->stream));
+        GP_CUDA(c, cudaEventRecord(c->stage_ev, c->stream));
+        c->stage_busy = 1;
+    } else {
+        GP_CUDA(c, cudaMemcpyAsync(dst, image, bytes, cudaMemcpyHostToDevice, c->stream));
+        GP_CUDA(c, cudaStreamSynchronize(c->stream));
+    }
     c->have_image = 1;
     return GPAIR_OK;
 }
 
 static int d2h(gpair_ctx *c, void *dst, const void *src, size_t bytes)
 {
+    if (bytes <= GP_STAGE_BYTES) {
+        GP_CUDA(c, cudaMemcpyAsync(c->stage, src, bytes, cudaMemcpyDeviceToHost, c->stream));
+        GP_CUDA(c, cudaStreamSynchronize(c->stream));
+        c->stage_busy = 0;
+        memcpy(dst, c->stage, bytes);
+        return GPAIR_OK;
+    }
     GP_CUDA(c, cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, c->stream));
     GP_CUDA(c, cudaStreamSynchronize(c->stream));
     return GPAIR_OK;
@@ -491,27 +530,42 @@ int gp_eval_gradient(gpair_ctx *c, int which, float alpha)
     return rc;
 }
 
+// End of a blocking evaluation whose last kernel wrote c->hres
+static int wait_result(gpair_ctx *c)
+{
+    GP_CUDA(c, cudaStreamSynchronize(c->stream));
+    c->stage_busy = 0;
+    return c->hres->tc_err ? gp_sync_scalars(c) : GPAIR_OK;  // reports the wait that gave up, and clears it
+}
+
+// chi2 and regulariser of the evaluation just waited for
+static int criterion_result(const gpair_ctx *c, double *chi2, double *entropy)
+{
+    if (chi2) *chi2 = c->hres->chi2;
+    if (entropy) *entropy = c->hres->entropy;
+    return (c->hres->nonfinite & 3u) ? GPAIR_ERR_NUMERIC : GPAIR_OK;
+}
+
 extern "C" int gpair_criterion(gpair_ctx *c, int which, double *chi2, double *entropy)
 {
     if (!c || !c->have_problem) return GPAIR_ERR_STATE;
     GP_CUDA(c, cudaSetDevice(c->device));
-    // the non-finite flag describes this evaluation, not an earlier one
-    GP_CUDA(c, cudaMemsetAsync(&c->sc->nonfinite, 0, sizeof(unsigned int), c->stream));
+    // the non-finite flag describes this evaluation, not an earlier one: the image prep sets it afresh
+    c->direct_result = 1;
     int rc = gp_eval_criterion(c, which, 0);
-    if (rc) return rc;
-    if ((rc = gp_sync_scalars(c))) return rc;
-    if (chi2) *chi2 = c->sc_host->chi2;
-    if (entropy) *entropy = c->sc_host->entropy;
-    return (c->sc_host->nonfinite & 3u) ? GPAIR_ERR_NUMERIC : GPAIR_OK;
+    c->direct_result = 0;
+    if (rc || (rc = wait_result(c))) return rc;
+    return criterion_result(c, chi2, entropy);
 }
 
 extern "C" int gpair_gradient(gpair_ctx *c, int which, float alpha)
 {
     if (!c || !c->have_problem || c->last_image_src < 0) return GPAIR_ERR_STATE;
     GP_CUDA(c, cudaSetDevice(c->device));
+    c->direct_result = 1;
     int rc = gp_eval_gradient(c, which, alpha);
-    if (rc) return rc;
-    return gp_sync_scalars(c);
+    c->direct_result = 0;
+    return rc ? rc : wait_result(c);
 }
 
 extern "C" int gpair_get_visibilities(gpair_ctx *c, gpair_float2 *visi)
@@ -584,13 +638,11 @@ extern "C" int gpair_update_pixel(gpair_ctx *c, int x, int y, float value, doubl
     if (c->last_image_src != GPAIR_IMG_CURR) return GPAIR_ERR_STATE;  // V must be the current image's
     if (x < 0 || y < 0 || x >= c->N || y >= c->N || !(value == value)) return GPAIR_ERR_INVALID;
     GP_CUDA(c, cudaSetDevice(c->device));
-    GP_CUDA(c, cudaMemsetAsync(&c->sc->nonfinite, 0, sizeof(unsigned int), c->stream));
+    c->direct_result = 1;
     int rc = gp_update_pixel(c, x, y, value);
-    if (rc) return rc;
-    if ((rc = gp_sync_scalars(c))) return rc;
-    if (chi2) *chi2 = c->sc_host->chi2;
-    if (entropy) *entropy = c->sc_host->entropy;
-    return (c->sc_host->nonfinite & 3u) ? GPAIR_ERR_NUMERIC : GPAIR_OK;
+    c->direct_result = 0;
+    if (rc || (rc = wait_result(c))) return rc;
+    return criterion_result(c, chi2, entropy);
 }
 
 // ---------------------------------------------------------- checkpoints
@@ -720,33 +772,16 @@ static int read_action(gpair_ctx *c, int *action)
 // flight at once (gpair_cg_run_many): prepare (parameters, controller reset,
 // graph build, start event), launch, finish (end event, wait, results).
 struct CgRun {
-    cudaEvent_t e0, e1;
     long long launches0;
     int want_trace;
 };
 
-static int cg_validate(gpair_ctx *c, const gpair_cg_params *p)
+// device state of a run with parameters p
+static CgState cg_params_state(const gpair_cg_params *p)
 {
-    if (!c || !p || !c->have_problem) return GPAIR_ERR_STATE;
-    if (p->iterations < 0 || p->method < 0 || p->method > 4) return GPAIR_ERR_INVALID;
-    if (p->line_search != GPAIR_LS_WOLFE && p->line_search != GPAIR_LS_BATCH) return GPAIR_ERR_INVALID;
-    if (!(p->target_J >= 0.0)) return GPAIR_ERR_INVALID;
-    return GPAIR_OK;
-}
-
-static int cg_prepare(gpair_ctx *c, const gpair_cg_params *p, int want_trace, CgRun *r, int build_graph = 1)
-{
-    int rc = cg_validate(c, p);
-    if (rc) return rc;
-    GP_CUDA(c, cudaSetDevice(c->device));
-    c->fuse_ctrl = -1;
-    c->fuse_handles = 0;
-    // parameters into the device state
     CgState h;
     memset(&h, 0, sizeof(h));
     h.method = p->method;
-    c->cg_method = p->method;
-    if (p->method == 4 && (rc = gp_lbfgs_alloc(c))) return rc;
     h.max_zoom = p->max_zoom > 0 ? p->max_zoom : 200;
     h.max_bracket = p->max_bracket > 0 ? p->max_bracket : 100;
     h.alpha = p->alpha;
@@ -758,38 +793,39 @@ static int cg_prepare(gpair_ctx *c, const gpair_cg_params *p, int want_trace, Cg
     h.ls_mode = p->line_search;
     h.target_J = p->target_J;
     h.batch_step_max = p->batch_step_max > 0.0 ? p->batch_step_max : 1e12;
-    // stop flag shared with racing runs (device pointer or null)
-    GP_CUDA(c, cudaMemcpyAsync(&c->sc->stop_flag, &p->stop_flag, sizeof(int *), cudaMemcpyHostToDevice, c->stream));
-    if (h.ls_mode == GPAIR_LS_BATCH && (rc = gp_batch_alloc(c))) return rc;
-    if (p->resume) {
-        // parameters only; the iteration state of the previous run is kept
-        GP_CUDA(c, cudaMemcpyAsync(&c->sc->cg, &h, offsetof(CgState, it), cudaMemcpyHostToDevice, c->stream));
-        if ((rc = gp_cg_kernel(c, CTRL_RESUME))) return rc;
-    } else {
-        GP_CUDA(c, cudaMemcpyAsync(&c->sc->cg, &h, sizeof(CgState), cudaMemcpyHostToDevice, c->stream));
-        if ((rc = gp_cg_kernel(c, CTRL_INIT))) return rc;
-    }
+    return h;
+}
+
+static int cg_validate(gpair_ctx *c, const gpair_cg_params *p)
+{
+    if (!c || !p || !c->have_problem) return GPAIR_ERR_STATE;
+    if (p->iterations < 0 || p->method < 0 || p->method > 4) return GPAIR_ERR_INVALID;
+    if (p->line_search != GPAIR_LS_WOLFE && p->line_search != GPAIR_LS_BATCH) return GPAIR_ERR_INVALID;
+    if (!(p->target_J >= 0.0)) return GPAIR_ERR_INVALID;
+    return GPAIR_OK;
+}
+
+static int cg_prepare(gpair_ctx *c, const gpair_cg_params *p, int want_trace, CgRun *r)
+{
+    int rc = cg_validate(c, p);
+    if (rc) return rc;
+    GP_CUDA(c, cudaSetDevice(c->device));
+    c->fuse_ctrl = -1;
+    c->fuse_handles = 0;
+    c->cg_method = p->method;
+    if (p->method == 4 && (rc = gp_lbfgs_alloc(c))) return rc;
+    if (p->line_search == GPAIR_LS_BATCH && (rc = gp_batch_alloc(c))) return rc;
+    if ((rc = gp_cg_start(c, cg_params_state(p), p->stop_flag, p->resume))) return rc;
     c->st_n = 0;
     r->want_trace = want_trace;
     r->launches0 = c->launches;
-    if (!p->host_loop && build_graph) {
+    if (!p->host_loop) {
         // build (or reuse) the graph before the timed region
         long long dummy = 0;
         if ((rc = gp_cg_graph_run(c, 0, want_trace, p->line_search, &dummy))) return rc;
         if (c->stage_timing) c->st_n = 0;
     }
-    GP_CUDA(c, cudaEventCreate(&r->e0));
-    if (cudaEventCreate(&r->e1) != cudaSuccess) {
-        cudaEventDestroy(r->e0);
-        snprintf(c->last_error, sizeof(c->last_error), "cudaEventCreate failed");
-        return GPAIR_ERR_CUDA;
-    }
-    if (cudaEventRecord(r->e0, c->stream) != cudaSuccess) {
-        cudaEventDestroy(r->e0);
-        cudaEventDestroy(r->e1);
-        snprintf(c->last_error, sizeof(c->last_error), "cudaEventRecord failed");
-        return GPAIR_ERR_CUDA;
-    }
+    GP_CUDA(c, cudaEventRecord(c->run_e0, c->stream));
     return GPAIR_OK;
 }
 
@@ -843,52 +879,50 @@ static int cg_host_loop(gpair_ctx *c, const gpair_cg_params *p, double *tJ, doub
     return status;
 }
 
-static void cg_mark_end(gpair_ctx *c, CgRun *r) { cudaEventRecord(r->e1, c->stream); }
+static void cg_mark_end(gpair_ctx *c) { cudaEventRecord(c->run_e1, c->stream); }
+
+// a run's counts and results into the context's statistics and the caller's struct
+static void cg_report(gpair_ctx *c, double ms, long long launches0, int it, const GpRunResult &r, int status,
+                      gpair_cg_result *res)
+{
+    c->last_ms = ms;
+    const double per = 4.0 * (double)c->npix * c->nuv + 8.0 * c->N * (double)c->nuv;
+    c->last_flops = per * (r.criterion_evals + r.grad_evals);
+    c->last_launches = c->launches - launches0;
+    if (!res) return;
+    res->iterations_done = it;
+    res->criterion_evals = r.criterion_evals;
+    res->grad_evals = r.grad_evals;
+    res->J = r.J;
+    res->chi2 = r.chi2;
+    res->entropy = r.entropy;
+    res->last_step = r.sel;
+    res->last_beta = r.beta;
+    res->status = status;
+    res->reached = r.reached;
+    res->stopped = r.stopped;
+}
 
 static int cg_finish(gpair_ctx *c, const gpair_cg_params *p, gpair_cg_result *res, double *tJ, double *tchi2,
-                     double *tS, double *tstep, double *tbeta, CgRun *r, int status, int it,
-                     void *batch_graph = nullptr, int batch_index = 0)
+                     double *tS, double *tstep, double *tbeta, CgRun *r, int status, int it)
 {
-    cudaError_t e = cudaEventSynchronize(r->e1);
+    int rc2 = gp_sync_scalars(c);  // waits for the run
+    c->stage_busy = 0;
+    if (rc2 == GPAIR_ERR_CUDA) return rc2;
     float ms = 0.f;
-    if (e == cudaSuccess) cudaEventElapsedTime(&ms, r->e0, r->e1);
-    cudaEventDestroy(r->e0);
-    cudaEventDestroy(r->e1);
-    if (e != cudaSuccess) {
-        snprintf(c->last_error, sizeof(c->last_error), "CG run: %s", cudaGetErrorString(e));
-        return GPAIR_ERR_CUDA;
-    }
+    cudaEventElapsedTime(&ms, c->run_e0, c->run_e1);
     if (c->stage_timing) stage_collect(c);
-    int rc2 = gp_sync_scalars(c);
     if (rc2 && !status) status = rc2;
     const CgState &s = c->sc_host->cg;
     if (!p->host_loop) {
         it = s.run_it;
-        if (r->want_trace && !status && !batch_graph) status = gp_cg_graph_trace(c, it, tJ, tchi2, tS, tstep, tbeta);
+        if (r->want_trace && !status) status = gp_cg_graph_trace(c, it, tJ, tchi2, tS, tstep, tbeta);
         if (!status && c->sc_host->nonfinite) status = GPAIR_ERR_NUMERIC;
-        c->launches = r->launches0 + (batch_graph ? gp_batch_graph_launches(batch_graph, batch_index, it,
-                                                                            s.criterion_evals, s.grad_evals,
-                                                                            s.batches)
-                                                  : gp_cg_graph_launches(c, it, s.criterion_evals, s.grad_evals,
-                                                                         s.batches));
+        c->launches = r->launches0 + gp_cg_graph_launches(c, it, s.criterion_evals, s.grad_evals, s.batches);
     }
-    c->last_ms = ms;
-    double per = 4.0 * (double)c->npix * c->nuv + 8.0 * c->N * (double)c->nuv;
-    c->last_flops = per * (s.criterion_evals + s.grad_evals);
-    c->last_launches = c->launches - r->launches0;
-    if (res) {
-        res->iterations_done = it;
-        res->criterion_evals = s.criterion_evals;
-        res->grad_evals = s.grad_evals;
-        res->J = s.J;
-        res->chi2 = s.chi2;
-        res->entropy = s.entropy;
-        res->last_step = s.sel;
-        res->last_beta = s.beta;
-        res->status = status;
-        res->reached = s.reached;
-        res->stopped = s.stopped;
-    }
+    const GpRunResult rr = {s.run_it, s.criterion_evals, s.grad_evals, s.batches, s.reached, s.stopped,
+                            c->sc_host->nonfinite, 0, s.J, s.chi2, s.entropy, s.sel, s.beta};
+    cg_report(c, ms, r->launches0, it, rr, status, res);
     return status;
 }
 
@@ -905,7 +939,7 @@ extern "C" int gpair_cg_run(gpair_ctx *c, const gpair_cg_params *p, gpair_cg_res
     } else {
         status = cg_host_loop(c, p, tJ, tchi2, tS, tstep, tbeta, &it);
     }
-    cg_mark_end(c, &r);
+    cg_mark_end(c);
     return cg_finish(c, p, res, tJ, tchi2, tS, tstep, tbeta, &r, status, it);
 }
 
@@ -916,8 +950,9 @@ struct gpair_batch {
     gpair_ctx **ctx;
     void *graph;
     cudaStream_t stream;
-    cudaEvent_t *ready;
-    cudaEvent_t done, e0, e1;
+    cudaEvent_t ready, e0, e1;
+    DevScalars **scs;    // device: every context's scalars
+    GpRunResult *hres;   // pinned: every context's results
 };
 
 extern "C" int gpair_batch_destroy(gpair_batch *b)
@@ -926,14 +961,12 @@ extern "C" int gpair_batch_destroy(gpair_batch *b)
     cudaSetDevice(b->device);
     if (b->stream) cudaStreamSynchronize(b->stream);
     gp_batch_graph_free(b->graph);
-    if (b->ready)
-        for (int i = 0; i < b->n; i++)
-            if (b->ready[i]) cudaEventDestroy(b->ready[i]);
-    if (b->done) cudaEventDestroy(b->done);
+    if (b->ready) cudaEventDestroy(b->ready);
+    if (b->scs) cudaFree(b->scs);
+    if (b->hres) cudaFreeHost(b->hres);
     if (b->e0) cudaEventDestroy(b->e0);
     if (b->e1) cudaEventDestroy(b->e1);
     if (b->stream) cudaStreamDestroy(b->stream);
-    free(b->ready);
     free(b->ctx);
     free(b);
     return GPAIR_OK;
@@ -975,19 +1008,25 @@ extern "C" int gpair_batch_create_ex(gpair_batch **out, gpair_ctx **ctx, int n, 
     b->ls_mode = line_search;
     b->device = ctx[0]->device;
     b->ctx = (gpair_ctx **)calloc((size_t)n, sizeof(gpair_ctx *));
-    b->ready = (cudaEvent_t *)calloc((size_t)n, sizeof(cudaEvent_t));
-    if (!b->ctx || !b->ready) {
+    if (!b->ctx) {
         gpair_batch_destroy(b);
         return GPAIR_ERR_ALLOC;
     }
     memcpy(b->ctx, ctx, sizeof(gpair_ctx *) * n);
     int rc = GPAIR_OK;
     if (cudaSetDevice(b->device) != cudaSuccess || cudaStreamCreateWithFlags(&b->stream, cudaStreamNonBlocking) ||
-        cudaEventCreateWithFlags(&b->done, cudaEventDisableTiming) || cudaEventCreate(&b->e0) ||
+        cudaEventCreateWithFlags(&b->ready, cudaEventDisableTiming) || cudaEventCreate(&b->e0) ||
         cudaEventCreate(&b->e1))
         rc = GPAIR_ERR_CUDA;
-    for (int i = 0; i < n && !rc; i++)
-        if (cudaEventCreateWithFlags(&b->ready[i], cudaEventDisableTiming) != cudaSuccess) rc = GPAIR_ERR_CUDA;
+    if (!rc) {
+        std::vector<DevScalars *> scs((size_t)n);
+        for (int i = 0; i < n; i++) scs[i] = ctx[i]->sc;
+        if (cudaMalloc(&b->scs, sizeof(DevScalars *) * (size_t)n) != cudaSuccess ||
+            cudaMallocHost(&b->hres, sizeof(GpRunResult) * (size_t)n) != cudaSuccess)
+            rc = GPAIR_ERR_ALLOC;
+        else if (cudaMemcpy(b->scs, scs.data(), sizeof(DevScalars *) * (size_t)n, cudaMemcpyHostToDevice) != cudaSuccess)
+            rc = GPAIR_ERR_CUDA;
+    }
     for (int i = 0; i < n && !rc; i++) {
         ctx[i]->fuse_ctrl = -1;
         ctx[i]->fuse_handles = 0;
@@ -1018,37 +1057,45 @@ extern "C" int gpair_batch_run(gpair_batch *b, const gpair_cg_params *p, gpair_c
             gp_batch_graph_buf_gen(b->graph, i) != b->ctx[i]->buf_gen)
             return GPAIR_ERR_STATE;
     }
-    std::vector<CgRun> r((size_t)b->n);
-    GP_CUDA(b->ctx[0], cudaSetDevice(b->device));
-    int prepared = 0, rc = GPAIR_OK;
-    for (; prepared < b->n; prepared++) {
-        gpair_ctx *c = b->ctx[prepared];
-        if ((rc = cg_prepare(c, p, 0, &r[prepared], 0))) break;
-        cudaEventRecord(b->ready[prepared], c->stream);
-        cudaStreamWaitEvent(b->stream, b->ready[prepared], 0);
-    }
-    float ms = 0.f;
-    if (!rc) {
-        cudaEventRecord(b->e0, b->stream);
-        rc = gp_batch_graph_launch(b->graph, b->stream);
-        cudaEventRecord(b->e1, b->stream);
-        cudaEventRecord(b->done, b->stream);
-        if (!rc && cudaEventSynchronize(b->e1) == cudaSuccess) cudaEventElapsedTime(&ms, b->e0, b->e1);
-    }
-    int first_err = rc;
-    for (int i = 0; i < prepared; i++) {
+    gpair_ctx *c0 = b->ctx[0];
+    GP_CUDA(c0, cudaSetDevice(b->device));
+    for (int i = 0; i < b->n; i++) {
         gpair_ctx *c = b->ctx[i];
-        if (rc) {
-            cudaEventDestroy(r[i].e0);
-            cudaEventDestroy(r[i].e1);
-            continue;
+        c->fuse_ctrl = -1;
+        c->fuse_handles = 0;
+        c->cg_method = p->method;
+        c->st_n = 0;
+        // after what the context has queued (an image upload); an idle stream needs no event
+        if (cudaStreamQuery(c->stream) != cudaSuccess) {
+            cudaGetLastError();
+            GP_CUDA(c, cudaEventRecord(b->ready, c->stream));
+            GP_CUDA(c, cudaStreamWaitEvent(b->stream, b->ready, 0));
         }
-        cudaStreamWaitEvent(c->stream, b->done, 0);
-        cg_mark_end(c, &r[i]);
-        int rci = cg_finish(c, p, res ? &res[i] : nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, &r[i],
-                            GPAIR_OK, 0, b->graph, i);
-        c->last_ms = ms;
-        if (rci && !first_err) first_err = rci;
+    }
+    // one launch sets every context's parameters, one gathers every context's results: 24 contexts spend 110 us
+    // outside the graph (1,000 with two copies, a kernel, events and a read per context)
+    int rc = gp_cg_start_many(c0, b->scs, b->n, cg_params_state(p), p->stop_flag, p->resume, b->stream);
+    if (rc) return rc;
+    cudaEventRecord(b->e0, b->stream);
+    rc = gp_batch_graph_launch(b->graph, b->stream);
+    cudaEventRecord(b->e1, b->stream);
+    if (!rc) rc = gp_run_results(c0, b->scs, b->n, b->hres, b->stream);
+    GP_CUDA(c0, cudaStreamSynchronize(b->stream));
+    if (rc) return rc;
+    float ms = 0.f;
+    cudaEventElapsedTime(&ms, b->e0, b->e1);
+    int first_err = GPAIR_OK;
+    for (int i = 0; i < b->n; i++) {
+        gpair_ctx *c = b->ctx[i];
+        const GpRunResult &r = b->hres[i];
+        int status = GPAIR_OK;
+        if (c->stage_timing) stage_collect(c);
+        if (r.tc_err) status = gp_sync_scalars(c);  // reports the wait that gave up, and clears it
+        if (!status && r.nonfinite) status = GPAIR_ERR_NUMERIC;
+        const long long launches0 = c->launches;
+        c->launches += gp_batch_graph_launches(b->graph, i, r.run_it, r.criterion_evals, r.grad_evals, r.batches);
+        cg_report(c, ms, launches0, r.run_it, r, status, res ? &res[i] : nullptr);
+        if (status && !first_err) first_err = status;
     }
     return first_err;
 }
@@ -1071,6 +1118,7 @@ extern "C" int gpair_cg_run_many(gpair_ctx **ctx, int n, const gpair_cg_params *
         return GPAIR_ERR_ALLOC;
     }
     int first_err = GPAIR_OK, prepared = 0;
+    bool launched = false;
     // every run is prepared (graphs built) before any is launched: a graph
     // capture must not overlap another context's work on the legacy stream
     for (; prepared < n; prepared++) {
@@ -1081,18 +1129,15 @@ extern "C" int gpair_cg_run_many(gpair_ctx **ctx, int n, const gpair_cg_params *
         }
     }
     if (!first_err) {
+        launched = true;
         for (int i = 0; i < n; i++) {
             long long dummy = 0;
             st[i] = gp_cg_graph_run(ctx[i], p->iterations, 0, p->line_search, &dummy);
-            cg_mark_end(ctx[i], &r[i]);
+            cg_mark_end(ctx[i]);
         }
     }
     for (int i = 0; i < prepared; i++) {
-        if (first_err) {
-            cudaEventDestroy(r[i].e0);
-            cudaEventDestroy(r[i].e1);
-            continue;
-        }
+        if (first_err && !launched) continue;
         int rc = cg_finish(ctx[i], p, res ? &res[i] : nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, &r[i],
                            st[i], 0);
         if (rc && !first_err) first_err = rc;

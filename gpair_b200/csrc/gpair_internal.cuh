@@ -120,8 +120,6 @@ struct DevScalars {
     unsigned int t_counter[GP_NTR + 1];
     int *stop_flag;  // shared with racing runs (device memory), or null
     int reg_kind;    // GPAIR_REG_GULL_SKILLING / GPAIR_REG_L2
-    // single-pixel update: old total flux and flux change of the last update
-    double upd_flux_old, upd_delta;
     // projected L-BFGS reductions
     double lb_pdots[GP_LB_NPD], lb_qdots[GP_LB_NQD];
     CgState cg;
@@ -212,6 +210,23 @@ __device__ __forceinline__ float reg_grad(float I, float m, float prev, int kind
     return (I > 0.f && m > 0.f) ? (float)(-log((double)I / (double)m)) : prev;
 }
 
+// What a blocking evaluation call returns, in pinned host memory: written by the last block of the
+// evaluation's last kernel, so that the call needs no copy after it
+struct GpHostResult {
+    double chi2, entropy;
+    unsigned int nonfinite, tc_err;
+};
+__device__ __forceinline__ void gp_host_result(GpHostResult *h, const DevScalars *sc)
+{
+    if (!h) return;
+    volatile GpHostResult *v = h;
+    v->chi2 = sc->chi2;
+    v->entropy = sc->entropy;
+    v->nonfinite = sc->nonfinite;
+    v->tc_err = sc->tc_err;
+    __threadfence_system();
+}
+
 struct gpair_buf {
     float *ptr;
     size_t count;  // floats
@@ -251,6 +266,15 @@ struct gpair_ctx {
     double *partials;  // RED_NSLOTS * GP_MAX_PARTIALS * 4 doubles
     DevScalars *sc;
     DevScalars *sc_host;  // pinned mirror for reads
+    // blocking evaluation calls: their result (pinned), passed to the kernels while `direct_result` is set, which
+    // also makes the image prep clear the non-finite flag
+    GpHostResult *hres;
+    int direct_result;
+    // pinned staging of small host arrays (images, results): stage_busy while an upload from it may be in flight
+    void *stage;
+    int stage_busy;
+    cudaEvent_t stage_ev;
+    cudaEvent_t run_e0, run_e1;  // around the last CG run
 
     // tensor-core operand buffers (GPAIR_PREC_SPLIT16 / TF32), see umma path
     void *tc_state;
@@ -423,6 +447,18 @@ int gp_descent_dir(gpair_ctx *c, int beta_from_state, double beta_host);
 int gp_update_image(gpair_ctx *c, int step_from_state, double step_host, double minval, int backup);
 int gp_update_temp(gpair_ctx *c, double step, double minval, int clamp);
 int gp_cg_kernel(gpair_ctx *c, int which_ctrl);
+// Run parameters into the device state and the controller reset (resume: parameters only, counters
+// cleared), of one context or, on stream st, of the n contexts whose scalars are scs[0..n-1]
+int gp_cg_start(gpair_ctx *c, const CgState &h, int *stop_flag, int resume);
+int gp_cg_start_many(gpair_ctx *c, DevScalars *const *scs, int n, const CgState &h, int *stop_flag, int resume,
+                     cudaStream_t st);
+// A finished run's results of n contexts into pinned host memory
+struct GpRunResult {
+    int run_it, criterion_evals, grad_evals, batches, reached, stopped;
+    unsigned int nonfinite, tc_err;
+    double J, chi2, entropy, sel, beta;
+};
+int gp_run_results(gpair_ctx *c, DevScalars *const *scs, int n, GpRunResult *out, cudaStream_t st);
 // graph-captured controller: also sets the conditional handles of the CG graph
 int gp_cg_kernel_graph(gpair_ctx *c, int which_ctrl, unsigned long long h_iter, unsigned long long h_ls,
                        unsigned long long h_grad, double *trace, int trace_cap);

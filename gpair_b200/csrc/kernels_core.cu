@@ -27,6 +27,7 @@
 //                    with FP64 scalars that stay on the device.
 #include <cuda_fp16.h>
 #include <math.h>
+#include <stddef.h>
 #include <string.h>
 
 #include "gpair_internal.cuh"
@@ -135,7 +136,7 @@ __global__ void __launch_bounds__(GP_THREADS) k_prep(const float *__restrict__ s
                                                      float *__restrict__ dst, const float *__restrict__ model,
                                                      int npix, int trial, double step, int step_from_state,
                                                      double minval, double *__restrict__ partials,
-                                                     DevScalars *__restrict__ sc)
+                                                     DevScalars *__restrict__ sc, int reset)
 {
     __shared__ double smem[2 * 32];
     double s = step_from_state ? sc->cg.s : step;
@@ -179,7 +180,8 @@ __global__ void __launch_bounds__(GP_THREADS) k_prep(const float *__restrict__ s
             sc->flux_f = (float)v[0];
             sc->invflux_f = (float)(1.0 / v[0]);
             sc->entropy_f = (float)v[1];
-            if (!isfinite(v[0]) || !isfinite(v[1])) sc->nonfinite |= 1u;
+            const unsigned int bad = !isfinite(v[0]) || !isfinite(v[1]) ? 1u : 0u;
+            sc->nonfinite = reset ? bad : sc->nonfinite | bad;
             sc->counter[RED_PREP] = 0;
         }
     }
@@ -193,7 +195,7 @@ int gp_prep_image(gpair_ctx *c, int which, int trial_mode, double step_host, int
     const int g = red_grid(c->npix);  // one wave, several pixels per thread: a short reduction tail
     k_prep<<<g, GP_THREADS, 0, c->stream>>>(src, c->descent_dir, c->image_temp, c->model, c->npix, trial_mode,
                                             step_host, step_from_state, (double)1e-8, slot_partials(c, RED_PREP),
-                                            c->sc);
+                                            c->sc, c->direct_result);
     GP_LAUNCH_CHECK(c);
     return GPAIR_OK;
 }
@@ -325,6 +327,7 @@ struct VisDataArgs {
     DevScalars *sc;
     FusedCtrl fc;
     int direct;
+    GpHostResult *hres;  // result of a blocking call, or null
     GP_VGRID_FIELDS;
 };
 
@@ -410,6 +413,7 @@ __device__ __forceinline__ void vis_data_body(const VisDataArgs &A, const GpVGri
             sc->chi2_f = (float)out[0];
             if (!isfinite(out[0])) sc->nonfinite |= 2u;
             sc->counter[RED_CHI2] = 0;
+            gp_host_result(A.hres, sc);
             run_fused_ctrl(sc, A.fc);
         }
     }
@@ -437,7 +441,7 @@ static VisDataArgs vis_data_args(gpair_ctx *c, int direct, FusedCtrl fc)
     if (nbt > 1536) nbt = 1536;
     VisDataArgs a = {c->vpart, c->mt, c->nuv, c->npow, c->nbis, c->data, c->data_err, c->tri, c->phasor, nbu,
                      c->visd, c->visi, c->mock, c->cw, c->trib, slot_partials(c, RED_CHI2), c->sc, fc, direct,
-                     nbu + nbt, 1};
+                     c->direct_result ? c->hres : nullptr, nbu + nbt, 1};
     return a;
 }
 
@@ -741,6 +745,7 @@ struct GradFinalizeArgs {
     double *partials;
     DevScalars *sc;
     FusedCtrl fc;
+    GpHostResult *hres;
     int parts;  // threads per four pixels (a power of two); 1: one thread sums all splits
     GP_VGRID_FIELDS;
 };
@@ -868,6 +873,7 @@ __device__ __forceinline__ void grad_finalize_body(const GradFinalizeArgs &A, co
             for (int i = 0; i < 4; i++) sc->grad_dots[dot_slot][i] = o[i];
             if (!isfinite(o[0])) sc->nonfinite |= 4u;
             sc->counter[RED_GRAD] = 0;
+            gp_host_result(A.hres, sc);
             run_fused_ctrl(sc, A.fc);
         }
     }
@@ -903,7 +909,8 @@ static GradFinalizeArgs grad_finalize_args(gpair_ctx *c, int which, int mode, fl
     if (g < 1) g = 1;
     GradFinalizeArgs a = {c->gpart, c->splits, c->npix, mode, img, c->model, alpha, alpha_from_state,
                           c->data_grad, c->entropy_grad, out, c->full_grad, c->descent_dir,
-                          which == GPAIR_IMG_TEMP ? 1 : 0, slot_partials(c, RED_GRAD), c->sc, fc, P, g, 1};
+                          which == GPAIR_IMG_TEMP ? 1 : 0, slot_partials(c, RED_GRAD), c->sc, fc,
+                          c->direct_result ? c->hres : nullptr, P, g, 1};
     return a;
 }
 
@@ -925,6 +932,7 @@ struct UgGradArgs {
     double *partials;
     DevScalars *sc;
     FusedCtrl fc;
+    GpHostResult *hres;
     GP_VGRID_FIELDS;
 };
 
@@ -1046,6 +1054,7 @@ __device__ __forceinline__ void ug_grad_body(const UgGradArgs &A, const GpVGrid 
             for (int i = 0; i < 4; i++) sc->grad_dots[A.dot_slot][i] = o[i];
             if (!isfinite(o[0])) sc->nonfinite |= 4u;
             sc->counter[RED_GRAD] = 0;
+            gp_host_result(A.hres, sc);
             run_fused_ctrl(sc, A.fc);
         }
     }
@@ -1080,7 +1089,7 @@ static UgGradArgs ug_grad_args(gpair_ctx *c, int which, int mode, float alpha, F
                     c->model, alpha, alpha < 0.f, c->data_grad, c->entropy_grad,
                     which == GPAIR_IMG_TEMP ? c->grad_temp : c->full_grad_new, c->full_grad, c->descent_dir,
                     which == GPAIR_IMG_TEMP ? 1 : 0, slot_partials(c, RED_GRAD), c->sc, fc,
-                    gp_cdiv(g->N, T) * gp_cdiv(g->H, T), 1};
+                    c->direct_result ? c->hres : nullptr, gp_cdiv(g->N, T) * gp_cdiv(g->H, T), 1};
     return a;
 }
 
@@ -1837,73 +1846,65 @@ int gp_eval_batch_timed(gpair_ctx *c, cudaEvent_t *ev) { return eval_batch(c, ev
 
 // --------------------------------------------- single-pixel update
 
-// One pixel changes from I_old to `value`: the total flux, the regulariser
-// sum and the image are updated on one thread; V follows in k_update_pixel_vis.
-// Corrected form of the reference's single-pixel flux change
-// (gpair1/trunk/cpu.c:477-486, gpair1/trunk/gpu.c:2137-2182): with the total
-// flux going from F to F' = F + delta, V'_k = (F V_k + delta e_k(x, y)) / F'.
-__global__ void k_update_pixel_scalar(float *__restrict__ img, const float *__restrict__ model, int p, float value,
-                                      DevScalars *__restrict__ sc)
+// One pixel changes from I_old to `value`. Corrected form of the reference's
+// single-pixel flux change (gpair1/trunk/cpu.c:477-486, gpair1/trunk/gpu.c:2137-2182):
+// with the total flux going from F to F' = F + delta, V'_k = (F V_k + delta e_k(x, y)) / F'.
+// The last block then writes the image, the flux and the regulariser sum (the
+// others have read the old ones) and clears the non-finite flag. Fx[k][x] and
+// Fy[k][y] come from the tables, or from (u, v) as k_gen_twiddles forms them
+// where the problem keeps none.
+__global__ void __launch_bounds__(256) k_update_pixel(float *__restrict__ img, const float *__restrict__ model, int N,
+                                                      int x, int y, float value, const float2 *__restrict__ fx,
+                                                      const float2 *__restrict__ fy, const float2 *__restrict__ uvc,
+                                                      float pix, int nuv, double2 *__restrict__ visd,
+                                                      DevScalars *__restrict__ sc)
 {
-    if (threadIdx.x != 0 || blockIdx.x != 0) return;
-    const double old = img[p], nv = value, m = model[p];
-    const double F = sc->flux, Fn = F + (nv - old);
-    sc->upd_flux_old = F;
-    sc->upd_delta = nv - old;
-    sc->flux = Fn;
-    sc->invflux = 1.0 / Fn;
-    sc->flux_f = (float)Fn;
-    sc->invflux_f = (float)(1.0 / Fn);
-    sc->entropy += reg_term(nv, m, sc->reg_kind) - reg_term(old, m, sc->reg_kind);
-    sc->entropy_f = (float)sc->entropy;
-    sc->imax = fmax(sc->imax, fabs(nv));
-    img[p] = value;
-}
-
-__global__ void k_update_pixel_vis(const float2 *__restrict__ fx, const float2 *__restrict__ fy, int N, int nuv,
-                                   int x, int y, double2 *__restrict__ visd, const DevScalars *__restrict__ sc)
-{
+    gp_pdl_enter();
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k >= nuv) return;
-    const float2 a = fx[(size_t)k * N + x], b = fy[(size_t)k * N + y];
-    const double er = (double)a.x * b.x - (double)a.y * b.y, ei = (double)a.x * b.y + (double)a.y * b.x;
-    const double F = sc->upd_flux_old, d = sc->upd_delta, inv = sc->invflux;
-    const double2 V = visd[k];
-    visd[k] = make_double2((F * V.x + d * er) * inv, (F * V.y + d * ei) * inv);
-}
-
-// The same where the problem keeps no tables: Fx[k][x] and Fy[k][y] as k_gen_twiddles forms them
-__global__ void k_update_pixel_vis_uv(const float2 *__restrict__ uvc, float pix, int nuv, int x, int y,
-                                      double2 *__restrict__ visd, const DevScalars *__restrict__ sc)
-{
-    const int k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k >= nuv) return;
-    const float2 uv = uvc[k];
-    double tu = RPMAS_D * (double)pix * (double)uv.x * (double)x, tv = RPMAS_D * (double)pix * (double)uv.y * (double)y;
-    tu -= rint(tu);
-    tv -= rint(tv);
-    double su, cu, sv, cv;
-    sincospi(2.0 * tu, &su, &cu);
-    sincospi(2.0 * tv, &sv, &cv);
-    const double er = cu * cv + su * sv, ei = su * cv - cu * sv;
-    const double F = sc->upd_flux_old, d = sc->upd_delta, inv = sc->invflux;
-    const double2 V = visd[k];
-    visd[k] = make_double2((F * V.x + d * er) * inv, (F * V.y + d * ei) * inv);
+    const int p = x + y * N;
+    const double old = img[p], F = sc->flux, d = (double)value - old, Fn = F + d, inv = 1.0 / Fn;
+    if (k < nuv) {
+        double er, ei;
+        if (fx) {
+            const float2 a = fx[(size_t)k * N + x], b = fy[(size_t)k * N + y];
+            er = (double)a.x * b.x - (double)a.y * b.y;
+            ei = (double)a.x * b.y + (double)a.y * b.x;
+        } else {
+            const float2 uv = uvc[k];
+            double tu = RPMAS_D * (double)pix * (double)uv.x * (double)x;
+            double tv = RPMAS_D * (double)pix * (double)uv.y * (double)y;
+            tu -= rint(tu);
+            tv -= rint(tv);
+            double su, cu, sv, cv;
+            sincospi(2.0 * tu, &su, &cu);
+            sincospi(2.0 * tv, &sv, &cv);
+            er = cu * cv + su * sv;
+            ei = su * cv - cu * sv;
+        }
+        const double2 V = visd[k];
+        visd[k] = make_double2((F * V.x + d * er) * inv, (F * V.y + d * ei) * inv);
+    }
+    if (last_block(&sc->counter[RED_ADJ]) && threadIdx.x == 0) {
+        const double nv = value, m = model[p];
+        sc->flux = Fn;
+        sc->invflux = inv;
+        sc->flux_f = (float)Fn;
+        sc->invflux_f = (float)inv;
+        sc->entropy += reg_term(nv, m, sc->reg_kind) - reg_term(old, m, sc->reg_kind);
+        sc->entropy_f = (float)sc->entropy;
+        sc->imax = fmax(sc->imax, fabs(nv));
+        sc->nonfinite = 0;
+        sc->counter[RED_ADJ] = 0;
+        img[p] = value;
+    }
 }
 
 int gp_update_pixel(gpair_ctx *c, int x, int y, float value)
 {
-    const int p = x + y * c->N;
-    k_update_pixel_scalar<<<1, 32, 0, c->stream>>>(c->image, c->model, p, value, c->sc);
-    GP_LAUNCH_CHECK(c);
-    if (c->ug) {
-        k_update_pixel_vis_uv<<<gp_cdiv(c->nuv, 256), 256, 0, c->stream>>>(c->uvc, c->pix, c->nuv, x, y, c->visd, c->sc);
-        GP_LAUNCH_CHECK(c);
-    } else if (c->nuv) {
-        k_update_pixel_vis<<<gp_cdiv(c->nuv, 256), 256, 0, c->stream>>>(c->fx, c->fy, c->N, c->nuv, x, y, c->visd,
-                                                                       c->sc);
-        GP_LAUNCH_CHECK(c);
-    }
+    const int nb = c->nuv ? gp_cdiv(c->nuv, 256) : 1;
+    GP_LAUNCH(c, gp_launch(c, k_update_pixel, dim3(nb), dim3(256), 0, c->image, (const float *)c->model, c->N, x, y,
+                           value, (const float2 *)(c->ug ? nullptr : c->fx), (const float2 *)(c->ug ? nullptr : c->fy),
+                           (const float2 *)c->uvc, c->pix, c->nuv, c->visd, c->sc));
     c->fuse_ctrl = -1;
     return vis_data_launch(c, 1);  // V2, T3, chi2 and the adjoint weights from the updated V
 }
@@ -2423,6 +2424,58 @@ int gp_cg_kernel_graph(gpair_ctx *c, int which_ctrl, unsigned long long h_iter, 
 {
     const CtrlArgs a = {c->sc, which_ctrl, h_iter, h_ls, h_grad, trace, trace_cap, 1, 1};
     GP_LAUNCH(c, gp_launch(c, k_cg_ctrl_g, dim3(1), dim3(32), 0, a));
+    return GPAIR_OK;
+}
+
+// Parameters of a run (the kernel's own copy) into the device state, then the
+// controller's reset; one block per context.
+__global__ void k_cg_start(DevScalars *const *__restrict__ scs, DevScalars *__restrict__ one,
+                           const __grid_constant__ CgState h, int *stop_flag, int resume)
+{
+    DevScalars *sc = scs ? scs[blockIdx.x] : one;
+    // a continued run takes the parameters (the members before `it`) and keeps the iteration state
+    const int words = (int)((resume ? offsetof(CgState, it) : sizeof(CgState)) / sizeof(int));
+    static_assert(offsetof(CgState, it) % sizeof(int) == 0 && sizeof(CgState) % sizeof(int) == 0, "whole words");
+    const int *src = reinterpret_cast<const int *>(&h);
+    int *dst = reinterpret_cast<int *>(&sc->cg);
+    for (int i = threadIdx.x; i < words; i += blockDim.x) dst[i] = src[i];
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        sc->stop_flag = stop_flag;
+        cg_control(sc, resume ? CTRL_RESUME : CTRL_INIT);
+    }
+}
+
+int gp_cg_start(gpair_ctx *c, const CgState &h, int *stop_flag, int resume)
+{
+    k_cg_start<<<1, 128, 0, c->stream>>>(nullptr, c->sc, h, stop_flag, resume);
+    GP_LAUNCH_CHECK(c);
+    return GPAIR_OK;
+}
+
+int gp_cg_start_many(gpair_ctx *c, DevScalars *const *scs, int n, const CgState &h, int *stop_flag, int resume,
+                     cudaStream_t st)
+{
+    k_cg_start<<<n, 128, 0, st>>>(scs, nullptr, h, stop_flag, resume);
+    GP_LAUNCH_CHECK(c);
+    return GPAIR_OK;
+}
+
+__global__ void k_run_results(DevScalars *const *__restrict__ scs, int n, GpRunResult *__restrict__ out)
+{
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    const DevScalars *sc = scs[i];
+    const CgState &s = sc->cg;
+    GpRunResult r = {s.run_it, s.criterion_evals, s.grad_evals, s.batches, s.reached, s.stopped, sc->nonfinite,
+                     sc->tc_err, s.J, s.chi2, s.entropy, s.sel, s.beta};
+    out[i] = r;
+}
+
+int gp_run_results(gpair_ctx *c, DevScalars *const *scs, int n, GpRunResult *out, cudaStream_t st)
+{
+    k_run_results<<<gp_cdiv(n, 64), 64, 0, st>>>(scs, n, out);
+    GP_LAUNCH_CHECK(c);
     return GPAIR_OK;
 }
 

@@ -927,6 +927,7 @@ struct PrepRowsArgs {
     double *partials;
     DevScalars *sc;
     const int *gate;
+    int reset;  // clear the non-finite flag (a blocking call's evaluation)
     GP_VGRID_FIELDS;
 };
 
@@ -1128,7 +1129,8 @@ __device__ __forceinline__ void tc_prep_rows_body(const PrepRowsArgs &A, const G
             sc->flux_f = (float)v3[0];
             sc->invflux_f = (float)(1.0 / v3[0]);
             sc->entropy_f = (float)v3[1];
-            if (!isfinite(v3[0]) || !isfinite(v3[1])) sc->nonfinite |= 1u;
+            const unsigned int bad = !isfinite(v3[0]) || !isfinite(v3[1]) ? 1u : 0u;
+            sc->nonfinite = A.reset ? bad : sc->nonfinite | bad;
             sc->counter[RED_PREP] = 0;
         }
     }
@@ -1889,6 +1891,7 @@ static PrepRowsArgs tc_prep_rows_args(gpair_ctx *c, TcState *t, int mode, int re
     a.partials = partials;
     a.sc = c->sc;
     a.gate = b ? c->gate : nullptr;
+    a.reset = c->direct_result;
     a.nbx = gx;
     a.nby = b ? GP_NTR : 1;
     return a;
