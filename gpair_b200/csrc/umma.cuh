@@ -243,10 +243,13 @@ __device__ __forceinline__ uint32_t mapa_shared(uint32_t smem_addr, uint32_t ran
     return r;
 }
 
-// arrive on an mbarrier given by its shared::cluster address (possibly the peer CTA's)
+// arrive on an mbarrier given by its shared::cluster address (possibly the peer CTA's).
+// The default scope (the CTA): what the arrival orders is the reading of tensor memory,
+// which the tcgen05 fences cover. With .release.cluster every arrival also waited until
+// this thread's earlier global stores had reached the cluster's scope.
 __device__ __forceinline__ void mbar_arrive_cluster(uint32_t cluster_addr)
 {
-    asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
+    asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
 }
 
 // every thread of both CTAs of the cluster

@@ -31,7 +31,8 @@
 // issues TMA loads (a ring of 2 stages of 96 KB, or 3 of 64 KB per CTA of a
 // pair), warp 1 owns TMEM (512 columns = two FP32 accumulators of 256
 // columns) and one of its threads issues tcgen05.mma; warps 2-9 drain TMEM,
-// two per lane quarter, each taking 128 of the accumulator's 256 columns.
+// two per lane quarter, each taking 128 of the accumulator's 256 columns. The
+// last tile of an image stops at the image's last rows, in steps of 32 columns.
 // All waits are bounded; a timeout sets an error code, the roles stop, TMEM is
 // released, and the host reports GPAIR_ERR_TIMEOUT.
 #include <cuda.h>
@@ -66,10 +67,14 @@
 #define TC_TMEM_COLS 512
 // after the stages: barriers (256 B), the unit prefix sums of a grouped launch
 // (up to TC_GROUP_MAX instances), then the forward epilogue's row scales of a
-// unit, one copy per epilogue warp and accumulator buffer
+// unit, one copy per epilogue warp and accumulator buffer, and likewise the
+// anchors and rotations of its 16 uv points
 #define TC_RS_OFF (256 + 4 * 272)
 #define TC_RS_BYTES (TC_EPI_WARPS * 2 * TC_EPI_COLS * 4)
-#define TC_SMEM_BYTES (1024 + TC_STAGES * TC_STAGE_BYTES + TC_RS_OFF + TC_RS_BYTES)
+#define TC_AN_OFF (TC_RS_OFF + TC_RS_BYTES)
+#define TC_AN_PTS (16 * (TC_EPI_COLS / 16 + 1))  // float2 of one warp and buffer: [anchor, then the rotation][uv point]
+#define TC_AN_BYTES (TC_EPI_WARPS * 2 * TC_AN_PTS * 8)
+#define TC_SMEM_BYTES (1024 + TC_STAGES * TC_STAGE_BYTES + TC_AN_OFF + TC_AN_BYTES)
 #define TC_SMEM_GROUP_BYTES TC_SMEM_BYTES
 #define TC_WAIT_BUDGET 4000000000LL  // default clock cycles (~2 s) per pipeline wait
 #define RPMAS_TC ((3.14159265358979323 / 180.0) / 3600000.0)  // radians per milliarcsecond
@@ -151,10 +156,11 @@ struct TcArgs {
     const float2 *fya, *fyr;
     int nanc;
     int N, nuv;
-    // image-side rows: lpad rows per image, partial entries of 2^elog2 rows;
+    // image-side rows: lpad rows per image, of which `live` are the image's own (the
+    // rest are zero); partial entries of 2^elog2 rows;
     // rsc[row]: power-of-two factor of every image-side row (operand scale and
     // twiddle scale removed in the epilogue)
-    int lpad, elog2;
+    int lpad, live, elog2;
     const float *rsc;
     float2 *vpart;
     // store epilogue
@@ -183,7 +189,7 @@ struct __align__(64) TcGroupInst {
     int m_tiles, n_tiles, kb_total, units;
     // forward epilogue
     const float2 *fya, *fyr;
-    int nanc, nuv, lpad, elog2;
+    int nanc, nuv, lpad, live, elog2;
     const float *rsc;
     float2 *vpart;
     // store epilogue (adjoint): split-K partial images
@@ -262,13 +268,23 @@ __device__ __forceinline__ void tc_decode(const TcArgs &a, int u, int &m, int &n
     }
 }
 
-// Unit u of a launch: tile (m, n), K-blocks [kb0, kb1), split. GROUP = 1: u
-// counts the units of the gated instances in instance order (prefix sums
-// gpre[0..ninst]); `ci` is the caller's instance cursor, which only moves
+// Columns of tile n that hold rows of an image, in whole chunk pairs of the
+// epilogue (32): the MMA of an image's last tile stops there. 192 rows take 192
+// columns instead of 256, and so 3/4 of the tensor-core time and of the epilogue.
+__device__ __forceinline__ int tc_cols(int n, int lpad, int live)
+{
+    if (lpad < TC_BN) return TC_BN;  // whole images in a tile
+    const int left = live - (n * TC_BN) % lpad;
+    return left >= TC_BN ? TC_BN : (left + 31) & ~31;
+}
+
+// Unit u of a launch: tile (m, n) of nv columns, K-blocks [kb0, kb1), split.
+// GROUP = 1: u counts the units of the gated instances in instance order (prefix
+// sums gpre[0..ninst]); `ci` is the caller's instance cursor, which only moves
 // forward because every role visits its units in increasing order.
 template <int EPI, int GROUP>
-__device__ __forceinline__ void tc_unit(const TcArgs &a, const int *gpre, int u, int &ci, int &m, int &n, int &kb0,
-                                        int &kb1, int &split)
+__device__ __forceinline__ void tc_unit(const TcArgs &a, const int *gpre, int u, int &ci, int &m, int &n, int &nv,
+                                        int &kb0, int &kb1, int &split)
 {
     if (GROUP) {
         while (gpre[ci + 1] <= u) ci++;
@@ -287,9 +303,121 @@ __device__ __forceinline__ void tc_unit(const TcArgs &a, const int *gpre, int u,
             kb0 = split * gi.kb_per_split;
             kb1 = min(gi.kb_total, kb0 + gi.kb_per_split);
         }
+        nv = tc_cols(n, gi.lpad, gi.live);
     } else {
         tc_decode<EPI>(a, u, m, n, kb0, kb1, split);
+        nv = tc_cols(n, a.lpad, a.live);
     }
+}
+
+// ------------------------------------------------ forward epilogue
+//
+// A thread sums its accumulator row over its 128 columns against Fy: an
+// FP64-accurate anchor every 16 rows (a chunk), rotated within the chunk.
+// The epilogue, not the operand traffic, is what keeps contractions of K <= 256
+// from the tensor cores' rate: with the loads taken out 8 trials at 256^2 ran as
+// before, with the epilogue taken out 1.2 (f16, single CTAs) to 1.5 times faster
+// (E4M3, pairs). It waited for a unit's anchors (two dependent loads), for every
+// chunk's TMEM load, for the chain of rotations, for instructions (900 in a row
+// without a loop), and in a pair for its own stores at the release of the
+// accumulator. So the next unit's anchors and row scales are copied to shared memory
+// during the current one (epi_fetch), two chunks' rotations run side by side in
+// packed arithmetic (half the instructions, the same roundings) while their TMEM
+// loads are in flight, the pairs of chunks are a loop, and the accumulator is
+// released as soon as it has been read. The sums keep their order, row by row.
+// 8 trials, 21,120 uv points, E4M3 pairs: 256^2 78 -> 70 us, 192^2 73 -> 57 (with
+// the cut tiles), 128^2 41 -> 35; 7,680 points, f16, single CTAs: 256^2 43 -> 40;
+// 24 instances of 64^2 to 256^2 in one launch: 240 -> 208.
+
+typedef unsigned long long f32x2;
+__device__ __forceinline__ f32x2 pack2(float lo, float hi)
+{
+    f32x2 d;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "f"(lo), "f"(hi));
+    return d;
+}
+__device__ __forceinline__ float2 unpack2(f32x2 v)
+{
+    float2 d;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(d.x), "=f"(d.y) : "l"(v));
+    return d;
+}
+__device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b)
+{
+    f32x2 d;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+    return d;
+}
+__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c)
+{
+    f32x2 d;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+    return d;
+}
+
+// asynchronous copies of 8 and 16 bytes into shared memory (ok = false: zeros)
+__device__ __forceinline__ void cp_async8(void *dst, const void *src, bool ok)
+{
+    const int bytes = ok ? 8 : 0;
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(umma::smem_u32(dst)), "l"(src), "r"(bytes)
+                 : "memory");
+}
+__device__ __forceinline__ void cp_async16(void *dst, const void *src)
+{
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(umma::smem_u32(dst)), "l"(src) : "memory");
+}
+__device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+
+// one unit of the forward epilogue, besides the accumulator, row scales and anchors
+struct EpiUnit {
+    float2 *vpart;
+    int k, nuv, y0, lpad, live, elog2;
+};
+
+// Starts the copies of unit u: the row scales of the warp's columns into rsw, the
+// anchors and rotations of its 16 uv points (a Re and an Im row each) into anw.
+// row0: the warp's first row of the twiddle-side operand within a tile.
+template <int PAIR, int GROUP>
+__device__ __forceinline__ void epi_fetch(const TcArgs &a, const int *gpre, int u, int &ci, int row0, int lane, int c0,
+                                          float *rsw, float2 *anw, EpiUnit &e)
+{
+    int m, n, nv, kb0, kb1, split;
+    tc_unit<EPI_FWD, GROUP>(a, gpre, u, ci, m, n, nv, kb0, kb1, split);
+    const float2 *fya = a.fya, *fyr = a.fyr;
+    const float *rsc = a.rsc;
+    int nanc = a.nanc;
+    e.vpart = a.vpart;
+    e.nuv = a.nuv;
+    e.lpad = a.lpad;
+    e.live = a.live;
+    e.elog2 = a.elog2;
+    if (GROUP) {
+        const TcGroupInst &gi = a.grp[ci];
+        fya = gi.fya;
+        fyr = gi.fyr;
+        rsc = gi.rsc;
+        nanc = gi.nanc;
+        e.vpart = gi.vpart;
+        e.nuv = gi.nuv;
+        e.lpad = gi.lpad;
+        e.live = gi.live;
+        e.elog2 = gi.elog2;
+    }
+    e.y0 = n * TC_BN;  // first image row of the columns
+    const int k0 = (m * (PAIR ? 256 : 128) + row0) >> 1, k = k0 + (lane & 15);
+    e.k = k0 + (lane >> 1);  // uv point of this thread's row
+    const bool vk = k < e.nuv;
+    const float2 *anc = fya + (size_t)(vk ? k : 0) * nanc;
+#pragma unroll
+    for (int i = 0; i < TC_EPI_COLS / 32; i++) {
+        const int c = 2 * i + (lane >> 4);
+        const int j = ((e.y0 + c0 + 16 * c) % e.lpad) >> 4;  // anchor of the chunk within its image
+        const bool ok = vk && j < nanc;
+        cp_async8(&anw[c * 16 + (lane & 15)], ok ? anc + j : fya, ok);
+    }
+    if (lane < 16) cp_async8(&anw[(TC_EPI_COLS / 16) * 16 + lane], vk ? fyr + k : fyr, vk);
+    static_assert(TC_EPI_COLS == 128, "one 16-byte copy per lane");
+    cp_async16(rsw + 4 * lane, rsc + e.y0 + c0 + 4 * lane);
 }
 
 // PAIR = 0: one CTA per tile of 128 (A rows) x 256 (B rows), 2 stages of 96 KB.
@@ -353,7 +481,7 @@ __global__ void __launch_bounds__(tc_threads<EPI>(), 1)
         }
         for (int b = 0; b < 2; b++) {
             umma::mbar_init(&tfull[b], 1);
-            umma::mbar_init(&tempty[b], (PAIR ? 2 : 1) * 32 * tc_epi_warps<EPI>());  // pair: both CTAs' epilogues release
+            umma::mbar_init(&tempty[b], (PAIR ? 2 : 1) * tc_epi_warps<EPI>());  // pair: both CTAs' epilogues release
         }
         umma::mbar_init(done_bar, 1);
         *abort_flag = 0;
@@ -411,8 +539,8 @@ __global__ void __launch_bounds__(tc_threads<EPI>(), 1)
             const uint32_t tx = (NPROD == 3 ? G::STAGE : TC_A_BYTES + G::B_BYTES) * (PAIR ? 2 : 1);
             int it = 0, ci = 0, cur = -1;
             for (int u = unit0; u < units && !*abort_flag; u += ustep) {
-                int m, n, kb0, kb1, split;
-                tc_unit<EPI, GROUP>(a, gpre, u, ci, m, n, kb0, kb1, split);
+                int m, n, nv, kb0, kb1, split;
+                tc_unit<EPI, GROUP>(a, gpre, u, ci, m, n, nv, kb0, kb1, split);
                 if (GROUP && ci != cur) {
                     // this instance's maps, written to global memory before the launch
                     cur = ci;
@@ -431,7 +559,7 @@ __global__ void __launch_bounds__(tc_threads<EPI>(), 1)
                         umma::tensormap_acquire(mBx);
                     }
                 }
-                const int arow0 = m * G::MT + (int)rank * 128, brow0 = n * TC_BN + (int)rank * G::BROWS;
+                const int arow0 = m * G::MT + (int)rank * 128, brow0 = n * TC_BN + (int)rank * (nv / 2);
                 for (int kb = kb0; kb < kb1; kb++) {
                     const int s = it % G::STAGES;
                     const uint32_t ph = (uint32_t)(it / G::STAGES) & 1u;
@@ -492,12 +620,12 @@ __global__ void __launch_bounds__(tc_threads<EPI>(), 1)
     } else if (warp == 1) {
         if (lane == 0 && leader) {
             // ------------------------------------------------ MMA issuer
-            const uint32_t idesc = umma::idesc_f16(G::MT, TC_BN, OP == OP_TF32 ? 2 : 0);  // f16, tf32; E4M3 for f8f6f4
             int it = 0, t = 0, ci = 0;
             bool ok = true, issued = false;
             for (int u = unit0; u < units && ok && !*abort_flag; u += ustep, t++) {
-                int m, n, kb0, kb1, split;
-                tc_unit<EPI, GROUP>(a, gpre, u, ci, m, n, kb0, kb1, split);
+                int m, n, nv, kb0, kb1, split;
+                tc_unit<EPI, GROUP>(a, gpre, u, ci, m, n, nv, kb0, kb1, split);
+                const uint32_t idesc = umma::idesc_f16(G::MT, nv, OP == OP_TF32 ? 2 : 0);  // f16, tf32; E4M3 for f8f6f4
                 const int b = t & 1;
                 if (!umma::mbar_wait(&tempty[b], ((uint32_t)(t >> 1) & 1u) ^ 1u, a.budget)) {
                     tc_fail(a.err, abort_flag, 2u);
@@ -605,67 +733,48 @@ __global__ void __launch_bounds__(tc_threads<EPI>(), 1)
         // the accumulator buffers are released on the leader's barriers
         const uint32_t te0 = PAIR ? umma::mapa_shared(umma::smem_u32(&tempty[0]), 0) : 0u;
         const uint32_t te1 = PAIR ? umma::mapa_shared(umma::smem_u32(&tempty[1]), 0) : 0u;
+        const int row = (int)rank * 128 + q * 32 + lane;         // row of the twiddle-side operand within a tile
         int t = 0, ci = 0;
+        EpiUnit nxt;
+        float *rsw0 = rsbuf + ew * 2 * TC_EPI_COLS;  // row scales of accumulator buffers 0 and 1
+        float2 *anw0 = (float2 *)(smem + G::STAGES * G::STAGE + TC_AN_OFF) + ew * 2 * TC_AN_PTS;  // likewise anchors
+        if (EPI == EPI_FWD && unit0 < units)
+            epi_fetch<PAIR, GROUP>(a, gpre, unit0, ci, row - lane, lane, c0, rsw0, anw0, nxt);
         for (int u = unit0; u < units; u += ustep, t++) {
-            int m, n, kb0, kb1, split;
-            tc_unit<EPI, GROUP>(a, gpre, u, ci, m, n, kb0, kb1, split);
             const int b = t & 1;
-            const int arow = m * G::MT + (int)rank * 128 + q * 32 + lane;  // row of the twiddle-side operand
-            const int y0 = n * TC_BN;                                      // first image row of the columns
             const uint32_t taddr = tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(b * TC_BN + c0);
+            // the accumulator has been read into this warp's registers: one arrival per warp
+            auto release = [&]() {
+                umma::tc_fence_before();
+                __syncwarp();
+                if (lane == 0) {
+                    if (PAIR) umma::mbar_arrive_cluster(b ? te1 : te0);
+                    else umma::mbar_arrive(&tempty[b]);
+                }
+            };
             if (EPI == EPI_FWD) {
-                // Fy[k][y] along this thread's TC_EPI_COLS columns: an FP64-accurate anchor
-                // every 16 rows, rotated by r_k = e^{-2 pi i s v_k} within the chunk (<= 15
-                // steps). Partial entries hold at most TC_EPI_COLS rows (elog2 <= 7), so
-                // that no entry spans two epilogue warps.
-                const float2 *fya = a.fya, *fyr = a.fyr;
-                const float *rsc = a.rsc;
-                float2 *vpart = a.vpart;
-                int nuv = a.nuv, nanc = a.nanc, lpad = a.lpad, elog2 = a.elog2;
-                if (GROUP) {
-                    const TcGroupInst &gi = a.grp[ci];
-                    fya = gi.fya;
-                    fyr = gi.fyr;
-                    rsc = gi.rsc;
-                    vpart = gi.vpart;
-                    nuv = gi.nuv;
-                    nanc = gi.nanc;
-                    lpad = gi.lpad;
-                    elog2 = gi.elog2;
-                }
-                const int k = arow >> 1;
-                const bool vk = k < nuv;
-                const float2 rot = vk ? __ldg(&fyr[k]) : make_float2(0.f, 0.f);
-                const float2 *anc = fya + (size_t)(vk ? k : 0) * nanc;
-                float2 an[TC_EPI_COLS / 16];
-#pragma unroll
-                for (int c = 0; c < TC_EPI_COLS / 16; c++) {
-                    const int j = ((y0 + c0 + 16 * c) % lpad) >> 4;  // anchor of the row within its image
-                    an[c] = (vk && j < nanc) ? __ldg(&anc[j]) : make_float2(0.f, 0.f);
-                }
-                // the row scales of this warp's columns into its shared copy (one L2
-                // round trip per unit, issued before the accumulator is ready; the copy
-                // of buffer b was last read by this warp two units ago)
-                float *rsw = rsbuf + (ew * 2 + b) * TC_EPI_COLS;
-                __syncwarp();
-                {
-                    static_assert(TC_EPI_COLS == 128, "one float4 per lane");
-                    const float4 *src = reinterpret_cast<const float4 *>(rsc + y0 + c0);
-                    reinterpret_cast<float4 *>(rsw)[lane] = __ldg(src + lane);
-                }
-                __syncwarp();
+                const EpiUnit cur = nxt;
+                const float *rsw = rsw0 + b * TC_EPI_COLS;
+                cp_async_wait();
+                __syncwarp();  // the copies come from every lane
+                const float2 *anw = anw0 + b * TC_AN_PTS + (lane >> 1);
+                const float2 rot = anw[(TC_EPI_COLS / 16) * 16];
+                // the next unit's copies (this warp last read buffer 1 - b before the barrier above)
+                if (u + ustep < units)
+                    epi_fetch<PAIR, GROUP>(a, gpre, u + ustep, ci, row - lane, lane, c0,
+                                           rsw0 + (1 - b) * TC_EPI_COLS, anw0 + (1 - b) * TC_AN_PTS, nxt);
                 if (!umma::mbar_wait(&tfull[b], (uint32_t)(t >> 1) & 1u, a.budget)) {
                     tc_fail(a.err, abort_flag, 8u);
                     break;
                 }
                 umma::tc_fence_after();
-                const int emask = (1 << elog2) - 1;
-                if (lpad < TC_EPI_COLS) {
+                const bool vk = cur.k < cur.nuv;
+                if (cur.lpad < TC_EPI_COLS) {
                     // several images in this warp's columns (a batch stack of lpad = 32 or
                     // 64 rows each; y0 + c0 is a multiple of lpad): chunk q of every image
                     // has the same 16 values of Fy, formed once for all of them. Each
                     // image's sum takes its chunks and rows in the order of the loop below.
-                    const int per = lpad >> 4, nimg = TC_EPI_COLS / lpad;
+                    const int per = cur.lpad >> 4, nimg = TC_EPI_COLS / cur.lpad;
                     float are[TC_EPI_COLS / 32], aim[TC_EPI_COLS / 32];
 #pragma unroll
                     for (int i = 0; i < TC_EPI_COLS / 32; i++) {
@@ -673,80 +782,112 @@ __global__ void __launch_bounds__(tc_threads<EPI>(), 1)
                         aim[i] = 0.f;
                     }
 #pragma unroll 1
-                    for (int qq = 0; qq < per; qq++) {  // a loop, not unrolled: the tile code stays in the instruction cache
+                    for (int qq = 0; qq < per && 16 * qq < cur.live; qq++) {  // not unrolled: the code stays in the instruction cache
+                        uint32_t r[2][16];  // two images at a time: the registers
+                        umma::tmem_ld16(taddr + (uint32_t)(qq * 16), r[0]);
+                        umma::tmem_ld16(taddr + (uint32_t)((per + qq) * 16), r[1]);
                         float2 wv[16];
-                        wv[0] = (vk && qq < nanc) ? __ldg(&anc[qq]) : make_float2(0.f, 0.f);
+                        wv[0] = anw[qq * 16];
 #pragma unroll
                         for (int j = 1; j < 16; j++) wv[j] = fy_step(wv[j - 1], rot);
 #pragma unroll
-                        for (int ti = 0; ti < TC_EPI_COLS / 32; ti++) {
-                            if (ti < nimg) {  // warp-uniform
-                                const int c = ti * per + qq;
-                                uint32_t r[16];
-                                umma::tmem_ld16(taddr + (uint32_t)(c * 16), r);
-                                float rs[16];
-                                const float4 *rp = reinterpret_cast<const float4 *>(rsw + 16 * c);
-#pragma unroll
-                                for (int v4 = 0; v4 < 4; v4++) *reinterpret_cast<float4 *>(&rs[4 * v4]) = rp[v4];
-                                umma::tmem_ld_wait();
-                                float sr = are[ti], si = aim[ti];
-#pragma unroll
-                                for (int j = 0; j < 16; j++) {
-                                    const float tv = __uint_as_float(r[j]) * rs[j];
-                                    sr = fmaf(tv, wv[j].x, sr);
-                                    si = fmaf(tv, wv[j].y, si);
+                        for (int t2 = 0; t2 < TC_EPI_COLS / 32; t2 += 2) {
+                            if (t2 < nimg) {  // warp-uniform
+                                if (t2) {
+                                    umma::tmem_ld16(taddr + (uint32_t)((t2 * per + qq) * 16), r[0]);
+                                    umma::tmem_ld16(taddr + (uint32_t)(((t2 + 1) * per + qq) * 16), r[1]);
                                 }
-                                are[ti] = sr;
-                                aim[ti] = si;
+                                umma::tmem_ld_wait();
+                                if (t2 + 2 >= nimg && (qq + 1 >= per || 16 * (qq + 1) >= cur.live)) release();
+#pragma unroll
+                                for (int h = 0; h < 2; h++) {
+                                    const float4 *rp = reinterpret_cast<const float4 *>(rsw + 16 * ((t2 + h) * per + qq));
+                                    float sr = are[t2 + h], si = aim[t2 + h];
+#pragma unroll
+                                    for (int j = 0; j < 16; j += 4) {
+                                        const float4 rs = rp[j / 4];
+                                        const float rv[4] = {rs.x, rs.y, rs.z, rs.w};
+#pragma unroll
+                                        for (int i = 0; i < 4; i++) {
+                                            const float tv = __uint_as_float(r[h][j + i]) * rv[i];
+                                            sr = fmaf(tv, wv[j + i].x, sr);
+                                            si = fmaf(tv, wv[j + i].y, si);
+                                        }
+                                    }
+                                    are[t2 + h] = sr;
+                                    aim[t2 + h] = si;
+                                }
                             }
                         }
                     }
 #pragma unroll
                     for (int ti = 0; ti < TC_EPI_COLS / 32; ti++) {
                         if (ti < nimg) {
-                            const int entry = (y0 + c0 + ti * lpad) >> elog2;
+                            const int entry = (cur.y0 + c0 + ti * cur.lpad) >> cur.elog2;
                             const float re = are[ti], im = aim[ti];
                             const float ore = __shfl_xor_sync(0xffffffffu, re, 1);
                             const float oim = __shfl_xor_sync(0xffffffffu, im, 1);
                             if ((lane & 1) == 0 && vk)
-                                vpart[(size_t)entry * nuv + k] = make_float2(re - oim, im + ore);
+                                cur.vpart[(size_t)entry * cur.nuv + cur.k] = make_float2(re - oim, im + ore);
                         }
                     }
                 } else {
+                    // 128 rows of one image: one partial entry (elog2 = 7)
+                    const f32x2 rx = pack2(rot.x, rot.x), ry = pack2(rot.y, rot.y);
+                    const f32x2 nry = pack2(-rot.y, -rot.y);
+                    const int y1 = (cur.y0 + c0) % cur.lpad;  // first row within its image
                     float sre = 0.f, sim = 0.f;
+                    const int nc = min(TC_EPI_COLS, cur.live - y1);  // columns that hold rows (the rest are zero)
+                    if (nc <= 0) release();
+#pragma unroll 1
+                    for (int c = 0; 16 * c < nc; c += 2) {  // not unrolled, as above
+                        {
+                            uint32_t r[2][16];
+                            umma::tmem_ld16(taddr + (uint32_t)(c * 16), r[0]);
+                            umma::tmem_ld16(taddr + (uint32_t)(c * 16 + 16), r[1]);
+                            // (Re, Im) of Fy along both chunks: X, Y hold rows j of chunk c and chunk c + 1
+                            f32x2 X[16], Y[16];
+                            const float2 w0 = anw[c * 16], w1 = anw[c * 16 + 16];
+                            X[0] = pack2(w0.x, w1.x);
+                            Y[0] = pack2(w0.y, w1.y);
 #pragma unroll
-                    for (int c = 0; c < TC_EPI_COLS / 16; c++) {
-                        uint32_t r[16];
-                        umma::tmem_ld16(taddr + (uint32_t)(c * 16), r);
-                        // power-of-two scales of the 16 image rows (shared memory, same address in every lane)
-                        float rs[16];
-                        const float4 *rp = reinterpret_cast<const float4 *>(rsw + 16 * c);
+                            for (int j = 1; j < 16; j++) {  // fy_step
+                                X[j] = fma2(X[j - 1], rx, mul2(Y[j - 1], nry));
+                                Y[j] = fma2(X[j - 1], ry, mul2(Y[j - 1], rx));
+                            }
+                            umma::tmem_ld_wait();
+                            if (16 * (c + 2) >= nc) release();
 #pragma unroll
-                        for (int v4 = 0; v4 < 4; v4++) *reinterpret_cast<float4 *>(&rs[4 * v4]) = rp[v4];
-                        umma::tmem_ld_wait();
-                        float2 w = an[c];
+                            for (int h = 0; h < 2; h++) {
+                                // power-of-two scales of the 16 image rows (shared memory, same address in every lane)
+                                const float4 *rp = reinterpret_cast<const float4 *>(rsw + 16 * (c + h));
 #pragma unroll
-                        for (int j = 0; j < 16; j++) {
-                            const float tv = __uint_as_float(r[j]) * rs[j];
-                            sre = fmaf(tv, w.x, sre);
-                            sim = fmaf(tv, w.y, sim);
-                            w = fy_step(w, rot);
-                        }
-                        if (((y0 + c0 + 16 * c + 16) & emask) == 0) {
-                            // end of a partial entry (warp-uniform): combine the Re/Im row
-                            // pair, store. even row: (sum T_re F_re, sum T_re F_im);
-                            // odd row: (sum T_im F_re, sum T_im F_im)
-                            const int entry = (y0 + c0 + 16 * c) >> elog2;
-                            const float re = sre, im = sim;
-                            const float ore = __shfl_xor_sync(0xffffffffu, re, 1);
-                            const float oim = __shfl_xor_sync(0xffffffffu, im, 1);
-                            if ((lane & 1) == 0 && vk) vpart[(size_t)entry * nuv + k] = make_float2(re - oim, im + ore);
-                            sre = 0.f;
-                            sim = 0.f;
+                                for (int j = 0; j < 16; j += 4) {
+                                    const float4 rs = rp[j / 4];
+                                    const float rv[4] = {rs.x, rs.y, rs.z, rs.w};
+#pragma unroll
+                                    for (int i = 0; i < 4; i++) {
+                                        const float tv = __uint_as_float(r[h][j + i]) * rv[i];
+                                        const float2 x = unpack2(X[j + i]), y = unpack2(Y[j + i]);
+                                        sre = fmaf(tv, h ? x.y : x.x, sre);
+                                        sim = fmaf(tv, h ? y.y : y.x, sim);
+                                    }
+                                }
+                            }
                         }
                     }
+                    // combine the Re/Im row pair, store. even row: (sum T_re F_re, sum T_re F_im);
+                    // odd row: (sum T_im F_re, sum T_im F_im)
+                    const int entry = (cur.y0 + c0) >> cur.elog2;
+                    const float ore = __shfl_xor_sync(0xffffffffu, sre, 1);
+                    const float oim = __shfl_xor_sync(0xffffffffu, sim, 1);
+                    if ((lane & 1) == 0 && vk)
+                        cur.vpart[(size_t)entry * cur.nuv + cur.k] = make_float2(sre - oim, sim + ore);
                 }
             } else {
+                int m, n, nv, kb0, kb1, split;
+                tc_unit<EPI, GROUP>(a, gpre, u, ci, m, n, nv, kb0, kb1, split);
+                const int y0 = n * TC_BN;  // first image row of the columns
                 if (!umma::mbar_wait(&tfull[b], (uint32_t)(t >> 1) & 1u, a.budget)) {
                     tc_fail(a.err, abort_flag, 8u);
                     break;
@@ -762,25 +903,24 @@ __global__ void __launch_bounds__(tc_threads<EPI>(), 1)
                     out_cols = gi.out_cols;
                 }
                 float *out = gpart + (size_t)split * out_rows * out_ld;
-                const int x = arow;
+                const int x = m * G::MT + row;  // twiddle-side row: an image column
                 const bool xv = x < out_cols;
 #pragma unroll 1
-                for (int c = 0; c < ECOLS / 16; c++) {
-                    uint32_t r[16];
-                    umma::tmem_ld16(taddr + (uint32_t)(c * 16), r);
+                for (int c = 0; c < nv; c += 32) {
+                    uint32_t r[2][16];
+                    umma::tmem_ld16(taddr + (uint32_t)c, r[0]);
+                    umma::tmem_ld16(taddr + (uint32_t)(c + 16), r[1]);
                     umma::tmem_ld_wait();
+                    if (c + 32 >= nv) release();
                     if (xv) {
+                        float *o = out + (size_t)(y0 + c) * out_ld + x;
 #pragma unroll
-                        for (int j = 0; j < 16; j++) {
-                            const int y = y0 + c0 + c * 16 + j;
-                            if (y < out_rows) out[(size_t)y * out_ld + x] = __uint_as_float(r[j]);
+                        for (int j = 0; j < 32; j++) {
+                            if (y0 + c + j < out_rows) o[(size_t)j * out_ld] = __uint_as_float(r[j >> 4][j & 15]);
                         }
                     }
                 }
             }
-            umma::tc_fence_before();
-            if (PAIR) umma::mbar_arrive_cluster(b ? te1 : te0);
-            else umma::mbar_arrive(&tempty[b]);
         }
     }
     __syncthreads();
@@ -1928,6 +2068,10 @@ static TcArgs tc_grid_args(gpair_ctx *c, TcState *t, int images)
     a.out_ld = g->ldT;
     a.out_rows = images > 1 ? images * t->Lb : c->N;
     a.out_cols = 2 * g->nbx;
+    if (images == 1) {  // a stack's rows are all written
+        a.lpad = t->M_pad;
+        a.live = c->N;
+    }
     return a;
 }
 
@@ -1967,6 +2111,7 @@ int gp_tc_forward_gemm(gpair_ctx *c)
     a.N = c->N;
     a.nuv = c->nuv;
     a.lpad = t->M_pad;  // one image, partial entries of TC_EPI_COLS rows (one epilogue warp's columns)
+    a.live = c->N;
     a.elog2 = 7;
     a.rsc = t->rsc;
     a.vpart = c->vpart;
@@ -2056,6 +2201,7 @@ int gp_tc_forward_batch_gemm(gpair_ctx *c)
     a.N = c->N;
     a.nuv = c->nuv;
     a.lpad = t->Lb;
+    a.live = c->N;
     const int erows = t->Lb < TC_EPI_COLS ? t->Lb : TC_EPI_COLS;
     a.elog2 = erows == 32 ? 5 : erows == 64 ? 6 : 7;
     a.rsc = t->rscb;
@@ -2148,6 +2294,8 @@ int gp_tc_adjoint_gemm(gpair_ctx *c)
     a.out_ld = c->N;
     a.out_rows = c->N;
     a.out_cols = c->N;
+    a.lpad = t->M_pad;
+    a.live = c->N;
     const TcMaps m = {&t->m_fxt_hi, &t->m_fxt_lo, &t->m_fxt_hi, &t->m_w_hi, &t->m_w_lo, &t->m_w_hi};
     if ((rc = tc_launch<EPI_STORE>(c, t, m, a))) return rc;
     c->splits = t->splits;
@@ -2218,6 +2366,8 @@ static void tc_group_inst(gpair_ctx *c, TcState *t, int kind, TcGroupInst &g)
         g.out_ld = c->N;
         g.out_rows = c->N;
         g.out_cols = c->N;
+        g.lpad = t->M_pad;
+        g.live = c->N;
         return;
     }
     const bool batch = kind == GP_TCG_TRIALS;
@@ -2232,6 +2382,8 @@ static void tc_group_inst(gpair_ctx *c, TcState *t, int kind, TcGroupInst &g)
         g.out_ld = a.out_ld;
         g.out_rows = a.out_rows;
         g.out_cols = a.out_cols;
+        g.lpad = a.lpad;
+        g.live = a.live;
     }
     const TcMaps fm = tc_fwd_maps(t, batch);
     g.A_hi = *fm.a_hi;
@@ -2250,6 +2402,7 @@ static void tc_group_inst(gpair_ctx *c, TcState *t, int kind, TcGroupInst &g)
     g.fyr = t->fyr;
     g.nanc = t->nanc;
     g.nuv = c->nuv;
+    g.live = c->N;
     if (batch) {
         g.lpad = t->Lb;
         const int erows = t->Lb < TC_EPI_COLS ? t->Lb : TC_EPI_COLS;
