@@ -306,7 +306,7 @@ struct gpair_ctx {
     // steps s and gradient changes y, and the image the last direction started from
     float *lb_s, *lb_y, *lb_xold;
     float2 *vpart_b;
-    double2 *visb;  // visibilities of the GP_NTR trials [GP_NTR][K], when their partial entries are many
+    double2 *visb;  // visibilities of the GP_NTR trials [K][GP_NTR], when their partial entries are many
     double *partials_b;
     int batch_wave[2];  // blocks per trial that fill one wave: [0] trial prep, [1] trial chi2
     int epp;  // forward partial entries per trial image

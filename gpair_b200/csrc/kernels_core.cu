@@ -295,10 +295,13 @@ int gp_forward(gpair_ctx *c, int which)
 
 // ------------------------------------------------- V2, T3, chi2, weights
 
+// The roundings are fixed (one product, then a fused multiply-add), so that a stage gives the same bits in
+// its own kernel and in a grouped launch, whatever the compiler fuses around it.
 __device__ __forceinline__ double2 cmul(double2 a, double2 b)
 {
-    return make_double2(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x);
+    return make_double2(fma(a.x, b.x, -__dmul_rn(a.y, b.y)), fma(a.x, b.y, __dmul_rn(a.y, b.x)));
 }
+__device__ __forceinline__ double sqr2(double x, double y) { return fma(x, x, __dmul_rn(y, y)); }  // x^2 + y^2
 __device__ __forceinline__ double2 cconj(double2 a) { return make_double2(a.x, -a.y); }
 
 __device__ __forceinline__ double2 sum_vpart(const float2 *__restrict__ vpart, int mt, int nuv, int k, double invF)
@@ -311,6 +314,8 @@ __device__ __forceinline__ double2 sum_vpart(const float2 *__restrict__ vpart, i
     }
     return make_double2(re * invF, im * invF);
 }
+
+__device__ __forceinline__ int gp_div_up(int a, int b) { return (a + b - 1) / b; }
 
 struct VisDataArgs {
     const float2 *vpart;
@@ -354,47 +359,54 @@ __device__ __forceinline__ void vis_data_body(const VisDataArgs &A, const GpVGri
     if (vg.bx < nblk_uv) {
         for (int k = vg.bx * blockDim.x + threadIdx.x; k < nuv; k += nblk_uv * blockDim.x) {
             double2 V = VIS_AT(k);
-            visd[k] = V;
+            if (!direct) visd[k] = V;
             visi[k] = make_float2((float)V.x, (float)V.y);
             float2 a = make_float2(0.f, 0.f);
             if (k < npow) {
-                double m2 = V.x * V.x + V.y * V.y;
+                double m2 = sqr2(V.x, V.y);
                 mock[k] = (float)m2;
-                double w = data_err[k], res = m2 - (double)data[k], r = res * w;
-                chi[0] += r * r;
+                double w = data_err[k], res = m2 - (double)data[k], r = __dmul_rn(res, w);
+                chi[0] = fma(r, r, chi[0]);
                 double f = 4.0 * w * w * res * invF; // a_k = f conj(V_k)
                 a = make_float2((float)(f * V.x), (float)(-f * V.y));
             }
             cw[k] = a;
         }
     } else {
-        const int nblk_tri = vg.nbx - nblk_uv;
-        for (int t = (vg.bx - nblk_uv) * blockDim.x + threadIdx.x; t < nbis; t += nblk_tri * blockDim.x) {
-            int4 q = tri[t];
+        // a run of consecutive triangles per block (those of an observation share its baselines: L1), the
+        // next triangle's index in flight
+        const int run = gp_div_up(gp_div_up(nbis, vg.nbx - nblk_uv), (int)blockDim.x) * (int)blockDim.x;
+        const int end = min(nbis, (vg.bx - nblk_uv + 1) * run);
+        int t = (vg.bx - nblk_uv) * run + (int)threadIdx.x;
+        int4 qn = t < end ? __ldg(&tri[t]) : make_int4(0, 0, 0, 0);
+        for (; t < end; t += blockDim.x) {
+            const int4 q = qn;
+            if (t + (int)blockDim.x < end) qn = __ldg(&tri[t + blockDim.x]);
             double2 va = VIS_AT(q.x);
             double2 vb = VIS_AT(q.y);
             double2 vc = VIS_AT(q.z);
+            const float2 phf = __ldg(&phasor[t]);
+            const int r0 = npow + 2 * t;
+            const float d0 = __ldg(&data[r0]), d1 = __ldg(&data[r0 + 1]);
+            const double wre = __ldg(&data_err[r0]), wim = __ldg(&data_err[r0 + 1]);
             if (q.w & 1) va = cconj(va);
             if (q.w & 2) vb = cconj(vb);
             if (q.w & 4) vc = cconj(vc);
-            float2 phf = phasor[t];
-            double2 ph = make_double2(phf.x, phf.y);
-            double2 t3 = cmul(cmul(cmul(va, vb), vc), ph);
-            int r0 = npow + 2 * t;
+            const double2 ph = make_double2(phf.x, phf.y);
+            const double2 ab = cmul(va, vb), t3 = cmul(cmul(ab, vc), ph);
             mock[r0] = (float)t3.x;
             mock[r0 + 1] = (float)t3.y;
-            double wre = data_err[r0], wim = data_err[r0 + 1];
-            double rre = t3.x - (double)data[r0], rim = t3.y - (double)data[r0 + 1];
-            chi[0] += (rre * wre) * (rre * wre) + (rim * wim) * (rim * wim);
+            const double rre = t3.x - (double)d0, rim = t3.y - (double)d1;
+            chi[0] += sqr2(__dmul_rn(rre, wre), __dmul_rn(rim, wim));
             // adjoint: Re(conj(g) * t3der) with g = 2 w_re^2 (T3re - d_re) + i 2 w_im^2 T3im
             // (the reference uses the mock imaginary part alone, gpair1/trunk/cpu.c:364-365)
-            double2 g = make_double2(2.0 * wre * wre * rre, 2.0 * wim * wim * t3.y);
+            const double2 g = make_double2(2.0 * wre * wre * rre, 2.0 * wim * wim * t3.y);
             double2 base = cmul(cconj(g), ph);
             base.x *= invF;
             base.y *= invF;
             double2 bab = cmul(base, cmul(vb, vc));
             double2 bbc = cmul(base, cmul(va, vc));
-            double2 bca = cmul(base, cmul(va, vb));
+            double2 bca = cmul(base, ab);
             if (q.w & 1) bab = cconj(bab);
             if (q.w & 2) bbc = cconj(bbc);
             if (q.w & 4) bca = cconj(bca);
@@ -421,7 +433,7 @@ __device__ __forceinline__ void vis_data_body(const VisDataArgs &A, const GpVGri
 
 #undef VIS_AT
 
-__global__ void __launch_bounds__(GP_THREADS) k_vis_data(const VisDataArgs a)
+__global__ void __launch_bounds__(GP_THREADS, 4) k_vis_data(const VisDataArgs a)
 {
     gp_pdl_enter();
     vis_data_body(a, gp_vgrid_hw());
@@ -434,11 +446,13 @@ struct VisDataOp {
 
 static VisDataArgs vis_data_args(gpair_ctx *c, int direct, FusedCtrl fc)
 {
+    // one wave of blocks (four per SM), more of them for the triangles: 1024^2 workload 37 us in three and a
+    // half waves, 25 in one (and four blocks per SM in 64 registers; 33 with three blocks, 28 with five)
     int nbu = gp_cdiv(c->nuv, GP_THREADS);
-    if (nbu > 512) nbu = 512;
+    if (nbu > 96) nbu = 96;
     if (nbu < 1) nbu = 1;
     int nbt = gp_cdiv(c->nbis, GP_THREADS);
-    if (nbt > 1536) nbt = 1536;
+    if (nbt > 496) nbt = 496;
     VisDataArgs a = {c->vpart, c->mt, c->nuv, c->npow, c->nbis, c->data, c->data_err, c->tri, c->phasor, nbu,
                      c->visd, c->visi, c->mock, c->cw, c->trib, slot_partials(c, RED_CHI2), c->sc, fc, direct,
                      c->direct_result ? c->hres : nullptr, nbu + nbt, 1};
@@ -1578,13 +1592,49 @@ __global__ void __launch_bounds__(GP_THREADS) k_trials_prep(const float *__restr
     }
 }
 
-// chi2 of every trial of a batch (blockIdx.y = trial): V = (sum of the trial's
-// epp partial entries) / F_j, then V2 and T3 residuals as in k_vis_data; mock
-// data and adjoint weights are not needed for trials. The last block of the
-// whole grid sums each trial's partials in block order and runs the controller.
-struct VisChi2BatchArgs {
+// Partial visibilities of a batch: entry e of trial j at uv point k lies at
+// vpart[j sj + e se + k sk]. The tensor forward writes a uv point's entries side
+// by side (sj = epp, se = 1, sk = GP_NTR epp), so that gathering a uv point for
+// all trials reads whole lines; the CUDA-core forward trial by trial
+// (sj = epp nuv, se = nuv, sk = 1).
+struct TrialVis {
     const float2 *vpart;
-    int epp, nuv, npow, nbis;
+    long long sj, se, sk;
+    int epp;
+};
+__device__ __forceinline__ double2 sum_trial(const TrialVis &T, int j, int k, double invF)
+{
+    const float2 *p = T.vpart + j * T.sj + k * T.sk;
+    double re = 0.0, im = 0.0;
+    if (T.epp == 2 && T.se == 1) {  // 129 to 256 pixels on the tensor path: both entries in one load
+        const float4 v = __ldg(reinterpret_cast<const float4 *>(p));
+        re += v.x;
+        im += v.y;
+        re += v.z;
+        im += v.w;
+        return make_double2(re * invF, im * invF);
+    }
+    for (int e = 0; e < T.epp; e++, p += T.se) {
+        const float2 v = __ldg(p);
+        re += v.x;
+        im += v.y;
+    }
+    return make_double2(re * invF, im * invF);
+}
+
+// chi2 of every trial of a batch: V = (sum of the trial's epp partial entries) /
+// F_j, then V2 and T3 residuals as in k_vis_data; mock data and adjoint weights are
+// not needed for trials. Bound by the latency of the gathers (index, then three uv
+// points): eight neighbouring lanes take the eight trials of one datum, so that
+// its index, data and errors are read once and a uv point's eight values come as one
+// 128-byte line (a thread per datum of one trial used 16 of every 32 bytes).
+// 1024^2 workload, 194,560 + 1,167,360 data: 60 us against 101 (five blocks per SM;
+// 68 with four, 83 with six and spills); 24 instances in one launch: 36 against 40. Every block sums its trials' data in a
+// fixed order; the last block sums each trial's partials in block order and runs
+// the controller.
+struct VisChi2BatchArgs {
+    TrialVis tv;
+    int npow, nbis;
     const float *data, *data_err;
     const int4 *tri;
     const float2 *phasor;
@@ -1592,61 +1642,77 @@ struct VisChi2BatchArgs {
     DevScalars *sc;
     FusedCtrl fc;
     const int *gate;
-    const double2 *visb;  // the trials' visibilities summed beforehand (k_vis_sum_batch), or null
+    const double2 *visb;  // the trials' visibilities [nuv][GP_NTR] summed beforehand, or null
     GP_VGRID_FIELDS;
 };
+static_assert(GP_NTR == 8, "eight lanes per datum");
 
 __device__ __forceinline__ void vis_chi2_batch_body(const VisChi2BatchArgs &A, const GpVGrid &vg)
 {
-    const float2 *__restrict__ vpart = A.vpart;
-    const int epp = A.epp, nuv = A.nuv, npow = A.npow, nbis = A.nbis;
+    const int npow = A.npow, nitems = A.npow + A.nbis;
     const float *__restrict__ data = A.data;
     const float *__restrict__ data_err = A.data_err;
     const int4 *__restrict__ tri = A.tri;
     const float2 *__restrict__ phasor = A.phasor;
+    const double2 *__restrict__ vb = A.visb;
     double *__restrict__ partials = A.partials;
     DevScalars *__restrict__ sc = A.sc;
-    __shared__ double smem[32];
+    __shared__ double smem[GP_THREADS / 32][GP_NTR];
     if (A.gate && !*A.gate) return;  // lockstep batches: this instance's line search is over
-    const int j = vg.by;
+    const int j = threadIdx.x & (GP_NTR - 1);
     const double invF = sc->t_invflux[j];
-    const float2 *vp = vpart + (size_t)j * epp * nuv;
-    const double2 *vb = A.visb ? A.visb + (size_t)j * nuv : nullptr;
-#define VIS_B(k) (vb ? vb[(k)] : sum_vpart(vp, epp, nuv, (k), invF))
-    double chi[1] = {0.0};
-    const int nitems = npow + nbis;
-    for (int i = vg.bx * blockDim.x + threadIdx.x; i < nitems; i += vg.nbx * blockDim.x) {
-        if (i < npow) {
-            double2 V = VIS_B(i);
-            double m2 = V.x * V.x + V.y * V.y;
-            double r = (m2 - (double)data[i]) * data_err[i];
-            chi[0] += r * r;
-        } else {
-            const int t = i - npow;
-            int4 q = tri[t];
-            double2 va = VIS_B(q.x);
-            double2 vbb = VIS_B(q.y);
-            double2 vc = VIS_B(q.z);
-            if (q.w & 1) va = cconj(va);
-            if (q.w & 2) vbb = cconj(vbb);
-            if (q.w & 4) vc = cconj(vc);
-            float2 phf = phasor[t];
-            double2 t3 = cmul(cmul(cmul(va, vbb), vc), make_double2(phf.x, phf.y));
-            const int r0 = npow + 2 * t;
-            double rre = (t3.x - (double)data[r0]) * data_err[r0];
-            double rim = (t3.y - (double)data[r0 + 1]) * data_err[r0 + 1];
-            chi[0] += rre * rre + rim * rim;
-        }
+    const TrialVis tv = A.tv;
+    auto vis = [&](int k) { return vb ? __ldg(&vb[(size_t)k * GP_NTR + j]) : sum_trial(tv, j, k, invF); };
+    double chi = 0.0;
+    // a run of consecutive data per block: the triangles of an observation share its baselines, whose values
+    // then come from L1
+    const int step = GP_THREADS / GP_NTR, run = gp_div_up(gp_div_up(nitems, vg.nbx), step) * step;
+    const int end = min(nitems, (vg.bx + 1) * run), end_pow = min(npow, end);
+    int i = vg.bx * run + threadIdx.x / GP_NTR;
+#pragma unroll 2
+    for (; i < end_pow; i += step) {
+        const double2 V = vis(i);
+        const double r = __dmul_rn(sqr2(V.x, V.y) - (double)__ldg(&data[i]), __ldg(&data_err[i]));
+        chi = fma(r, r, chi);
     }
-    block_sum<1>(chi, smem);
-    if (threadIdx.x == 0) partials[(size_t)j * vg.nbx + vg.bx] = chi[0];
-    if (last_block_of(&sc->t_counter[GP_NTR], vg.nbx * vg.nby)) {
+    int4 qn = i < end ? __ldg(&tri[i - npow]) : make_int4(0, 0, 0, 0);
+    for (; i < end; i += step) {
+        const int4 q = qn;
+        const int t = i - npow;
+        if (i + step < end) qn = __ldg(&tri[t + step]);  // the next index in flight
+        double2 va = vis(q.x), vbb = vis(q.y), vc = vis(q.z);
+        const float2 phf = __ldg(&phasor[t]);
+        const float d0 = __ldg(&data[npow + 2 * t]), d1 = __ldg(&data[npow + 2 * t + 1]);
+        const float w0 = __ldg(&data_err[npow + 2 * t]), w1 = __ldg(&data_err[npow + 2 * t + 1]);
+        if (q.w & 1) va = cconj(va);
+        if (q.w & 2) vbb = cconj(vbb);
+        if (q.w & 4) vc = cconj(vc);
+        const double2 t3 = cmul(cmul(cmul(va, vbb), vc), make_double2(phf.x, phf.y));
+        chi += sqr2(__dmul_rn(t3.x - (double)d0, w0), __dmul_rn(t3.y - (double)d1, w1));
+    }
+    // over the lanes of one trial, then over the warps
+    chi += __shfl_down_sync(0xffffffffu, chi, 16);
+    chi += __shfl_down_sync(0xffffffffu, chi, 8);
+    if ((threadIdx.x & 31) < GP_NTR) smem[threadIdx.x >> 5][j] = chi;
+    __syncthreads();
+    if (threadIdx.x < GP_NTR) {
+        double v = 0.0;
+        for (int w = 0; w < GP_THREADS / 32; w++) v += smem[w][threadIdx.x];
+        partials[(size_t)threadIdx.x * vg.nbx + vg.bx] = v;
+    }
+    if (last_block_of(&sc->t_counter[GP_NTR], vg.nbx)) {
         // one warp per trial, all trials at once; fixed lane order and shuffle tree
         const int lane = threadIdx.x & 31;
-        for (int jj = threadIdx.x >> 5; jj < vg.nby; jj += blockDim.x >> 5) {
+        for (int jj = threadIdx.x >> 5; jj < GP_NTR; jj += blockDim.x >> 5) {
             const double *pp = partials + (size_t)jj * vg.nbx;
             double v = 0.0;
-            for (int b = lane; b < vg.nbx; b += 32) v += __ldcg(&pp[b]);
+            for (int b0 = lane; b0 < vg.nbx; b0 += 8 * 32) {
+                double p[8];  // eight loads in flight
+#pragma unroll
+                for (int i = 0; i < 8; i++) p[i] = b0 + 32 * i < vg.nbx ? __ldcg(&pp[b0 + 32 * i]) : 0.0;
+#pragma unroll
+                for (int i = 0; i < 8; i++) v += p[i];
+            }
             for (int off = 16; off > 0; off >>= 1) v += __shfl_down_sync(0xffffffffu, v, off);
             if (lane == 0) sc->t_chi2[jj] = v;
         }
@@ -1658,25 +1724,22 @@ __device__ __forceinline__ void vis_chi2_batch_body(const VisChi2BatchArgs &A, c
     }
 }
 
-#undef VIS_B
-
-// the trials' visibilities V_jk = (sum of trial j's partial entries) / F_j into visb,
+// the trials' visibilities V_jk = (sum of trial j's partial entries) / F_j into visb [nuv][GP_NTR],
 // summed once instead of once per gathering triangle vertex (the same sum)
-__global__ void __launch_bounds__(GP_THREADS) k_vis_sum_batch(const float2 *__restrict__ vpart, int epp, int nuv,
+__global__ void __launch_bounds__(GP_THREADS) k_vis_sum_batch(const TrialVis tv, int nuv,
                                                               const DevScalars *__restrict__ sc,
                                                               double2 *__restrict__ visb,
                                                               const int *__restrict__ gate)
 {
     gp_pdl_enter();
     if (gate && !*gate) return;  // lockstep batches: this instance's line search is over
-    const int j = blockIdx.y;
+    const int j = threadIdx.x & (GP_NTR - 1);
     const double invF = sc->t_invflux[j];
-    const float2 *vp = vpart + (size_t)j * epp * nuv;
-    for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < nuv; k += gridDim.x * blockDim.x)
-        visb[(size_t)j * nuv + k] = sum_vpart(vp, epp, nuv, k, invF);
+    for (int k = (blockIdx.x * blockDim.x + threadIdx.x) / GP_NTR; k < nuv; k += gridDim.x * (GP_THREADS / GP_NTR))
+        visb[(size_t)k * GP_NTR + j] = sum_trial(tv, j, k, invF);
 }
 
-__global__ void __launch_bounds__(GP_THREADS) k_vis_chi2_batch(const VisChi2BatchArgs a)
+__global__ void __launch_bounds__(GP_THREADS, 5) k_vis_chi2_batch(const VisChi2BatchArgs a)
 {
     gp_pdl_enter();
     vis_chi2_batch_body(a, gp_vgrid_hw());
@@ -1698,12 +1761,13 @@ static int batch_blocks_per_trial(gpair_ctx *c)
     return g < 1 ? 1 : g;
 }
 
-static int batch_wave_blocks(const void *kernel, int nsm)
+// one wave of blocks of `kernel` in a grid of `rows` rows
+static int batch_wave_blocks(const void *kernel, int nsm, int rows)
 {
     int per_sm = 1;
     if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, GP_THREADS, 0) != cudaSuccess || per_sm < 1)
         per_sm = 1;
-    const int w = per_sm * nsm / GP_NTR;
+    const int w = per_sm * nsm / rows;
     return w < 1 ? 1 : w;
 }
 
@@ -1731,8 +1795,8 @@ int gp_batch_alloc(gpair_ctx *c)
     GP_CUDA(c, cudaMalloc(&c->partials_b, sizeof(double) * (size_t)GP_NTR * 1024 * 2));
     int nsm = 148;
     GP_CUDA(c, cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, c->device));
-    c->batch_wave[0] = batch_wave_blocks((const void *)k_trials_prep, nsm);
-    c->batch_wave[1] = batch_wave_blocks((const void *)k_vis_chi2_batch, nsm);
+    c->batch_wave[0] = batch_wave_blocks((const void *)k_trials_prep, nsm, GP_NTR);
+    c->batch_wave[1] = batch_wave_blocks((const void *)k_vis_chi2_batch, nsm, 1);
     return GPAIR_OK;
 }
 
@@ -1764,13 +1828,20 @@ int gp_trials_prep_launch(gpair_ctx *c)
 // partial entries are many; grouped launches pass 0
 static VisChi2BatchArgs batch_chi2_args(gpair_ctx *c, int epp, FusedCtrl fc, const int *gate, int presum = 0)
 {
-    int nb = gp_cdiv(c->npow + c->nbis, GP_THREADS * 2);
-    if (nb > c->batch_wave[1]) nb = c->batch_wave[1];  // one wave over the batch
+    // four data per eight lanes (24 instances in one launch: 265 us in 7 launches, 296 with two, 270 with eight), two
+    // while that leaves the blocks few (64^2: 10 us against 12); at most one wave. A grouped launch takes
+    // the same, so that its sums are the same.
+    const int items = c->npow + c->nbis, per = GP_THREADS / GP_NTR;
+    int nb = gp_cdiv(items, 4 * per);
+    if (nb < 32) nb = gp_cdiv(items, 2 * per) < 32 ? gp_cdiv(items, 2 * per) : 32;
+    if (nb > c->batch_wave[1]) nb = c->batch_wave[1];
     if (nb > 1024) nb = 1024;
     if (nb < 1) nb = 1;
     const double2 *vb = (c->ug || (presum && epp > VIS_PRESUM_ENTRIES && c->visb)) ? c->visb : nullptr;
-    VisChi2BatchArgs a = {c->vpart_b, epp, c->nuv, c->npow, c->nbis, c->data, c->data_err, c->tri, c->phasor,
-                          c->partials_b, c->sc, fc, gate, vb, nb, GP_NTR};
+    const bool tc = c->precision != GPAIR_PREC_FP32;
+    const TrialVis tv = {c->vpart_b, tc ? epp : (long long)epp * c->nuv, tc ? 1 : c->nuv, tc ? GP_NTR * epp : 1, epp};
+    VisChi2BatchArgs a = {tv, c->npow, c->nbis, c->data, c->data_err, c->tri, c->phasor, c->partials_b, c->sc, fc,
+                          gate, vb, nb, 1};
     return a;
 }
 
@@ -1778,10 +1849,10 @@ static int batch_chi2(gpair_ctx *c, int epp)
 {
     const VisChi2BatchArgs a = batch_chi2_args(c, epp, take_fused_ctrl(c), c->gate, 1);
     if (a.visb && !c->ug) {  // the grid's forward leaves the trials' V there
-        int nb = gp_cdiv(c->nuv, GP_THREADS);
-        if (nb > 148) nb = 148;  // 8 trials: about eight blocks per SM
-        GP_LAUNCH(c, gp_launch(c, k_vis_sum_batch, dim3(nb, GP_NTR), dim3(GP_THREADS), 0, (const float2 *)c->vpart_b,
-                               epp, c->nuv, (const DevScalars *)c->sc, c->visb, c->gate));
+        int nb = gp_cdiv(c->nuv, GP_THREADS / GP_NTR);
+        if (nb > 8 * 148) nb = 8 * 148;
+        GP_LAUNCH(c, gp_launch(c, k_vis_sum_batch, dim3(nb), dim3(GP_THREADS), 0, a.tv, c->nuv,
+                               (const DevScalars *)c->sc, c->visb, c->gate));
     }
     GP_LAUNCH(c, gp_launch(c, k_vis_chi2_batch, dim3(a.nbx, a.nby), dim3(GP_THREADS), 0, a));
     return GPAIR_OK;

@@ -162,7 +162,8 @@ struct TcArgs {
     // twiddle scale removed in the epilogue)
     int lpad, live, elog2;
     const float *rsc;
-    float2 *vpart;
+    float2 *vpart;  // entry e of uv point k at vpart[e es + k ks]
+    int es, ks;
     // store epilogue
     float *gpart;
     int out_ld, out_rows, out_cols;
@@ -192,6 +193,7 @@ struct __align__(64) TcGroupInst {
     int nanc, nuv, lpad, live, elog2;
     const float *rsc;
     float2 *vpart;
+    int es, ks;
     // store epilogue (adjoint): split-K partial images
     int kb_per_split;
     float *gpart;
@@ -371,7 +373,7 @@ __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_al
 // one unit of the forward epilogue, besides the accumulator, row scales and anchors
 struct EpiUnit {
     float2 *vpart;
-    int k, nuv, y0, lpad, live, elog2;
+    int k, nuv, y0, lpad, live, elog2, es, ks;
 };
 
 // Starts the copies of unit u: the row scales of the warp's columns into rsw, the
@@ -391,6 +393,8 @@ __device__ __forceinline__ void epi_fetch(const TcArgs &a, const int *gpre, int 
     e.lpad = a.lpad;
     e.live = a.live;
     e.elog2 = a.elog2;
+    e.es = a.es;
+    e.ks = a.ks;
     if (GROUP) {
         const TcGroupInst &gi = a.grp[ci];
         fya = gi.fya;
@@ -402,6 +406,8 @@ __device__ __forceinline__ void epi_fetch(const TcArgs &a, const int *gpre, int 
         e.lpad = gi.lpad;
         e.live = gi.live;
         e.elog2 = gi.elog2;
+        e.es = gi.es;
+        e.ks = gi.ks;
     }
     e.y0 = n * TC_BN;  // first image row of the columns
     const int k0 = (m * (PAIR ? 256 : 128) + row0) >> 1, k = k0 + (lane & 15);
@@ -828,7 +834,7 @@ __global__ void __launch_bounds__(tc_threads<EPI>(), 1)
                             const float ore = __shfl_xor_sync(0xffffffffu, re, 1);
                             const float oim = __shfl_xor_sync(0xffffffffu, im, 1);
                             if ((lane & 1) == 0 && vk)
-                                cur.vpart[(size_t)entry * cur.nuv + cur.k] = make_float2(re - oim, im + ore);
+                                cur.vpart[(size_t)entry * cur.es + (size_t)cur.k * cur.ks] = make_float2(re - oim, im + ore);
                         }
                     }
                 } else {
@@ -882,7 +888,7 @@ __global__ void __launch_bounds__(tc_threads<EPI>(), 1)
                     const float ore = __shfl_xor_sync(0xffffffffu, sre, 1);
                     const float oim = __shfl_xor_sync(0xffffffffu, sim, 1);
                     if ((lane & 1) == 0 && vk)
-                        cur.vpart[(size_t)entry * cur.nuv + cur.k] = make_float2(sre - oim, sim + ore);
+                        cur.vpart[(size_t)entry * cur.es + (size_t)cur.k * cur.ks] = make_float2(sre - oim, sim + ore);
                 }
             } else {
                 int m, n, nv, kb0, kb1, split;
@@ -2115,6 +2121,8 @@ int gp_tc_forward_gemm(gpair_ctx *c)
     a.elog2 = 7;
     a.rsc = t->rsc;
     a.vpart = c->vpart;
+    a.es = c->nuv;
+    a.ks = 1;
     if ((rc = tc_launch<EPI_FWD>(c, t, tc_fwd_maps(t, false), a))) return rc;
     c->mt = t->M_pad / TC_EPI_COLS;
     return GPAIR_OK;
@@ -2205,7 +2213,9 @@ int gp_tc_forward_batch_gemm(gpair_ctx *c)
     const int erows = t->Lb < TC_EPI_COLS ? t->Lb : TC_EPI_COLS;
     a.elog2 = erows == 32 ? 5 : erows == 64 ? 6 : 7;
     a.rsc = t->rscb;
-    a.vpart = c->vpart_b;
+    a.vpart = c->vpart_b;  // a uv point's entries side by side (VisChi2BatchArgs)
+    a.es = 1;
+    a.ks = GP_NTR * t->epp_b;
     return tc_launch<EPI_FWD>(c, t, tc_fwd_maps(t, true), a);
 }
 
@@ -2409,11 +2419,15 @@ static void tc_group_inst(gpair_ctx *c, TcState *t, int kind, TcGroupInst &g)
         g.elog2 = erows == 32 ? 5 : erows == 64 ? 6 : 7;
         g.rsc = t->rscb;
         g.vpart = c->vpart_b;
+        g.es = 1;
+        g.ks = GP_NTR * t->epp_b;
     } else {
         g.lpad = t->M_pad;  // one image, partial entries of TC_EPI_COLS rows
         g.elog2 = 7;
         g.rsc = t->rsc;
         g.vpart = c->vpart;
+        g.es = c->nuv;
+        g.ks = 1;
     }
 }
 

@@ -346,19 +346,31 @@ __global__ void __launch_bounds__(256) k_ug_x(const UgXArgs a)
         }
 }
 
+// four doubles in 16-byte halves of shared memory
+struct __align__(16) double4_a16 {
+    double x, y, z, w;
+};
+
 // ------------------------------------------------------ y contraction
 //
-// G[+-j][jx] of UGR_C columns jx and 32 rows j per block: lane = j, the eight
-// warps take every eighth folded image row h (pixels h and N-1-h), whose
-// folded T values (sum and difference of the two rows, partial sums added,
-// row scales removed) wait in shared memory. cos and sin serve +j and -j.
-// Bound by the L2 reads of the row twiddles (H x 32 x 8 B per block).
-#define UGR_H 256  // folded rows staged at once
+// G[+-j][jx] of C columns jx and 32 rows j per block: lane = j, the W warps take
+// every W-th folded image row h (pixels h and N-1-h), whose folded T values (sum and
+// difference of the two rows, partial sums added, row scales removed) wait in
+// shared memory, in FP64: converted where they are used they would be converted
+// by every warp, at a quarter of the FP64 rate. cos and sin serve +j and -j. Bound by
+// latency: T's partial sums (all loads of a row in flight), then the row twiddles
+// (H x 32 x 8 B per block). 1024^2, 60 x 119 grid points: 14.2 us (19.6 with
+// conversions, loads one by one and 8 warps), 8 trials 30.4 (49).
+template <int C> struct UgRowsGeo {
+    static constexpr int W = C == 1 ? 16 : 8;          // warps
+    static constexpr int HB = C == 1 ? 512 : 256;      // folded rows staged at once
+    static constexpr int BYTES = HB * C * 32 > W * 32 * C * 32 ? HB * C * 32 : W * 32 * C * 32;
+};
 struct UgRowsArgs {
     const float *T;  // image b: rows b lrows .. b lrows + N - 1
     const float *rsc;  // power-of-two factor of every row (tensor path), or null
     const float2 *ctab;
-    float2 *grid;  // image b at grid + b cells
+    float2 *grid;  // cell e at grid[e], of trial b of a batch at grid[GP_NTR e + b]
     int N, H, gw, J, ldT, cells, splits, lrows;  // gw: grid columns
     size_t split_stride;
     const int *gate;
@@ -368,63 +380,74 @@ struct UgRowsArgs {
 template <int C>
 __device__ __forceinline__ void ug_rows_body(const UgRowsArgs &A, const GpVGrid &vg)
 {
-    __shared__ __align__(16) float4 Ts[UGR_H * C];
-    __shared__ double red[8][32][C][4];
+    using G = UgRowsGeo<C>;
+    __shared__ __align__(16) unsigned char raw[G::BYTES];
+    double4_a16(*Ts)[C] = reinterpret_cast<double4_a16(*)[C]>(raw);          // [h][column]: sum, difference
+    double(*red)[32][C][4] = reinterpret_cast<double(*)[32][C][4]>(raw);     // [warp][j], once Ts has been used
     if (A.gate && !*A.gate) return;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int ctiles = (A.gw + C - 1) / C;
     const int c0 = (vg.bx % ctiles) * C, j = (vg.bx / ctiles) * 32 + lane;
     const int image = vg.by;
-    const int N = A.N, H = A.H, J1 = A.J + 1;
+    const int N = A.N, H = A.H, J1 = A.J + 1, splits = A.splits;
     const size_t row0 = (size_t)image * A.lrows;
     double acc[C][4];
 #pragma unroll
     for (int q = 0; q < C; q++)
 #pragma unroll
         for (int i = 0; i < 4; i++) acc[q][i] = 0.0;
-    for (int hb = 0; hb < H; hb += UGR_H) {
-        const int nh = min(UGR_H, H - hb);
-        for (int e = threadIdx.x; e < nh * C; e += blockDim.x) {
+    for (int hb = 0; hb < H; hb += G::HB) {
+        const int nh = min(G::HB, H - hb);
+        for (int e = threadIdx.x; e < nh * C; e += 32 * G::W) {
             const int h = hb + e / C, col = c0 + e % C;
             float2 p = make_float2(0.f, 0.f), m = make_float2(0.f, 0.f);
             if (col < A.gw) {
                 const size_t rp = row0 + (N - 1 - h), rm = row0 + h;
                 const bool two = rp != rm;
-                for (int s = 0; s < A.splits; s++) {
-                    const float *T = A.T + s * A.split_stride;
-                    const float2 a = __ldg(reinterpret_cast<const float2 *>(T + rp * A.ldT + 2 * col));
-                    p.x += a.x;
-                    p.y += a.y;
-                    if (two) {
-                        const float2 b = __ldg(reinterpret_cast<const float2 *>(T + rm * A.ldT + 2 * col));
-                        m.x += b.x;
-                        m.y += b.y;
-                    }
+                float2 a[UG_MAX_SPLITS], b[UG_MAX_SPLITS];
+#pragma unroll
+                for (int s = 0; s < UG_MAX_SPLITS; s++) {
+                    if (s >= splits) break;
+                    const float *T = A.T + s * A.split_stride + 2 * col;
+                    a[s] = __ldg(reinterpret_cast<const float2 *>(T + rp * A.ldT));
+                    b[s] = __ldg(reinterpret_cast<const float2 *>(T + rm * A.ldT));
                 }
-                if (A.rsc) {
-                    const float sp = __ldg(&A.rsc[rp]), sm = __ldg(&A.rsc[rm]);
-                    p.x *= sp;
-                    p.y *= sp;
-                    m.x *= sm;
-                    m.y *= sm;
+                const float sp = A.rsc ? __ldg(&A.rsc[rp]) : 1.f, sm = A.rsc ? __ldg(&A.rsc[rm]) : 1.f;
+#pragma unroll
+                for (int s = 0; s < UG_MAX_SPLITS; s++) {
+                    if (s >= splits) break;
+                    p.x += a[s].x;
+                    p.y += a[s].y;
+                    m.x += b[s].x;
+                    m.y += b[s].y;
                 }
+                p.x *= sp;
+                p.y *= sp;
+                m.x *= sm;
+                m.y *= sm;
+                if (!two) m = make_float2(0.f, 0.f);  // the middle row
             }
-            Ts[e] = make_float4(p.x + m.x, p.y + m.y, p.x - m.x, p.y - m.y);
+            double4_a16 t;
+            t.x = p.x + m.x;
+            t.y = p.y + m.y;
+            t.z = p.x - m.x;
+            t.w = p.y - m.y;
+            Ts[e / C][e % C] = t;
         }
         __syncthreads();
         if (j < J1) {
             const float2 *ct = A.ctab + (size_t)hb * J1 + j;
 #pragma unroll 8
-            for (int h = warp; h < nh; h += 8) {
+            for (int h = warp; h < nh; h += G::W) {
                 const float2 wf = __ldg(&ct[(size_t)h * J1]);
                 const double wc = wf.x, ws = wf.y;
 #pragma unroll
                 for (int q = 0; q < C; q++) {
-                    const float4 t = Ts[h * C + q];
-                    acc[q][0] = fma(wc, (double)t.x, acc[q][0]);
-                    acc[q][1] = fma(wc, (double)t.y, acc[q][1]);
-                    acc[q][2] = fma(ws, (double)t.z, acc[q][2]);
-                    acc[q][3] = fma(ws, (double)t.w, acc[q][3]);
+                    const double4_a16 t = Ts[h][q];
+                    acc[q][0] = fma(wc, t.x, acc[q][0]);
+                    acc[q][1] = fma(wc, t.y, acc[q][1]);
+                    acc[q][2] = fma(ws, t.z, acc[q][2]);
+                    acc[q][3] = fma(ws, t.w, acc[q][3]);
                 }
             }
         }
@@ -435,7 +458,7 @@ __device__ __forceinline__ void ug_rows_body(const UgRowsArgs &A, const GpVGrid 
 #pragma unroll
         for (int i = 0; i < 4; i++) red[warp][lane][q][i] = acc[q][i];
     __syncthreads();
-    for (int e = threadIdx.x; e < 32 * C; e += blockDim.x) {
+    for (int e = threadIdx.x; e < 32 * C; e += 32 * G::W) {
         const int l = e / C, q = e % C, jj = (vg.bx / ctiles) * 32 + l, col = c0 + q;
         if (jj >= J1 || col >= A.gw) continue;
         double t[4];
@@ -443,17 +466,18 @@ __device__ __forceinline__ void ug_rows_body(const UgRowsArgs &A, const GpVGrid 
         for (int i = 0; i < 4; i++) {
             t[i] = red[0][l][q][i];
 #pragma unroll
-            for (int w = 1; w < 8; w++) t[i] += red[w][l][q][i];
+            for (int w = 1; w < G::W; w++) t[i] += red[w][l][q][i];
         }
         // sum T e^{-+i theta} = (even . cos) -+ i (odd . sin)
-        float2 *g = A.grid + (size_t)image * A.cells + col;
-        g[(size_t)(A.J + jj) * A.gw] = make_float2((float)(t[0] + t[3]), (float)(t[1] - t[2]));
-        g[(size_t)(A.J - jj) * A.gw] = make_float2((float)(t[0] - t[3]), (float)(t[1] + t[2]));
+        const int st = vg.nby > 1 ? GP_NTR : 1;
+        float2 *g = A.grid + image + (size_t)col * st;
+        g[(size_t)(A.J + jj) * A.gw * st] = make_float2((float)(t[0] + t[3]), (float)(t[1] - t[2]));
+        g[(size_t)(A.J - jj) * A.gw * st] = make_float2((float)(t[0] - t[3]), (float)(t[1] + t[2]));
     }
 }
 
 template <int C>
-__global__ void __launch_bounds__(256) k_ug_rows(const UgRowsArgs a)
+__global__ void __launch_bounds__(32 * UgRowsGeo<C>::W) k_ug_rows(const UgRowsArgs a)
 {
     gp_pdl_enter();
     ug_rows_body<C>(a, gp_vgrid_hw());
@@ -467,8 +491,8 @@ template <int C> struct UgRowsOp {
 // ------------------------------------------------------- interpolation
 //
 // V_k / F of one sorted uv point per thread. The points of a warp share a grid
-// cell or lie in neighbouring ones, so the 64 grid loads are served by one or
-// two sectors each; the window weights stream (64 B per point).
+// cell or lie in neighbouring ones, so the 64 grid loads are served by one or two
+// sectors each; the window weights stream (64 B per point).
 #define UGI_THREADS 128
 struct UgInterpArgs {
     const float2 *grid;
@@ -476,22 +500,30 @@ struct UgInterpArgs {
     const float *wts;
     const float2 *phase;
     const DevScalars *sc;
-    double2 *out;  // [nuv], or [GP_NTR][nuv] (trials)
-    int nuv, gw, cells, trials;
+    double2 *out;  // [nuv], or [nuv][GP_NTR] (trials)
+    int nuv, gw, nchunk;
+    const int2 *chunk;
     const int *gate;
     GP_VGRID_FIELDS;
 };
 
+__device__ __forceinline__ double2 ug_vis_out(float re, float im, float2 ph, bool conj, double invF)
+{
+    const double vr = (double)re * ph.x - (double)im * ph.y;
+    const double vi = (double)re * ph.y + (double)im * ph.x;
+    return make_double2(vr * invF, (conj ? -vi : vi) * invF);
+}
+
 __device__ __forceinline__ void ug_interp_body(const UgInterpArgs &A, const GpVGrid &vg)
 {
     if (A.gate && !*A.gate) return;
-    const int p = vg.bx * blockDim.x + threadIdx.x, image = vg.by;
+    const int p = vg.bx * blockDim.x + threadIdx.x;
     if (p >= A.nuv) return;
     const float4 *w4 = reinterpret_cast<const float4 *>(A.wts + (size_t)p * (2 * UG_W));
     float w[2 * UG_W];
 #pragma unroll
     for (int i = 0; i < 4; i++) *reinterpret_cast<float4 *>(&w[4 * i]) = __ldg(&w4[i]);
-    const float2 *g = A.grid + (size_t)image * A.cells + __ldg(&A.base[p]);
+    const float2 *g = A.grid + __ldg(&A.base[p]);
     float re = 0.f, im = 0.f;
 #pragma unroll
     for (int i = 0; i < UG_W; i++) {
@@ -506,13 +538,88 @@ __device__ __forceinline__ void ug_interp_body(const UgInterpArgs &A, const GpVG
         re = fmaf(w[UG_W + i], rr, re);
         im = fmaf(w[UG_W + i], ri, im);
     }
-    const float2 ph = __ldg(&A.phase[p]);
     const int s = __ldg(&A.src[p]);
-    const double invF = A.trials ? A.sc->t_invflux[image] : A.sc->invflux;
-    const double vr = (double)re * ph.x - (double)im * ph.y;
-    const double vi = (double)re * ph.y + (double)im * ph.x;
-    A.out[(size_t)image * A.nuv + (s & 0x7fffffff)] = make_double2(vr * invF, (s < 0 ? -vi : vi) * invF);
+    A.out[s & 0x7fffffff] = ug_vis_out(re, im, __ldg(&A.phase[p]), s < 0, A.sc->invflux);
 }
+
+// The trials of a batch: one warp per run of at most 32 uv points of one grid cell
+// (the adjoint's runs), lane = (group of 8 of its points, trial). A lane reads each
+// of the cell's 64 grid values once for its 8 points (the 8 trials' values of a grid
+// point lie side by side) and keeps their x weights in registers, so the
+// multiply-adds bound it (1,152 a warp and run); with a thread per point and trial
+// the loads of the grid values did. The sums are those of ug_interp_body.
+// 194,560 points: 28 us against 46.
+__device__ __forceinline__ void ug_interp_trials_body(const UgInterpArgs &A, const GpVGrid &vg)
+{
+    __shared__ __align__(16) float ws[UGI_THREADS / 32][2 * UG_W][32];  // the run's weights, [weight][point]
+    if (A.gate && !*A.gate) return;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int ch = vg.bx * (UGI_THREADS / 32) + warp;
+    if (ch >= A.nchunk) return;  // warp-uniform
+    const int2 q = __ldg(&A.chunk[ch]);
+    {
+        float w[2 * UG_W];
+        const float4 *w4 = reinterpret_cast<const float4 *>(A.wts + (size_t)(q.x + lane) * (2 * UG_W));
+#pragma unroll
+        for (int i = 0; i < 4; i++)
+            *reinterpret_cast<float4 *>(&w[4 * i]) = lane < q.y ? __ldg(&w4[i]) : make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+        for (int i = 0; i < 2 * UG_W; i++) ws[warp][i][lane] = w[i];
+    }
+    __syncwarp();
+    const int trial = lane & 7, p0 = lane & 24;
+    float wx[UG_W][8];
+#pragma unroll
+    for (int j = 0; j < UG_W; j++) {
+        *reinterpret_cast<float4 *>(&wx[j][0]) = *reinterpret_cast<const float4 *>(&ws[warp][j][p0]);
+        *reinterpret_cast<float4 *>(&wx[j][4]) = *reinterpret_cast<const float4 *>(&ws[warp][j][p0 + 4]);
+    }
+    const float2 *g = A.grid + (size_t)__ldg(&A.base[q.x]) * GP_NTR + trial;
+    float re[8], im[8];
+#pragma unroll
+    for (int n = 0; n < 8; n++) re[n] = im[n] = 0.f;
+#pragma unroll 2
+    for (int i = 0; i < UG_W; i++) {
+        float2 v[UG_W];
+#pragma unroll
+        for (int j = 0; j < UG_W; j++) v[j] = __ldg(&g[j * GP_NTR]);
+        g += (size_t)A.gw * GP_NTR;
+        float wy[8];
+        *reinterpret_cast<float4 *>(&wy[0]) = *reinterpret_cast<const float4 *>(&ws[warp][UG_W + i][p0]);
+        *reinterpret_cast<float4 *>(&wy[4]) = *reinterpret_cast<const float4 *>(&ws[warp][UG_W + i][p0 + 4]);
+#pragma unroll
+        for (int n = 0; n < 8; n++) {
+            float rr = 0.f, ri = 0.f;
+#pragma unroll
+            for (int j = 0; j < UG_W; j++) {
+                rr = fmaf(wx[j][n], v[j].x, rr);
+                ri = fmaf(wx[j][n], v[j].y, ri);
+            }
+            re[n] = fmaf(wy[n], rr, re[n]);
+            im[n] = fmaf(wy[n], ri, im[n]);
+        }
+    }
+    const double invF = A.sc->t_invflux[trial];
+#pragma unroll
+    for (int n = 0; n < 8; n++) {
+        if (p0 + n < q.y) {
+            const int s = __ldg(&A.src[q.x + p0 + n]);
+            A.out[(size_t)(s & 0x7fffffff) * GP_NTR + trial] =
+                ug_vis_out(re[n], im[n], __ldg(&A.phase[q.x + p0 + n]), s < 0, invF);
+        }
+    }
+}
+
+__global__ void __launch_bounds__(UGI_THREADS) k_ug_interp_trials(const UgInterpArgs a)
+{
+    gp_pdl_enter();
+    ug_interp_trials_body(a, gp_vgrid_hw());
+}
+
+struct UgInterpTrialsOp {
+    using Args = UgInterpArgs;
+    static __device__ __forceinline__ void run(const Args &a, const GpVGrid &v) { ug_interp_trials_body(a, v); }
+};
 
 __global__ void __launch_bounds__(UGI_THREADS) k_ug_interp(const UgInterpArgs a)
 {
@@ -528,7 +635,11 @@ struct UgInterpOp {
 // ------------------------------------------------------------ spreading
 //
 // One warp per run of at most 32 uv points of one grid cell: their 8 x 8 patch
-// sum_k c_k wx wy, two patch points per lane, in point order.
+// sum_k c_k wx wy, two patch points per lane, in point order. The run's weights pass
+// through shared memory, loaded a point per lane: bound by the chain run -> point ->
+// weight c_k, not by a load per point. 1024^2: 13.4 us, 15 with the weights read
+// point by point.
+#define UGS_LD 20  // floats per point in shared memory: 16 weights, padded against bank conflicts
 struct UgSpreadArgs {
     const float2 *cw;
     const int *src;
@@ -542,12 +653,17 @@ struct UgSpreadArgs {
 
 __device__ __forceinline__ void ug_spread_body(const UgSpreadArgs &A, const GpVGrid &vg)
 {
-    const int lane = threadIdx.x & 31;
-    const int ch = vg.bx * (int)(blockDim.x >> 5) + (int)(threadIdx.x >> 5);
+    __shared__ __align__(16) float ws[8][32][UGS_LD];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int ch = vg.bx * 8 + warp;
     if (ch >= A.nchunk) return;  // warp-uniform
     const int2 q = __ldg(&A.chunk[ch]);
     float2 cv = make_float2(0.f, 0.f);
+    float4 w4[4];
     if (lane < q.y) {
+#pragma unroll
+        for (int n = 0; n < 4; n++)
+            w4[n] = __ldg(reinterpret_cast<const float4 *>(A.wts + (size_t)(q.x + lane) * (2 * UG_W)) + n);
         // c_k e^{2 pi i (a - b)(N-1)/2}; a conjugated point contributes conj(c_k) (only the real part of the image is kept)
         const int s = __ldg(&A.src[q.x + lane]);
         float2 c = __ldg(&A.cw[s & 0x7fffffff]);
@@ -555,19 +671,23 @@ __device__ __forceinline__ void ug_spread_body(const UgSpreadArgs &A, const GpVG
         const float2 ph = __ldg(&A.phase[q.x + lane]);
         cv = make_float2(c.x * ph.x - c.y * ph.y, c.x * ph.y + c.y * ph.x);
     }
-    const float *w = A.wts + (size_t)q.x * (2 * UG_W);
+#pragma unroll
+    for (int n = 0; n < 4; n++)
+        if (lane < q.y) *reinterpret_cast<float4 *>(&ws[warp][lane][4 * n]) = w4[n];
+    __syncwarp();
+    const float *w = ws[warp][0];
     const int i = lane >> 3, j = lane & 7;
     float2 a0 = make_float2(0.f, 0.f), a1 = make_float2(0.f, 0.f);
 #pragma unroll 4
     for (int n = 0; n < q.y; n++) {
         const float cx = __shfl_sync(0xffffffffu, cv.x, n), cy = __shfl_sync(0xffffffffu, cv.y, n);
-        const float wx = __ldg(&w[j]);
-        const float f0 = wx * __ldg(&w[UG_W + i]), f1 = wx * __ldg(&w[UG_W + 4 + i]);
+        const float wx = w[j];
+        const float f0 = wx * w[UG_W + i], f1 = wx * w[UG_W + 4 + i];
         a0.x = fmaf(f0, cx, a0.x);
         a0.y = fmaf(f0, cy, a0.y);
         a1.x = fmaf(f1, cx, a1.x);
         a1.y = fmaf(f1, cy, a1.y);
-        w += 2 * UG_W;
+        w += UGS_LD;
     }
     float2 *out = A.patch + (size_t)ch * (UG_W * UG_W);
     out[lane] = a0;
@@ -585,8 +705,10 @@ struct UgSpreadOp {
     static __device__ __forceinline__ void run(const Args &a, const GpVGrid &v) { ug_spread_body(a, v); }
 };
 
-// Grid point (jy, jx) = the patches of the cells (jy - i, jx - j) at (i, j): eight
-// threads per grid point (one per i), FP64, cells and runs in order.
+// Grid point (jy, jx) = the patches of the cells (jy - i, jx - j) at (i, j): one
+// warp per grid point, lane = (i, j mod 4), two cells a lane, FP64, in a fixed order. Few
+// loads, so bound by the longest chain of them: a cell of a dense coverage has dozens of
+// runs. 1024^2: 9.3 us, 20 with eight threads a grid point and eight cells each.
 struct UgGatherArgs {
     const int *cst;
     const float2 *patch;
@@ -597,32 +719,39 @@ struct UgGatherArgs {
 
 __device__ __forceinline__ void ug_gather_body(const UgGatherArgs &A, const GpVGrid &vg)
 {
-    const int t = vg.bx * (int)blockDim.x + (int)threadIdx.x;
-    const int q = t >> 3, i = t & 7;
+    const int q = (vg.bx * (int)blockDim.x + (int)threadIdx.x) >> 5, lane = threadIdx.x & 31;
+    if (q >= A.cells) return;  // warp-uniform
+    const int i = lane >> 2, jy = q / A.gw - i, jx = q % A.gw;
     double re = 0.0, im = 0.0;
-    if (q < A.cells) {
-        const int jy = q / A.gw - i, jx = q % A.gw;
-        if (jy >= 0) {
+    int st[2], end[2];  // runs of its two cells
 #pragma unroll
-            for (int j = 0; j < UG_W; j++) {
-                if (jx - j >= 0) {
-                    const int cell = jy * A.gw + jx - j;
-                    const int e = __ldg(&A.cst[cell + 1]);
-                    for (int s = __ldg(&A.cst[cell]); s < e; s++) {
-                        const float2 v = __ldg(&A.patch[(size_t)s * (UG_W * UG_W) + i * UG_W + j]);
-                        re += v.x;
-                        im += v.y;
-                    }
-                }
+    for (int n = 0; n < 2; n++) {
+        const int j = (lane & 3) + 4 * n;
+        const bool ok = jy >= 0 && jx >= j;
+        st[n] = ok ? __ldg(&A.cst[jy * A.gw + jx - j]) : 0;
+        end[n] = ok ? __ldg(&A.cst[jy * A.gw + jx - j + 1]) : 0;
+    }
+#pragma unroll
+    for (int n = 0; n < 2; n++) {
+        const float2 *p = A.patch + i * UG_W + (lane & 3) + 4 * n;
+        for (int s = st[n]; s < end[n]; s += 8) {
+            float2 v[8];  // eight loads in flight
+#pragma unroll
+            for (int m = 0; m < 8; m++)
+                v[m] = s + m < end[n] ? __ldg(&p[(size_t)(s + m) * (UG_W * UG_W)]) : make_float2(0.f, 0.f);
+#pragma unroll
+            for (int m = 0; m < 8; m++) {
+                re += v[m].x;
+                im += v[m].y;
             }
         }
     }
 #pragma unroll
-    for (int o = 4; o > 0; o >>= 1) {
-        re += __shfl_down_sync(0xffffffffu, re, o, 8);
-        im += __shfl_down_sync(0xffffffffu, im, o, 8);
+    for (int o = 16; o > 0; o >>= 1) {
+        re += __shfl_down_sync(0xffffffffu, re, o);
+        im += __shfl_down_sync(0xffffffffu, im, o);
     }
-    if (i == 0 && q < A.cells) A.cgrid[q] = make_float2((float)re, (float)im);
+    if (lane == 0) A.cgrid[q] = make_float2((float)re, (float)im);
 }
 
 __global__ void __launch_bounds__(256) k_ug_gather(const UgGatherArgs a)
@@ -638,11 +767,12 @@ struct UgGatherOp {
 
 // ------------------------------------------------- adjoint y contraction
 //
-// S[y][jx] for 32 columns (lane = jx) and 8 UGC_H folded image rows per block
-// (a warp takes UGC_H of them, image rows h and N-1-h). The sums and
-// differences of the grid rows +-j wait in shared memory.
-#define UGC_H 2
-#define UGC_J 64
+// S[y][jx] for 32 columns (lane = jx) and 8 folded image rows per block (a warp
+// takes one, image rows h and N-1-h). The sums and differences of the grid rows +-j and
+// the twiddles wait in shared memory in FP64 (converted once, not by every warp); the
+// next UGC_J rows are loaded meanwhile. Bound by latency. 1024^2: 10.4 us (14.6 with
+// two rows a warp, 64 blocks, and conversions where they are used).
+#define UGC_J 32
 struct UgColsArgs {
     const float2 *cgrid, *ctab;
     float2 *S;
@@ -652,59 +782,55 @@ struct UgColsArgs {
 
 __device__ __forceinline__ void ug_cols_body(const UgColsArgs &A, const GpVGrid &vg)
 {
-    __shared__ __align__(16) float4 Cs[UGC_J][32];  // (sum, difference)
-    __shared__ float2 Ws[8 * UGC_H][UGC_J];
+    __shared__ __align__(16) double4_a16 Cs[UGC_J][32];  // (sum, difference)
+    __shared__ __align__(16) double2 Ws[8][UGC_J];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int xt = (A.gw + 31) / 32;
-    const int jx = (vg.bx % xt) * 32 + lane, hb = (vg.bx / xt) * 8 * UGC_H;
+    const int jx = (vg.bx % xt) * 32 + lane, h = (vg.bx / xt) * 8 + warp;
     const int J1 = A.J + 1;
-    double acc[UGC_H][4];  // even (re, im), odd (re, im)
+    float2 p[UGC_J / 8], m[UGC_J / 8], w;  // the next UGC_J rows: +-j = warp, warp + 8, ..; twiddle of row h
+    auto load = [&](int jb) {
 #pragma unroll
-    for (int r = 0; r < UGC_H; r++)
-#pragma unroll
-        for (int i = 0; i < 4; i++) acc[r][i] = 0.0;
+        for (int n = 0; n < UGC_J / 8; n++) {
+            const int j = jb + warp + 8 * n;
+            const bool ok = j < J1 && jx < A.gw;
+            p[n] = ok ? __ldg(&A.cgrid[(size_t)(A.J + j) * A.gw + jx]) : make_float2(0.f, 0.f);
+            m[n] = ok && j ? __ldg(&A.cgrid[(size_t)(A.J - j) * A.gw + jx]) : make_float2(0.f, 0.f);
+        }
+        w = h < A.H && jb + lane < J1 ? __ldg(&A.ctab[(size_t)h * J1 + jb + lane]) : make_float2(0.f, 0.f);
+    };
+    double acc[4] = {0.0, 0.0, 0.0, 0.0};  // even (re, im), odd (re, im)
+    load(0);
     for (int jb = 0; jb < J1; jb += UGC_J) {
         const int nj = min(UGC_J, J1 - jb);
-        for (int jj = warp; jj < nj; jj += 8) {
-            const int j = jb + jj;
-            float2 p = make_float2(0.f, 0.f), m = make_float2(0.f, 0.f);
-            if (jx < A.gw) {
-                p = __ldg(&A.cgrid[(size_t)(A.J + j) * A.gw + jx]);
-                if (j) m = __ldg(&A.cgrid[(size_t)(A.J - j) * A.gw + jx]);
-            }
-            Cs[jj][lane] = make_float4(p.x + m.x, p.y + m.y, p.x - m.x, p.y - m.y);
+#pragma unroll
+        for (int n = 0; n < UGC_J / 8; n++) {
+            double4_a16 t;
+            t.x = p[n].x + m[n].x;
+            t.y = p[n].y + m[n].y;
+            t.z = p[n].x - m[n].x;
+            t.w = p[n].y - m[n].y;
+            Cs[warp + 8 * n][lane] = t;
         }
-        for (int e = threadIdx.x; e < 8 * UGC_H * UGC_J; e += blockDim.x) {
-            const int r = e / UGC_J, jj = e % UGC_J, h = hb + r;
-            if (jj < nj) Ws[r][jj] = h < A.H ? __ldg(&A.ctab[(size_t)h * J1 + jb + jj]) : make_float2(0.f, 0.f);
-        }
+        Ws[warp][lane] = make_double2(w.x, w.y);
         __syncthreads();
-#pragma unroll 4
+        if (jb + UGC_J < J1) load(jb + UGC_J);
+#pragma unroll 8
         for (int jj = 0; jj < nj; jj++) {
-            const float4 v = Cs[jj][lane];
-#pragma unroll
-            for (int r = 0; r < UGC_H; r++) {
-                const float2 w = Ws[warp * UGC_H + r][jj];
-                acc[r][0] = fma((double)w.x, (double)v.x, acc[r][0]);
-                acc[r][1] = fma((double)w.x, (double)v.y, acc[r][1]);
-                acc[r][2] = fma((double)w.y, (double)v.z, acc[r][2]);
-                acc[r][3] = fma((double)w.y, (double)v.w, acc[r][3]);
-            }
+            const double4_a16 v = Cs[jj][lane];
+            const double2 c = Ws[warp][jj];
+            acc[0] = fma(c.x, v.x, acc[0]);
+            acc[1] = fma(c.x, v.y, acc[1]);
+            acc[2] = fma(c.y, v.z, acc[2]);
+            acc[3] = fma(c.y, v.w, acc[3]);
         }
         __syncthreads();
     }
-    if (jx >= A.gw) return;
-#pragma unroll
-    for (int r = 0; r < UGC_H; r++) {
-        const int h = hb + warp * UGC_H + r;
-        if (h >= A.H) continue;
-        // C[j] e^{-i theta} + C[-j] e^{i theta} = sum . cos - i difference . sin, theta -> -theta at row h
-        A.S[(size_t)(A.N - 1 - h) * A.gw + jx] = 
-            make_float2((float)(acc[r][0] + acc[r][3]), (float)(acc[r][1] - acc[r][2]));
-        if (h != A.N - 1 - h)
-            A.S[(size_t)h * A.gw + jx] =
-                make_float2((float)(acc[r][0] - acc[r][3]), (float)(acc[r][1] + acc[r][2]));
-    }
+    if (jx >= A.gw || h >= A.H) return;
+    // C[j] e^{-i theta} + C[-j] e^{i theta} = sum . cos - i difference . sin, theta -> -theta at row h
+    A.S[(size_t)(A.N - 1 - h) * A.gw + jx] = make_float2((float)(acc[0] + acc[3]), (float)(acc[1] - acc[2]));
+    if (h != A.N - 1 - h)
+        A.S[(size_t)h * A.gw + jx] = make_float2((float)(acc[0] - acc[3]), (float)(acc[1] + acc[2]));
 }
 
 __global__ void __launch_bounds__(256) k_ug_cols(const UgColsArgs a)
@@ -799,11 +925,11 @@ static UgInterpArgs ug_interp_args(gpair_ctx *c, int images, const int *gate)
     a.out = images > 1 ? c->visb : c->visd;
     a.nuv = c->nuv;
     a.gw = g->nbx;
-    a.cells = g->cells;
-    a.trials = images > 1;
+    a.chunk = g->chunk;
+    a.nchunk = g->nchunk;
     a.gate = gate;
-    a.nbx = gp_cdiv(c->nuv, UGI_THREADS);
-    a.nby = images;
+    a.nbx = images > 1 ? gp_cdiv(g->nchunk, UGI_THREADS / 32) : gp_cdiv(c->nuv, UGI_THREADS);
+    a.nby = 1;
     return a;
 }
 
@@ -817,7 +943,7 @@ static UgSpreadArgs ug_spread_args(gpair_ctx *c)
 static UgGatherArgs ug_gather_args(gpair_ctx *c)
 {
     UgState *g = (UgState *)c->ug;
-    UgGatherArgs a = {g->cst, g->patch, g->cgrid, g->nbx, g->cells, gp_cdiv(8LL * g->cells, 256), 1};
+    UgGatherArgs a = {g->cst, g->patch, g->cgrid, g->nbx, g->cells, gp_cdiv(32LL * g->cells, 256), 1};
     return a;
 }
 
@@ -825,7 +951,7 @@ static UgColsArgs ug_cols_args(gpair_ctx *c)
 {
     UgState *g = (UgState *)c->ug;
     UgColsArgs a = {g->cgrid, g->ctab, g->S, g->N, g->H, g->nbx, g->J,
-                    gp_cdiv(g->nbx, 32) * gp_cdiv(g->H, 8 * UGC_H), 1};
+                    gp_cdiv(g->nbx, 32) * gp_cdiv(g->H, 8), 1};
     return a;
 }
 
@@ -841,10 +967,12 @@ int gp_ug_vis(gpair_ctx *c, int images)
     }
     const int *gate = images > 1 ? c->gate : nullptr;
     const UgRowsArgs r = ug_rows_args(c, images, splits, rsc, lrows, gate);
-    GP_LAUNCH(c, gp_launch(c, images > 1 ? k_ug_rows<UGR_COLS_BATCH> : k_ug_rows<1>, dim3(r.nbx, r.nby), dim3(256), 0,
+    GP_LAUNCH(c, gp_launch(c, images > 1 ? k_ug_rows<UGR_COLS_BATCH> : k_ug_rows<1>, dim3(r.nbx, r.nby),
+                           dim3(32 * (images > 1 ? UgRowsGeo<UGR_COLS_BATCH>::W : UgRowsGeo<1>::W)), 0,
                            r));
     const UgInterpArgs t = ug_interp_args(c, images, gate);
-    GP_LAUNCH(c, gp_launch(c, k_ug_interp, dim3(t.nbx, t.nby), dim3(UGI_THREADS), 0, t));
+    GP_LAUNCH(c, gp_launch(c, images > 1 ? k_ug_interp_trials : k_ug_interp, dim3(t.nbx, t.nby), dim3(UGI_THREADS), 0,
+                           t));
     return GPAIR_OK;
 }
 
@@ -917,10 +1045,12 @@ int gp_ug_stage_group_launch(gpair_ctx *c, int stage, const void *d_args, const 
 {
     if (total < 1 || n < 1) return GPAIR_ERR_INVALID;
     switch (stage) {
-    case GS_UG_ROWS: return group_launch<UgRowsOp<1>, 256>(c, d_args, d_start, n, total, gate);
-    case GS_UG_ROWS_T: return group_launch<UgRowsOp<UGR_COLS_BATCH>, 256>(c, d_args, d_start, n, total, gate);
-    case GS_UG_INTERP:
-    case GS_UG_INTERP_T: return group_launch<UgInterpOp, UGI_THREADS>(c, d_args, d_start, n, total, gate);
+    case GS_UG_ROWS: return group_launch<UgRowsOp<1>, 32 * UgRowsGeo<1>::W>(c, d_args, d_start, n, total, gate);
+    case GS_UG_ROWS_T:
+        return group_launch<UgRowsOp<UGR_COLS_BATCH>, 32 * UgRowsGeo<UGR_COLS_BATCH>::W>(c, d_args, d_start, n, total,
+                                                                                         gate);
+    case GS_UG_INTERP: return group_launch<UgInterpOp, UGI_THREADS>(c, d_args, d_start, n, total, gate);
+    case GS_UG_INTERP_T: return group_launch<UgInterpTrialsOp, UGI_THREADS>(c, d_args, d_start, n, total, gate);
     case GS_UG_SPREAD: return group_launch<UgSpreadOp, 256>(c, d_args, d_start, n, total, gate);
     case GS_UG_GATHER: return group_launch<UgGatherOp, 256>(c, d_args, d_start, n, total, gate);
     case GS_UG_COLS: return group_launch<UgColsOp, 256>(c, d_args, d_start, n, total, gate);

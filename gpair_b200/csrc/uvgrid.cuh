@@ -44,6 +44,6 @@ struct UgState {
     float2 *S;           // [N][nbx]
     // batched trials
     float *Tb;           // [splits][GP_NTR rows per image][ldT]
-    float2 *gridb;       // [GP_NTR][cells]
+    float2 *gridb;       // [cells][GP_NTR]
     int splits, splitsb; // partial sums of the last CUDA-core x contraction
 };
