@@ -138,6 +138,7 @@ __global__ void __launch_bounds__(GP_THREADS) k_prep(const float *__restrict__ s
                                                      double minval, double *__restrict__ partials,
                                                      DevScalars *__restrict__ sc, int reset)
 {
+    gp_pdl_enter();
     __shared__ double smem[2 * 32];
     double s = step_from_state ? sc->cg.s : step;
     if (step_from_state) minval = sc->cg.minvalue;
@@ -187,91 +188,134 @@ __global__ void __launch_bounds__(GP_THREADS) k_prep(const float *__restrict__ s
     }
 }
 
-static int red_grid(long long n) { int g = gp_cdiv(n, GP_THREADS * 4); return g < 1 ? 1 : (g > 1184 ? 1184 : g); }
+// Blocks of a pass over n pixels that ends in a sum: a pixel per thread until every SM has a block (64^2 in 16
+// blocks: the FP64 logarithms of four pixels in one thread took as long as the rest of the kernel), then up to
+// four, for a short sum over the blocks
+static int red_grid(long long n)
+{
+    int g = gp_cdiv(n, GP_THREADS * 4), one = gp_cdiv(n, GP_THREADS);
+    if (one > 148) one = 148;
+    if (g < one) g = one;
+    return g < 1 ? 1 : (g > 1184 ? 1184 : g);
+}
 
 int gp_prep_image(gpair_ctx *c, int which, int trial_mode, double step_host, int step_from_state)
 {
     const float *src = (which == GPAIR_IMG_TEMP && !trial_mode) ? c->image_temp : c->image;
     const int g = red_grid(c->npix);  // one wave, several pixels per thread: a short reduction tail
-    k_prep<<<g, GP_THREADS, 0, c->stream>>>(src, c->descent_dir, c->image_temp, c->model, c->npix, trial_mode,
-                                            step_host, step_from_state, (double)1e-8, slot_partials(c, RED_PREP),
-                                            c->sc, c->direct_result);
-    GP_LAUNCH_CHECK(c);
+    GP_LAUNCH(c, gp_launch(c, k_prep, dim3(g), dim3(GP_THREADS), 0, src, (const float *)c->descent_dir, c->image_temp,
+                           (const float *)c->model, c->npix, trial_mode, step_host, step_from_state, (double)1e-8,
+                           slot_partials(c, RED_PREP), c->sc, c->direct_result));
     return GPAIR_OK;
 }
 
 // ----------------------------------------------------- forward, CUDA cores
 
+// V of KT uv points over FB_M image rows per block: T[y][k] = sum_x I[y][x] Fx[k][x]
+// in shared-memory tiles of FB_X pixels (the next tile's loads in flight), then
+// the sum over y against Fy. A problem of this path is small (the uv grid takes the
+// others), so a block's latency bounds it: narrow tiles where wide ones would leave
+// SMs without a block. 64^2, 900 points: 29 blocks of 32 points, loads and
+// products in turn 11.0 us with its launch; 57 of 16, prefetched 8.8.
 #define FB_M 64
-#define FB_K 32
 #define FB_X 32
 
+template <int KT>
 __global__ void __launch_bounds__(256) k_fwd_simt(const float *__restrict__ img, const float2 *__restrict__ fx,
                                                   const float2 *__restrict__ fy, int N, int nuv,
                                                   float2 *__restrict__ vpart, const int *__restrict__ gate)
 {
+    constexpr int Q = KT / 16;  // uv points per thread
+    gp_pdl_enter();
     if (gate && !*gate) return;  // lockstep batches: this instance's line search is over
     __shared__ float As[FB_X][FB_M + 1];
-    __shared__ float2 Bs[FB_X][FB_K + 1];
-    __shared__ float2 red[16][FB_K + 1];
+    __shared__ float2 Bs[FB_X][KT + 1];
+    __shared__ float2 red[16][KT + 1];
     const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
-    const int k0 = blockIdx.x * FB_K, y0 = blockIdx.y * FB_M;
+    const int k0 = blockIdx.x * KT, y0 = blockIdx.y * FB_M;
     // batched trials: image z of a stack, partials of image z after those of images < z
     img += (size_t)blockIdx.z * N * N;
     vpart += (size_t)blockIdx.z * gridDim.y * nuv;
-    float2 acc[4][2];
+    float2 acc[4][Q], f[4][Q];
 #pragma unroll
-    for (int r = 0; r < 4; r++) acc[r][0] = acc[r][1] = make_float2(0.f, 0.f);
-    for (int x0 = 0; x0 < N; x0 += FB_X) {
+    for (int r = 0; r < 4; r++)
+#pragma unroll
+        for (int j = 0; j < Q; j++) {
+            const int k = k0 + tx * Q + j, y = y0 + ty * 4 + r;
+            acc[r][j] = make_float2(0.f, 0.f);
+            f[r][j] = k < nuv && y < N ? __ldg(&fy[(size_t)k * N + y]) : make_float2(0.f, 0.f);
+        }
+    const int cx = tid & 31, rw = tid >> 5;
+    float an[8];
+    float2 bn[KT / 8];
+    auto load = [&](int x) {
 #pragma unroll
         for (int i = 0; i < 8; i++) {
-            int r = (tid >> 5) + 8 * i, cx = tid & 31, y = y0 + r, x = x0 + cx;
-            As[cx][r] = (y < N && x < N) ? img[(size_t)y * N + x] : 0.f;
+            const int y = y0 + rw + 8 * i;
+            an[i] = (y < N && x < N) ? img[(size_t)y * N + x] : 0.f;
         }
 #pragma unroll
-        for (int i = 0; i < 4; i++) {
-            int kk = (tid >> 5) + 8 * i, cx = tid & 31, k = k0 + kk, x = x0 + cx;
-            Bs[cx][kk] = (k < nuv && x < N) ? fx[(size_t)k * N + x] : make_float2(0.f, 0.f);
+        for (int i = 0; i < KT / 8; i++) {
+            const int k = k0 + rw + 8 * i;
+            bn[i] = (k < nuv && x < N) ? __ldg(&fx[(size_t)k * N + x]) : make_float2(0.f, 0.f);
         }
+    };
+    load(cx);
+    for (int x0 = 0; x0 < N; x0 += FB_X) {
+#pragma unroll
+        for (int i = 0; i < 8; i++) As[cx][rw + 8 * i] = an[i];
+#pragma unroll
+        for (int i = 0; i < KT / 8; i++) Bs[cx][rw + 8 * i] = bn[i];
         __syncthreads();
+        if (x0 + FB_X < N) load(x0 + FB_X + cx);
 #pragma unroll 8
-        for (int cx = 0; cx < FB_X; cx++) {
-            float2 b0 = Bs[cx][tx * 2], b1 = Bs[cx][tx * 2 + 1];
+        for (int xx = 0; xx < FB_X; xx++) {
+            float2 b[Q];
+#pragma unroll
+            for (int j = 0; j < Q; j++) b[j] = Bs[xx][tx * Q + j];
 #pragma unroll
             for (int r = 0; r < 4; r++) {
-                float a = As[cx][ty * 4 + r];
-                acc[r][0].x = fmaf(a, b0.x, acc[r][0].x);
-                acc[r][0].y = fmaf(a, b0.y, acc[r][0].y);
-                acc[r][1].x = fmaf(a, b1.x, acc[r][1].x);
-                acc[r][1].y = fmaf(a, b1.y, acc[r][1].y);
-            }
-        }
-        __syncthreads();
-    }
+                const float a = As[xx][ty * 4 + r];
 #pragma unroll
-    for (int j = 0; j < 2; j++) {
-        int k = k0 + tx * 2 + j;
-        float2 part = make_float2(0.f, 0.f);
-        if (k < nuv) {
-#pragma unroll
-            for (int r = 0; r < 4; r++) {
-                int y = y0 + ty * 4 + r;
-                if (y < N) {
-                    float2 f = fy[(size_t)k * N + y];
-                    part.x += acc[r][j].x * f.x - acc[r][j].y * f.y;
-                    part.y += acc[r][j].x * f.y + acc[r][j].y * f.x;
+                for (int j = 0; j < Q; j++) {
+                    acc[r][j].x = fmaf(a, b[j].x, acc[r][j].x);
+                    acc[r][j].y = fmaf(a, b[j].y, acc[r][j].y);
                 }
             }
         }
-        red[ty][tx * 2 + j] = part;
+        __syncthreads();
+    }
+#pragma unroll
+    for (int j = 0; j < Q; j++) {
+        float2 part = make_float2(0.f, 0.f);
+#pragma unroll
+        for (int r = 0; r < 4; r++) {
+            if (k0 + tx * Q + j < nuv && y0 + ty * 4 + r < N) {
+                part.x += acc[r][j].x * f[r][j].x - acc[r][j].y * f[r][j].y;
+                part.y += acc[r][j].x * f[r][j].y + acc[r][j].y * f[r][j].x;
+            }
+        }
+        red[ty][tx * Q + j] = part;
     }
     __syncthreads();
-    if (tid < FB_K) {
+    if (tid < KT) {
         float2 s = make_float2(0.f, 0.f);
+#pragma unroll
         for (int r = 0; r < 16; r++) { s.x += red[r][tid].x; s.y += red[r][tid].y; }
         int k = k0 + tid;
         if (k < nuv) vpart[(size_t)blockIdx.y * nuv + k] = s;
     }
+}
+
+// `images` images (a stack from img): tiles of 16 uv points while those of 32 leave SMs without a block
+static int fwd_simt(gpair_ctx *c, const float *img, float2 *vpart, int images, const int *gate)
+{
+    const int mt = gp_cdiv(c->N, FB_M);
+    const bool narrow = gp_cdiv(c->nuv, 32) * mt * images < 148;
+    GP_LAUNCH(c, gp_launch(c, narrow ? k_fwd_simt<16> : k_fwd_simt<32>,
+                           dim3(gp_cdiv(c->nuv, narrow ? 16 : 32), mt, images), dim3(256), 0, img,
+                           (const float2 *)c->fx, (const float2 *)c->fy, c->N, c->nuv, vpart, gate));
+    return GPAIR_OK;
 }
 
 int gp_forward(gpair_ctx *c, int which)
@@ -287,10 +331,7 @@ int gp_forward(gpair_ctx *c, int which)
         return rc ? rc : gp_ug_vis(c, 1);
     }
     c->mt = gp_cdiv(c->N, FB_M);
-    dim3 grid(gp_cdiv(c->nuv, FB_K), c->mt);
-    k_fwd_simt<<<grid, 256, 0, c->stream>>>(img, c->fx, c->fy, c->N, c->nuv, c->vpart, nullptr);
-    GP_LAUNCH_CHECK(c);
-    return GPAIR_OK;
+    return fwd_simt(c, img, c->vpart, 1, nullptr);
 }
 
 // ------------------------------------------------- V2, T3, chi2, weights
@@ -592,72 +633,89 @@ static AdjWeightsArgs adj_weights_args(gpair_ctx *c)
 
 // ----------------------------------------------------- adjoint, CUDA cores
 
-#define AB_M 64
-#define AB_N 64
+// Partial image of one split of the uv points over a tile of 16 R x 16 R pixels per
+// block, AB_K uv points at a time (the next ones' loads in flight). Bound by a
+// block's latency, as the forward: tiles of 32 pixels where those of 64 leave SMs
+// without a block (at least 32 uv points each). 64^2, 900 points: 15 blocks of 64
+// pixels, loads and products in turn 15.7 us with its launch; 60 of 32, prefetched 8.8.
+#define AB_M 64  // widest tile
 #define AB_K 16  // complex uv per k-step
 
+template <int R>
 __global__ void __launch_bounds__(256) k_adj_simt(const float2 *__restrict__ fx, const float2 *__restrict__ fy,
                                                   const float2 *__restrict__ cw, int N, int nuv, int kchunk,
                                                   float *__restrict__ gpart)
 {
-    __shared__ float As[2 * AB_K][AB_M + 4];
-    __shared__ float Bs[2 * AB_K][AB_N + 4];
+    constexpr int T = 16 * R, NL = AB_K * T / 256;  // uv points loaded per thread
+    gp_pdl_enter();
+    __shared__ __align__(16) float As[2 * AB_K][T + 4];
+    __shared__ __align__(16) float Bs[2 * AB_K][T + 4];
     const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
-    const int x0 = blockIdx.x * AB_N, y0 = blockIdx.y * AB_M;
+    const int x0 = blockIdx.x * T, y0 = blockIdx.y * T;
     const int kb = blockIdx.z * kchunk, ke = min(nuv, kb + kchunk);
-    float acc[4][4];
+    const int cc = tid % T, y = y0 + cc, x = x0 + cc;
+    float2 wn[NL], fyn[NL], fxn[NL];
+    auto load = [&](int k0) {
 #pragma unroll
-    for (int i = 0; i < 4; i++)
+        for (int i = 0; i < NL; i++) {
+            const int k = k0 + tid / T + (256 / T) * i;
+            const bool ok = k < ke;
+            wn[i] = ok ? __ldg(&cw[k]) : make_float2(0.f, 0.f);
+            fyn[i] = ok && y < N ? __ldg(&fy[(size_t)k * N + y]) : make_float2(0.f, 0.f);
+            fxn[i] = ok && x < N ? __ldg(&fx[(size_t)k * N + x]) : make_float2(0.f, 0.f);
+        }
+    };
+    float acc[R][R];
 #pragma unroll
-        for (int j = 0; j < 4; j++) acc[i][j] = 0.f;
+    for (int i = 0; i < R; i++)
+#pragma unroll
+        for (int j = 0; j < R; j++) acc[i][j] = 0.f;
+    load(kb);
     for (int k0 = kb; k0 < ke; k0 += AB_K) {
 #pragma unroll
-        for (int i = 0; i < 4; i++) {
-            int kk = (tid >> 6) + 4 * i, cc = tid & 63, k = k0 + kk;
-            float2 wa = make_float2(0.f, 0.f), fb = make_float2(0.f, 0.f);
-            if (k < ke) {
-                int y = y0 + cc, x = x0 + cc;
-                float2 cwk = cw[k];
-                if (y < N) {
-                    float2 f = fy[(size_t)k * N + y];
-                    wa = make_float2(cwk.x * f.x - cwk.y * f.y, cwk.x * f.y + cwk.y * f.x);
-                }
-                if (x < N) fb = fx[(size_t)k * N + x];
-            }
-            As[2 * kk][cc] = wa.x;
-            As[2 * kk + 1][cc] = -wa.y;
-            Bs[2 * kk][cc] = fb.x;
-            Bs[2 * kk + 1][cc] = fb.y;
+        for (int i = 0; i < NL; i++) {
+            const int kk = tid / T + (256 / T) * i;
+            const float2 w = wn[i], f = fyn[i];
+            As[2 * kk][cc] = w.x * f.x - w.y * f.y;
+            As[2 * kk + 1][cc] = -(w.x * f.y + w.y * f.x);
+            Bs[2 * kk][cc] = fxn[i].x;
+            Bs[2 * kk + 1][cc] = fxn[i].y;
         }
         __syncthreads();
+        if (k0 + AB_K < ke) load(k0 + AB_K);
 #pragma unroll 8
         for (int kp = 0; kp < 2 * AB_K; kp++) {
-            float4 a = *reinterpret_cast<const float4 *>(&As[kp][ty * 4]);
-            float4 b = *reinterpret_cast<const float4 *>(&Bs[kp][tx * 4]);
-            float av[4] = {a.x, a.y, a.z, a.w}, bv[4] = {b.x, b.y, b.z, b.w};
+            float av[R], bv[R];
+            if (R == 4) {
+                *reinterpret_cast<float4 *>(av) = *reinterpret_cast<const float4 *>(&As[kp][ty * 4]);
+                *reinterpret_cast<float4 *>(bv) = *reinterpret_cast<const float4 *>(&Bs[kp][tx * 4]);
+            } else {
+                *reinterpret_cast<float2 *>(av) = *reinterpret_cast<const float2 *>(&As[kp][ty * 2]);
+                *reinterpret_cast<float2 *>(bv) = *reinterpret_cast<const float2 *>(&Bs[kp][tx * 2]);
+            }
 #pragma unroll
-            for (int i = 0; i < 4; i++)
+            for (int i = 0; i < R; i++)
 #pragma unroll
-                for (int j = 0; j < 4; j++) acc[i][j] = fmaf(av[i], bv[j], acc[i][j]);
+                for (int j = 0; j < R; j++) acc[i][j] = fmaf(av[i], bv[j], acc[i][j]);
         }
         __syncthreads();
     }
     float *out = gpart + (size_t)blockIdx.z * N * N;
 #pragma unroll
-    for (int i = 0; i < 4; i++) {
-        int y = y0 + ty * 4 + i;
-        if (y >= N) continue;
+    for (int i = 0; i < R; i++) {
+        const int yo = y0 + ty * R + i;
+        if (yo >= N) continue;
 #pragma unroll
-        for (int j = 0; j < 4; j++) {
-            int x = x0 + tx * 4 + j;
-            if (x < N) out[(size_t)y * N + x] = acc[i][j];
+        for (int j = 0; j < R; j++) {
+            const int xo = x0 + tx * R + j;
+            if (xo < N) out[(size_t)yo * N + xo] = acc[i][j];
         }
     }
 }
 
 static int adj_splits(int N, int nuv)
 {
-    int tiles = gp_cdiv(N, AB_M) * gp_cdiv(N, AB_N);
+    int tiles = gp_cdiv(N, AB_M) * gp_cdiv(N, AB_M);
     int s = gp_cdiv(148 * 3, tiles);
     int maxs = gp_cdiv(nuv, 64);
     if (s > maxs) s = maxs;
@@ -732,14 +790,16 @@ int gp_adjoint_contraction(gpair_ctx *c, int which)
     if (S < 1) S = 1;
     c->splits_simt = S;
     c->splits = S;
-    dim3 grid(gp_cdiv(c->N, AB_N), gp_cdiv(c->N, AB_M), S);
     if (c->nuv == 0) {
         GP_CUDA(c, cudaMemsetAsync(c->gpart, 0, sizeof(float) * c->npix, c->stream));
         c->splits = 1;
         return GPAIR_OK;
     }
-    k_adj_simt<<<grid, 256, 0, c->stream>>>(c->fx, c->fy, c->cw, c->N, c->nuv, kchunk, c->gpart);
-    GP_LAUNCH_CHECK(c);
+    const int wide = gp_cdiv(c->N, AB_M);
+    const int T = wide * wide * S < 148 ? 32 : AB_M;
+    GP_LAUNCH(c, gp_launch(c, T == 32 ? k_adj_simt<2> : k_adj_simt<4>, dim3(gp_cdiv(c->N, T), gp_cdiv(c->N, T), S),
+                           dim3(256), 0, (const float2 *)c->fx, (const float2 *)c->fy, (const float2 *)c->cw, c->N,
+                           c->nuv, kchunk, c->gpart));
     return GPAIR_OK;
 }
 
@@ -842,9 +902,10 @@ __device__ __forceinline__ void grad_finalize_body(const GradFinalizeArgs &A, co
 #pragma unroll
             for (int j = 0; j < 4; j++) psum[threadIdx.x][j] = g[j];
             __syncthreads();
-            if (pp == 0 && q < nq) {
-#pragma unroll
-                for (int j = 0; j < 4; j++) {
+            // the four pixels are shared among the P threads (their FP64 logarithms one after
+            // another in one thread took half of the kernel at 64^2)
+            if (q < nq) {
+                for (int j = pp; j < 4; j += P) {
                     double t = psum[lq][j];
                     for (int r = 1; r < P; r++) t += psum[r * qpb + lq][j];
                     finish(4 * q + j, t);
@@ -1883,10 +1944,8 @@ static int eval_batch(gpair_ctx *c, cudaEvent_t *ev)
         epp = gp_cdiv(c->N, FB_M);
         if (c->ug) {
             if ((rc = gp_ug_x(c, c->image_trials, GP_NTR)) || (rc = gp_ug_vis(c, GP_NTR))) return rc;
-        } else {
-            dim3 grid(gp_cdiv(c->nuv, FB_K), epp, GP_NTR);
-            k_fwd_simt<<<grid, 256, 0, c->stream>>>(c->image_trials, c->fx, c->fy, c->N, c->nuv, c->vpart_b, c->gate);
-            GP_LAUNCH_CHECK(c);
+        } else if (c->nuv) {
+            if ((rc = fwd_simt(c, c->image_trials, c->vpart_b, GP_NTR, c->gate))) return rc;
         }
     }
     gp_stage_end(c);
