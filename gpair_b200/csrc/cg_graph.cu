@@ -75,14 +75,18 @@ static int emit(gpair_ctx *c, CgGraph *G, int seq, cudaGraphConditionalHandle hi
             rc = gp_eval_batch(c);
         } else {
             c->fuse_ctrl = CTRL_AFTER_CRIT;
+            c->chi2_only = gp_vis_chi2_only(c);
             rc = gp_eval_criterion(c, GPAIR_IMG_TEMP, 1);
+            c->chi2_only = 0;
         }
         break;
     case SEQ_GRAD:
+        if (gp_vis_chi2_only(c) && (rc = gp_vis_data_again(c, 0))) break;
         c->fuse_ctrl = CTRL_AFTER_GRAD;
         rc = gp_eval_gradient(c, GPAIR_IMG_TEMP, -1.f);
         break;
     default:
+        if (G->ls_mode != GPAIR_LS_BATCH && gp_vis_chi2_only(c) && (rc = gp_vis_data_again(c, 1))) break;
         if ((rc = gp_update_image(c, 1, 0.0, 1e-8, 1))) break;
         rc = gp_cg_kernel_graph(c, CTRL_END, hi, hl, hg, G->trace, G->trace_cap);
         break;

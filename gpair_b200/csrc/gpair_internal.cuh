@@ -120,6 +120,7 @@ struct DevScalars {
     unsigned int t_counter[GP_NTR + 1];
     int *stop_flag;  // shared with racing runs (device memory), or null
     int reg_kind;    // GPAIR_REG_GULL_SKILLING / GPAIR_REG_L2
+    int vis_stale;   // the last pass over the data formed chi2 alone (k_vis_chi2)
     // projected L-BFGS reductions
     double lb_pdots[GP_LB_NPD], lb_qdots[GP_LB_NQD];
     CgState cg;
@@ -270,6 +271,7 @@ struct gpair_ctx {
     // also makes the image prep clear the non-finite flag
     GpHostResult *hres;
     int direct_result;
+    int chi2_only;  // the next pass over the data forms chi2 alone (trials of a captured Wolfe search)
     // pinned staging of small host arrays (images, results): stage_busy while an upload from it may be in flight
     void *stage;
     int stage_busy;
@@ -436,6 +438,8 @@ int gp_build_incidence(gpair_ctx *c, const int64_t *uvpnt);
 int gp_prep_image(gpair_ctx *c, int which, int trial_mode, double step_host, int step_from_state);
 int gp_forward(gpair_ctx *c, int which);
 int gp_vis_data(gpair_ctx *c);
+bool gp_vis_chi2_only(const gpair_ctx *c);
+int gp_vis_data_again(gpair_ctx *c, int if_stale);
 int gp_adjoint(gpair_ctx *c, int which);
 int gp_adj_weights_only(gpair_ctx *c);
 int gp_adjoint_contraction(gpair_ctx *c, int which);

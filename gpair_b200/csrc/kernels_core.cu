@@ -374,9 +374,12 @@ struct VisDataArgs {
     FusedCtrl fc;
     int direct;
     GpHostResult *hres;  // result of a blocking call, or null
+    int if_stale;        // return unless the last pass formed chi2 alone
     GP_VGRID_FIELDS;
 };
 
+// FULL: V, mock data and the adjoint's weights beside chi2; else chi2 alone (the same sums)
+template <bool FULL>
 __device__ __forceinline__ void vis_data_body(const VisDataArgs &A, const GpVGrid &vg)
 {
     const float2 *__restrict__ vpart = A.vpart;
@@ -394,24 +397,28 @@ __device__ __forceinline__ void vis_data_body(const VisDataArgs &A, const GpVGri
     DevScalars *__restrict__ sc = A.sc;
     // direct: the visibilities are already in visd (a single-pixel update), not in vpart
     __shared__ double smem[32];
+    if (FULL && A.if_stale && !sc->vis_stale) return;  // uniform over the grid: the last block clears it
     const double invF = sc->invflux;
 #define VIS_AT(k) (direct ? visd[(k)] : sum_vpart(vpart, mt, nuv, (k), invF))
     double chi[1] = {0.0};
     if (vg.bx < nblk_uv) {
         for (int k = vg.bx * blockDim.x + threadIdx.x; k < nuv; k += nblk_uv * blockDim.x) {
+            if (!FULL && k >= npow) break;
             double2 V = VIS_AT(k);
-            if (!direct) visd[k] = V;
-            visi[k] = make_float2((float)V.x, (float)V.y);
+            if (FULL) {
+                if (!direct) visd[k] = V;
+                visi[k] = make_float2((float)V.x, (float)V.y);
+            }
             float2 a = make_float2(0.f, 0.f);
             if (k < npow) {
                 double m2 = sqr2(V.x, V.y);
-                mock[k] = (float)m2;
+                if (FULL) mock[k] = (float)m2;
                 double w = data_err[k], res = m2 - (double)data[k], r = __dmul_rn(res, w);
                 chi[0] = fma(r, r, chi[0]);
                 double f = 4.0 * w * w * res * invF; // a_k = f conj(V_k)
                 a = make_float2((float)(f * V.x), (float)(-f * V.y));
             }
-            cw[k] = a;
+            if (FULL) cw[k] = a;
         }
     } else {
         // a run of consecutive triangles per block (those of an observation share its baselines: L1), the
@@ -435,10 +442,13 @@ __device__ __forceinline__ void vis_data_body(const VisDataArgs &A, const GpVGri
             if (q.w & 4) vc = cconj(vc);
             const double2 ph = make_double2(phf.x, phf.y);
             const double2 ab = cmul(va, vb), t3 = cmul(cmul(ab, vc), ph);
-            mock[r0] = (float)t3.x;
-            mock[r0 + 1] = (float)t3.y;
+            if (FULL) {
+                mock[r0] = (float)t3.x;
+                mock[r0 + 1] = (float)t3.y;
+            }
             const double rre = t3.x - (double)d0, rim = t3.y - (double)d1;
             chi[0] += sqr2(__dmul_rn(rre, wre), __dmul_rn(rim, wim));
+            if (!FULL) continue;
             // adjoint: Re(conj(g) * t3der) with g = 2 w_re^2 (T3re - d_re) + i 2 w_im^2 T3im
             // (the reference uses the mock imaginary part alone, gpair1/trunk/cpu.c:364-365)
             const double2 g = make_double2(2.0 * wre * wre * rre, 2.0 * wim * wim * t3.y);
@@ -465,6 +475,7 @@ __device__ __forceinline__ void vis_data_body(const VisDataArgs &A, const GpVGri
             sc->chi2 = out[0];
             sc->chi2_f = (float)out[0];
             if (!isfinite(out[0])) sc->nonfinite |= 2u;
+            sc->vis_stale = FULL ? 0 : 1;
             sc->counter[RED_CHI2] = 0;
             gp_host_result(A.hres, sc);
             run_fused_ctrl(sc, A.fc);
@@ -477,12 +488,19 @@ __device__ __forceinline__ void vis_data_body(const VisDataArgs &A, const GpVGri
 __global__ void __launch_bounds__(GP_THREADS, 4) k_vis_data(const VisDataArgs a)
 {
     gp_pdl_enter();
-    vis_data_body(a, gp_vgrid_hw());
+    vis_data_body<true>(a, gp_vgrid_hw());
+}
+
+// chi2 alone, for the trials of a Wolfe search over large data (gp_vis_chi2)
+__global__ void __launch_bounds__(GP_THREADS, 5) k_vis_chi2(const VisDataArgs a)
+{
+    gp_pdl_enter();
+    vis_data_body<false>(a, gp_vgrid_hw());
 }
 
 struct VisDataOp {
     using Args = VisDataArgs;
-    static __device__ __forceinline__ void run(const Args &a, const GpVGrid &v) { vis_data_body(a, v); }
+    static __device__ __forceinline__ void run(const Args &a, const GpVGrid &v) { vis_data_body<true>(a, v); }
 };
 
 static VisDataArgs vis_data_args(gpair_ctx *c, int direct, FusedCtrl fc)
@@ -496,7 +514,7 @@ static VisDataArgs vis_data_args(gpair_ctx *c, int direct, FusedCtrl fc)
     if (nbt > 496) nbt = 496;
     VisDataArgs a = {c->vpart, c->mt, c->nuv, c->npow, c->nbis, c->data, c->data_err, c->tri, c->phasor, nbu,
                      c->visd, c->visi, c->mock, c->cw, c->trib, slot_partials(c, RED_CHI2), c->sc, fc, direct,
-                     c->direct_result ? c->hres : nullptr, nbu + nbt, 1};
+                     c->direct_result ? c->hres : nullptr, 0, nbu + nbt, 1};
     return a;
 }
 
@@ -531,6 +549,25 @@ static int vis_data_launch(gpair_ctx *c, int direct)
         direct = 1;
     }
     const VisDataArgs a = vis_data_args(c, direct, take_fused_ctrl(c));
+    GP_LAUNCH(c, gp_launch(c, c->chi2_only ? k_vis_chi2 : k_vis_data, dim3(a.nbx), dim3(GP_THREADS), 0, a));
+    return GPAIR_OK;
+}
+
+// A Wolfe search takes the gradient at few of its trials (1024^2 workload: 40 objectives, 2
+// gradients an iteration). Where the pass writes this much, its trials form chi2 alone, and the
+// full pass follows where a gradient is taken and at the end of the iteration, so that a run leaves the
+// same V, mock data and weights. 46 MB: 25 us full, 12 chi2 alone. 3 MB (256^2, 21,120 points): 12 either way.
+#define VIS_CHI2_ONLY_BYTES 32e6
+bool gp_vis_chi2_only(const gpair_ctx *c) { return 36.0 * c->nbis + 20.0 * c->nuv >= VIS_CHI2_ONLY_BYTES; }
+
+// the full pass after one that formed chi2 alone (if_stale: returns at once after a full one)
+int gp_vis_data_again(gpair_ctx *c, int if_stale)
+{
+    const int direct = c->ug || c->mt > VIS_PRESUM_ENTRIES;  // V is in visd already
+    FusedCtrl none = {};
+    none.what = -1;
+    VisDataArgs a = vis_data_args(c, direct, none);
+    a.if_stale = if_stale;
     GP_LAUNCH(c, gp_launch(c, k_vis_data, dim3(a.nbx), dim3(GP_THREADS), 0, a));
     return GPAIR_OK;
 }
