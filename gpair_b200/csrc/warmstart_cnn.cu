@@ -174,99 +174,289 @@ __global__ void __launch_bounds__(TW4 *TH *(CB / CT)) k_conv3(const float *__res
     }
 }
 
-// Weight and bias gradient partials: block (CO output channels, input channel,
-// slice) sums over the images [slice*bps, (slice+1)*bps) and all pixels;
+// Weight and bias gradient partials: block (NG groups of CO output channels, input
+// channel, slice) sums over the images [slice*bps, (slice+1)*bps) and all pixels;
 // part[slice][co][ci][tap], bpart[slice][co] (bias, from the blocks of the first
-// input channel). Thread t sums the pixels p = t mod 256 in order, image by
+// input channel). Thread t of a group sums the pixels p = t mod 256 in order, image by
 // image; the threads' sums go through a shuffle tree and then over the warps
-// in order. Bound by instruction issue: 9 predicated input loads and CO of g for
-// 9 CO FMAs, the pixel's coordinates advanced without a division, and U pixels
-// loaded before the first is used. (One output and 8 input channels per block
-// made 32 blocks of a 16 -> 16 layer, each waiting for one pixel's loads at a
-// time: 16 images of 64^2 took 765 us, now 66; 128 -> 128 at 8^2 318, now 41.)
+// in order. The input passes through shared memory with its zero border, a chunk of
+// whole images or of 256 nstep pixels of one image at a time, the next chunk's copies
+// in flight: a pixel is then 9 shared loads and CO loads of g, also ahead, for 9 CO
+// FMAs. Masked pixels (g = 0) add nothing and taps outside the image are left out,
+// also beside infinities: the products are formed regardless, and a block whose sums
+// come out non-finite forms them again pixel by pixel (wg_careful). (With
+// the inputs loaded per pixel and every mask applied, 90 instructions went to 9
+// FMAs: 16 images of 64^2, 16 -> 16 channels 68 us, now 51; 8^2, 128 -> 128
+// 41, now 35.)
 #define WG_THREADS 256
-template <int CO, int U>
-__global__ void __launch_bounds__(WG_THREADS) k_conv3_wgrad(const float *__restrict__ in, const float *__restrict__ g,
-                                                            float *__restrict__ part, float *__restrict__ bpart, int B,
-                                                            int Cin, int Cout, int H, int W, int bps)
+#define WG_BUF 5120  // floats of a chunk
+struct WgPlan {
+    int threads, nimg, nstep;  // threads per group; images per chunk, or steps of 256 pixels of one image
+    int ld, xo;                // floats per row of a chunk, offset of a row's first pixel
+    int vec, wshift;           // 16-byte copies, of which a row takes 1 << wshift
+};
+// false: a chunk of one step does not fit
+static bool wg_plan(const float *in, int B, int H, int W, WgPlan *p)
+{
+    const int HW = H * W;
+    p->vec = W >= 4 && (W & (W - 1)) == 0 && ((uintptr_t)in & 15) == 0;
+    p->wshift = 0;
+    while (p->vec && 4 << p->wshift < W) p->wshift++;
+    p->xo = p->vec ? 4 : 1;
+    p->ld = W + 2 * p->xo;
+    p->threads = HW >= WG_THREADS ? WG_THREADS : (HW + 31) / 32 * 32;
+    p->nstep = (HW + WG_THREADS - 1) / WG_THREADS;
+    p->nimg = (long long)(H + 2) * p->ld <= WG_BUF ? WG_BUF / ((H + 2) * p->ld) : 0;
+    if (p->nimg) {
+        if (p->nimg > B) p->nimg = B;
+        return true;
+    }
+    p->nimg = 1;
+    // the rows that 256 nstep consecutive pixels touch, one above and one below
+    int n = (int)((long long)(WG_BUF / p->ld - 3) * W / WG_THREADS);
+    if (n > p->nstep) n = p->nstep;
+    p->nstep = n;
+    return n >= 1;
+}
+
+// the sums of one thread pixel by pixel: acc [co][tap], then the bias sums
+template <int CO>
+__device__ __noinline__ void wg_careful(const float *__restrict__ in, const float *__restrict__ g, int b0, int b1, int ci,
+                                        int co0, int Cin, int Cout, int H, int W, int t, float *acc)
+{
+    const int HW = H * W;
+    for (int i = 0; i < CO * NTAP + CO; i++) acc[i] = 0.f;
+    for (int b = b0; b < b1; b++)
+        for (int p = t; p < HW; p += WG_THREADS) {
+            const int y = p / W, x = p - y * W;
+            const float *ip = in + ((size_t)b * Cin + ci) * HW + p;
+            for (int o = 0; o < CO && co0 + o < Cout; o++) {
+                const float gv = g[((size_t)b * Cout + co0 + o) * HW + p];
+                if (gv == 0.f) continue;
+                acc[CO * NTAP + o] += gv;
+                for (int k = 0; k < NTAP; k++) {
+                    const int dy = k / 3 - 1, dx = k % 3 - 1;
+                    if (y + dy < 0 || y + dy >= H || x + dx < 0 || x + dx >= W) continue;
+                    acc[o * NTAP + k] = fmaf(gv, ip[dy * W + dx], acc[o * NTAP + k]);
+                }
+            }
+        }
+}
+
+// Sums of N values (at most 32) over the lanes of a warp, into out[0..N-1]: at every level of
+// the tree half of the lanes go on with half of the values. The pairs are those of a shuffle tree per value, so
+// the sums are the same; 4 instructions a pair instead of 10 a value.
+template <int N>
+__device__ __forceinline__ void wg_warp_sums(const float *acc, int lane, float *out)
+{
+    constexpr int M = N > 16 ? 32 : N > 8 ? 16 : N > 4 ? 8 : N > 2 ? 4 : N;  // a power of two
+    float v[M];
+#pragma unroll
+    for (int i = 0; i < M; i++) v[i] = i < N ? acc[i] : 0.f;
+    int idx = 0, off = 16;
+#pragma unroll
+    for (int m = M; off > 0; off >>= 1) {
+        if (m > 1) {
+            m >>= 1;
+            const bool hi = lane & off;
+#pragma unroll
+            for (int i = 0; i < M / 2; i++)
+                if (i < m) {
+                    const float keep = hi ? v[i + m] : v[i], send = hi ? v[i] : v[i + m];
+                    v[i] = keep + __shfl_xor_sync(0xffffffffu, send, off);
+                }
+            if (hi) idx += m;
+        } else {
+            v[0] += __shfl_xor_sync(0xffffffffu, v[0], off);
+        }
+    }
+    if (idx < N && (lane & (32 / M - 1)) == 0) out[idx] = v[0];
+}
+
+// How a thread steps through a chunk: from row to row (any width), by a fixed stride (the width divides
+// 256), or from image to image (an image is one step). WG_WIDE: images of which no chunk of 256
+// pixels fits (W > 1,278), pixel by pixel.
+enum { WG_ROWS, WG_FIXED, WG_IMAGES, WG_WIDE };
+template <int CO, int NG, int U, int MODE>
+__global__ void __launch_bounds__(WG_THREADS *NG) k_conv3_wgrad(const float *__restrict__ in,
+                                                                const float *__restrict__ g,
+                                                                float *__restrict__ part, float *__restrict__ bpart,
+                                                                int B, int Cin, int Cout, int H, int W, int bps,
+                                                                const WgPlan P)
 {
     constexpr int NV = CO * NTAP + CO;
-    __shared__ float red[WG_THREADS / 32][NV];
-    const int co0 = blockIdx.x * CO, ci = blockIdx.y, slice = blockIdx.z;
+    constexpr bool STAGED = MODE != WG_WIDE;
+    __shared__ __align__(16) float xs[STAGED ? 2 : 1][STAGED ? WG_BUF : 4];
+    __shared__ float red[NG][WG_THREADS / 32][NV];
+    const int t = threadIdx.x % P.threads, grp = threadIdx.x / P.threads;
+    const int co0 = (blockIdx.x * NG + grp) * CO, ci = blockIdx.y, slice = blockIdx.z;
     const int b0 = slice * bps, b1 = min(B, b0 + bps);
+    const int HW = H * W, LD = P.ld;
+    const int lane = threadIdx.x & 31;
     float acc[NV];  // [co][tap], then the bias sums
 #pragma unroll
     for (int i = 0; i < NV; i++) acc[i] = 0.f;
-    const int HW = H * W;
-    // this thread's pixels of an image (a block smaller than 256 threads has one per thread), over the slice's images
-    const int per = (int)threadIdx.x < HW ? (HW - (int)threadIdx.x + WG_THREADS - 1) / WG_THREADS : 0;
-    const int steps = per * (b1 - b0);
-    const int dy = WG_THREADS / W, dx = WG_THREADS - dy * W, yt = (int)threadIdx.x / W, xt = (int)threadIdx.x - yt * W;
-    const float *gp = g + ((size_t)b0 * Cout + co0) * HW + threadIdx.x;
-    const float *ip = in + ((size_t)b0 * Cin + ci) * HW + threadIdx.x;
-    const int no = min(CO, Cout - co0);
-    int left = per, y = yt, x = xt;
-    for (int s = 0; s < steps; s += U) {
-        float gv[U][CO], v[U][NTAP];
-#pragma unroll
-        for (int u = 0; u < U; u++) {
-            const bool live = s + u < steps;
-            const bool r0 = live && y > 0, r2 = live && y + 1 < H, c0 = x > 0, c2 = x + 1 < W;
-#pragma unroll
-            for (int o = 0; o < CO; o++) gv[u][o] = live && o < no ? __ldg(gp + (size_t)o * HW) : 0.f;
-            const float *u0 = ip - W, *u2 = ip + W;
-            v[u][0] = r0 && c0 ? __ldg(u0 - 1) : 0.f;
-            v[u][1] = r0 ? __ldg(u0) : 0.f;
-            v[u][2] = r0 && c2 ? __ldg(u0 + 1) : 0.f;
-            v[u][3] = live && c0 ? __ldg(ip - 1) : 0.f;
-            v[u][4] = live ? __ldg(ip) : 0.f;
-            v[u][5] = live && c2 ? __ldg(ip + 1) : 0.f;
-            v[u][6] = r2 && c0 ? __ldg(u2 - 1) : 0.f;
-            v[u][7] = r2 ? __ldg(u2) : 0.f;
-            v[u][8] = r2 && c2 ? __ldg(u2 + 1) : 0.f;
-            if (--left > 0) {
-                gp += WG_THREADS;
-                ip += WG_THREADS;
-                y += dy;
-                x += dx;
-                if (x >= W) {
-                    x -= W;
-                    y++;
-                }
-            } else {  // the next image
-                const int back = (per - 1) * WG_THREADS;
-                gp += (ptrdiff_t)Cout * HW - back;
-                ip += (ptrdiff_t)Cin * HW - back;
-                y = yt;
-                x = xt;
-                left = per;
+    if (STAGED) {
+        const int total_steps = (HW + WG_THREADS - 1) / WG_THREADS;
+        const bool whole = P.nstep == total_steps;
+        const int spi = whole ? 1 : (total_steps + P.nstep - 1) / P.nstep;  // chunks per image
+        const int nchunk = whole ? (b1 - b0 + P.nimg - 1) / P.nimg : (b1 - b0) * spi;
+        // the borders stay zero
+        const int used = whole ? P.nimg * (H + 2) * LD : WG_BUF, nbuf = nchunk > 1 ? 2 : 1;
+        for (int b = 0; b < nbuf; b++)
+            for (int i = threadIdx.x; i < (used + 3) / 4; i += blockDim.x)
+                reinterpret_cast<float4 *>(xs[b])[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+        __syncthreads();
+        // chunk c: images [ib, ib + ni), steps [s0, s1) of each, rows from ylo
+        auto range = [&](int c, int &ib, int &ni, int &s0, int &s1, int &ylo, int &rows) {
+            if (whole) {
+                ib = b0 + c * P.nimg;
+                ni = min(P.nimg, b1 - ib);
+                s0 = 0;
+                s1 = total_steps;
+                ylo = -1;
+                rows = H + 2;
+            } else {
+                ib = b0 + c / spi;
+                ni = 1;
+                s0 = (c % spi) * P.nstep;
+                s1 = min(total_steps, s0 + P.nstep);
+                ylo = WG_THREADS * s0 / W - 1;
+                rows = (min(HW, WG_THREADS * s1) - 1) / W + 1 - ylo + 1;
             }
+        };
+        // the rows of chunk c (zeros for those outside the image), 16 bytes or one pixel a copy
+        auto stage = [&](int c) {
+            int ib, ni, s0, s1, ylo, rows;
+            range(c, ib, ni, s0, s1, ylo, rows);
+            const uint32_t buf = (uint32_t)__cvta_generic_to_shared(&xs[c & 1][P.xo]);
+            const float *src = in + ((size_t)ib * Cin + ci) * HW;
+            const int lo = whole ? 1 : 0, nr = whole ? H : rows;  // of whole images the border rows stay zero
+            for (int im = 0; im < ni; im++, src += (size_t)Cin * HW) {
+                const uint32_t dst = buf + 4u * (uint32_t)(im * rows * LD);
+                if (P.vec) {
+                    for (int e = threadIdx.x; e < nr << P.wshift; e += blockDim.x) {
+                        const int r = lo + (e >> P.wshift), x = 4 * (e & ((1 << P.wshift) - 1)), y = ylo + r;
+                        const bool ok = y >= 0 && y < H;
+                        const int bytes = ok ? 16 : 0;
+                        asm volatile("cp.async.ca.shared.global [%0], [%1], 16, %2;" ::"r"(dst + 4u * (uint32_t)(r * LD + x)),
+                                     "l"(ok ? src + (size_t)y * W + x : src), "r"(bytes)
+                                     : "memory");
+                    }
+                } else {
+                    for (int e = threadIdx.x; e < nr * W; e += blockDim.x) {
+                        const int q = e / W, r = lo + q, x = e - q * W, y = ylo + r;
+                        const bool ok = y >= 0 && y < H;
+                        const int bytes = ok ? 4 : 0;
+                        asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(dst + 4u * (uint32_t)(r * LD + x)),
+                                     "l"(ok ? src + (size_t)y * W + x : src), "r"(bytes)
+                                     : "memory");
+                    }
+                }
+            }
+            asm volatile("cp.async.commit_group;" ::: "memory");
+        };
+        const int dy = WG_THREADS / W, dx = WG_THREADS - dy * W;
+        stage(0);
+        for (int c = 0; c < nchunk; c++) {
+            if (c + 1 < nchunk) {
+                stage(c + 1);
+                asm volatile("cp.async.wait_group 1;" ::: "memory");
+            } else {
+                asm volatile("cp.async.wait_group 0;" ::: "memory");
+            }
+            __syncthreads();
+            int ib, ni, s0, s1, ylo, rows;
+            range(c, ib, ni, s0, s1, ylo, rows);
+            // this thread's pixels of the chunk: `per` of each image from pixel t + 256 s0
+            const int p0 = t + WG_THREADS * s0;
+            const int per = p0 < HW ? min(s1 - s0, (HW - p0 + WG_THREADS - 1) / WG_THREADS) : 0;
+            const int y0 = p0 / W, x0 = p0 - y0 * W;
+            const int n = MODE == WG_IMAGES ? per * ni : per, outer = MODE == WG_IMAGES ? 1 : ni;
+            const int gs = MODE == WG_IMAGES ? Cout * HW : WG_THREADS;
+            const int os = MODE == WG_IMAGES ? rows * LD : dy * LD + dx;
+            for (int im = 0; im < outer; im++) {
+                const float *gp = g + (size_t)(ib + im) * Cout * HW + p0;
+                const float *bp = &xs[c & 1][im * rows * LD + (y0 - ylo) * LD + x0 + P.xo];
+                const float *gc[CO];  // (channels past the last repeat it; their sums are not stored)
+#pragma unroll
+                for (int o = 0; o < CO; o++) gc[o] = gp + (size_t)min(co0 + o, Cout - 1) * HW;
+                int x = x0;
+                float gn[U][CO];
+                // g of the next k pixels
+                auto fetch = [&](int k) {
+#pragma unroll
+                    for (int u = 0; u < U; u++)
+                        if (u < k) {
+#pragma unroll
+                            for (int o = 0; o < CO; o++) gn[u][o] = __ldg(gc[o] + u * gs);
+                        }
+#pragma unroll
+                    for (int o = 0; o < CO; o++) gc[o] += U * gs;
+                };
+                // the sums of k pixels, g of the kn after them in flight
+                auto run = [&](int k, int kn) {
+                    float gv[U][CO], v[U][NTAP];
+#pragma unroll
+                    for (int u = 0; u < U; u++)
+                        if (u < k) {
+#pragma unroll
+                            for (int o = 0; o < CO; o++) gv[u][o] = gn[u][o];
+                            const float *q = MODE == WG_ROWS ? bp : bp + u * os;
+#pragma unroll
+                            for (int t9 = 0; t9 < NTAP; t9++) v[u][t9] = q[(t9 / 3 - 1) * LD + t9 % 3 - 1];
+                            if (MODE == WG_ROWS) {
+                                bp += os;
+                                x += dx;
+                                if (x >= W) {
+                                    x -= W;
+                                    bp += LD - W;
+                                }
+                            }
+                        }
+                    if (MODE != WG_ROWS) bp += U * os;
+                    fetch(kn);
+#pragma unroll
+                    for (int u = 0; u < U; u++)
+                        if (u < k) {
+#pragma unroll
+                            for (int o = 0; o < CO; o++) {
+                                acc[CO * NTAP + o] += gv[u][o];
+#pragma unroll
+                                for (int t9 = 0; t9 < NTAP; t9++)
+                                    acc[o * NTAP + t9] = fmaf(gv[u][o], v[u][t9], acc[o * NTAP + t9]);
+                            }
+                        }
+                };
+                int left = n;
+                fetch(min(left, U));
+                for (; left >= 2 * U; left -= U) run(U, U);
+                for (; left > 0; left -= U) run(min(left, U), min(max(left - U, 0), U));
+            }
+            __syncthreads();  // the chunk after the next takes this buffer
         }
-#pragma unroll
-        for (int u = 0; u < U; u++)
-#pragma unroll
-            for (int o = 0; o < CO; o++) {
-                acc[CO * NTAP + o] += gv[u][o];
-                if (gv[u][o] != 0.f) {  // masked pixels add nothing
-#pragma unroll
-                    for (int k = 0; k < NTAP; k++) acc[o * NTAP + k] = fmaf(gv[u][o], v[u][k], acc[o * NTAP + k]);
-                }
-            }
     }
-    // fixed-order block reduction: warp shuffles, then one pass over the warps
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    bool redo = !STAGED;
 #pragma unroll
-    for (int i = 0; i < NV; i++) {
-        float v = acc[i];
+    for (int i = 0; i < NV; i++) redo |= !(fabsf(acc[i]) <= 3.402823466e38f);
+    if (__syncthreads_or(redo)) {
+        float again[NV];
+        wg_careful<CO>(in, g, b0, b1, ci, co0, Cin, Cout, H, W, t, again);
 #pragma unroll
-        for (int off = 16; off > 0; off >>= 1) v += __shfl_down_sync(0xffffffffu, v, off);
-        if (lane == 0) red[warp][i] = v;
+        for (int i = 0; i < NV; i++) acc[i] = again[i];
+    }
+    // fixed-order block reduction: warp shuffles, then one pass over the group's warps
+    const int gw = P.threads >> 5;
+#pragma unroll
+    for (int i = 0; i < NV; i += 32) {
+        if constexpr (NV <= 32) wg_warp_sums<NV>(&acc[i], lane, &red[grp][t >> 5][i]);
+        else if (i + 32 <= NV) wg_warp_sums<32>(&acc[i], lane, &red[grp][t >> 5][i]);
+        else wg_warp_sums<NV % 32 ? NV % 32 : 32>(&acc[i], lane, &red[grp][t >> 5][i]);
     }
     __syncthreads();
-    const int nw = (int)(blockDim.x >> 5);
-    for (int i = threadIdx.x; i < NV; i += blockDim.x) {
+    for (int i = t; i < NV; i += P.threads) {
         float v = 0.f;
-        for (int w = 0; w < nw; w++) v += red[w][i];
+        for (int w = 0; w < gw; w++) v += red[grp][w][i];
         if (i < CO * NTAP) {
             const int co = co0 + i / NTAP, k = i % NTAP;
             if (co < Cout) part[(((size_t)slice * Cout + co) * Cin + ci) * NTAP + k] = v;
@@ -576,17 +766,28 @@ extern "C" int gpair_cnn_conv3x3_bwd_weight(const float *in, const float *gpre, 
     const long long nw = (long long)Cout * Cin * NTAP;
     if ((long long)slices * (nw + Cout) > scratch_floats) return GPAIR_ERR_INVALID;
     float *part = scratch, *bpart = scratch + (size_t)slices * nw;
-    // a thread per pixel of an image, up to 256: the warps past them would add zeros
-    const int threads = H * W >= WG_THREADS ? WG_THREADS : (H * W + 31) / 32 * 32;
-    // four output channels a block (9 input loads for 36 FMAs) where that still makes two blocks per SM
     const cudaStream_t st = CNN_STREAM(stream);
-    auto go = [&](auto kernel, int co) {
-        kernel<<<dim3(cdiv_ll(Cout, co), Cin, slices), threads, 0, st>>>(in, gpre, part, bpart, B, Cin, Cout, H, W, bps);
-    };
     const long long blocks = (long long)Cout * Cin * slices;
-    if (blocks >= 4 * 2 * 148) go(k_conv3_wgrad<4, 2>, 4);
-    else if (blocks >= 2 * 2 * 148) go(k_conv3_wgrad<2, 4>, 2);
-    else go(k_conv3_wgrad<1, 4>, 1);
+    WgPlan p;
+    const bool staged = wg_plan(in, B, H, W, &p);
+    auto go = [&](auto kernel, int co, int ng) {
+        kernel<<<dim3(cdiv_ll(Cout, co * ng), Cin, slices), p.threads * ng, 0, st>>>(in, gpre, part, bpart, B, Cin, Cout,
+                                                                                    H, W, bps, p);
+    };
+    // four output channels a block (9 input loads for 36 FMAs) where that still makes two blocks per SM; one
+    // each in two groups that share a chunk where blocks are few
+#define WG_GO(CO, NG, U)                                                                      \
+    do {                                                                                      \
+        if (H * W <= WG_THREADS) go(k_conv3_wgrad<CO, NG, U, WG_IMAGES>, CO, NG);             \
+        else if (WG_THREADS % W == 0) go(k_conv3_wgrad<CO, NG, U, WG_FIXED>, CO, NG);         \
+        else go(k_conv3_wgrad<CO, NG, U, WG_ROWS>, CO, NG);                                   \
+    } while (0)
+    if (!staged) go(k_conv3_wgrad<1, 1, 1, WG_WIDE>, 1, 1);
+    else if (blocks >= 4 * 2 * 148) WG_GO(4, 1, 2);
+    else if (blocks >= 2 * 2 * 148) WG_GO(2, 1, 4);
+    else if (blocks >= 148) WG_GO(1, 2, 4);
+    else WG_GO(1, 1, 4);
+#undef WG_GO
     k_reduce_wgrad<<<cdiv_ll(nw + Cout, 256), 256, 0, st>>>(part, (int)nw, bpart, Cout, slices, dw, db);
     return cnn_status();
 }
