@@ -161,6 +161,7 @@ struct TcArgs {
     // rsc[row]: power-of-two factor of every image-side row (operand scale and
     // twiddle scale removed in the epilogue)
     int lpad, live, elog2;
+    int bn;  // columns of a tile: TC_BN, or fewer for short units (store epilogue)
     const float *rsc;
     float2 *vpart;  // entry e of uv point k at vpart[e es + k ks]
     int es, ks;
@@ -190,7 +191,7 @@ struct __align__(64) TcGroupInst {
     int m_tiles, n_tiles, kb_total, units;
     // forward epilogue
     const float2 *fya, *fyr;
-    int nanc, nuv, lpad, live, elog2;
+    int nanc, nuv, lpad, live, elog2, bn;
     const float *rsc;
     float2 *vpart;
     int es, ks;
@@ -273,11 +274,11 @@ __device__ __forceinline__ void tc_decode(const TcArgs &a, int u, int &m, int &n
 // Columns of tile n that hold rows of an image, in whole chunk pairs of the
 // epilogue (32): the MMA of an image's last tile stops there. 192 rows take 192
 // columns instead of 256, and so 3/4 of the tensor-core time and of the epilogue.
-__device__ __forceinline__ int tc_cols(int n, int lpad, int live)
+__device__ __forceinline__ int tc_cols(int n, int lpad, int live, int bn)
 {
     if (lpad < TC_BN) return TC_BN;  // whole images in a tile
-    const int left = live - (n * TC_BN) % lpad;
-    return left >= TC_BN ? TC_BN : (left + 31) & ~31;
+    const int left = live - (n * bn) % lpad;
+    return left >= bn ? bn : (left + 31) & ~31;
 }
 
 // Unit u of a launch: tile (m, n) of nv columns, K-blocks [kb0, kb1), split.
@@ -305,10 +306,10 @@ __device__ __forceinline__ void tc_unit(const TcArgs &a, const int *gpre, int u,
             kb0 = split * gi.kb_per_split;
             kb1 = min(gi.kb_total, kb0 + gi.kb_per_split);
         }
-        nv = tc_cols(n, gi.lpad, gi.live);
+        nv = tc_cols(n, gi.lpad, gi.live, gi.bn);
     } else {
         tc_decode<EPI>(a, u, m, n, kb0, kb1, split);
-        nv = tc_cols(n, a.lpad, a.live);
+        nv = tc_cols(n, a.lpad, a.live, a.bn);
     }
 }
 
@@ -565,7 +566,7 @@ __global__ void __launch_bounds__(tc_threads<EPI>(), 1)
                         umma::tensormap_acquire(mBx);
                     }
                 }
-                const int arow0 = m * G::MT + (int)rank * 128, brow0 = n * TC_BN + (int)rank * (nv / 2);
+                const int arow0 = m * G::MT + (int)rank * 128, brow0 = n * (GROUP ? a.grp[ci].bn : a.bn) + (int)rank * (nv / 2);
                 for (int kb = kb0; kb < kb1; kb++) {
                     const int s = it % G::STAGES;
                     const uint32_t ph = (uint32_t)(it / G::STAGES) & 1u;
@@ -893,7 +894,7 @@ __global__ void __launch_bounds__(tc_threads<EPI>(), 1)
             } else {
                 int m, n, nv, kb0, kb1, split;
                 tc_unit<EPI, GROUP>(a, gpre, u, ci, m, n, nv, kb0, kb1, split);
-                const int y0 = n * TC_BN;  // first image row of the columns
+                const int y0 = n * (GROUP ? a.grp[ci].bn : a.bn);  // first image row of the columns
                 if (!umma::mbar_wait(&tfull[b], (uint32_t)(t >> 1) & 1u, a.budget)) {
                     tc_fail(a.err, abort_flag, 8u);
                     break;
@@ -1974,6 +1975,7 @@ template <int EPI>
 static int tc_launch(gpair_ctx *c, TcState *t, const TcMaps &m, TcArgs &a)
 {
     a.err = &c->sc->tc_err;
+    if (!a.bn) a.bn = TC_BN;
     a.budget = c->tc_wait_budget > 0 ? c->tc_wait_budget : TC_WAIT_BUDGET;
     a.skip_loads = c->tc_skip_loads;
     cudaError_t e;
@@ -2066,18 +2068,22 @@ static TcArgs tc_grid_args(gpair_ctx *c, TcState *t, int images)
     TcArgs a;
     memset(&a, 0, sizeof(a));
     a.m_tiles = t->rows_pad / TC_BM;
-    a.n_tiles = images > 1 ? images * t->Lb / TC_BN : t->M_pad / TC_BN;
     a.kb_total = t->Kx_pad / t->bk;
     a.kb_per_split = t->gkb;
-    a.units = a.m_tiles * a.n_tiles * t->gsplits;
     a.gpart = images > 1 ? g->Tb : g->T;
     a.out_ld = g->ldT;
     a.out_rows = images > 1 ? images * t->Lb : c->N;
     a.out_cols = 2 * g->nbx;
-    if (images == 1) {  // a stack's rows are all written
-        a.lpad = t->M_pad;
-        a.live = c->N;
-    }
+    // tiles of fewer image rows while the units leave half of the SMs idle: a unit's few products and its stores
+    // are its time (with its two successors, 1024^2: 38.8 us in 32 units of 256 rows, 30.9 in 128 of 64; 256^2:
+    // 27.8 in 2, 19.4 in 16 of 32). A stack's rows are all written.
+    const int rows = images == 1 ? c->N : images * t->Lb;
+    a.bn = TC_BN;
+    while (a.bn > 32 && 2 * a.m_tiles * gp_cdiv(rows, a.bn) * t->gsplits <= t->nsm) a.bn /= 2;
+    a.n_tiles = gp_cdiv(rows, a.bn);
+    a.units = a.m_tiles * a.n_tiles * t->gsplits;
+    a.lpad = images == 1 ? t->M_pad : rows;
+    a.live = rows;
     return a;
 }
 
@@ -2360,6 +2366,7 @@ int gp_tc_group_key(gpair_ctx *c)
 static void tc_group_inst(gpair_ctx *c, TcState *t, int kind, TcGroupInst &g)
 {
     const int mt = t->pair ? 256 : TC_BM;
+    g.bn = TC_BN;
     if (kind == GP_TCG_ADJOINT) {
         g.A_hi = t->m_fxt_hi;
         g.A_lo = t->m_fxt_lo;
@@ -2394,6 +2401,7 @@ static void tc_group_inst(gpair_ctx *c, TcState *t, int kind, TcGroupInst &g)
         g.out_cols = a.out_cols;
         g.lpad = a.lpad;
         g.live = a.live;
+        g.bn = a.bn;
     }
     const TcMaps fm = tc_fwd_maps(t, batch);
     g.A_hi = *fm.a_hi;
