@@ -14,7 +14,10 @@ A step is one plain PR+ nonlinear-CG iteration with the reference's strong
 Wolfe line search (criterion + gradient of the current image, direction
 update, bracketing/zoom trials, image update), continuing from the previous
 step. Metric: algorithmic DFT + adjoint TFLOP/s over the timed steps, i.e.
-(criterion + gradient evaluations) x (4 N^2 nuv + 8 N nuv) / time.
+(criterion + gradient evaluations) x (4 N^2 nuv + 8 N nuv) / time. The FLOPs are
+those of the direct sums; where the library takes the uv grid, whose result is
+the same to the same bounds, it executes far fewer, and the rate may exceed the
+tensor cores' peak.
 
     python bench.py [--gpus N] [--steps K] [--warmup W] [--impl ours|reference]
 
@@ -642,15 +645,32 @@ def _executed_mult(precision, stage):
     return 1.0
 
 
+GRID_NOTE = ("the contraction goes through a grid of the uv plane and does not execute the direct sums' FLOPs; "
+             "bytes: image (or gradient), window weights and phases of every uv point, V (or c_k)")
+
+
+def _grid_bytes(p, images=1):
+    """Bytes a contraction through the uv grid cannot do without: images 4 B/px, 76 B of window data per uv
+    point, 16 B of V per uv point and image."""
+    return images * 4 * p.npix + 76 * p.nuv + images * 16 * p.nuv
+
+
 def roofline(p, m, precision, workload):
     """Roofline of the dominant stage (largest total time over the timed steps)."""
     hbm, tflops_peak, peak_kind = _peaks()
     stage_ms, stage_n = m["stage_ms"], m["stage_n"]
     dom = max(stage_ms, key=lambda k: stage_ms[k])
     per_launch_ms = stage_ms[dom] / max(stage_n[dom], 1)
-    if dom in ("forward_dft", "adjoint_dft"):
+    achieved = p.dft_flops() / (per_launch_ms * 1e-3) / 1e12
+    contraction = dom in ("forward_dft", "adjoint_dft")
+    if contraction and _executed_mult(precision, dom) * achieved > 1.2 * tflops_peak:
+        # more than the tensor cores can execute: the uv grid
+        work = _grid_bytes(p)
+        gbs = work / (per_launch_ms * 1e-3) / 1e9
+        roof = {"bound": "hbm", "achieved": gbs, "peak": hbm, "unit": "GB/s", "frac": gbs / hbm,
+                "work_per_launch": work, "work_note": GRID_NOTE, "algorithmic_tflops": achieved}
+    elif contraction:
         work = p.dft_flops()
-        achieved = work / (per_launch_ms * 1e-3) / 1e12
         roof = {"bound": "tensor", "achieved": achieved, "peak": tflops_peak, "unit": "TFLOP/s",
                 "frac": achieved / tflops_peak, "work_per_launch": work,
                 "work_note": "algorithmic FLOPs 4 N^2 nuv + 8 N nuv per launch (one image)"}
@@ -699,12 +719,18 @@ def batched_block(rec, p, args, flush, img, precision, workload):
     mult = _executed_mult(precision, "forward_dft")
     fb_ms = st_b["forward_dft_batch"]
     fb_ach = 8 * p.dft_flops() / (fb_ms * 1e-3) / 1e12
+    if mult * fb_ach > 1.2 * tflops_peak:  # the uv grid
+        gbs = _grid_bytes(p, 8) / (fb_ms * 1e-3) / 1e9
+        roof = {"bound": "hbm", "achieved": gbs, "peak": hbm, "unit": "GB/s", "frac": gbs / hbm,
+                "work_note": GRID_NOTE, "algorithmic_tflops": fb_ach}
+    else:
+        roof = {"bound": "tensor", "achieved": fb_ach, "peak": tflops_peak, "unit": "TFLOP/s",
+                "frac": fb_ach / tflops_peak, "executed_tflops": mult * fb_ach,
+                "executed_frac": mult * fb_ach / tflops_peak}
     return {"value": bat_flops / max(bat_ms * 1e-3, 1e-12) / 1e12, "unit": UNIT,
             "ms_per_step": bat_ms / max(args.steps, 1), "evaluations": bat_evals,
             "note": "CG iterations with 8 trial images per batched evaluation (rank 0, device time)",
-            "roofline": {"bound": "tensor", "kernel": "forward_dft_batch (8 stacked trial images)",
-                         "achieved": fb_ach, "peak": tflops_peak, "unit": "TFLOP/s", "frac": fb_ach / tflops_peak,
-                         "executed_tflops": mult * fb_ach, "executed_frac": mult * fb_ach / tflops_peak,
+            "roofline": {**roof, "kernel": "forward_dft_batch (8 stacked trial images)",
                          "peak_source": peak_kind,
                          "traffic": _traffic(f"forward_dft_batch8@{workload}@{precision}"),
                          "stage_ms_per_launch": st_b,
@@ -793,7 +819,10 @@ def run_ours(args, rank, world, local):
         if not args.no_batched:
             line["batched_line_search"] = batched_block(rec, p, args, flush, m["img"], args.precision, args.workload)
         if world == 1 and not args.no_cpu_baseline:
-            line["cpu_baseline"] = cpu_baseline(reference_sample(args.workload, oi))
+            try:
+                line["cpu_baseline"] = cpu_baseline(reference_sample(args.workload, oi))
+            except FileNotFoundError as e:  # the reference's compiled sources are not there
+                line["cpu_baseline"] = {"unavailable": str(e)}
         if not args.no_time_to_objective and args.tto_workload_iters > 0:
             line["time_to_objective_workload"] = time_to_objective_workload(
                 rec, p, args.tto_workload_iters, args.tto_workload_iters, args.tto_method)
@@ -841,6 +870,8 @@ def run_ours(args, rank, world, local):
             if cpu_small is not None:
                 try:
                     cpu = cpu_small.result()
+                except FileNotFoundError:  # as for cpu_baseline
+                    cpu = None
                 finally:
                     cpu_pool.shutdown()
                     os.dup2(saved_fd, 1)
