@@ -33,10 +33,9 @@ __device__ __forceinline__ GpVGrid gp_vgrid_hw()
 
 // Op: struct with `using Args = ...;` and `static __device__ void run(const Args &, const GpVGrid &)`.
 // start[0..n]: first block of every instance, start[n] = the launch's blocks.
-template <class Op, int THREADS>
-__global__ void __launch_bounds__(THREADS) k_grouped(const typename Op::Args *__restrict__ args,
-                                                     const int *__restrict__ start, int n,
-                                                     const int *__restrict__ gate)
+template <class Op>
+__device__ __forceinline__ void grouped_body(const typename Op::Args *__restrict__ args, const int *__restrict__ start,
+                                             int n, const int *__restrict__ gate)
 {
     gp_pdl_enter();  // after the kernel before it on the stream (programmatic dependent launch)
     const int b = (int)blockIdx.x;
@@ -55,4 +54,21 @@ __global__ void __launch_bounds__(THREADS) k_grouped(const typename Op::Args *__
     vg.bx = local % vg.nbx;
     vg.by = local / vg.nbx;
     Op::run(a, vg);
+}
+
+template <class Op, int THREADS>
+__global__ void __launch_bounds__(THREADS) k_grouped(const typename Op::Args *__restrict__ args,
+                                                     const int *__restrict__ start, int n,
+                                                     const int *__restrict__ gate)
+{
+    grouped_body<Op>(args, start, n, gate);
+}
+
+// with the registers of MINB blocks per SM (an explicit 1 would let every other stage take more registers, and run slower)
+template <class Op, int THREADS, int MINB>
+__global__ void __launch_bounds__(THREADS, MINB) k_grouped_min(const typename Op::Args *__restrict__ args,
+                                                               const int *__restrict__ start, int n,
+                                                               const int *__restrict__ gate)
+{
+    grouped_body<Op>(args, start, n, gate);
 }

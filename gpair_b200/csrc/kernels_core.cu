@@ -13,6 +13,10 @@
 //                    the adjoint weights of every V2 point and triangle vertex
 //                    (kernel_pow_spec.cl, kernel_bispec.cl, kernel_chi2.cl,
 //                    cpu.c:758-802, cpu.c:371-383)
+//   k_vis_chi2       chi2 alone, by the same sums (trials of a Wolfe search over large data);
+//                    k_vis_chi2_batch of the eight trials of a batched search
+//   k_ug_grad        on the uv grid: the adjoint's x contraction with the gradient assembly of
+//                    k_grad_finalize (the grid's other stages are in uvgrid.cu)
 //   k_adj_weights    c_k = a_k + sum of incident triangle-vertex weights (CSR
 //                    gather, fixed order), C = Re sum c_k V_k
 //   k_adj_simt       adjoint image G[y][x] = Re sum_k c_k Fy[k][y] Fx[k][x],
@@ -188,13 +192,13 @@ __global__ void __launch_bounds__(GP_THREADS) k_prep(const float *__restrict__ s
     }
 }
 
-// Blocks of a pass over n pixels that ends in a sum: a pixel per thread until every SM has a block (64^2 in 16
-// blocks: the FP64 logarithms of four pixels in one thread took as long as the rest of the kernel), then up to
-// four, for a short sum over the blocks
+// Blocks of a pass over n pixels that ends in a sum: a pixel per thread up to 64 blocks (64^2 in 16 blocks: the
+// FP64 logarithms of four pixels in one thread took as long as the rest of the kernel), then up to four, for
+// a short sum over the blocks (up to 148 made the direction updates of 24 instances 35 us instead of 26)
 static int red_grid(long long n)
 {
     int g = gp_cdiv(n, GP_THREADS * 4), one = gp_cdiv(n, GP_THREADS);
-    if (one > 148) one = 148;
+    if (one > 64) one = 64;
     if (g < one) g = one;
     return g < 1 ? 1 : (g > 1184 ? 1184 : g);
 }
@@ -1727,7 +1731,7 @@ __device__ __forceinline__ double2 sum_trial(const TrialVis &T, int j, int k, do
 // its index, data and errors are read once and a uv point's eight values come as one
 // 128-byte line (a thread per datum of one trial used 16 of every 32 bytes).
 // 1024^2 workload, 194,560 + 1,167,360 data: 60 us against 101 (five blocks per SM;
-// 68 with four, 83 with six and spills); 24 instances in one launch: 36 against 40. Every block sums its trials' data in a
+// 68 with four, 83 with six and spills); 24 instances in one launch: 28 against 40. Every block sums its trials' data in a
 // fixed order; the last block sums each trial's partials in block order and runs
 // the controller.
 struct VisChi2BatchArgs {
@@ -2712,11 +2716,14 @@ int gp_stage_args(gpair_ctx *c, int stage, double *trace, void *out, int *nblock
     }
 }
 
-template <class Op, int THREADS>
+template <class Op, int THREADS, int MINB = 0>
 static int group_launch(gpair_ctx *c, const void *d_args, const int *d_start, int n, int total, const int *gate)
 {
-    GP_LAUNCH(c, gp_launch(c, k_grouped<Op, THREADS>, dim3(total), dim3(THREADS), 0,
-                           (const typename Op::Args *)d_args, d_start, n, gate));
+    const auto *args = (const typename Op::Args *)d_args;
+    if constexpr (MINB > 0)
+        GP_LAUNCH(c, gp_launch(c, k_grouped_min<Op, THREADS, MINB>, dim3(total), dim3(THREADS), 0, args, d_start, n, gate));
+    else
+        GP_LAUNCH(c, gp_launch(c, k_grouped<Op, THREADS>, dim3(total), dim3(THREADS), 0, args, d_start, n, gate));
     return GPAIR_OK;
 }
 
@@ -2725,11 +2732,11 @@ int gp_stage_group_launch(gpair_ctx *c, int stage, const void *d_args, const int
 {
     if (total < 1 || n < 1) return GPAIR_ERR_INVALID;
     switch (stage) {
-    case GS_VIS_DATA: return group_launch<VisDataOp, GP_THREADS>(c, d_args, d_start, n, total, gate);
+    case GS_VIS_DATA: return group_launch<VisDataOp, GP_THREADS, 4>(c, d_args, d_start, n, total, gate);
     case GS_ADJ_WEIGHTS: return group_launch<AdjWeightsOp, GP_THREADS>(c, d_args, d_start, n, total, gate);
     case GS_GRAD_FINALIZE: return group_launch<GradFinalizeOp, GP_THREADS>(c, d_args, d_start, n, total, gate);
     case GS_DESCENT: return group_launch<DescentOp, GP_THREADS>(c, d_args, d_start, n, total, gate);
-    case GS_CHI2_BATCH: return group_launch<VisChi2BatchOp, GP_THREADS>(c, d_args, d_start, n, total, gate);
+    case GS_CHI2_BATCH: return group_launch<VisChi2BatchOp, GP_THREADS, 5>(c, d_args, d_start, n, total, gate);
     case GS_UPDATE: return group_launch<UpdateImageOp, 256>(c, d_args, d_start, n, total, gate);
     case GS_CTRL_END: return group_launch<CtrlOp, 32>(c, d_args, d_start, n, total, gate);
     case GS_UG_GRAD: return group_launch<UgGradOp, 256>(c, d_args, d_start, n, total, gate);

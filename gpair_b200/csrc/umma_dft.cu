@@ -1052,6 +1052,9 @@ __device__ __forceinline__ float warp_max_f(float v)
 // fixed order (kernel_update_tempimage.cl, kernel_entropy_gs.cl;
 // gpu.c:860-884).
 #define PR_THREADS 256
+// blocks per SM: 64 registers instead of 80, without spills. Issue-bound (about 150 instructions a trial pixel) with
+// waits between; 8 trials at 1024^2 54 us against 60, 24 instances 40 against 43.
+#define PR_BLOCKS 4
 #define PR_WARPS_MAX (PR_THREADS / 32)
 
 // warps per image row: a power of two, at most PR_WARPS_MAX
@@ -1284,7 +1287,7 @@ __device__ __forceinline__ void tc_prep_rows_body(const PrepRowsArgs &A, const G
 }
 
 template <typename OT, int MODE>
-__global__ void __launch_bounds__(PR_THREADS) k_tc_prep_rows(const PrepRowsArgs a)
+__global__ void __launch_bounds__(PR_THREADS, PR_BLOCKS) k_tc_prep_rows(const PrepRowsArgs a)
 {
     gp_pdl_enter();
     tc_prep_rows_body<OT, MODE>(a, gp_vgrid_hw());
@@ -2640,9 +2643,9 @@ int gp_tc_prep_trials_passes(gpair_ctx *const *ctx, int n, int op)
         return 1;
     const cudaError_t e =
         op == OP_F16
-            ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_grouped<PrepRowsOp<__half, 2>, PR_THREADS>,
+            ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_grouped_min<PrepRowsOp<__half, 2>, PR_THREADS, PR_BLOCKS>,
                                                             PR_THREADS, 0)
-            : cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_grouped<PrepRowsOp<float, 2>, PR_THREADS>,
+            : cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_grouped_min<PrepRowsOp<float, 2>, PR_THREADS, PR_BLOCKS>,
                                                             PR_THREADS, 0);
     if (e != cudaSuccess || per < 1) return 1;
     const long long waves4 = 4LL * per * nsm;
@@ -2655,11 +2658,14 @@ int gp_tc_prep_trials_passes(gpair_ctx *const *ctx, int n, int op)
     return p;
 }
 
-template <class Op, int THREADS>
+template <class Op, int THREADS, int MINB = 0>
 static int tc_group_stage(gpair_ctx *c, const void *d_args, const int *d_start, int n, int total, const int *gate)
 {
-    GP_LAUNCH(c, gp_launch(c, k_grouped<Op, THREADS>, dim3(total), dim3(THREADS), 0,
-                           (const typename Op::Args *)d_args, d_start, n, gate));
+    const auto *args = (const typename Op::Args *)d_args;
+    if constexpr (MINB > 0)
+        GP_LAUNCH(c, gp_launch(c, k_grouped_min<Op, THREADS, MINB>, dim3(total), dim3(THREADS), 0, args, d_start, n, gate));
+    else
+        GP_LAUNCH(c, gp_launch(c, k_grouped<Op, THREADS>, dim3(total), dim3(THREADS), 0, args, d_start, n, gate));
     return GPAIR_OK;
 }
 
@@ -2670,11 +2676,11 @@ int gp_tc_stage_group_launch(gpair_ctx *c, int stage, int op, const void *d_args
     const bool f16 = op == OP_F16;
     switch (stage) {
     case GS_PREP_IMAGE:
-        return f16 ? tc_group_stage<PrepRowsOp<__half, 0>, PR_THREADS>(c, d_args, d_start, n, total, gate)
-                   : tc_group_stage<PrepRowsOp<float, 0>, PR_THREADS>(c, d_args, d_start, n, total, gate);
+        return f16 ? tc_group_stage<PrepRowsOp<__half, 0>, PR_THREADS, PR_BLOCKS>(c, d_args, d_start, n, total, gate)
+                   : tc_group_stage<PrepRowsOp<float, 0>, PR_THREADS, PR_BLOCKS>(c, d_args, d_start, n, total, gate);
     case GS_PREP_TRIALS:
-        return f16 ? tc_group_stage<PrepRowsOp<__half, 2>, PR_THREADS>(c, d_args, d_start, n, total, gate)
-                   : tc_group_stage<PrepRowsOp<float, 2>, PR_THREADS>(c, d_args, d_start, n, total, gate);
+        return f16 ? tc_group_stage<PrepRowsOp<__half, 2>, PR_THREADS, PR_BLOCKS>(c, d_args, d_start, n, total, gate)
+                   : tc_group_stage<PrepRowsOp<float, 2>, PR_THREADS, PR_BLOCKS>(c, d_args, d_start, n, total, gate);
     case GS_BUILD_W:
         return f16 ? tc_group_stage<BuildWOp<__half>, 256>(c, d_args, d_start, n, total, gate)
                    : tc_group_stage<BuildWOp<float>, 256>(c, d_args, d_start, n, total, gate);
