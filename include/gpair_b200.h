@@ -222,6 +222,10 @@ int gpair_dft_tables(int image_width, int nuv, const gpair_uv *uv, float pixella
 
 /* ---- device contexts ---- */
 
+/* Precision modes. In every mode a problem given by (u, v), at least 96 pixels wide and large
+ * enough for its mode goes through a grid of the uv plane (csrc/uvgrid.cu), whose results meet
+ * the mode's bounds; the operands below are then those of its x contraction (GPAIR_PREC_SPLIT16F8:
+ * as GPAIR_PREC_SPLIT16), the other stages FP32 products with FP64 sums. */
 #define GPAIR_PREC_FP32 0     /* CUDA-core FP32 DFT/adjoint (FP32 twiddles) */
 #define GPAIR_PREC_SPLIT16 1  /* tcgen05 f16 hi+lo split operands, 3 products, FP32 accumulate */
 #define GPAIR_PREC_TF32 2     /* tcgen05 kind::tf32, TF32 operands, 1 product, FP32 accumulate */
@@ -459,14 +463,15 @@ int gpair_cg_run(gpair_ctx *ctx, const gpair_cg_params *p, gpair_cg_result *res,
                  double *trace_chi2, double *trace_entropy, double *trace_step, double *trace_beta);
 
 /* Timing hooks for benchmarks: device time of the last gpair_cg_run (ms) and
- * the algorithmic DFT + adjoint flop count it executed. */
+ * the algorithmic DFT + adjoint flop count of its evaluations (the direct sums', also where the
+ * uv grid executes fewer). */
 int gpair_last_run_stats(gpair_ctx *ctx, double *device_ms, double *dft_flops, int *kernel_launches);
 
 /* Stages of one criterion + gradient evaluation, timed with CUDA events on
  * the context's stream (average ms over `reps` repetitions, on the current
  * image): [0] image prep (flux, entropy), [1] forward DFT, [2] V2/T3/chi2 and
- * adjoint weights, [3] per-uv weight gather, [4] adjoint DFT, [5] gradient
- * finalize. Returns the number of stages written (<= max_stages). */
+ * adjoint weights, [3] per-uv weight gather (tensor paths without the uv grid: and the adjoint's
+ * weight operand), [4] adjoint DFT, [5] gradient finalize (uv grid: and its x contraction). Returns the number of stages written (<= max_stages). */
 #define GPAIR_NSTAGES 6
 int gpair_time_stages(gpair_ctx *ctx, int reps, double *stage_ms, int max_stages);
 
