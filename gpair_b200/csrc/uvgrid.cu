@@ -28,8 +28,8 @@
 // contractions measure 2e-6 to 2e-5 (their accumulation truncates; the x
 // contraction's partial sums here are 128 products long).
 // Measured on a B200, one objective with its gradient (events around the
-// stages): 1024^2 and 194,560 uv points 3,240 -> 205 us on the tensor path,
-// 57,000 -> 205 us in FP32; 256^2 and 21,120 uv points 120 -> 99 us and 495 -> 86 us.
+// stages, launches included): 1024^2 and 194,560 uv points 3,240 -> 147 us on the tensor
+// path, 57,000 -> 157 us in FP32; 256^2 and 21,120 uv points 120 -> 80 us and 483 -> 78 us.
 //
 // Everything is summed in a fixed order: uv points are sorted by their grid
 // cell, and the adjoint adds per-cell patches, so there are no atomics.

@@ -12,11 +12,11 @@
 // UG_MIN_WIDTH: on narrower images hundreds of uv points share a grid point, and its FP32 rounding no
 // longer averages out of the gradient (2e-7 to 4e-7 at 55 to 67 pixels, the direct sums 1e-7).
 // UG_MIN_WORK_FP32: where the CUDA-core contractions start to cost more than the grid's fixed launches
-// (147^2 x 1,904 uv: forward 22 against 17 us; 128^2 x 960: 16 against 15).
-// UG_MIN_WORK_TC, _F8: the tensor contractions are within a few us of the grid up to there (256^2 x 960
-// uv: 85 against 91 us for an objective with its gradient; 256^2 x 21,120: 120 against 99). Below it they also keep
-// what long runs reproduce: their rounding, 1e-6 to 1e-5 of the gradient and largest with E4M3 cross
-// terms, is a hundred times the grid's, and a CG run a few iterations on differs by up to 5e-5 with it.
+// (an objective with its gradient, 147^2 x 1,904 uv: 81 us directly, 74 through the grid; 128^2 x 960: 59, 66).
+// UG_MIN_WORK_TC, _F8: below them the direct contractions keep what long runs reproduce: their rounding, 1e-6
+// to 1e-5 of the gradient and largest with E4M3 cross terms, is a hundred times the grid's, and a CG run a
+// few iterations on differs by up to 5e-5 with it. They cost little there (256^2 x 960 uv: 86 us directly, 76
+// through the grid; x 8,960: 95, 79; x 21,120: 120, 80; 128^2 x 960: 74, 70).
 #define UG_MIN_WIDTH 96
 #define UG_MIN_WORK_FP32 4e7
 #define UG_MIN_WORK_TC 1.2e9
