@@ -124,8 +124,10 @@ __global__ void __launch_bounds__(TW4 *TH *(CB / CT)) k_conv3(const float *__res
                 for (int o = 0; o < CT; o += (CT < 4 ? CT : 4)) {
                     if constexpr (CT >= 4)
                         *reinterpret_cast<float4 *>(&wk[o]) = *reinterpret_cast<const float4 *>(&ws[c][k][og * CT + o]);
-                    else
+                    else if constexpr (CT >= 2)
                         *reinterpret_cast<float2 *>(&wk[o]) = *reinterpret_cast<const float2 *>(&ws[c][k][og * CT + o]);
+                    else
+                        wk[o] = ws[c][k][og];
                 }
 #pragma unroll
                 for (int o = 0; o < CT; o++)
@@ -721,7 +723,11 @@ static void conv3_go(int B, int Cout, int H, int W, cudaStream_t st, A... a)
 
 // The widest tile whose blocks still give every SM two: a wider tile reads less
 // halo and more outputs share a thread's loads, but one image of a small level
-// has few tiles, and its chain of Cin x 9 FMAs per output then runs on few SMs.
+// has few tiles, and its chain of Cin x 9 FMAs per output then runs on few SMs. The
+// smallest tile gives a thread one channel, for a second warp beside the chain (the six such
+// layers of one 128^2 image: 187 us with two channels, 138 with one). On the wider tiles
+// fewer channels per thread were slower (4 -> 2: 298 -> 334 us, 2 -> 1: 268 -> 347 of a training step), and
+// so was the smallest tile up to twice its blocks (304 -> 343).
 static void conv3_launch(const float *in, const __nv_bfloat16 *w, const float *bias, const float *skip, float *out,
                          int B, int Cin, int Cout, int H, int W, int relu, int flip, int accumulate, cudaStream_t st)
 {
@@ -733,7 +739,7 @@ static void conv3_launch(const float *in, const __nv_bfloat16 *w, const float *b
     else if (conv3_blocks<2, 8, 16, 2>(B, Cout, H, W) >= want / 4)
         conv3_go<2, 8, 16, 2>(B, Cout, H, W, st, in, w, bias, skip, out, Cin, Cout, H, W, relu, flip, accumulate);
     else
-        conv3_go<2, 4, 8, 2>(B, Cout, H, W, st, in, w, bias, skip, out, Cin, Cout, H, W, relu, flip, accumulate);
+        conv3_go<2, 4, 8, 1>(B, Cout, H, W, st, in, w, bias, skip, out, Cin, Cout, H, W, relu, flip, accumulate);
 }
 
 extern "C" int gpair_cnn_conv3x3(const float *in, const void *w_bf16, const float *bias, const float *skip, float *out,
