@@ -226,6 +226,7 @@ static int build(gpair_ctx *c, int trace_cap, int ls_mode)
     GP_CUDA(c, cudaMalloc(&G->trace, sizeof(double) * 5 * (size_t)trace_cap));
     GP_CUDA(c, cudaGraphCreate(&G->g, 0));
     int rc = add_loop(c, G, G->g);
+    G->buf_gen = c->buf_gen;
     if (!rc) {
         cudaError_t e = cudaGraphInstantiate(&G->exec, G->g, 0);
         if (e != cudaSuccess) {
@@ -976,7 +977,8 @@ int gp_cg_graph_run(gpair_ctx *c, int iterations, int want_trace, int ls_mode, l
     c->cg_graph_mode = ls_mode;
     CgGraph *G = (CgGraph *)c->cg_graph[ls_mode];
     int cap = iterations > 4096 ? iterations : 4096;
-    if (!G || G->precision != c->precision || G->lbfgs != (c->cg_method == 4) ||
+    // buf_gen: a change of the precision mode and back leaves the mode as it was but not the operand buffers
+    if (!G || G->precision != c->precision || G->buf_gen != c->buf_gen || G->lbfgs != (c->cg_method == 4) ||
         (want_trace && G->trace_cap < iterations)) {
         int rc = build(c, cap, ls_mode);
         if (rc) return rc;

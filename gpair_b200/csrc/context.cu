@@ -61,6 +61,7 @@ static void free_problem(gpair_ctx *c)
     gp_tc_free(c);
     gp_ug_free(c);
     c->have_problem = 0;
+    c->buf_gen++;  // a batch's graph holds what was freed
 }
 
 static void free_images(gpair_ctx *c)
