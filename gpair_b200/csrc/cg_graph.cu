@@ -213,6 +213,23 @@ static int add_loop(gpair_ctx *c, CgGraph *G, cudaGraph_t parent)
     return rc;
 }
 
+static int build_into(gpair_ctx *c, CgGraph *G)
+{
+    GP_CUDA(c, cudaMalloc(&G->trace, sizeof(double) * 5 * (size_t)G->trace_cap));
+    GP_CUDA(c, cudaGraphCreate(&G->g, 0));
+    int rc = add_loop(c, G, G->g);
+    G->buf_gen = c->buf_gen;
+    if (!rc) {
+        cudaError_t e = cudaGraphInstantiate(&G->exec, G->g, 0);
+        if (e != cudaSuccess) {
+            snprintf(c->last_error, sizeof(c->last_error), "CG graph instantiate: %s", cudaGetErrorString(e));
+            cudaGetLastError();
+            rc = GPAIR_ERR_CUDA;
+        }
+    }
+    return rc;
+}
+
 static int build(gpair_ctx *c, int trace_cap, int ls_mode)
 {
     graph_free_one(c, ls_mode);
@@ -223,18 +240,8 @@ static int build(gpair_ctx *c, int trace_cap, int ls_mode)
     G->ls_mode = ls_mode;
     G->lbfgs = c->cg_method == 4;
     G->trace_cap = trace_cap;
-    GP_CUDA(c, cudaMalloc(&G->trace, sizeof(double) * 5 * (size_t)trace_cap));
-    GP_CUDA(c, cudaGraphCreate(&G->g, 0));
-    int rc = add_loop(c, G, G->g);
-    G->buf_gen = c->buf_gen;
-    if (!rc) {
-        cudaError_t e = cudaGraphInstantiate(&G->exec, G->g, 0);
-        if (e != cudaSuccess) {
-            snprintf(c->last_error, sizeof(c->last_error), "CG graph instantiate: %s", cudaGetErrorString(e));
-            rc = GPAIR_ERR_CUDA;
-        }
-    }
-    if (rc) graph_free_one(c, ls_mode);
+    const int rc = build_into(c, G);
+    if (rc) graph_free_one(c, ls_mode);  // a graph without its end is not one of this mode
     return rc;
 }
 

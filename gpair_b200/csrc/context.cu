@@ -225,7 +225,9 @@ int gp_direct_prepare(gpair_ctx *c)
     if (!c->gpart) GP_CUDA(c, cudaMalloc(&c->gpart, (size_t)c->gpart_cap * c->npix * sizeof(float)));
     if (!c->fy) GP_CUDA(c, cudaMalloc(&c->fy, nk * c->N * sizeof(float2)));
     GP_CUDA(c, cudaMalloc(&c->fx, nk * c->N * sizeof(float2)));  // last: its presence says that all exist
-    return c->have_uv ? gp_gen_twiddles(c) : GPAIR_OK;
+    const int rc = c->have_uv ? gp_gen_twiddles(c) : GPAIR_OK;
+    if (rc) FREE_DEV(c->fx);
+    return rc;
 }
 
 // Problem upload. uv may be NULL when the twiddles are supplied as tables

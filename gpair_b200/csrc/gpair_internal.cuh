@@ -358,6 +358,7 @@ struct gpair_ctx {
         if (e_ != cudaSuccess) {                                                                    \
             snprintf((ctx)->last_error, sizeof((ctx)->last_error), "%s: %s (%s:%d)", #call,        \
                      cudaGetErrorString(e_), __FILE__, __LINE__);                                   \
+            cudaGetLastError(); /* reported here, not by the next launch's check */                 \
             return GPAIR_ERR_CUDA;                                                                  \
         }                                                                                           \
     } while (0)

@@ -1530,9 +1530,9 @@ int gp_lbfgs_alloc(gpair_ctx *c)
 {
     if (c->lb_s) return GPAIR_OK;
     const size_t n = (size_t)(GP_LB_PAIRS + 1) * c->npix;
-    GP_CUDA(c, cudaMalloc(&c->lb_s, n * sizeof(float)));
-    GP_CUDA(c, cudaMalloc(&c->lb_y, n * sizeof(float)));
-    GP_CUDA(c, cudaMalloc(&c->lb_xold, (size_t)c->npix * sizeof(float)));
+    if (!c->lb_y) GP_CUDA(c, cudaMalloc(&c->lb_y, n * sizeof(float)));
+    if (!c->lb_xold) GP_CUDA(c, cudaMalloc(&c->lb_xold, (size_t)c->npix * sizeof(float)));
+    GP_CUDA(c, cudaMalloc(&c->lb_s, n * sizeof(float)));  // last: its presence says that all exist
     GP_CUDA(c, cudaMemsetAsync(c->lb_s, 0, n * sizeof(float), c->stream));
     GP_CUDA(c, cudaMemsetAsync(c->lb_y, 0, n * sizeof(float), c->stream));
     GP_CUDA(c, cudaMemsetAsync(c->lb_xold, 0, (size_t)c->npix * sizeof(float), c->stream));
@@ -1893,18 +1893,18 @@ int gp_batch_alloc(gpair_ctx *c)
     if (!c->ug && !c->vpart_b) GP_CUDA(c, cudaMalloc(&c->vpart_b, sizeof(float2) * epp_max * nk));
     if (!c->visb && (c->ug || epp_max > VIS_PRESUM_ENTRIES)) GP_CUDA(c, cudaMalloc(&c->visb, sizeof(double2) * nk));
     if (c->image_trials) return GPAIR_OK;
-    GP_CUDA(c, cudaMalloc(&c->image_trials, sizeof(float) * (size_t)GP_NTR * c->npix));
-    GP_CUDA(c, cudaMalloc(&c->partials_b, sizeof(double) * (size_t)GP_NTR * 1024 * 2));
+    if (!c->partials_b) GP_CUDA(c, cudaMalloc(&c->partials_b, sizeof(double) * (size_t)GP_NTR * 1024 * 2));
     int nsm = 148;
     GP_CUDA(c, cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, c->device));
     c->batch_wave[0] = batch_wave_blocks((const void *)k_trials_prep, nsm, GP_NTR);
     c->batch_wave[1] = batch_wave_blocks((const void *)k_vis_chi2_batch, nsm, 1);
+    GP_CUDA(c, cudaMalloc(&c->image_trials, sizeof(float) * (size_t)GP_NTR * c->npix));  // last: its presence says that all exist
     return GPAIR_OK;
 }
 
 void gp_batch_free(gpair_ctx *c)
 {
-    if (c->image_trials || c->vpart_b || c->visb) c->buf_gen++;
+    if (c->image_trials || c->vpart_b || c->partials_b || c->visb) c->buf_gen++;
     if (c->image_trials) cudaFree(c->image_trials);
     if (c->vpart_b) cudaFree(c->vpart_b);
     if (c->partials_b) cudaFree(c->partials_b);

@@ -1672,9 +1672,20 @@ static int tc_set_smem(gpair_ctx *c)
     return GPAIR_OK;
 }
 
+static int tc_build(gpair_ctx *c);
+
+// The tensor state of the context's mode. A state that could not be built to its end (device memory) does not
+// stay: the next call would take its empty buffers for finished ones.
 int gp_tc_prepare(gpair_ctx *c)
 {
     if (!c->have_problem) return GPAIR_OK;  // prepared when the problem is loaded
+    const int rc = tc_build(c);
+    if (rc) gp_tc_free(c);
+    return rc;
+}
+
+static int tc_build(gpair_ctx *c)
+{
     int op, nprod, fop;
     tc_mode(c, &op, &nprod, &fop);
     const int pair = tc_pair_of(c);
@@ -2142,39 +2153,51 @@ int gp_tc_forward_gemm(gpair_ctx *c)
 // whole images, else N rounded up to 256); partial entries of min(Lb, 256) rows.
 int gp_tc_stack_rows(int N) { return N <= 32 ? 32 : N <= 64 ? 64 : N <= 128 ? 128 : round_up(N, TC_BN); }
 
+static int tc_batch_build(gpair_ctx *c, TcState *t)
+{
+    int rc;
+    const int N = c->N;
+    t->Lb = gp_tc_stack_rows(N);
+    const int erows = t->Lb < TC_EPI_COLS ? t->Lb : TC_EPI_COLS;
+    t->epp_b = t->Lb / erows;
+    const size_t rows = (size_t)GP_NTR * t->Lb, n = rows * t->Kx_pad;
+    GP_CUDA(c, cudaMalloc(&t->rscb, sizeof(float) * rows));
+    GP_CUDA(c, cudaMemsetAsync(t->rscb, 0, sizeof(float) * rows, c->stream));
+    GP_CUDA(c, cudaMalloc(&t->imgb_hi, n * t->esz));
+    GP_CUDA(c, cudaMemsetAsync(t->imgb_hi, 0, n * t->esz, c->stream));
+    const int bbox = t->pair ? 128 : TC_BN;
+    if ((rc = tc_make_map(c, &t->m_imgb_hi, t->imgb_hi, (long long)rows, t->Kx_pad, bbox, t->esz))) return rc;
+    if (t->fop == OP_F16F8) {
+        GP_CUDA(c, cudaMalloc(&t->imgb8h, n));
+        GP_CUDA(c, cudaMemsetAsync(t->imgb8h, 0, n, c->stream));
+        GP_CUDA(c, cudaMalloc(&t->imgb8l, n));
+        GP_CUDA(c, cudaMemsetAsync(t->imgb8l, 0, n, c->stream));
+        if ((rc = tc_make_map8(c, &t->m_imgb8h, t->imgb8h, (long long)rows, t->Kx_pad, bbox))) return rc;
+        if ((rc = tc_make_map8(c, &t->m_imgb8l, t->imgb8l, (long long)rows, t->Kx_pad, bbox))) return rc;
+        t->m_imgb_lo = t->m_imgb_hi;  // not loaded by the OP_F16F8 forward
+    } else if (t->nprod == 3) {
+        GP_CUDA(c, cudaMalloc(&t->imgb_lo, n * t->esz));
+        GP_CUDA(c, cudaMemsetAsync(t->imgb_lo, 0, n * t->esz, c->stream));
+        if ((rc = tc_make_map(c, &t->m_imgb_lo, t->imgb_lo, (long long)rows, t->Kx_pad, bbox, t->esz))) return rc;
+    } else {
+        t->m_imgb_lo = t->m_imgb_hi;
+    }
+    return GPAIR_OK;
+}
+
 int gp_tc_batch_prepare(gpair_ctx *c, int *epp)
 {
     int rc;
     TcState *t = tc_state_ready(c, &rc);
     if (rc) return rc;
-    if (!t->imgb_hi) {
-        const int N = c->N;
-        t->Lb = gp_tc_stack_rows(N);
-        const int erows = t->Lb < TC_EPI_COLS ? t->Lb : TC_EPI_COLS;
-        t->epp_b = t->Lb / erows;
-        const size_t rows = (size_t)GP_NTR * t->Lb, n = rows * t->Kx_pad;
-        GP_CUDA(c, cudaMalloc(&t->rscb, sizeof(float) * rows));
-        GP_CUDA(c, cudaMemsetAsync(t->rscb, 0, sizeof(float) * rows, c->stream));
-        GP_CUDA(c, cudaMalloc(&t->imgb_hi, n * t->esz));
-        GP_CUDA(c, cudaMemsetAsync(t->imgb_hi, 0, n * t->esz, c->stream));
-        const int bbox = t->pair ? 128 : TC_BN;
-        if ((rc = tc_make_map(c, &t->m_imgb_hi, t->imgb_hi, (long long)rows, t->Kx_pad, bbox, t->esz))) return rc;
-        if (t->fop == OP_F16F8) {
-            GP_CUDA(c, cudaMalloc(&t->imgb8h, n));
-            GP_CUDA(c, cudaMemsetAsync(t->imgb8h, 0, n, c->stream));
-            GP_CUDA(c, cudaMalloc(&t->imgb8l, n));
-            GP_CUDA(c, cudaMemsetAsync(t->imgb8l, 0, n, c->stream));
-            if ((rc = tc_make_map8(c, &t->m_imgb8h, t->imgb8h, (long long)rows, t->Kx_pad, bbox))) return rc;
-            if ((rc = tc_make_map8(c, &t->m_imgb8l, t->imgb8l, (long long)rows, t->Kx_pad, bbox))) return rc;
-            t->m_imgb_lo = t->m_imgb_hi;  // not loaded by the OP_F16F8 forward
-        } else if (t->nprod == 3) {
-            GP_CUDA(c, cudaMalloc(&t->imgb_lo, n * t->esz));
-            GP_CUDA(c, cudaMemsetAsync(t->imgb_lo, 0, n * t->esz, c->stream));
-            if ((rc = tc_make_map(c, &t->m_imgb_lo, t->imgb_lo, (long long)rows, t->Kx_pad, bbox, t->esz)))
-                return rc;
-        } else {
-            t->m_imgb_lo = t->m_imgb_hi;
+    if (!t->imgb_hi && (rc = tc_batch_build(c, t))) {
+        // the whole stack or none of it
+        void **bufs[] = {(void **)&t->rscb, &t->imgb_hi, &t->imgb_lo, &t->imgb8h, &t->imgb8l};
+        for (void **b : bufs) {
+            if (*b) cudaFree(*b);
+            *b = nullptr;
         }
+        return rc;
     }
     if (t->grid && (rc = gp_ug_batch_alloc(c))) return rc;
     c->epp = t->epp_b;

@@ -853,8 +853,8 @@ int gp_ug_batch_alloc(gpair_ctx *c)
     UgState *g = (UgState *)c->ug;
     if (g->gridb) return GPAIR_OK;
     const size_t rows = (size_t)GP_NTR * gp_tc_stack_rows(c->N);
-    GP_CUDA(c, cudaMalloc(&g->Tb, sizeof(float) * UG_MAX_SPLITS * rows * g->ldT));
-    GP_CUDA(c, cudaMalloc(&g->gridb, sizeof(float2) * GP_NTR * (size_t)g->cells));
+    if (!g->Tb) GP_CUDA(c, cudaMalloc(&g->Tb, sizeof(float) * UG_MAX_SPLITS * rows * g->ldT));
+    GP_CUDA(c, cudaMalloc(&g->gridb, sizeof(float2) * GP_NTR * (size_t)g->cells));  // last: its presence says that both exist
     return GPAIR_OK;
 }
 
