@@ -329,6 +329,7 @@ extern "C" int gpair_set_problem(gpair_ctx *c, int N, float pix, int nuv, const 
 extern "C" int gpair_set_precision(gpair_ctx *c, int mode)
 {
     if (!c || mode < GPAIR_PREC_FP32 || mode > GPAIR_PREC_SPLIT16F8) return GPAIR_ERR_INVALID;
+    GP_CUDA(c, cudaSetDevice(c->device));  // the mode's buffers are allocated here
     int old = c->precision;
     c->precision = mode;
     if (c->have_problem) {
@@ -435,6 +436,7 @@ static void stage_collect(gpair_ctx *c)
 extern "C" int gpair_set_tc_pair(gpair_ctx *c, int on)
 {
     if (!c) return GPAIR_ERR_INVALID;
+    GP_CUDA(c, cudaSetDevice(c->device));
     c->tc_pair = on ? 1 : 0;
     gp_cg_graph_free(c);  // captured graphs hold the other kernel variant
     if (c->precision != GPAIR_PREC_FP32 && c->have_problem && c->have_uv) return gp_tc_prepare(c);

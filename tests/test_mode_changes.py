@@ -57,3 +57,26 @@ def test_batch_after_a_new_problem_is_refused(precision, search):
     b.close()
     for r in recs:
         r.close()
+
+
+def _devices():
+    import torch
+    return torch.cuda.device_count() if torch.cuda.is_available() else 0
+
+
+@pytest.mark.skipif(_devices() < 2, reason="needs two devices")
+def test_mode_of_a_context_on_another_device():
+    """One thread with a context on each device: a change of the first one's mode allocates on its own device."""
+    p = _problem(330, _freq("inner", 20001, 1), 300, 2)
+    recs = [g.Reconstructor(d) for d in (0, 1)]
+    for r in recs:
+        r.set_problem(p)
+        r.set_image(_image(330, 3))
+    got = []
+    for r in recs[::-1] + recs:  # the current device is the other one's at every second step
+        r.set_precision(g.PREC_SPLIT16)
+        got.append(r.criterion()[0])
+        r.set_precision(g.PREC_FP32)
+    assert len(set(got)) == 1
+    for r in recs:
+        r.close()
