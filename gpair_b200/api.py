@@ -130,6 +130,7 @@ def lib() -> C.CDLL:
         L.gpair_set_problem.argtypes = [vp, i, f, i, vp, i, i, vp, vp, vp, vp, vp, vp]
         L.gpair_set_precision.argtypes = [vp, i]
         L.gpair_get_precision.argtypes = [vp]
+        L.gpair_uv_grid.argtypes = [vp, i]
         L.gpair_set_image.argtypes = [vp, i, vp]
         L.gpair_get_image.argtypes = [vp, i, vp]
         L.gpair_criterion.argtypes = [vp, i, C.POINTER(d), C.POINTER(d)]
@@ -473,6 +474,13 @@ class Reconstructor:
 
     def set_precision(self, mode: int):
         self._c(self._L.gpair_set_precision(self.h, mode))
+
+    def uv_grid(self, mode: int = -1) -> bool:
+        """Whether the problem's contractions go through the uv grid in a precision mode (-1: the current one)."""
+        rc = self._L.gpair_uv_grid(self.h, mode)
+        if rc < 0:
+            self._c(rc)
+        return rc == 1
 
     def set_image(self, img: np.ndarray, which: int = IMG_CURR):
         a = np.ascontiguousarray(img, np.float32).ravel()

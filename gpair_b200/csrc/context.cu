@@ -347,6 +347,13 @@ extern "C" int gpair_set_precision(gpair_ctx *c, int mode)
 
 extern "C" int gpair_get_precision(gpair_ctx *c) { return c ? c->precision : -1; }
 
+extern "C" int gpair_uv_grid(gpair_ctx *c, int mode)
+{
+    if (!c || mode < -1 || mode > GPAIR_PREC_SPLIT16F8) return GPAIR_ERR_INVALID;
+    if (!c->have_problem) return GPAIR_ERR_STATE;
+    return gp_ug_takes(c, mode < 0 ? c->precision : mode) ? 1 : 0;
+}
+
 extern "C" int gpair_set_image(gpair_ctx *c, int which, const float *image)
 {
     if (!c || !image || !c->image) return GPAIR_ERR_STATE;

@@ -551,10 +551,11 @@ int gp_tc_stage_group_launch(gpair_ctx *c, int stage, int op, const void *d_args
                              int total, const int *gate);
 // tables and partial-sum buffers of the direct contractions (no-op when they exist)
 int gp_direct_prepare(gpair_ctx *c);
-// uv grid (uvgrid.cu): plan of a problem (none where no mode would take it), the choice for the
-// context's precision mode (sets c->ug), x contraction on the CUDA cores, visibilities from T
+// uv grid (uvgrid.cu): plan of a problem (none where no mode would take it), whether a precision mode
+// takes it, the choice for the context's mode (sets c->ug), x contraction on the CUDA cores, visibilities from T
 // (1 or GP_NTR images), adjoint up to S
 int gp_ug_plan(gpair_ctx *c, const gpair_uv *uv);
+bool gp_ug_takes(const gpair_ctx *c, int precision);
 void gp_ug_choose(gpair_ctx *c);
 void gp_ug_free(gpair_ctx *c);
 int gp_ug_batch_alloc(gpair_ctx *c);

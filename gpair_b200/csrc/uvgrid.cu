@@ -167,10 +167,12 @@ static double ug_min_work(int precision)
     return precision == GPAIR_PREC_SPLIT16F8 ? UG_MIN_WORK_F8 : UG_MIN_WORK_TC;
 }
 
-void gp_ug_choose(gpair_ctx *c)
+bool gp_ug_takes(const gpair_ctx *c, int precision)
 {
-    c->ug = c->ug_plan && 2.0 * (double)c->N * c->N * (double)c->nuv >= ug_min_work(c->precision) ? c->ug_plan : nullptr;
+    return c->ug_plan && 2.0 * (double)c->N * c->N * (double)c->nuv >= ug_min_work(precision);
 }
+
+void gp_ug_choose(gpair_ctx *c) { c->ug = gp_ug_takes(c, c->precision) ? c->ug_plan : nullptr; }
 
 void gp_ug_free(gpair_ctx *c)
 {

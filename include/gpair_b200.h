@@ -255,6 +255,9 @@ int gpair_set_problem(gpair_ctx *ctx, int image_width, float pixellation, int nu
                       const int64_t *uvpnt, const int16_t *sign, const float *default_model);
 int gpair_set_precision(gpair_ctx *ctx, int mode);
 int gpair_get_precision(gpair_ctx *ctx);
+/* Whether the loaded problem's contractions go through the grid of the uv plane in a precision mode (1)
+ * or are direct sums (0); mode -1: the current one. */
+int gpair_uv_grid(gpair_ctx *ctx, int mode);
 int gpair_set_image(gpair_ctx *ctx, int which, const float *image);
 int gpair_get_image(gpair_ctx *ctx, int which, float *image);
 
