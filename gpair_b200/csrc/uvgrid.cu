@@ -167,9 +167,20 @@ static double ug_min_work(int precision)
     return precision == GPAIR_PREC_SPLIT16F8 ? UG_MIN_WORK_F8 : UG_MIN_WORK_TC;
 }
 
+// The mode's direct sums 2 N nuv an image row against the grid's y contractions nbx J (uvgrid.cuh); 0: not asked
+static double ug_wide_ratio(int precision)
+{
+    if (precision == GPAIR_PREC_FP32 || precision == GPAIR_PREC_TF32X3) return 0.0;
+    return precision == GPAIR_PREC_SPLIT16 ? UG_WIDE_RATIO_TC : UG_WIDE_RATIO_F8;
+}
+
 bool gp_ug_takes(const gpair_ctx *c, int precision)
 {
-    return c->ug_plan && 2.0 * (double)c->N * c->N * (double)c->nuv >= ug_min_work(precision);
+    const UgState *g = (const UgState *)c->ug_plan;
+    if (!g) return false;
+    const double row = 2.0 * (double)c->N * (double)c->nuv;
+    return row * (double)c->N >= ug_min_work(precision) &&
+           row >= ug_wide_ratio(precision) * (double)g->nbx * (double)g->J;
 }
 
 void gp_ug_choose(gpair_ctx *c) { c->ug = gp_ug_takes(c, c->precision) ? c->ug_plan : nullptr; }

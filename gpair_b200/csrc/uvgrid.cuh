@@ -8,7 +8,8 @@
 #define UG_MAX_SPLITS 8  // partial sums of the x contraction
 
 // A problem takes the grid when the image is at least UG_MIN_WIDTH wide, its direct work 2 N^2 nuv is at
-// least UG_MIN_WORK_* of the precision mode and UG_GRID_RATIO times the grid's own contractions.
+// least UG_MIN_WORK_* of the precision mode and UG_GRID_RATIO times the grid's own contractions, and the
+// coverage is not too wide for the mode (UG_WIDE_RATIO_*).
 // UG_MIN_WIDTH: on narrower images hundreds of uv points share a grid point, and its FP32 rounding no
 // longer averages out of the gradient (2e-7 to 4e-7 at 55 to 67 pixels, the direct sums 1e-7).
 // UG_MIN_WORK_FP32: where the CUDA-core contractions start to cost more than the grid's fixed launches
@@ -17,6 +18,18 @@
 // to 1e-5 of the gradient and largest with E4M3 cross terms, is a hundred times the grid's, and a CG run a
 // few iterations on differs by up to 5e-5 with it. They cost little there (256^2 x 960 uv: 86 us directly, 76
 // through the grid; x 8,960: 95, 79; x 21,120: 120, 80; 128^2 x 960: 74, 70).
+// UG_WIDE_RATIO_TC (SPLIT16), _F8 (SPLIT16F8 and TF32, whose direct forwards cost two thirds): on a wide
+// coverage the grid's y contractions, FP64 on nbx (2 J + 1) grid points, are slower than the tensor cores' direct sums,
+// which the ratio above does not see. One objective with its gradient + eight trials, direct and through the grid, split-f16:
+// half a cycle per pixel each way, 1024^2 x 8,924 uv 335 + 626 us and 3,880 + 6,060, 512^2 x 8,412 112 + 127 and 613 + 722,
+// x 134,607 717 + 1,938 and 729 + 954; a quarter of a cycle, 512^2 x 12,907 131 + 183 and 224 + 252, x 51,631
+// 311 + 749 and 232 + 315. At the lines an objective with its gradient and two batches of eight trials cost the same within a
+// fifth; an ordinary coverage (1024^2: 60 x 119 grid points) is far above them. The direct sums are less accurate there, within
+// the modes' bounds (515^2 x 9,001 over the whole plane, adjoint of given weights: 7e-6 against 1.5e-7). FP32 and
+// TF32X3 have no such line, because that difference passes their bounds: TF32X3 1.4e-5 directly (bound 1e-5), FP32 gradient
+// 1.6e-5 directly and 1.8e-6 through the grid.
+#define UG_WIDE_RATIO_TC 300.0
+#define UG_WIDE_RATIO_F8 450.0
 #define UG_MIN_WIDTH 96
 #define UG_MIN_WORK_FP32 4e7
 #define UG_MIN_WORK_TC 1.2e9

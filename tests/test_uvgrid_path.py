@@ -1,6 +1,6 @@
 """Which path a problem takes: the uv grid or direct sums, by the context's own answer (gpair_uv_grid).
 
-No tolerances here: paths are compared with what the rule says, runs with runs bit for bit.
+Paths are compared with what the rule says, runs with runs bit for bit; the one tolerance is the library's 1e-5.
 """
 import numpy as np
 import pytest
@@ -107,3 +107,55 @@ def test_wolfe_batch_with_instances_on_the_grid():
     finally:
         for r in recs:
             r.close()
+
+
+def _extent(p):
+    """Grid columns and rows each way (nbx, J) of a problem: first window points floor(2 N |f|) - 3, 8 of them."""
+    f = U.RPMAS * np.float64(np.float32(p.pixellation)) * p.uv[:, :2].astype(np.float64)
+    f -= np.rint(f)
+    f[f[:, 0] < 0] *= -1
+    j = np.floor(f * 2 * p.width).astype(int) - 3
+    return j[:, 0].max() - j[:, 0].min() + 8, max((-j[:, 1]).max(), (j[:, 1] + 7).max())
+
+
+@pytest.mark.parametrize("N", [256, 301])
+@pytest.mark.parametrize("mode,ratio", [(g.PREC_SPLIT16, 300), (g.PREC_SPLIT16F8, 450), (g.PREC_TF32, 450)])
+def test_wide_coverage_line(N, mode, ratio):
+    """A few points at the edge of the plane, the others inside: the last uv count left to the direct sums, the first on the grid."""
+    edge = np.array([[0.49, 0.49], [0.49, -0.49], [0.0, 0.0]])
+
+    def problem(nuv):
+        f = _freq("inner", nuv, 1)
+        f[:3] = edge
+        return _problem(N, f, 10, 2)
+
+    nbx, J = _extent(problem(10))
+    first = int(np.ceil(ratio * nbx * J / (2 * N)))
+    for nuv, grid in ((first - 1, False), (first, True)):
+        p = problem(nuv)
+        assert _extent(p) == (nbx, J)
+        with g.Reconstructor(0) as r:
+            r.set_problem(p)
+            assert r.uv_grid(mode) == grid
+            assert r.uv_grid(g.PREC_FP32) and r.uv_grid(g.PREC_TF32X3)
+
+
+@pytest.mark.parametrize("N,nuv", [(515, 9001), (330, 8200)])
+def test_wide_coverage_on_either_path(N, nuv):
+    """Points over the whole plane: V, chi2 and the adjoint of given weights within 1e-5 on the path that each mode takes."""
+    p = _problem(N, _freq("full", nuv, 5), 500, 6)
+    img = _image(N, 7)
+    V, chi2, _ = U._direct(p, img)
+    rng = np.random.default_rng(4)
+    w = (rng.standard_normal(nuv) + 1j * rng.standard_normal(nuv)).astype(np.complex64)
+    adj = U._adjoint(p, w)
+    with g.Reconstructor(0) as r:
+        r.set_problem(p)
+        for mode, grid in ((g.PREC_SPLIT16, False), (g.PREC_FP32, True), (g.PREC_SPLIT16F8, False), (g.PREC_TF32X3, True)):
+            r.set_precision(mode)
+            assert r.uv_grid() == grid
+            r.set_image(img)
+            c, _ = r.criterion()
+            assert np.abs(r.visibilities() - V).max() <= 1e-5
+            assert abs(c - chi2) <= 1e-5 * chi2
+            assert np.linalg.norm(r.adjoint_image(w) - adj) <= 1e-5 * np.linalg.norm(adj)
