@@ -55,12 +55,15 @@ static void free_problem(gpair_ctx *c)
     gp_cg_graph_free(c);
     FREE_DEV(c->data); FREE_DEV(c->data_err); FREE_DEV(c->mock);
     FREE_DEV(c->tri); FREE_DEV(c->phasor); FREE_DEV(c->uvc);
-    FREE_DEV(c->fx); FREE_DEV(c->fy); FREE_DEV(c->vpart); FREE_DEV(c->visd); FREE_DEV(c->visi);
-    FREE_DEV(c->trib); FREE_DEV(c->cw); FREE_DEV(c->inc_off); FREE_DEV(c->inc_idx); FREE_DEV(c->gpart);
+    FREE_DEV(c->direct_mem); FREE_DEV(c->visd); FREE_DEV(c->visi);
+    c->fx = c->fy = c->vpart = nullptr;
+    c->gpart = nullptr;
+    FREE_DEV(c->trib); FREE_DEV(c->cw); FREE_DEV(c->inc_off); FREE_DEV(c->inc_idx);
     gp_batch_free(c);
     gp_tc_free(c);
     gp_ug_free(c);
     c->have_problem = 0;
+    c->path_ready = 0;
     c->buf_gen++;  // a batch's graph holds what was freed
 }
 
@@ -214,19 +217,37 @@ int gp_build_incidence(gpair_ctx *c, const int64_t *uvpnt)
 
 // What the direct contractions need: tables, partial visibility entries (the
 // CUDA-core forward's row tiles or the tensor forward's entries) and split-K
-// partial images. A problem on the uv grid has none until a precision mode
-// that takes the direct contractions is set.
+// partial images, in one allocation (an allocation costs 0.3 to 0.4 ms). A problem on the uv grid has none until a
+// precision mode that takes the direct contractions is set.
 int gp_direct_prepare(gpair_ctx *c)
 {
-    if (c->fx) return GPAIR_OK;
+    if (c->direct_mem) return GPAIR_OK;
     const size_t nk = c->nuv ? c->nuv : 1;
     const int mt = gp_cdiv(c->N, 64), mt_cap = mt > gp_tc_forward_entries(c->N) ? mt : gp_tc_forward_entries(c->N);
-    if (!c->vpart) GP_CUDA(c, cudaMalloc(&c->vpart, (size_t)mt_cap * nk * sizeof(float2)));
-    if (!c->gpart) GP_CUDA(c, cudaMalloc(&c->gpart, (size_t)c->gpart_cap * c->npix * sizeof(float)));
-    if (!c->fy) GP_CUDA(c, cudaMalloc(&c->fy, nk * c->N * sizeof(float2)));
-    GP_CUDA(c, cudaMalloc(&c->fx, nk * c->N * sizeof(float2)));  // last: its presence says that all exist
+    auto padded = [](size_t n) { return (n + 255) & ~(size_t)255; };
+    const size_t table = padded(nk * c->N * sizeof(float2)), vis = padded((size_t)mt_cap * nk * sizeof(float2));
+    GP_CUDA(c, cudaMalloc(&c->direct_mem, 2 * table + vis + (size_t)c->gpart_cap * c->npix * sizeof(float)));
+    unsigned char *p = (unsigned char *)c->direct_mem;
+    c->fx = (float2 *)p;
+    c->fy = (float2 *)(p + table);
+    c->vpart = (float2 *)(p + 2 * table);
+    c->gpart = (float *)(p + 2 * table + vis);
     const int rc = c->have_uv ? gp_gen_twiddles(c) : GPAIR_OK;
-    if (rc) FREE_DEV(c->fx);
+    if (rc) {
+        FREE_DEV(c->direct_mem);
+        c->fx = c->fy = c->vpart = nullptr;
+        c->gpart = nullptr;
+    }
+    return rc;
+}
+
+int gp_path_prepare(gpair_ctx *c)
+{
+    if (c->path_ready) return GPAIR_OK;
+    int rc = gp_ug_choose(c);
+    if (!rc && !c->ug) rc = gp_direct_prepare(c);
+    if (!rc && c->precision != GPAIR_PREC_FP32) rc = gp_tc_prepare(c);
+    c->path_ready = !rc;
     return rc;
 }
 
@@ -302,17 +323,16 @@ int gp_set_problem_core(gpair_ctx *c, int N, float pix, int nuv, const gpair_uv 
         std::vector<float2> uvc(nuv);
         for (int k = 0; k < nuv; k++) uvc[k] = make_float2(uv[k].u, uv[k].v);
         GP_CUDA(c, cudaMemcpyAsync(c->uvc, uvc.data(), nuv * sizeof(float2), cudaMemcpyHostToDevice, c->stream));
-        if ((rc = gp_ug_plan(c, uv))) return rc;
+        if ((rc = gp_ug_scan(c, uv))) return rc;
     }
-    gp_ug_choose(c);
-    if (!c->ug && (rc = gp_direct_prepare(c))) return rc;
-    rc = gp_build_incidence(c, uvpnt);
-    if (rc) return rc;
     c->have_problem = 1;
-    if (c->precision != GPAIR_PREC_FP32 && uv) {
-        // with reference tables (uv == NULL) the operands are built lazily, once the tables are on the device
-        rc = gp_tc_prepare(c);
-        if (rc) return rc;
+    // the path of the mode, whose kernels run beside the host's sorting of the triangles; with reference
+    // tables (uv == NULL) its tensor operands are built once the tables are on the device
+    rc = uv ? gp_path_prepare(c) : gp_direct_prepare(c);
+    if (!rc) rc = gp_build_incidence(c, uvpnt);
+    if (rc) {
+        c->have_problem = 0;
+        return rc;
     }
     GP_CUDA(c, cudaStreamSynchronize(c->stream));
     return GPAIR_OK;
@@ -333,12 +353,11 @@ extern "C" int gpair_set_precision(gpair_ctx *c, int mode)
     int old = c->precision;
     c->precision = mode;
     if (c->have_problem) {
-        gp_ug_choose(c);
-        int rc = c->ug ? GPAIR_OK : gp_direct_prepare(c);
-        if (!rc && mode != GPAIR_PREC_FP32) rc = gp_tc_prepare(c);
+        c->path_ready = 0;
+        const int rc = gp_path_prepare(c);
         if (rc) {
             c->precision = old;
-            gp_ug_choose(c);
+            c->ug = gp_ug_takes(c, old) ? c->ug_plan : nullptr;  // the next evaluation finishes it
             return rc;
         }
     }
@@ -507,7 +526,8 @@ extern "C" int gpair_last_run_stage_ms(gpair_ctx *c, double *ms, int *counts, in
 
 int gp_eval_criterion(gpair_ctx *c, int which, int trial)
 {
-    int rc;
+    int rc = gp_path_prepare(c);
+    if (rc) return rc;
     gp_stage_begin(c, 0);
     // tensor path: image (or trial image), its sums and its forward operand in one pass
     const bool tc = c->precision != GPAIR_PREC_FP32;
@@ -825,6 +845,7 @@ static int cg_prepare(gpair_ctx *c, const gpair_cg_params *p, int want_trace, Cg
     c->fuse_ctrl = -1;
     c->fuse_handles = 0;
     c->cg_method = p->method;
+    if ((rc = gp_path_prepare(c))) return rc;  // before the capture
     if (p->method == 4 && (rc = gp_lbfgs_alloc(c))) return rc;
     if (p->line_search == GPAIR_LS_BATCH && (rc = gp_batch_alloc(c))) return rc;
     if ((rc = gp_cg_start(c, cg_params_state(p), p->stop_flag, p->resume))) return rc;
@@ -1042,6 +1063,7 @@ extern "C" int gpair_batch_create_ex(gpair_batch **out, gpair_ctx **ctx, int n, 
     for (int i = 0; i < n && !rc; i++) {
         ctx[i]->fuse_ctrl = -1;
         ctx[i]->fuse_handles = 0;
+        rc = gp_path_prepare(ctx[i]);  // before the capture
     }
     // 2: every stage grouped where the instances allow it, 1: grouped forwards only, 0: independent
     int group = (flags & GPAIR_BATCH_INDEPENDENT) ? 0 : (flags & GPAIR_BATCH_FORWARDS_ONLY) ? 1 : 2;
@@ -1172,11 +1194,12 @@ extern "C" int gpair_time_stages(gpair_ctx *c, int reps, double *ms, int max_sta
 {
     if (!c || !c->have_problem || reps <= 0 || !ms) return GPAIR_ERR_INVALID;
     GP_CUDA(c, cudaSetDevice(c->device));
+    int rc = gp_path_prepare(c);  // not between the events
+    if (rc) return rc;
     const int ns = GPAIR_NSTAGES;
     std::vector<cudaEvent_t> ev((size_t)(ns + 1) * reps);
     for (auto &e : ev) GP_CUDA(c, cudaEventCreate(&e));
     const bool tc = c->precision != GPAIR_PREC_FP32;
-    int rc = GPAIR_OK;
     for (int r = 0; r < reps && !rc; r++) {
         // stages queued back to back: the events time kernels, not host launch gaps
         cudaEvent_t *E = &ev[(size_t)r * (ns + 1)];

@@ -256,6 +256,7 @@ struct gpair_ctx {
     int4 *tri;
     float2 *phasor;
     float2 *uvc;
+    void *direct_mem;  // what the direct contractions' fx, fy, vpart and gpart lie in
     float2 *fx, *fy;
     float2 *vpart;
     double2 *visd;
@@ -281,8 +282,13 @@ struct gpair_ctx {
     // tensor-core operand buffers (GPAIR_PREC_SPLIT16 / TF32), see umma path
     void *tc_state;
     // the DFT and its adjoint through a grid of the uv plane (uvgrid.cu): the problem's plan (UgState), or
-    // null; ug is the plan where the precision mode takes it, null: the direct contractions
+    // null; ug is the plan where the precision mode takes it, null: the direct contractions.
+    // ug_able: some mode may take the grid of ug_nbx columns from ug_jxf and rows -ug_J .. ug_J;
+    // ug_first: every uv point's first window point (x, and y with the conjugation in bit 0), until the plan is built
     void *ug_plan, *ug;
+    int ug_able, ug_nbx, ug_J, ug_jxf;
+    int2 *ug_first;
+    int path_ready;  // what the precision mode's path needs exists (gp_path_prepare)
 
     // handles for layer 1
     gpair_buf h_image, h_image_temp, h_fgn, h_fg, h_dd, h_tg, h_eg, h_dg, h_model;
@@ -551,12 +557,15 @@ int gp_tc_stage_group_launch(gpair_ctx *c, int stage, int op, const void *d_args
                              int total, const int *gate);
 // tables and partial-sum buffers of the direct contractions (no-op when they exist)
 int gp_direct_prepare(gpair_ctx *c);
-// uv grid (uvgrid.cu): plan of a problem (none where no mode would take it), whether a precision mode
-// takes it, the choice for the context's mode (sets c->ug), x contraction on the CUDA cores, visibilities from T
+// what the precision mode's path needs (no-op when it exists): the grid's plan or the direct sums' tables, the
+// tensor operands. Called before every evaluation, and before a capture
+int gp_path_prepare(gpair_ctx *c);
+// uv grid (uvgrid.cu): the grid's extent for a problem's points, whether a precision mode takes it, the
+// choice for the context's mode (sets c->ug, builds the plan if need be), x contraction on the CUDA cores, visibilities from T
 // (1 or GP_NTR images), adjoint up to S
-int gp_ug_plan(gpair_ctx *c, const gpair_uv *uv);
+int gp_ug_scan(gpair_ctx *c, const gpair_uv *uv);
 bool gp_ug_takes(const gpair_ctx *c, int precision);
-void gp_ug_choose(gpair_ctx *c);
+int gp_ug_choose(gpair_ctx *c);
 void gp_ug_free(gpair_ctx *c);
 int gp_ug_batch_alloc(gpair_ctx *c);
 int gp_tc_stack_rows(int N);  // rows per image of the batched trials' operand stack

@@ -330,10 +330,9 @@ int gp_forward(gpair_ctx *c, int which)
         return GPAIR_ERR_STATE; // tensor path requested but unavailable: fail loudly
     }
     const float *img = (which == GPAIR_IMG_TEMP) ? c->image_temp : c->image;
-    if (c->ug) {
-        int rc = gp_ug_x(c, img, 1);
-        return rc ? rc : gp_ug_vis(c, 1);
-    }
+    int rc = gp_path_prepare(c);
+    if (rc) return rc;
+    if (c->ug) return (rc = gp_ug_x(c, img, 1)) ? rc : gp_ug_vis(c, 1);
     c->mt = gp_cdiv(c->N, FB_M);
     return fwd_simt(c, img, c->vpart, 1, nullptr);
 }
@@ -822,6 +821,8 @@ int gp_adjoint(gpair_ctx *c, int which)
 
 int gp_adjoint_contraction(gpair_ctx *c, int which)
 {
+    const int rc = gp_path_prepare(c);
+    if (rc) return rc;
     if (c->ug) return gp_ug_adjoint(c);
     if (c->precision != GPAIR_PREC_FP32) return gp_tc_adjoint(c, which);
     int S = c->splits_simt;
@@ -1875,7 +1876,8 @@ static int batch_wave_blocks(const void *kernel, int nsm, int rows)
 
 int gp_batch_alloc(gpair_ctx *c)
 {
-    int epp_tc = 0;
+    int epp_tc = 0, rc0 = gp_path_prepare(c);
+    if (rc0) return rc0;
     if (c->precision != GPAIR_PREC_FP32) {
         // every time: the tensor state (and its trial operand stack) is rebuilt when
         // the precision or the tile layout changes, the trial images are not

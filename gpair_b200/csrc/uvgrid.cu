@@ -121,36 +121,6 @@ __global__ void k_ug_tables(const double *__restrict__ invphi, int N, int H, dou
     else ctab[i] = v;
 }
 
-// First window points of the uv points (host) and the grid's extent: columns
-// jxf .. jxf + nbx - 1, rows -J .. J. False when a coordinate is not finite.
-static bool ug_extent(const gpair_uv *uv, int nuv, float pix, double M, std::vector<int> &jx0, std::vector<int> &jy0,
-                      std::vector<unsigned char> &flip, int *jxf, int *nbx, int *J)
-{
-    int xmin = 1 << 30, xmax = -(1 << 30), ymax = 0;
-    for (int k = 0; k < nuv; k++) {
-        double a = UG_RPMAS * (double)pix * (double)uv[k].u, b = UG_RPMAS * (double)pix * (double)uv[k].v;
-        if (!isfinite(a) || !isfinite(b)) return false;
-        a -= rint(a);
-        b -= rint(b);
-        flip[k] = a < 0.0;
-        if (flip[k]) {
-            a = -a;
-            b = -b;
-        }
-        jx0[k] = (int)floor(a * M) - (UG_W / 2 - 1);
-        jy0[k] = (int)floor(b * M) - (UG_W / 2 - 1);
-        if (jx0[k] < xmin) xmin = jx0[k];
-        if (jx0[k] > xmax) xmax = jx0[k];
-        const int lo = -jy0[k], hi = jy0[k] + UG_W - 1;
-        if (lo > ymax) ymax = lo;
-        if (hi > ymax) ymax = hi;
-    }
-    *jxf = xmin;
-    *nbx = xmax - xmin + UG_W;
-    *J = ymax;
-    return true;
-}
-
 // Whether the grid's contractions are small beside the direct ones (UG_GRID_RATIO), with one partial sum
 // of the gradient's dot products per 64 x 64 tile
 static bool ug_small(int N, int nuv, int nbx, int J)
@@ -176,46 +146,93 @@ static double ug_wide_ratio(int precision)
 
 bool gp_ug_takes(const gpair_ctx *c, int precision)
 {
-    const UgState *g = (const UgState *)c->ug_plan;
-    if (!g) return false;
+    if (!c->ug_able) return false;
     const double row = 2.0 * (double)c->N * (double)c->nuv;
     return row * (double)c->N >= ug_min_work(precision) &&
-           row >= ug_wide_ratio(precision) * (double)g->nbx * (double)g->J;
+           row >= ug_wide_ratio(precision) * (double)c->ug_nbx * (double)c->ug_J;
 }
 
-void gp_ug_choose(gpair_ctx *c) { c->ug = gp_ug_takes(c, c->precision) ? c->ug_plan : nullptr; }
+// The points' first window points and the extent of the grid, columns ug_jxf .. ug_jxf + ug_nbx - 1 and rows -ug_J .. ug_J;
+// whether some precision mode may take it (c->ug_able; not with a coordinate that is not finite). The sizes of the
+// context are set.
+int gp_ug_scan(gpair_ctx *c, const gpair_uv *uv)
+{
+    const int N = c->N, nuv = c->nuv;
+    if (!uv || N < UG_MIN_WIDTH || 2.0 * (double)N * N * (double)nuv < UG_MIN_WORK_FP32) return GPAIR_OK;
+    const double M = UG_OVERSAMPLING * N, pix = (double)c->pix;
+    int2 *first = (int2 *)malloc(sizeof(int2) * (size_t)nuv);
+    if (!first) return GPAIR_ERR_ALLOC;
+    int xmin = 1 << 30, xmax = -(1 << 30), ymax = 0;
+    bool ok = true;
+    for (int k = 0; k < nuv && ok; k++) {
+        double a = UG_RPMAS * pix * (double)uv[k].u, b = UG_RPMAS * pix * (double)uv[k].v;
+        ok = isfinite(a) && isfinite(b);
+        if (!ok) break;
+        a -= rint(a);
+        b -= rint(b);
+        const bool flip = a < 0.0;
+        if (flip) {
+            a = -a;
+            b = -b;
+        }
+        const int jx = (int)floor(a * M) - (UG_W / 2 - 1), jy = (int)floor(b * M) - (UG_W / 2 - 1);
+        first[k] = make_int2(jx, 2 * jy + (flip ? 1 : 0));
+        if (jx < xmin) xmin = jx;
+        if (jx > xmax) xmax = jx;
+        const int lo = -jy, hi = jy + UG_W - 1;
+        if (lo > ymax) ymax = lo;
+        if (hi > ymax) ymax = hi;
+    }
+    const int nbx = xmax - xmin + UG_W;
+    if (!ok || !ug_small(N, nuv, nbx, ymax)) {
+        free(first);
+        return GPAIR_OK;
+    }
+    c->ug_first = first;
+    c->ug_jxf = xmin;
+    c->ug_nbx = nbx;
+    c->ug_J = ymax;
+    c->ug_able = 1;
+    return GPAIR_OK;
+}
 
-void gp_ug_free(gpair_ctx *c)
+static void ug_free_plan(gpair_ctx *c)
 {
     UgState *g = (UgState *)c->ug_plan;
-    if (!g) return;
-    void *bufs[] = {g->src, g->base, g->wts, g->phase, g->chunk, g->cst, g->ftab, g->ctab, g->invphi,
-                    g->T, g->grid, g->patch, g->cgrid, g->S, g->Tb, g->gridb};
-    for (void *b : bufs)
-        if (b) cudaFree(b);
-    free(g);
+    if (g) {
+        void *bufs[] = {g->mem, g->Tb, g->gridb};
+        for (void *b : bufs)
+            if (b) cudaFree(b);
+        free(g);
+    }
     c->ug_plan = nullptr;
     c->ug = nullptr;
 }
 
-// Builds the plan of a problem given by (u, v) when some precision mode would
-// take it. The sizes of the context are set.
-int gp_ug_plan(gpair_ctx *c, const gpair_uv *uv)
+void gp_ug_free(gpair_ctx *c)
 {
-    gp_ug_free(c);
-    const int N = c->N, nuv = c->nuv;
-    if (!uv || N < UG_MIN_WIDTH || 2.0 * (double)N * N * (double)nuv < UG_MIN_WORK_FP32) return GPAIR_OK;
+    ug_free_plan(c);
+    free(c->ug_first);
+    c->ug_first = nullptr;
+    c->ug_able = 0;
+}
+
+// Builds the plan of the problem that gp_ug_scan looked over, when a mode first takes it. A new context is in FP32, so a
+// program that goes on to a mode with direct sums has built a plan that it does not use. An allocation costs 0.3 to
+// 0.4 ms, so the plan is one, and so are the direct sums' buffers: such a context's preparation takes what it took without the
+// grid (set_problem and set_precision, 256^2, split-f16/E4M3: 8,000 uv points 4.2 to 4.4 ms without the grid, 4.8 to 5.0 with an
+// allocation per array, 4.3 now; 21,120 5.4, 6.0 to 6.3, 5.0 to 5.4). A context whose mode is set before the problem builds its mode's alone.
+static int ug_plan(gpair_ctx *c)
+{
+    const int N = c->N, nuv = c->nuv, jxf = c->ug_jxf, nbx = c->ug_nbx, J = c->ug_J;
     const double M = UG_OVERSAMPLING * N;
-    std::vector<int> jx0(nuv), jy0(nuv);
-    std::vector<unsigned char> flip(nuv);
-    int jxf, nbx, J;
-    if (!ug_extent(uv, nuv, c->pix, M, jx0, jy0, flip, &jxf, &nbx, &J)) return GPAIR_OK;
-    if (!ug_small(N, nuv, nbx, J)) return GPAIR_OK;
     const int cells = nbx * (2 * J + 1);
     // counting sort by cell (stable), then runs of at most 32 points of one cell
     std::vector<int> off((size_t)cells + 1, 0), src(nuv), base(nuv), cst((size_t)cells + 1, 0);
     std::vector<int2> chunk;
-    for (int k = 0; k < nuv; k++) off[(size_t)(jy0[k] + J) * nbx + (jx0[k] - jxf) + 1]++;
+    const int2 *first = c->ug_first;
+    auto cell_of = [&](int k) { return ((first[k].y >> 1) + J) * nbx + (first[k].x - jxf); };
+    for (int k = 0; k < nuv; k++) off[(size_t)cell_of(k) + 1]++;
     for (int q = 0; q < cells; q++) {
         cst[q] = (int)chunk.size();
         for (int s = 0; s < off[q + 1]; s += 32) {
@@ -227,9 +244,9 @@ int gp_ug_plan(gpair_ctx *c, const gpair_uv *uv)
     cst[cells] = (int)chunk.size();
     std::vector<int> pos(off.begin(), off.end() - 1);
     for (int k = 0; k < nuv; k++) {
-        const int cell = (jy0[k] + J) * nbx + (jx0[k] - jxf);
+        const int cell = cell_of(k);
         const int p = pos[cell]++;
-        src[p] = k | (flip[k] ? (int)0x80000000 : 0);
+        src[p] = k | ((first[k].y & 1) ? (int)0x80000000 : 0);
         base[p] = cell;
     }
     // 1 / phi over the folded coordinate: phi(x') = w sinh(z) / z / I0(beta), z^2 = beta^2 - (pi w x'/M)^2
@@ -258,32 +275,63 @@ int gp_ug_plan(gpair_ctx *c, const gpair_uv *uv)
     g->nchunk = (int)chunk.size();
     g->ldT = (2 * nbx + 3) & ~3;
     cudaStream_t st = c->stream;
-    GP_CUDA(c, cudaMalloc(&g->src, sizeof(int) * nuv));
-    GP_CUDA(c, cudaMalloc(&g->base, sizeof(int) * nuv));
-    GP_CUDA(c, cudaMalloc(&g->wts, sizeof(float) * 2 * UG_W * (size_t)nuv));
-    GP_CUDA(c, cudaMalloc(&g->phase, sizeof(float2) * nuv));
-    GP_CUDA(c, cudaMalloc(&g->chunk, sizeof(int2) * g->nchunk));
-    GP_CUDA(c, cudaMalloc(&g->cst, sizeof(int) * ((size_t)cells + 1)));
-    GP_CUDA(c, cudaMalloc(&g->ftab, sizeof(float2) * (size_t)nbx * H));
-    GP_CUDA(c, cudaMalloc(&g->ctab, sizeof(float2) * (size_t)H * (J + 1)));
-    GP_CUDA(c, cudaMalloc(&g->invphi, sizeof(double) * H));
-    GP_CUDA(c, cudaMalloc(&g->grid, sizeof(float2) * (size_t)cells));
-    GP_CUDA(c, cudaMalloc(&g->patch, sizeof(float2) * UG_W * UG_W * (size_t)g->nchunk));
-    GP_CUDA(c, cudaMalloc(&g->cgrid, sizeof(float2) * (size_t)cells));
-    GP_CUDA(c, cudaMalloc(&g->S, sizeof(float2) * (size_t)N * nbx));
-    GP_CUDA(c, cudaMalloc(&g->T, sizeof(float) * (size_t)UG_MAX_SPLITS * N * g->ldT));
-    GP_CUDA(c, cudaMemcpyAsync(g->src, src.data(), sizeof(int) * nuv, cudaMemcpyHostToDevice, st));
-    GP_CUDA(c, cudaMemcpyAsync(g->base, base.data(), sizeof(int) * nuv, cudaMemcpyHostToDevice, st));
-    GP_CUDA(c, cudaMemcpyAsync(g->chunk, chunk.data(), sizeof(int2) * g->nchunk, cudaMemcpyHostToDevice, st));
-    GP_CUDA(c, cudaMemcpyAsync(g->cst, cst.data(), sizeof(int) * ((size_t)cells + 1), cudaMemcpyHostToDevice, st));
-    GP_CUDA(c, cudaMemcpyAsync(g->invphi, invphi.data(), sizeof(double) * H, cudaMemcpyHostToDevice, st));
+    // one allocation for all, the arrays from the host first, in one copy
+    const struct {
+        void **p;
+        size_t bytes;
+        const void *host;
+    } arrays[] = {{(void **)&g->src, sizeof(int) * (size_t)nuv, src.data()},
+                  {(void **)&g->base, sizeof(int) * (size_t)nuv, base.data()},
+                  {(void **)&g->chunk, sizeof(int2) * (size_t)g->nchunk, chunk.data()},
+                  {(void **)&g->cst, sizeof(int) * ((size_t)cells + 1), cst.data()},
+                  {(void **)&g->invphi, sizeof(double) * (size_t)H, invphi.data()},
+                  {(void **)&g->wts, sizeof(float) * 2 * UG_W * (size_t)nuv, nullptr},
+                  {(void **)&g->phase, sizeof(float2) * (size_t)nuv, nullptr},
+                  {(void **)&g->ftab, sizeof(float2) * (size_t)nbx * H, nullptr},
+                  {(void **)&g->ctab, sizeof(float2) * (size_t)H * (J + 1), nullptr},
+                  {(void **)&g->grid, sizeof(float2) * (size_t)cells, nullptr},
+                  {(void **)&g->patch, sizeof(float2) * UG_W * UG_W * (size_t)g->nchunk, nullptr},
+                  {(void **)&g->cgrid, sizeof(float2) * (size_t)cells, nullptr},
+                  {(void **)&g->S, sizeof(float2) * (size_t)N * nbx, nullptr},
+                  {(void **)&g->T, sizeof(float) * (size_t)UG_MAX_SPLITS * N * g->ldT, nullptr}};
+    auto padded = [](size_t n) { return (n + 255) & ~(size_t)255; };
+    size_t total = 0, given = 0;
+    for (const auto &x : arrays) {
+        total += padded(x.bytes);
+        if (x.host) given = total;
+    }
+    GP_CUDA(c, cudaMalloc(&g->mem, total));
+    std::vector<unsigned char> host(given);
+    size_t at = 0;
+    for (const auto &x : arrays) {
+        *x.p = (unsigned char *)g->mem + at;
+        if (x.host) memcpy(&host[at], x.host, x.bytes);
+        at += padded(x.bytes);
+    }
+    GP_CUDA(c, cudaMemcpyAsync(g->mem, host.data(), given, cudaMemcpyHostToDevice, st));
     k_ug_points<<<gp_cdiv(nuv, 128), 128, 0, st>>>(c->uvc, g->src, g->base, nuv, (double)c->pix, N, M, jxf, J, nbx,
                                                    beta, g->wts, g->phase);
     GP_LAUNCH_CHECK(c);
     const long long nt = (long long)nbx * H + (long long)H * (J + 1);
     k_ug_tables<<<gp_cdiv(nt, 256), 256, 0, st>>>(g->invphi, N, H, M, jxf, nbx, J, g->ftab, g->ctab);
     GP_LAUNCH_CHECK(c);
-    GP_CUDA(c, cudaStreamSynchronize(st));  // the host arrays go out of scope
+    return GPAIR_OK;  // the copy has taken the host's arrays, pageable memory, before it returned
+}
+
+int gp_ug_choose(gpair_ctx *c)
+{
+    c->ug = nullptr;
+    if (!gp_ug_takes(c, c->precision)) return GPAIR_OK;
+    if (!c->ug_plan) {
+        const int rc = ug_plan(c);
+        if (rc) {
+            ug_free_plan(c);  // the whole plan or none
+            return rc;
+        }
+        free(c->ug_first);
+        c->ug_first = nullptr;
+    }
+    c->ug = c->ug_plan;
     return GPAIR_OK;
 }
 

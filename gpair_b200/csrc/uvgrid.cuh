@@ -41,6 +41,7 @@ struct UgState {
     int jxf, nbx, J;     // grid columns jxf .. jxf + nbx - 1, rows -J .. J
     int cells, nchunk;   // nbx (2 J + 1); runs of at most 32 uv points of one cell
     int ldT;             // floats per row of T
+    void *mem;           // what the arrays up to S lie in
     // uv points sorted by the cell of their first window point
     int *src;            // [nuv] uv index, bit 31: conjugated
     int *base;           // [nuv] cell

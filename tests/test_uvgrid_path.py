@@ -159,3 +159,81 @@ def test_wide_coverage_on_either_path(N, nuv):
             assert np.abs(r.visibilities() - V).max() <= 1e-5
             assert abs(c - chi2) <= 1e-5 * chi2
             assert np.linalg.norm(r.adjoint_image(w) - adj) <= 1e-5 * np.linalg.norm(adj)
+
+
+def _used():
+    import torch
+    free, total = torch.cuda.mem_get_info()
+    return total - free
+
+
+def test_plan_is_built_by_the_mode_that_takes_it():
+    """1024 pixels and points over the whole plane: the grid for FP32, direct sums for split-f16. The plan (S alone is
+    2 x 8.5 MB, the x contraction's sums 8.5 MB) exists once FP32 has been set, and not in a context that was split-f16 before the
+    problem was loaded."""
+    p = _problem(1024, _freq("full", 9500, 5), 100, 6)
+    img = _image(1024, 7)
+    want = []
+    used = []
+    for fp32 in (False, True):
+        with g.Reconstructor(0) as r:
+            u0 = _used()
+            r.set_precision(g.PREC_FP32 if fp32 else g.PREC_SPLIT16)
+            r.set_problem(p)
+            r.set_precision(g.PREC_SPLIT16)
+            assert r.uv_grid(g.PREC_FP32) and not r.uv_grid()
+            used.append(_used() - u0)
+            r.set_image(img)
+            one = r.criterion()
+            r.set_precision(g.PREC_FP32)
+            want += [one, r.criterion()]
+            r.set_precision(g.PREC_SPLIT16)
+            assert r.criterion() == one
+    assert want[:2] == want[2:]
+    assert used[1] - used[0] >= 16 << 20
+
+
+@pytest.mark.parametrize("first", ["criterion", "adjoint", "cg", "host_loop", "batch", "batched_search", "time_stages",
+                                   "time_batch_stages", "autotune", "checkpoint"])
+def test_first_call_in_fp32(first):
+    """Each entry point as a new context's first: the results are those after an evaluation."""
+    N, nuv = 147, 1904
+    rng = np.random.default_rng(4)
+    w = (rng.standard_normal(nuv) + 1j * rng.standard_normal(nuv)).astype(np.complex64)
+    got = []
+    for warm in (True, False):
+        with _context(N, nuv, nbis=900) as r:
+            assert r.uv_grid()
+            r.set_image(_image(N, 2))
+            if warm:
+                r.criterion()
+                r.gradient()
+                r.set_image(_image(N, 2))
+            if first == "criterion":
+                out = r.criterion()
+            elif first == "adjoint":
+                out = r.adjoint_image(w).tolist()
+            elif first == "cg":
+                out = r.cg(2)["J"]
+            elif first == "host_loop":
+                out = r.cg(2, host_loop=1)["J"]
+            elif first == "batch":
+                with g.api.Batch([r]) as b:
+                    out = b.run(2)[0]["J"]
+            elif first == "batched_search":
+                out = r.cg(2, line_search=g.LS_BATCH)["J"]
+            elif first == "time_stages":
+                out = len(r.time_stages(2))
+            elif first == "time_batch_stages":
+                out = len(r.time_batch_stages(2))
+            elif first == "autotune":
+                r.autotune(g.api.TUNE_SPLITS)
+                out = r.criterion()
+            else:
+                with _context(N, nuv, nbis=900) as other:
+                    other.set_image(_image(N, 2))
+                    other.cg(1)
+                    r.restore(other.checkpoint())
+                out = r.cg(1, resume=True)["J"]
+            got.append((out, r.get_image().tolist()))
+    assert got[0] == got[1]
