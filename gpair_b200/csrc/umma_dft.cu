@@ -1742,8 +1742,9 @@ static int tc_build(gpair_ctx *c)
         // partial sums of TC_GRID_PRODUCTS products: short FP32 chains, and more units than one per tile
         t->gkb = TC_GRID_PRODUCTS / t->bk;
         const int kb_total = t->Kx_pad / t->bk;
-        if (gp_cdiv(kb_total, t->gkb) > UG_MAX_SPLITS) t->gkb = gp_cdiv(kb_total, UG_MAX_SPLITS);
+        if (gp_cdiv(kb_total, t->gkb) > UG_MAX_SPLITS) t->gkb = gp_cdiv(kb_total, UG_MAX_SPLITS);  // N > 1,024
         t->gsplits = gp_cdiv(kb_total, t->gkb);
+        if (t->gsplits > ug_tc_splits(N)) return GPAIR_ERR_STATE;  // what T holds
     }
     t->nanc = (N + 15) / 16;
     if (!ug) {
@@ -2084,7 +2085,7 @@ static TcArgs tc_grid_args(gpair_ctx *c, TcState *t, int images)
     a.m_tiles = t->rows_pad / TC_BM;
     a.kb_total = t->Kx_pad / t->bk;
     a.kb_per_split = t->gkb;
-    a.gpart = images > 1 ? g->Tb : g->T;
+    a.gpart = images > 1 ? g->Tb[1] : g->T[1];
     a.out_ld = g->ldT;
     a.out_rows = images > 1 ? images * t->Lb : c->N;
     a.out_cols = 2 * g->nbx;

@@ -45,6 +45,7 @@
 #include "uvgrid.cuh"
 
 #define UG_PI 3.14159265358979323846
+#define UGX_T 32  // tile of the x contraction on the CUDA cores (k_ug_x): image rows, columns, folded pixels
 #define UG_RPMAS ((3.14159265358979323 / 180.0) / 3600000.0)  // radians per milliarcsecond, as k_gen_twiddles
 
 // ------------------------------------------------------------------ plan
@@ -200,7 +201,7 @@ static void ug_free_plan(gpair_ctx *c)
 {
     UgState *g = (UgState *)c->ug_plan;
     if (g) {
-        void *bufs[] = {g->mem, g->Tb, g->gridb};
+        void *bufs[] = {g->mem, g->t_mem[0], g->t_mem[1], g->Tb[0], g->Tb[1], g->gridb};
         for (void *b : bufs)
             if (b) cudaFree(b);
         free(g);
@@ -215,6 +216,29 @@ void gp_ug_free(gpair_ctx *c)
     free(c->ug_first);
     c->ug_first = nullptr;
     c->ug_able = 0;
+}
+
+// 0: the CUDA cores' x contraction, 1: the tensor cores'
+static int ug_class(const gpair_ctx *c) { return c->precision != GPAIR_PREC_FP32; }
+
+// Partial sums of the x contraction of `images` images on the CUDA cores, and folded pixels in each: slices
+// of whole tiles until the blocks fill two waves of 148 SMs
+static int ug_x_splits(const UgState *g, int images, int *hper)
+{
+    const int blocks = gp_cdiv(g->N, UGX_T) * gp_cdiv(g->nbx, UGX_T) * images;
+    int s = 1;
+    while (s < UG_MAX_SPLITS && 2 * s * UGX_T <= g->H && blocks * s < 2 * 148) s *= 2;
+    *hper = gp_cdiv(gp_cdiv(g->H, s), UGX_T) * UGX_T;
+    return gp_cdiv(g->H, *hper);
+}
+
+// floats of the x contraction's sums of one image or the batch's, in the context's mode (the tensor path's
+// operand stack has at least as many rows per image as the CUDA cores, N)
+static size_t ug_t_floats(const gpair_ctx *c, const UgState *g, int images)
+{
+    int hper;
+    if (!ug_class(c)) return (size_t)ug_x_splits(g, images, &hper) * images * g->N * g->ldT;
+    return (size_t)ug_tc_splits(g->N) * (images > 1 ? (size_t)images * gp_tc_stack_rows(g->N) : (size_t)g->N) * g->ldT;
 }
 
 // Builds the plan of the problem that gp_ug_scan looked over, when a mode first takes it. A new context is in FP32, so a
@@ -293,7 +317,7 @@ static int ug_plan(gpair_ctx *c)
                   {(void **)&g->patch, sizeof(float2) * UG_W * UG_W * (size_t)g->nchunk, nullptr},
                   {(void **)&g->cgrid, sizeof(float2) * (size_t)cells, nullptr},
                   {(void **)&g->S, sizeof(float2) * (size_t)N * nbx, nullptr},
-                  {(void **)&g->T, sizeof(float) * (size_t)UG_MAX_SPLITS * N * g->ldT, nullptr}};
+                  {(void **)&g->T[ug_class(c)], sizeof(float) * ug_t_floats(c, g, 1), nullptr}};
     auto padded = [](size_t n) { return (n + 255) & ~(size_t)255; };
     size_t total = 0, given = 0;
     for (const auto &x : arrays) {
@@ -331,6 +355,12 @@ int gp_ug_choose(gpair_ctx *c)
         free(c->ug_first);
         c->ug_first = nullptr;
     }
+    UgState *g = (UgState *)c->ug_plan;
+    const int cls = ug_class(c);
+    if (!g->T[cls]) {  // the plan was built by a mode on the other cores
+        GP_CUDA(c, cudaMalloc(&g->t_mem[cls], sizeof(float) * ug_t_floats(c, g, 1)));
+        g->T[cls] = (float *)g->t_mem[cls];
+    }
     c->ug = c->ug_plan;
     return GPAIR_OK;
 }
@@ -341,7 +371,6 @@ int gp_ug_choose(gpair_ctx *c)
 // row meets I[N-1-h] + I[h], the sine row I[N-1-h] - I[h]. A block makes 32
 // image rows x 32 columns over a slice of h; the slices are partial sums that
 // k_ug_rows adds.
-#define UGX_T 32
 struct UgXArgs {
     const float *img;  // image b at img + b npix
     const float2 *ftab;
@@ -907,15 +936,13 @@ struct UgColsOp {
 
 // ------------------------------------------------------------ host side
 
-// Buffers of the batched trials: rows for the tensor path's operand stack, which has at
-// least as many per image as the CUDA cores (N)
+// Buffers of the batched trials
 int gp_ug_batch_alloc(gpair_ctx *c)
 {
     UgState *g = (UgState *)c->ug;
-    if (g->gridb) return GPAIR_OK;
-    const size_t rows = (size_t)GP_NTR * gp_tc_stack_rows(c->N);
-    if (!g->Tb) GP_CUDA(c, cudaMalloc(&g->Tb, sizeof(float) * UG_MAX_SPLITS * rows * g->ldT));
-    GP_CUDA(c, cudaMalloc(&g->gridb, sizeof(float2) * GP_NTR * (size_t)g->cells));  // last: its presence says that both exist
+    const int cls = ug_class(c);
+    if (!g->Tb[cls]) GP_CUDA(c, cudaMalloc(&g->Tb[cls], sizeof(float) * ug_t_floats(c, g, GP_NTR)));
+    if (!g->gridb) GP_CUDA(c, cudaMalloc(&g->gridb, sizeof(float2) * GP_NTR * (size_t)g->cells));
     return GPAIR_OK;
 }
 
@@ -926,18 +953,14 @@ int gp_ug_x(gpair_ctx *c, const float *img, int images)
     UgXArgs a;
     a.img = img;
     a.ftab = g->ftab;
-    a.T = images > 1 ? g->Tb : g->T;
+    a.T = images > 1 ? g->Tb[0] : g->T[0];
     a.N = g->N;
     a.H = g->H;
     a.nbx = g->nbx;
     a.ldT = g->ldT;
     a.images = images;
     const int bx = gp_cdiv(g->N, UGX_T), by = gp_cdiv(g->nbx, UGX_T);
-    // slices of h (whole tiles) until the blocks fill two waves of 148 SMs
-    int s = 1;
-    while (s < UG_MAX_SPLITS && 2 * s * UGX_T <= g->H && bx * by * images * s < 2 * 148) s *= 2;
-    a.hper = gp_cdiv(gp_cdiv(g->H, s), UGX_T) * UGX_T;
-    a.splits = gp_cdiv(g->H, a.hper);
+    a.splits = ug_x_splits(g, images, &a.hper);
     a.gate = images > 1 ? c->gate : nullptr;
     GP_LAUNCH(c, gp_launch(c, k_ug_x, dim3(bx, by, a.splits * images), dim3(256), 0, a));
     (images > 1 ? g->splitsb : g->splits) = a.splits;
@@ -953,7 +976,7 @@ static UgRowsArgs ug_rows_args(gpair_ctx *c, int images, int splits, const float
     UgState *g = (UgState *)c->ug;
     UgRowsArgs a;
     memset(&a, 0, sizeof(a));
-    a.T = images > 1 ? g->Tb : g->T;
+    a.T = images > 1 ? g->Tb[ug_class(c)] : g->T[ug_class(c)];
     a.rsc = rsc;
     a.ctab = g->ctab;
     a.grid = images > 1 ? g->gridb : g->grid;

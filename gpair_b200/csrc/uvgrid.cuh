@@ -51,13 +51,19 @@ struct UgState {
     int *cst;            // [cells + 1] first run of every cell
     float2 *ftab, *ctab; // grid twiddles [nbx][H], [H][J + 1] (k_ug_tables)
     double *invphi;      // [H] 1 / window transform
-    float *T;            // [splits][N][ldT] x contraction of one image
+    // the x contraction's sums, on the CUDA cores [0] and on the tensor cores [1]: [splits][N][ldT] of one image, where a
+    // mode has taken them (t_mem: their own allocation, if any)
+    float *T[2];
+    void *t_mem[2];
     float2 *grid;        // [cells] G
     float2 *patch;       // [nchunk][64]
     float2 *cgrid;       // [cells] C
     float2 *S;           // [N][nbx]
     // batched trials
-    float *Tb;           // [splits][GP_NTR rows per image][ldT]
+    float *Tb[2];        // [splits][GP_NTR rows per image][ldT], likewise
     float2 *gridb;       // [cells][GP_NTR]
     int splits, splitsb; // partial sums of the last CUDA-core x contraction
 };
+
+// Partial sums of the tensor cores' x contraction at most (TC_GRID_PRODUCTS products each)
+static inline int ug_tc_splits(int N) { return gp_cdiv(N, 128) < UG_MAX_SPLITS ? gp_cdiv(N, 128) : UG_MAX_SPLITS; }

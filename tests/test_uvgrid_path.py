@@ -237,3 +237,48 @@ def test_first_call_in_fp32(first):
                 out = r.cg(1, resume=True)["J"]
             got.append((out, r.get_image().tolist()))
     assert got[0] == got[1]
+
+
+@pytest.mark.parametrize("mode", [g.PREC_FP32, g.PREC_TF32X3])
+def test_memory_of_a_wide_image(mode):
+    """1,500 pixels, a grid of 371 x 731 points: images (9 + 8 trials of 9 MB), the x contraction's sums as many as the mode takes (FP32
+    one of 744 floats a row; TF32X3 eight, and eight of its operand stack of 1,536 rows an image), grids and points."""
+    N, nuv = 1500, 20000
+    f = np.random.default_rng(1).uniform(-0.12, 0.12, (nuv, 2))
+    p = _problem(N, f, 100, 2)
+    nbx, J = _extent(p)
+    with g.Reconstructor(0) as r:
+        u0 = _used()
+        r.set_precision(mode)
+        r.set_problem(p)
+        assert r.uv_grid()
+        r.set_image(_image(N, 3))
+        r.cg(1, line_search=g.LS_BATCH)
+        sums = 4 * (2 * nbx + 4) * (N * 9 if mode == g.PREC_FP32 else 8 * (N + 8 * 1536))
+        operands = 0 if mode == g.PREC_FP32 else 8 * (9 * 1536 + 2 * nbx + 128) * 1504
+        rest = 8 * nbx * (2 * J + 1) * 10 + 8 * N * nbx + 1000 * nuv
+        assert _used() - u0 <= 17 * 4 * N * N + sums + operands + rest + (64 << 20)  # allocations in blocks of 2 MB, the run's graph
+
+
+def test_sums_of_both_kinds_of_core():
+    """FP32 and tensor modes on the grid keep sums of their own: changes between batched runs leave the other's alone, and a batch of a
+    mode still runs after evaluations in another."""
+    N, nuv = 330, 20001
+    want = {}
+    for mode in (g.PREC_FP32, g.PREC_SPLIT16):
+        with _context(N, nuv, nbis=2000) as r:
+            r.set_precision(mode)
+            r.set_image(_image(N, 2))
+            want[mode] = r.cg(2, line_search=g.LS_BATCH)["J"], r.get_image()
+    with _context(N, nuv, nbis=2000) as r:
+        r.set_precision(g.PREC_SPLIT16)
+        assert r.uv_grid() and r.uv_grid(g.PREC_FP32)
+        r.set_image(_image(N, 2))
+        with g.api.Batch([r], line_search=g.LS_BATCH) as b:
+            for mode in (g.PREC_SPLIT16, g.PREC_FP32, g.PREC_SPLIT16):
+                r.set_precision(mode)
+                r.set_image(_image(N, 2))
+                out = r.cg(2, line_search=g.LS_BATCH)
+                assert out["J"] == want[mode][0] and np.array_equal(r.get_image(), want[mode][1])
+            r.set_image(_image(N, 2))
+            assert b.run(2)[0]["J"] == want[g.PREC_SPLIT16][0]
