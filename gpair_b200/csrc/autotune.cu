@@ -14,10 +14,13 @@
 //   splits     the adjoint's K-blocks per split (tensor) or split count
 //              (CUDA cores): the heuristic's value, half and double of it,
 //              within the FP32-accumulation cap and the partial-image buffer
+// A precision whose contractions go through the uv grid is one candidate: the tile and the splits are the direct sums'.
 // Objective: one criterion + gradient evaluation, or (GPAIR_TUNE_BATCHED) that
 // plus two batched 8-trial evaluations, the work of a batched-line-search
 // iteration. Choices are cached per (device, width, uv count to 1/8, objective,
-// and the precision path and tile layout when those are not tuned).
+// the precision path and tile layout when those are not tuned, which of the candidate precisions
+// go through the uv grid, and the grid's extent in that case): the same sizes
+// with a wider coverage can take the direct sums, at many times the cost.
 #include <math.h>
 #include <stdlib.h>
 #include <string.h>
@@ -32,14 +35,35 @@
 namespace {
 
 struct Choice {
-    int precision, tc_kb_per, simt_splits, tc_pair;
+    int precision, tc_kb_per, simt_splits, tc_pair;  // on the uv grid: no splits (0), the context's own tile (-1)
     double ms;
 };
 
 std::mutex g_mu;
-std::map<std::tuple<int, int, int, int>, Choice> g_cache;
+std::map<std::tuple<int, int, int, int, int>, Choice> g_cache;
 
 int uv_bucket(int nuv) { return nuv <= 0 ? 0 : (int)floor(log2((double)nuv) * 8.0); }
+
+// which of the precisions take the uv grid, and the grid's size to a factor of two where one does
+int path_key(const gpair_ctx *c, const std::vector<int> &precs)
+{
+    int key = 0;
+    for (size_t i = 0; i < precs.size(); i++) key |= gp_ug_takes(c, precs[i]) ? 1 << i : 0;
+    return key ? key | (int)log2((double)c->ug_nbx * (double)c->ug_J) << 8 : 0;
+}
+
+// split count and tile rows of a choice, as reported
+int splits_of(gpair_ctx *c, const Choice &ch)
+{
+    if (gp_ug_takes(c, ch.precision)) return 0;
+    return ch.precision == GPAIR_PREC_FP32 ? ch.simt_splits : gp_tc_split_count(c, ch.tc_kb_per);
+}
+
+int tile_of(const gpair_ctx *c, const Choice &ch)
+{
+    if (ch.precision == GPAIR_PREC_FP32) return 0;
+    return !gp_ug_takes(c, ch.precision) && ch.tc_pair ? 256 : 128;
+}
 
 // average ms of one criterion + gradient evaluation of the current image, plus
 // (batched) two evaluations of 8 trial images: the work of one iteration of the
@@ -84,7 +108,8 @@ int time_evals(gpair_ctx *c, int reps, int batched, double *ms)
 
 int apply(gpair_ctx *c, const Choice &ch)
 {
-    if (c->tc_pair != ch.tc_pair) {
+    const bool grid = gp_ug_takes(c, ch.precision);
+    if (!grid && c->tc_pair != ch.tc_pair) {
         int rc = gpair_set_tc_pair(c, ch.tc_pair);  // rebuilds the tensor state on the tensor path
         if (rc) return rc;
     }
@@ -92,9 +117,9 @@ int apply(gpair_ctx *c, const Choice &ch)
     if (rc) return rc;
     if (ch.precision != GPAIR_PREC_FP32) {
         if ((rc = gp_tc_prepare(c))) return rc;
-        if ((rc = gp_tc_set_kb_per(c, ch.tc_kb_per))) return rc;
+        if (!grid && (rc = gp_tc_set_kb_per(c, ch.tc_kb_per))) return rc;
     }
-    c->splits_simt = ch.simt_splits;
+    if (!grid) c->splits_simt = ch.simt_splits;
     gp_cg_graph_free(c);  // a captured CG graph holds the old configuration
     return GPAIR_OK;
 }
@@ -110,10 +135,18 @@ extern "C" int gpair_autotune(gpair_ctx *c, int flags, int reps, gpair_tune_resu
     // fixed precision path or tile layout is not reused
     const int fixed = ((flags & GPAIR_TUNE_PRECISION) ? 0 : c->precision + 1) * 4 +
                       ((flags & GPAIR_TUNE_TILE) ? 0 : c->tc_pair + 1);
+    std::vector<int> precs;
+    if (flags & GPAIR_TUNE_PRECISION) {
+        precs.push_back(GPAIR_PREC_SPLIT16);
+        precs.push_back(GPAIR_PREC_SPLIT16F8);
+        precs.push_back(GPAIR_PREC_FP32);
+    } else {
+        precs.push_back(c->precision);
+    }
     const auto key = std::make_tuple(c->device, c->N,
                                      uv_bucket(c->nuv) * 4 + ((flags & GPAIR_TUNE_BATCHED) ? 1 : 0) +
                                          ((flags & GPAIR_TUNE_TILE) ? 2 : 0),
-                                     fixed);
+                                     fixed, path_key(c, precs));
     if (res) memset(res, 0, sizeof(*res));
     if (flags & GPAIR_TUNE_CACHE) {
         Choice ch;
@@ -137,35 +170,29 @@ extern "C" int gpair_autotune(gpair_ctx *c, int flags, int reps, gpair_tune_resu
         if (applied) {
             if (res) {
                 res->precision = ch.precision;
-                res->adjoint_splits = ch.precision == GPAIR_PREC_FP32 ? ch.simt_splits : gp_tc_split_count(c, ch.tc_kb_per);
+                res->adjoint_splits = splits_of(c, ch);
                 res->ms_per_eval = ch.ms;
                 res->from_cache = 1;
-                res->tile_m = ch.precision == GPAIR_PREC_FP32 ? 0 : (ch.tc_pair ? 256 : 128);
+                res->tile_m = tile_of(c, ch);
             }
             return GPAIR_OK;
         }
     }
-    std::vector<int> precs;
-    if (flags & GPAIR_TUNE_PRECISION) {
-        precs.push_back(GPAIR_PREC_SPLIT16);
-        precs.push_back(GPAIR_PREC_SPLIT16F8);
-        precs.push_back(GPAIR_PREC_FP32);
-    } else {
-        precs.push_back(c->precision);
-    }
-    const int simt0 = c->splits_simt > 0 ? c->splits_simt : 1;
+    const int simt0 = c->splits_simt > 0 ? c->splits_simt : 1, pair0 = c->tc_pair;
     std::vector<Choice> cand;
     for (int prec : precs) {
-        if (prec == GPAIR_PREC_FP32) {
+        if (gp_ug_takes(c, prec)) {
+            cand.push_back({prec, 0, 0, -1, 0.0});
+        } else if (prec == GPAIR_PREC_FP32) {
             std::vector<int> ss = {simt0};
             if (flags & GPAIR_TUNE_SPLITS) {
                 if (simt0 / 2 >= 1) ss.push_back(simt0 / 2);
                 if (2 * simt0 <= c->gpart_cap && 2 * simt0 <= 64) ss.push_back(2 * simt0);
             }
-            for (int s : ss) cand.push_back({prec, 0, s, c->tc_pair, 0.0});
+            for (int s : ss) cand.push_back({prec, 0, s, pair0, 0.0});
         } else {
-            std::vector<int> pairs = {c->tc_pair};
-            if (flags & GPAIR_TUNE_TILE) pairs.push_back(!c->tc_pair);
+            std::vector<int> pairs = {pair0};
+            if (flags & GPAIR_TUNE_TILE) pairs.push_back(!pair0);
             for (int pr : pairs) {
                 int rc = gpair_set_tc_pair(c, pr);
                 if (rc) return rc;
@@ -203,16 +230,14 @@ extern "C" int gpair_autotune(gpair_ctx *c, int flags, int reps, gpair_tune_resu
     }
     if (res) {
         res->precision = cand[best].precision;
-        res->adjoint_splits = cand[best].precision == GPAIR_PREC_FP32 ? cand[best].simt_splits
-                                                                       : gp_tc_split_count(c, cand[best].tc_kb_per);
+        res->adjoint_splits = splits_of(c, cand[best]);
         res->ms_per_eval = cand[best].ms;
         res->n_candidates = (int)cand.size();
-        res->tile_m = cand[best].precision == GPAIR_PREC_FP32 ? 0 : (cand[best].tc_pair ? 256 : 128);
+        res->tile_m = tile_of(c, cand[best]);
         for (size_t i = 0; i < cand.size(); i++) {
-            res->cand_tile_m[i] = cand[i].precision == GPAIR_PREC_FP32 ? 0 : (cand[i].tc_pair ? 256 : 128);
+            res->cand_tile_m[i] = tile_of(c, cand[i]);
             res->cand_precision[i] = cand[i].precision;
-            res->cand_splits[i] = cand[i].precision == GPAIR_PREC_FP32 ? cand[i].simt_splits
-                                                                      : gp_tc_split_count(c, cand[i].tc_kb_per);
+            res->cand_splits[i] = splits_of(c, cand[i]);
             res->cand_ms[i] = cand[i].ms;
         }
     }

@@ -494,7 +494,9 @@ int gpair_time_batch_stages(gpair_ctx *ctx, int reps, double *stage_ms, int max_
  * 256 x 256 output tiles on CTA pairs or 128 x 256 on single CTAs, as
  * gpair_set_tc_pair selects). GPAIR_TUNE_CACHE reuses the choice made for a
  * problem of the same device, width and uv count (to 1/8) and objective in this
- * process, made with the same precision path and tile when those are not tuned. */
+ * process, made with the same precision path and tile when those are not tuned, whose
+ * candidates take the uv grid alike (gpair_uv_grid). A precision on the uv grid is one
+ * candidate: it has no split-K adjoint and one tile. */
 #define GPAIR_TUNE_PRECISION 1
 #define GPAIR_TUNE_SPLITS 2
 #define GPAIR_TUNE_CACHE 4
@@ -504,11 +506,11 @@ int gpair_time_batch_stages(gpair_ctx *ctx, int reps, double *stage_ms, int max_
 #define GPAIR_TUNE_MAX_CANDIDATES 16
 typedef struct {
     int precision;       /* chosen precision mode */
-    int adjoint_splits;  /* chosen split-K count of the adjoint contraction */
+    int adjoint_splits;  /* chosen split-K count of the adjoint contraction; 0 on the uv grid */
     double ms_per_eval;  /* criterion + gradient, chosen configuration */
     int from_cache;
     int n_candidates;
-    int tile_m;          /* chosen tensor-core tile rows: 256 (CTA pairs), 128, or 0 (CUDA cores) */
+    int tile_m;          /* chosen tensor-core tile rows: 256 (CTA pairs), 128 (and on the uv grid), or 0 (CUDA cores) */
     int cand_precision[GPAIR_TUNE_MAX_CANDIDATES];
     int cand_splits[GPAIR_TUNE_MAX_CANDIDATES];
     int cand_tile_m[GPAIR_TUNE_MAX_CANDIDATES];

@@ -282,3 +282,37 @@ def test_sums_of_both_kinds_of_core():
                 assert out["J"] == want[mode][0] and np.array_equal(r.get_image(), want[mode][1])
             r.set_image(_image(N, 2))
             assert b.run(2)[0]["J"] == want[g.PREC_SPLIT16][0]
+
+
+def test_tuned_choice_is_not_taken_over_by_another_path():
+    """Equal widths and uv counts: a compact coverage on the grid, one too wide for it, and one on the grid in FP32 alone."""
+    flags = g.api.TUNE_PRECISION | g.api.TUNE_SPLITS | g.api.TUNE_TILE | g.api.TUNE_CACHE
+    seen = []
+    for kind, nuv, grid in (("inner", 5000, (True, False, True)), ("full", 5000, (False, False, True)),
+                            ("inner", 5001, (True, False, True))):
+        with _context(512, nuv, kind) as r:
+            assert (r.uv_grid(g.PREC_SPLIT16), r.uv_grid(g.PREC_SPLIT16F8), r.uv_grid(g.PREC_FP32)) == grid
+            r.set_image(_image(512, 3))
+            t = r.autotune(flags, reps=2)
+            seen.append(t)
+            tune = r.uv_grid(t["precision"])
+            assert (t["adjoint_splits"] == 0) == tune
+            for prec, splits, tile, _ in t["candidates"]:
+                assert (splits == 0) == r.uv_grid(prec)
+                assert tile == 0 if prec == g.PREC_FP32 else tile in ((128,) if r.uv_grid(prec) else (128, 256))
+            assert np.isfinite(r.criterion()).all()
+    assert [t["from_cache"] for t in seen] == [False, False, True]
+    assert seen[2]["precision"] == seen[0]["precision"]
+    # S16 and FP32 on the grid: one candidate each; F8 directly: two tiles, up to three splits each
+    assert sum(c[0] != g.PREC_SPLIT16F8 for c in seen[0]["candidates"]) == 2
+
+
+def test_tuning_on_the_grid_leaves_the_tile():
+    with _context(512, 20000) as r:
+        assert all(r.uv_grid(m) for m in (g.PREC_FP32, g.PREC_SPLIT16, g.PREC_SPLIT16F8))
+        r.set_image(_image(512, 3))
+        for pair in (True, False):
+            r.set_tc_pair(pair)
+            t = r.autotune(g.api.TUNE_PRECISION | g.api.TUNE_SPLITS | g.api.TUNE_TILE, reps=2)
+            assert len(t["candidates"]) == 3 and t["adjoint_splits"] == 0
+            assert r._L.gpair_get_tc_pair(r.h) == pair
