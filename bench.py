@@ -624,7 +624,7 @@ def measure_plain(rec, p, args, flush, local, dist):
         e2e_flops += rec.last_run_stats()[1]
     return {"dev_ms": dev_ms, "flops": flops, "launches": launches, "evals": crit_evals + grad_evals,
             "crit_evals": crit_evals, "grad_evals": grad_evals, "clocks": clocks, "stage_n": stage_n,
-            "stage_ms": stage_ms, "e2e_s": e2e_s, "e2e_flops": e2e_flops, "img": img}
+            "stage_ms": stage_ms, "e2e_s": e2e_s, "e2e_flops": e2e_flops, "img": img, "uv_grid": rec.uv_grid()}
 
 
 PRECISION_MODES = {"fp32": 0, "split16": 1, "split16f8": 4}
@@ -663,8 +663,7 @@ def roofline(p, m, precision, workload):
     per_launch_ms = stage_ms[dom] / max(stage_n[dom], 1)
     achieved = p.dft_flops() / (per_launch_ms * 1e-3) / 1e12
     contraction = dom in ("forward_dft", "adjoint_dft")
-    if contraction and _executed_mult(precision, dom) * achieved > 1.2 * tflops_peak:
-        # more than the tensor cores can execute: the uv grid
+    if contraction and m["uv_grid"]:
         work = _grid_bytes(p)
         gbs = work / (per_launch_ms * 1e-3) / 1e9
         roof = {"bound": "hbm", "achieved": gbs, "peak": hbm, "unit": "GB/s", "frac": gbs / hbm,
@@ -690,7 +689,9 @@ def roofline(p, m, precision, workload):
     roof["peak_source"] = peak_kind
     roof["timing"] = ("per-stage CUDA events, stages queued back to back; stage totals = per-launch time x "
                       "the timed steps' criterion (prep, forward, vis_data) or gradient evaluations")
-    roof["traffic"] = _traffic(f"{dom}@{workload}@{precision}")
+    roof["uv_grid"] = m["uv_grid"]
+    # captured on the direct sums' kernels
+    roof["traffic"] = None if m["uv_grid"] else _traffic(f"{dom}@{workload}@{precision}")
     roof["stage_ms_per_launch"] = {k: stage_ms[k] / max(stage_n[k], 1) for k in stage_ms}
     roof["stage_share"] = {k: stage_ms[k] / max(sum(stage_ms.values()), 1e-12) for k in stage_ms}
     return roof
@@ -719,7 +720,7 @@ def batched_block(rec, p, args, flush, img, precision, workload):
     mult = _executed_mult(precision, "forward_dft")
     fb_ms = st_b["forward_dft_batch"]
     fb_ach = 8 * p.dft_flops() / (fb_ms * 1e-3) / 1e12
-    if mult * fb_ach > 1.2 * tflops_peak:  # the uv grid
+    if rec.uv_grid():
         gbs = _grid_bytes(p, 8) / (fb_ms * 1e-3) / 1e9
         roof = {"bound": "hbm", "achieved": gbs, "peak": hbm, "unit": "GB/s", "frac": gbs / hbm,
                 "work_note": GRID_NOTE, "algorithmic_tflops": fb_ach}
@@ -732,7 +733,8 @@ def batched_block(rec, p, args, flush, img, precision, workload):
             "note": "CG iterations with 8 trial images per batched evaluation (rank 0, device time)",
             "roofline": {**roof, "kernel": "forward_dft_batch (8 stacked trial images)",
                          "peak_source": peak_kind,
-                         "traffic": _traffic(f"forward_dft_batch8@{workload}@{precision}"),
+                         "uv_grid": rec.uv_grid(),
+                         "traffic": None if rec.uv_grid() else _traffic(f"forward_dft_batch8@{workload}@{precision}"),
                          "stage_ms_per_launch": st_b,
                          "timing": "CUDA events around the three batched stages queued back to back"}}
 
@@ -803,8 +805,8 @@ def run_ours(args, rank, world, local):
                                     if args.line_search == "wolfe" else
                                     "one PR+ CG iteration with the batched 8-trial line search (continuing)"),
                            "precision": args.precision, "evaluations": m["evals"],
-                           "tensor_tiles": "CTA pairs (cta_group::2, 256x256)" if args.tc_pair else
-                           "single CTAs (128x256)",
+                           "tensor_tiles": "single CTAs (uv grid)" if m["uv_grid"] else
+                           "CTA pairs (cta_group::2, 256x256)" if args.tc_pair else "single CTAs (128x256)",
                            "criterion_evals": m["crit_evals"], "grad_evals": m["grad_evals"],
                            "flop_per_evaluation": p.dft_flops(),
                            "autotuned_adjoint_splits": tune["adjoint_splits"],
