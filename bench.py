@@ -276,7 +276,11 @@ def run_reference(args, rank):
     if rank != 0:
         return
     t_setup = time.perf_counter()
-    sample = reference_sample(args.workload)
+    try:
+        sample = reference_sample(args.workload)
+    except FileNotFoundError as e:  # its compiled sources are not there
+        print(json.dumps({"impl": "reference", "unavailable": str(e).replace(ROOT + os.sep, "").splitlines()[0]}), flush=True)
+        return
     t_setup = time.perf_counter() - t_setup
     cores = os.cpu_count() or 1
     ctx = mp.get_context("spawn")

@@ -26,3 +26,19 @@ def test_bound_follows_the_path():
             direct = bench.roofline(p, _measured(ms, False), precision, "precision")
             assert direct["bound"] == "tensor" and not direct["uv_grid"]
             assert direct["work_per_launch"] == p.dft_flops() and direct["executed_tflops"] >= direct["achieved"]
+
+
+def test_reference_arm_without_the_reference(monkeypatch, capsys):
+    """Where the reference's sources were never there to compile, its arm says so in its line."""
+    import argparse
+    import json
+
+    def missing(*_):
+        raise FileNotFoundError("libgpair_ref.so not built (reference sources unavailable)")
+
+    monkeypatch.setattr(bench, "reference_sample", missing)
+    bench.run_reference(argparse.Namespace(workload="tiny", gpus=1, steps=1, warmup=3), 0)
+    lines = capsys.readouterr().out.strip().splitlines()
+    assert len(lines) == 1
+    line = json.loads(lines[0])
+    assert line["impl"] == "reference" and "not built" in line["unavailable"] and len(line) == 2
