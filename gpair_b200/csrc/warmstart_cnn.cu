@@ -291,7 +291,9 @@ __global__ void __launch_bounds__(WG_THREADS *NG) k_conv3_wgrad(const float *__r
     __shared__ __align__(16) float xs[STAGED ? 2 : 1][STAGED ? WG_BUF : 4];
     __shared__ float red[NG][WG_THREADS / 32][NV];
     const int t = threadIdx.x % P.threads, grp = threadIdx.x / P.threads;
-    const int co0 = (blockIdx.x * NG + grp) * CO, ci = blockIdx.y, slice = blockIdx.z;
+    // (output channels, input channel) on one dimension of the grid: neither is held to 65,535 blocks
+    const int ncog = gridDim.x / Cin, ci = blockIdx.x / ncog;
+    const int co0 = ((blockIdx.x - ci * ncog) * NG + grp) * CO, slice = blockIdx.z;
     const int b0 = slice * bps, b1 = min(B, b0 + bps);
     const int HW = H * W, LD = P.ld;
     const int lane = threadIdx.x & 31;
@@ -462,7 +464,7 @@ __global__ void __launch_bounds__(WG_THREADS *NG) k_conv3_wgrad(const float *__r
         if (i < CO * NTAP) {
             const int co = co0 + i / NTAP, k = i % NTAP;
             if (co < Cout) part[(((size_t)slice * Cout + co) * Cin + ci) * NTAP + k] = v;
-        } else if (blockIdx.y == 0) {
+        } else if (ci == 0) {
             const int co = co0 + i - CO * NTAP;
             if (co < Cout) bpart[(size_t)slice * Cout + co] = v;
         }
@@ -777,8 +779,8 @@ extern "C" int gpair_cnn_conv3x3_bwd_weight(const float *in, const float *gpre, 
     WgPlan p;
     const bool staged = wg_plan(in, B, H, W, &p);
     auto go = [&](auto kernel, int co, int ng) {
-        kernel<<<dim3(cdiv_ll(Cout, co * ng), Cin, slices), p.threads * ng, 0, st>>>(in, gpre, part, bpart, B, Cin, Cout,
-                                                                                    H, W, bps, p);
+        kernel<<<dim3(cdiv_ll(Cout, co * ng) * Cin, 1, slices), p.threads * ng, 0, st>>>(in, gpre, part, bpart, B, Cin,
+                                                                                        Cout, H, W, bps, p);
     };
     // four output channels a block (9 input loads for 36 FMAs) where that still makes two blocks per SM; one
     // each in two groups that share a chunk where blocks are few
