@@ -851,7 +851,7 @@ extern "C" int gpair_cnn_head_bwd(const float *d, const float *w, const float *z
     if (B <= 0 || C <= 0 || HW <= 0) return GPAIR_ERR_INVALID;
     k_head_bwd<<<B * HD_CTAS, 256, 0, CNN_STREAM(stream)>>>(d, w, z, out, asum, gout, gd, scratch, C, HW);
     // dw[c] (c < C) and dbias (c = C): fixed-order sums over the images
-    k_reduce_slices<<<1, 256, 0, CNN_STREAM(stream)>>>(scratch, C + 1, B, dw);
+    k_reduce_slices<<<cdiv_ll(C + 1, 256), 256, 0, CNN_STREAM(stream)>>>(scratch, C + 1, B, dw);
     return cnn_status();
 }
 
