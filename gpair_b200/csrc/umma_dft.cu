@@ -120,7 +120,7 @@ __device__ __forceinline__ void split_f8(float v, float s_hi, float s_lo, __half
 // products per K step: 3 = hi*hi + hi*lo + lo*hi of split operands, 1 = hi*hi
 // At most TC_SPLIT_PRODUCTS products per adjoint split-K partial (FP32 accumulation)
 #define TC_SPLIT_PRODUCTS 4096
-// and per partial sum of the uv grid's x contraction
+// and per partial sum of the uv grid's x contraction, up to 1,024 pixels (UG_MAX_SPLITS partial sums at most)
 #define TC_GRID_PRODUCTS 128
 
 template <typename OT> struct OpSplit;

@@ -1,7 +1,7 @@
 """The network's kernels at channel counts beyond one pass or one dimension of a grid, against FP64.
 
 Tolerances as in test_cnn_kernels: n 2^-24 of the sum of the products' magnitudes for a chain of n FP32 products; for the head, whose sums
-are FP64, a few roundings (16 x 2^-24) of each term's magnitude.
+are FP64, a few roundings (64 x 2^-24) of each term's magnitude.
 """
 import pytest
 
