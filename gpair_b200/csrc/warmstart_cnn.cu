@@ -291,9 +291,7 @@ __global__ void __launch_bounds__(WG_THREADS *NG) k_conv3_wgrad(const float *__r
     __shared__ __align__(16) float xs[STAGED ? 2 : 1][STAGED ? WG_BUF : 4];
     __shared__ float red[NG][WG_THREADS / 32][NV];
     const int t = threadIdx.x % P.threads, grp = threadIdx.x / P.threads;
-    // (output channels, input channel) on one dimension of the grid: neither is held to 65,535 blocks
-    const int ncog = gridDim.x / Cin, ci = blockIdx.x / ncog;
-    const int co0 = ((blockIdx.x - ci * ncog) * NG + grp) * CO, slice = blockIdx.z;
+    const int co0 = (blockIdx.x * NG + grp) * CO, ci = blockIdx.y, slice = blockIdx.z;
     const int b0 = slice * bps, b1 = min(B, b0 + bps);
     const int HW = H * W, LD = P.ld;
     const int lane = threadIdx.x & 31;
@@ -464,7 +462,7 @@ __global__ void __launch_bounds__(WG_THREADS *NG) k_conv3_wgrad(const float *__r
         if (i < CO * NTAP) {
             const int co = co0 + i / NTAP, k = i % NTAP;
             if (co < Cout) part[(((size_t)slice * Cout + co) * Cin + ci) * NTAP + k] = v;
-        } else if (ci == 0) {
+        } else if (blockIdx.y == 0) {
             const int co = co0 + i - CO * NTAP;
             if (co < Cout) bpart[(size_t)slice * Cout + co] = v;
         }
@@ -779,8 +777,11 @@ extern "C" int gpair_cnn_conv3x3_bwd_weight(const float *in, const float *gpre, 
     WgPlan p;
     const bool staged = wg_plan(in, B, H, W, &p);
     auto go = [&](auto kernel, int co, int ng) {
-        kernel<<<dim3(cdiv_ll(Cout, co * ng) * Cin, 1, slices), p.threads * ng, 0, st>>>(in, gpre, part, bpart, B, Cin,
-                                                                                        Cout, H, W, bps, p);
+        // at most 65,535 input channels a launch (the grid's second dimension); each writes the same bias sums. (Both
+        // channels on the first dimension: 100 -> 122 registers and a training step 1 % slower.)
+        for (int c = 0; c < Cin; c += 65535)
+            kernel<<<dim3(cdiv_ll(Cout, co * ng), Cin - c < 65535 ? Cin - c : 65535, slices), p.threads * ng, 0, st>>>(
+                in + (size_t)c * H * W, gpre, part + (size_t)c * NTAP, bpart, B, Cin, Cout, H, W, bps, p);
     };
     // four output channels a block (9 input loads for 36 FMAs) where that still makes two blocks per SM; one
     // each in two groups that share a chunk where blocks are few
