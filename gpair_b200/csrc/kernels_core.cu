@@ -1195,7 +1195,7 @@ struct UgGradOp {
 
 // Pixels per thread and side: two where the tiles' partial sums fit, else four. The pixels' FP64
 // logarithms want warps more than the contraction wants register tiles: at 1024^2 four a side (128
-// blocks) took 62 us, two (512 blocks) 20.
+// blocks) take 53 us, two (512 blocks) 29; at 256^2 29 and 14.
 static int ug_grad_m(int N) { return gp_cdiv(N, 32) * gp_cdiv((N + 1) / 2, 32) <= GP_MAX_PARTIALS ? 2 : 4; }
 
 static UgGradArgs ug_grad_args(gpair_ctx *c, int which, int mode, float alpha, FusedCtrl fc)

@@ -13,11 +13,14 @@
 // UG_MIN_WIDTH: on narrower images hundreds of uv points share a grid point, and its FP32 rounding no
 // longer averages out of the gradient (2e-7 to 4e-7 at 55 to 67 pixels, the direct sums 1e-7).
 // UG_MIN_WORK_FP32: where the CUDA-core contractions start to cost more than the grid's fixed launches
-// (an objective with its gradient, 147^2 x 1,904 uv: 81 us directly, 74 through the grid; 128^2 x 960: 59, 66).
-// UG_MIN_WORK_TC, _F8: below them the direct contractions keep what long runs reproduce: their rounding, 1e-6
-// to 1e-5 of the gradient and largest with E4M3 cross terms, is a hundred times the grid's, and a CG run a
-// few iterations on differs by up to 5e-5 with it. They cost little there (256^2 x 960 uv: 86 us directly, 76
-// through the grid; x 8,960: 95, 79; x 21,120: 120, 80; 128^2 x 960: 74, 70).
+// (an objective with its gradient + eight trials, directly and through the grid: 147^2 x 1,904 uv 82 + 100 us, 77 + 42;
+// 128^2 x 1,300 67 + 61, 71 + 38; 128^2 x 960, objective and gradient: 59, 66).
+// UG_MIN_WORK_TC, _F8: not where the times cross (128^2 x 1,300 uv points, below 960 at 256^2), but how far the modes
+// keep the results of their direct sums: those sums' rounding, 1e-6 to 1e-5 of the gradient and largest with E4M3 cross terms, is a
+// hundred times the grid's, and a CG run a few iterations on differs by up to 5e-5 with it. What that costs (the same two
+// times): split-f16 128^2 x 4,480 79 + 42, 76 + 42; 192^2 x 6,000 83 + 55, 79 + 47; 256^2 x 960 86 + 39, 78 + 45; x 8,960
+// 95 + 71, 79 + 48; split-f16/E4M3 256^2 x 21,120 118 + 100, 79 + 48; x 30,000 132 + 129, 82 + 49. From 1.2e9 to 4e9
+// split-f16 is therefore the faster of the two.
 // UG_WIDE_RATIO_TC (SPLIT16), _F8 (SPLIT16F8 and TF32, whose direct forwards cost two thirds): on a wide
 // coverage the grid's y contractions, FP64 on nbx (2 J + 1) grid points, are slower than the tensor cores' direct sums,
 // which the ratio above does not see. One objective with its gradient + eight trials, direct and through the grid, split-f16:

@@ -222,10 +222,13 @@ int gpair_dft_tables(int image_width, int nuv, const gpair_uv *uv, float pixella
 
 /* ---- device contexts ---- */
 
-/* Precision modes. In every mode a problem given by (u, v), at least 96 pixels wide and large
- * enough for its mode goes through a grid of the uv plane (csrc/uvgrid.cu), whose results meet
+/* Precision modes. In every mode a problem given by (u, v), at least 96 pixels wide, large
+ * enough for its mode and (GPAIR_PREC_SPLIT16, TF32, SPLIT16F8) not too wide in its coverage goes
+ * through a grid of the uv plane (csrc/uvgrid.cu; gpair_uv_grid tells), whose results meet
  * the mode's bounds; the operands below are then those of its x contraction (GPAIR_PREC_SPLIT16F8:
- * as GPAIR_PREC_SPLIT16), the other stages FP32 products with FP64 sums. */
+ * as GPAIR_PREC_SPLIT16), the other stages FP32 products with FP64 sums between them. "Large enough" is 2 N^2 nuv
+ * >= 4e7 in FP32, 1.2e9 in the tensor modes, 4e9 in GPAIR_PREC_SPLIT16F8: between the last two (256^2: 9,156
+ * to 30,517 uv points) GPAIR_PREC_SPLIT16 is on the grid, and the faster and the more accurate of the two. */
 #define GPAIR_PREC_FP32 0     /* CUDA-core FP32 DFT/adjoint (FP32 twiddles) */
 #define GPAIR_PREC_SPLIT16 1  /* tcgen05 f16 hi+lo split operands, 3 products, FP32 accumulate */
 #define GPAIR_PREC_TF32 2     /* tcgen05 kind::tf32, TF32 operands, 1 product, FP32 accumulate */
