@@ -356,15 +356,15 @@ def combine_over_ranks(times, work, device=None):
 
 def many_instances(n: int, iters: int, precision: int) -> dict:
     """n independent reconstructions of uneven size (widths 64-256, 500-8,000 uv)
-    for `iters` batched-line-search CG iterations each: one after another, all
-    at once through gpair_cg_run_many (each context's graph on its own stream),
+    for `iters` batched-line-search CG iterations each: one after another, in one
+    call of gpair_cg_run_many (each context's graph on its own stream, in a line),
     (with one precision path and tile layout for all, chosen by timing staged batches,
     and gpair_set_shared_splits: the adjoint split-K lengths for instances that
     share the GPU) and as one graph launch (gpair_batch_run) in three layouts: the staged lockstep
     batch (every stage of an iteration one launch over all instances, every
     contraction one grouped tcgen05 launch per class), the lockstep batch with
-    grouped trial forwards only, and every CG loop an independent branch of the
-    graph. Host wall clock; problem loading and graph capture are outside the
+    grouped trial forwards only, and every CG loop a node of its own, one after
+    another. Host wall clock; problem loading and graph capture are outside the
     timings."""
     import gpair_b200 as g
     from gpair_b200.instances import instances

@@ -170,6 +170,7 @@ def lib() -> C.CDLL:
         L.gpair_batch_create_ex.argtypes = [C.POINTER(vp), C.POINTER(vp), i, i, i]
         L.gpair_batch_grouped.argtypes = [vp]
         L.gpair_batch_prep_passes.argtypes = [vp]
+        L.gpair_batch_branches.argtypes = [vp]
         L.gpair_batch_stage_stamps.argtypes = [vp, vp, i, i]
         L.gpair_batch_run.argtypes = [vp, C.POINTER(CgParams), C.POINTER(CgResult)]
         L.gpair_batch_destroy.argtypes = [vp]
@@ -670,8 +671,9 @@ def _result_dict(res: CgResult) -> dict:
 
 
 def cg_many(recs, iterations: int, method: int = 2, alpha: Optional[float] = None, resume: bool = False, **kw):
-    """The same CG run on several contexts at once (gpair_cg_run_many): each
-    context's graph runs on its own stream. Returns one result dict per context."""
+    """The same CG run on several contexts in one call (gpair_cg_run_many): each
+    context's graph runs on its own stream, after the one before it. Returns one
+    result dict per context."""
     L = lib()
     n = len(recs)
     prm = CgParams()
@@ -744,8 +746,9 @@ class Batch:
     lockstep: `grouped` is 2 when every stage of an iteration is one launch over all
     instances and every contraction one grouped tcgen05 launch per class (staged),
     1 when only the trial forwards are grouped (forwards_only=True, or instances
-    that cannot all be staged), 0 when every context's whole CG loop is an
-    independent branch of the graph (independent=True, or no tensor-core context).
+    that cannot all be staged), 0 when every context keeps its whole CG loop, one
+    after another (independent=True, or no tensor-core context). `branches` is the most
+    nodes of one level of the graph that can start together: 1.
     Build after the contexts hold their problems, images and configuration."""
 
     def __init__(self, recs, line_search: int = LS_BATCH, independent: bool = False, forwards_only: bool = False,
@@ -761,6 +764,7 @@ class Batch:
         self.h = h
         self.grouped = int(self._L.gpair_batch_grouped(self.h))
         self.prep_passes = int(self._L.gpair_batch_prep_passes(self.h))  # 0: not staged
+        self.branches = int(self._L.gpair_batch_branches(self.h))
 
     def run(self, iterations: int, method: int = 2, alpha: Optional[float] = None, resume: bool = False, **kw):
         prm = CgParams()

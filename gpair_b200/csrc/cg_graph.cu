@@ -154,8 +154,9 @@ static cudaGraphNode_t add_conditional(gpair_ctx *c, cudaGraph_t parent, cudaGra
 }
 
 // Adds one context's whole CG loop (the WHILE node and its bodies) to `parent`.
-// G carries the loop's line-search mode, trace buffer and launch counts.
-static int add_loop(gpair_ctx *c, CgGraph *G, cudaGraph_t parent)
+// G carries the loop's line-search mode, trace buffer and launch counts. `after`
+// (or nullptr) is the node that the loop waits for; `node` receives the WHILE node.
+static int add_loop(gpair_ctx *c, CgGraph *G, cudaGraph_t parent, cudaGraphNode_t after, cudaGraphNode_t *node)
 {
     if (c->precision != GPAIR_PREC_FP32) {
         int rc = gp_tc_prepare(c);  // operand buffers must exist before capture
@@ -173,8 +174,9 @@ static int add_loop(gpair_ctx *c, CgGraph *G, cudaGraph_t parent)
     cudaGraphConditionalHandle h_iter, h_ls, h_grad;
     GP_CUDA(c, cudaGraphConditionalHandleCreate(&h_iter, parent, 1, cudaGraphCondAssignDefault));
     cudaGraph_t B1, B2, B3;
-    add_conditional(c, parent, h_iter, cudaGraphCondTypeWhile, &B1, &rc);
+    *node = add_conditional(c, parent, h_iter, cudaGraphCondTypeWhile, &B1, &rc);
     if (rc) return rc;
+    if (after) GP_CUDA(c, cudaGraphAddDependencies(parent, &after, node, 1));
     GP_CUDA(c, cudaGraphConditionalHandleCreate(&h_ls, B1, 0, 0));
     cudaGraphNode_t n_ls = add_conditional(c, B1, h_ls, cudaGraphCondTypeWhile, &B2, &rc);
     if (rc) return rc;
@@ -217,7 +219,8 @@ static int build_into(gpair_ctx *c, CgGraph *G)
 {
     GP_CUDA(c, cudaMalloc(&G->trace, sizeof(double) * 5 * (size_t)G->trace_cap));
     GP_CUDA(c, cudaGraphCreate(&G->g, 0));
-    int rc = add_loop(c, G, G->g);
+    cudaGraphNode_t loop;
+    int rc = add_loop(c, G, G->g, nullptr, &loop);
     G->buf_gen = c->buf_gen;
     if (!rc) {
         cudaError_t e = cudaGraphInstantiate(&G->exec, G->g, 0);
@@ -247,15 +250,22 @@ static int build(gpair_ctx *c, int trace_cap, int ls_mode)
 
 // ------------------------------------------------ many contexts, one graph
 //
-// One graph holding every context's whole CG loop as an independent branch
-// (each a WHILE node with its own conditional handles), so that one launch
-// runs all the reconstructions and the device schedules their kernels side
-// by side.
+// One graph holding every context's whole CG loop (each a WHILE node with its
+// own conditional handles), so that one launch runs all the reconstructions.
+//
+// No two instances' chains of kernels are in flight together, in any layout:
+// every level of the graph is one line of nodes (gp_batch_graph_branches is 1).
+// With the chains of 64 instances side by side a launch now and then never
+// ended: one instance's chain stopped between two of its kernels, with no
+// wait that gave up and the other 63 done. What stops it is not known; chains
+// in a line leave it out. The staged layout, which fills the GPU with one
+// launch per stage, is a line by itself and was never seen to stop.
 struct BatchGraph {
     int n;
     cudaGraph_t g;
     cudaGraphExec_t exec;
     CgGraph *loops;  // per context: mode, trace buffer, launch counts (no graph of its own)
+    int branches;    // the most nodes of one level that can start together
     // lockstep batch with grouped forwards (instances in lockstep order: by class)
     int grouped;
     int ngrp;
@@ -342,7 +352,7 @@ void gp_batch_graph_free(void *bg)
 //   [route INIT]   act[i] = 1
 //   WHILE (h_any_iter)
 //     [route BEGIN]  h_pre[i] = h_post[i] = act[i]
-//     IF (h_pre[i])  criterion + gradient + direction of instance i   (each i, side by side)
+//     IF (h_pre[i])  criterion + gradient + direction of instance i   (each i, one after another)
 //     [route LS0]    ls[i] = act[i] and the line search of i goes on; h_any_ls
 //     WHILE (h_any_ls)
 //       trial images + operands of instance i, if ls[i]              (each tensor i)
@@ -459,8 +469,26 @@ static int lockstep_route(BatchGraph *B, gpair_ctx *c, int what, cudaGraphCondit
     return add_child(c, parent, g, deps, ndeps, node);
 }
 
+// raises *most to the most nodes of `g` (one level) that can start together: its
+// roots, or the nodes that wait for one and the same node
+static int count_branches(gpair_ctx *c, cudaGraph_t g, int *most)
+{
+    size_t nn = 0, nr = 0;
+    GP_CUDA(c, cudaGraphGetRootNodes(g, nullptr, &nr));
+    GP_CUDA(c, cudaGraphGetNodes(g, nullptr, &nn));
+    std::vector<cudaGraphNode_t> nodes(nn);
+    if (nn) GP_CUDA(c, cudaGraphGetNodes(g, nodes.data(), &nn));
+    if ((int)nr > *most) *most = (int)nr;
+    for (cudaGraphNode_t nd : nodes) {
+        size_t nd_out = 0;
+        GP_CUDA(c, cudaGraphNodeGetDependentNodes(nd, nullptr, &nd_out));
+        if ((int)nd_out > *most) *most = (int)nd_out;
+    }
+    return GPAIR_OK;
+}
+
 // GPAIR_ERR_STATE: no instance can take part in a grouped forward (the caller
-// builds the independent branches instead)
+// builds the instances' whole loops instead, one after another)
 static int build_lockstep(gpair_ctx **ctx_in, int n, BatchGraph *B)
 {
     // lockstep order: tensor instances by class (stable), then the CUDA-core ones
@@ -531,12 +559,12 @@ static int build_lockstep(gpair_ctx **ctx_in, int n, BatchGraph *B)
         cudaGraph_t body, s = nullptr;
         pre[k] = add_conditional(ctx[k], B1, hh[k], cudaGraphCondTypeIf, &body, &rc);
         if (rc) return rc;
-        GP_CUDA(c0, cudaGraphAddDependencies(B1, &n_begin, &pre[k], 1));
+        GP_CUDA(c0, cudaGraphAddDependencies(B1, k ? &pre[k - 1] : &n_begin, &pre[k], 1));
         if ((rc = capture(ctx[k], G, SEQ_PRE, 0, 0, 0, &s, &G->n_pre))) return rc;
         cudaGraphNode_t nn;
         if ((rc = add_child(ctx[k], body, s, nullptr, 0, &nn))) return rc;
     }
-    if ((rc = lockstep_route(B, c0, GR_LS0, h_ls, B1, pre.data(), pre.size(), &n_ls0))) return rc;
+    if ((rc = lockstep_route(B, c0, GR_LS0, h_ls, B1, &pre[n - 1], 1, &n_ls0))) return rc;
     n_lsw = add_conditional(c0, B1, h_ls, cudaGraphCondTypeWhile, &B2, &rc);
     if (rc) return rc;
     GP_CUDA(c0, cudaGraphAddDependencies(B1, &n_ls0, &n_lsw, 1));
@@ -545,25 +573,30 @@ static int build_lockstep(gpair_ctx **ctx_in, int n, BatchGraph *B)
         cudaGraph_t body, s = nullptr;
         post[k] = add_conditional(ctx[k], B1, hh[n + k], cudaGraphCondTypeIf, &body, &rc);
         if (rc) return rc;
-        GP_CUDA(c0, cudaGraphAddDependencies(B1, &n_lsw, &post[k], 1));
+        GP_CUDA(c0, cudaGraphAddDependencies(B1, k ? &post[k - 1] : &n_lsw, &post[k], 1));
         if ((rc = capture(ctx[k], G, SEQ_POST, 0, 0, 0, &s, &G->n_post))) return rc;
         cudaGraphNode_t nn;
         if ((rc = add_child(ctx[k], body, s, nullptr, 0, &nn))) return rc;
     }
-    if ((rc = lockstep_route(B, c0, GR_END, h_iter, B1, post.data(), post.size(), &n_end))) return rc;
+    if ((rc = lockstep_route(B, c0, GR_END, h_iter, B1, &post[n - 1], 1, &n_end))) return rc;
 
     // B2: per class, the trial prep of its instances, its grouped forward, their
-    // chi2 + controller; the CUDA-core instances' whole evaluations; LSN after all
-    std::vector<cudaGraphNode_t> last;  // what LSN waits for
+    // chi2 + controller; the CUDA-core instances' whole evaluations; LSN after all.
+    // Each node waits for the one before it.
+    cudaGraphNode_t last = nullptr;
+    auto add_last = [&](gpair_ctx *c, cudaGraph_t s) {
+        cudaGraphNode_t nd;
+        const int r = add_child(c, B2, s, &last, last ? 1 : 0, &nd);
+        if (!r) last = nd;
+        return r;
+    };
     for (int q = 0; q < B->ngrp && !rc; q++) {
         const int k0 = cls_begin[q], k1 = cls_begin[q + 1];
-        std::vector<cudaGraphNode_t> bprep;
         for (int k = k0; k < k1 && !rc; k++) {
             gpair_ctx *c = ctx[k];
             CgGraph *G = &B->loops[order[k]];
             const int *gate = B->flags + n + k;
             cudaGraph_t s = nullptr;
-            cudaGraphNode_t nd;
             rc = capture_fn(
                 c,
                 [&]() {
@@ -573,15 +606,13 @@ static int build_lockstep(gpair_ctx **ctx_in, int n, BatchGraph *B)
                     return r;
                 },
                 &s, &G->n_crit);
-            if (rc || (rc = add_child(c, B2, s, nullptr, 0, &nd))) return rc;
-            bprep.push_back(nd);
+            if (rc || (rc = add_last(c, s))) return rc;
         }
-        cudaGraphNode_t n_gemm;
         {
             gpair_ctx *c = ctx[k0];
             cudaGraph_t s = nullptr;
             rc = capture_fn(c, [&]() { return gp_tc_group_forward(B->grps[q], c); }, &s, nullptr);
-            if (rc || (rc = add_child(c, B2, s, bprep.data(), bprep.size(), &n_gemm))) return rc;
+            if (rc || (rc = add_last(c, s))) return rc;
         }
         for (int k = k0; k < k1 && !rc; k++) {
             gpair_ctx *c = ctx[k];
@@ -589,7 +620,6 @@ static int build_lockstep(gpair_ctx **ctx_in, int n, BatchGraph *B)
             const int *gate = B->flags + n + k;
             cudaGraph_t s = nullptr;
             int n2 = 0;
-            cudaGraphNode_t nd;
             rc = capture_fn(
                 c,
                 [&]() {
@@ -602,9 +632,8 @@ static int build_lockstep(gpair_ctx **ctx_in, int n, BatchGraph *B)
                     return r;
                 },
                 &s, &n2);
-            if (rc || (rc = add_child(c, B2, s, &n_gemm, 1, &nd))) return rc;
+            if (rc || (rc = add_last(c, s))) return rc;
             G->n_crit += n2;
-            last.push_back(nd);
         }
     }
     for (int k = ntc; k < n && !rc; k++) {
@@ -612,7 +641,6 @@ static int build_lockstep(gpair_ctx **ctx_in, int n, BatchGraph *B)
         CgGraph *G = &B->loops[order[k]];
         const int *gate = B->flags + n + k;
         cudaGraph_t s = nullptr;
-        cudaGraphNode_t nd;
         rc = capture_fn(
             c,
             [&]() {
@@ -625,11 +653,12 @@ static int build_lockstep(gpair_ctx **ctx_in, int n, BatchGraph *B)
                 return r;
             },
             &s, &G->n_crit);
-        if (rc || (rc = add_child(c, B2, s, nullptr, 0, &nd))) return rc;
-        last.push_back(nd);
+        if (rc || (rc = add_last(c, s))) return rc;
     }
     cudaGraphNode_t n_lsn;
-    return lockstep_route(B, c0, GR_LSN, h_ls, B2, last.data(), last.size(), &n_lsn);
+    if ((rc = lockstep_route(B, c0, GR_LSN, h_ls, B2, &last, 1, &n_lsn))) return rc;
+    if ((rc = count_branches(c0, B1, &B->branches))) return rc;
+    return count_branches(c0, B2, &B->branches);
 }
 
 // --------------------------------- staged lockstep batches (every stage grouped)
@@ -878,7 +907,8 @@ static int build_lockstep_staged(gpair_ctx **ctx_in, int n, BatchGraph *B, int w
         B->loops[i].n_grad = 0;
     }
     B->staged = 1;
-    return GPAIR_OK;
+    if ((rc = count_branches(c0, B1, &B->branches))) return rc;
+    return count_branches(c0, B2, &B->branches);
 }
 
 int gp_batch_graph_build(gpair_ctx **ctx, int n, int ls_mode, int allow_group, void **out)
@@ -921,7 +951,9 @@ int gp_batch_graph_build(gpair_ctx **ctx, int n, int ls_mode, int allow_group, v
             rc = cudaGraphCreate(&B->g, 0) == cudaSuccess ? GPAIR_OK : GPAIR_ERR_CUDA;
         }
     }
-    for (int i = 0; i < n && !rc && !B->grouped; i++) rc = add_loop(ctx[i], &B->loops[i], B->g);
+    cudaGraphNode_t loop = nullptr;
+    for (int i = 0; i < n && !rc && !B->grouped; i++) rc = add_loop(ctx[i], &B->loops[i], B->g, loop, &loop);
+    if (!rc) rc = count_branches(ctx[0], B->g, &B->branches);
     for (int i = 0; i < n && !rc; i++) B->loops[i].buf_gen = ctx[i]->buf_gen;
     if (!rc) {
         cudaError_t e = cudaGraphInstantiate(&B->exec, B->g, 0);
@@ -948,6 +980,7 @@ int gp_batch_graph_launch(void *bg, cudaStream_t stream)
 int gp_batch_graph_precision(void *bg, int i) { return ((BatchGraph *)bg)->loops[i].precision; }
 unsigned int gp_batch_graph_buf_gen(void *bg, int i) { return ((BatchGraph *)bg)->loops[i].buf_gen; }
 int gp_batch_graph_grouped(void *bg) { return bg ? ((BatchGraph *)bg)->grouped : 0; }
+int gp_batch_graph_branches(void *bg) { return bg ? ((BatchGraph *)bg)->branches : 0; }
 int gp_batch_graph_prep_passes(void *bg) { return bg && ((BatchGraph *)bg)->staged ? ((BatchGraph *)bg)->prep_passes : 0; }
 
 // the stage stamps of a staged batch (none recorded: 0); `reset` zeroes them

@@ -27,6 +27,7 @@ int gp_batch_graph_launch(void *bg, cudaStream_t stream);
 int gp_batch_graph_precision(void *bg, int i);
 unsigned int gp_batch_graph_buf_gen(void *bg, int i);
 int gp_batch_graph_grouped(void *bg);
+int gp_batch_graph_branches(void *bg);
 int gp_batch_graph_prep_passes(void *bg);
 int gp_batch_graph_stamps(void *bg, unsigned long long *out, int max, cudaStream_t st, int reset);
 long long gp_batch_graph_launches(void *bg, int i, int iterations_done, int criterion_evals, int grad_evals,
@@ -800,8 +801,8 @@ static int read_action(gpair_ctx *c, int *action)
     return GPAIR_OK;
 }
 
-// One CG run in three phases, so that several contexts can have their runs in
-// flight at once (gpair_cg_run_many): prepare (parameters, controller reset,
+// One CG run in three phases, so that several contexts can have their runs
+// queued at once (gpair_cg_run_many): prepare (parameters, controller reset,
 // graph build, start event), launch, finish (end event, wait, results).
 struct CgRun {
     long long launches0;
@@ -1011,6 +1012,7 @@ extern "C" int gpair_batch_create(gpair_batch **out, gpair_ctx **ctx, int n, int
 }
 
 extern "C" int gpair_batch_grouped(const gpair_batch *b) { return b ? gp_batch_graph_grouped(b->graph) : 0; }
+extern "C" int gpair_batch_branches(const gpair_batch *b) { return b ? gp_batch_graph_branches(b->graph) : 0; }
 extern "C" int gpair_batch_prep_passes(const gpair_batch *b) { return b ? gp_batch_graph_prep_passes(b->graph) : 0; }
 
 extern "C" int gpair_batch_stage_stamps(const gpair_batch *b, unsigned long long *ns, int max, int reset)
@@ -1166,7 +1168,19 @@ extern "C" int gpair_cg_run_many(gpair_ctx **ctx, int n, const gpair_cg_params *
         launched = true;
         for (int i = 0; i < n; i++) {
             long long dummy = 0;
-            st[i] = gp_cg_graph_run(ctx[i], p->iterations, 0, p->line_search, &dummy);
+            // after the run before it on the same device: with the loops of 64 contexts in flight
+            // together a call now and then never returned (BatchGraph, cg_graph.cu)
+            int prev = i - 1;
+            while (prev >= 0 && ctx[prev]->device != ctx[i]->device) prev--;
+            cudaError_t e = prev < 0 ? cudaSuccess : cudaStreamWaitEvent(ctx[i]->stream, ctx[prev]->run_e1, 0);
+            if (e == cudaSuccess) e = cudaEventRecord(ctx[i]->run_e0, ctx[i]->stream);  // its time without the wait
+            if (e != cudaSuccess) {
+                snprintf(ctx[i]->last_error, sizeof(ctx[i]->last_error), "run order: %s", cudaGetErrorString(e));
+                cudaGetLastError();
+                st[i] = GPAIR_ERR_CUDA;
+            } else {
+                st[i] = gp_cg_graph_run(ctx[i], p->iterations, 0, p->line_search, &dummy);
+            }
             cg_mark_end(ctx[i]);
         }
     }

@@ -332,10 +332,10 @@ typedef struct {
 } gpair_cg_result;
 
 /* Runs the same CG parameters on n contexts (one problem each, distinct contexts)
- * at once: every context's run is prepared, then every run's graph is launched on
- * its context's stream, then the host waits for all. Small problems that each fill
- * a few SMs run side by side this way (many independent reconstructions, e.g. a
- * survey or a training set). host_loop must be 0; res (length n) may be NULL.
+ * in one call: every context's run is prepared, then every run's graph is launched
+ * on its context's stream, on one device each after the one before it, then the host
+ * waits for all. Many small problems share the GPU in a staged batch (below).
+ * host_loop must be 0; res (length n) may be NULL.
  * Returns the first error; per-run status in res[i].status. */
 int gpair_cg_run_many(gpair_ctx **ctx, int n, const gpair_cg_params *p, gpair_cg_result *res);
 
@@ -365,8 +365,7 @@ int gpair_cg_checkpoint_save(gpair_ctx *ctx, void *buffer, size_t bytes);
 int gpair_cg_checkpoint_load(gpair_ctx *ctx, const void *buffer, size_t bytes);
 
 /* Batched reconstructions: one CUDA graph holds the whole CG loop of every context
- * (each an independent branch with its own conditional nodes), so one graph launch
- * runs all n reconstructions and the device schedules their kernels side by side.
+ * (with its own conditional nodes), so one graph launch runs all n reconstructions.
  * Create after every context holds its problem, image, precision and (optional)
  * autotuned configuration; those are fixed into the graph: rebuild the batch after
  * changing any of them. gpair_batch_run takes the same parameters as gpair_cg_run
@@ -388,8 +387,10 @@ int gpair_cg_checkpoint_load(gpair_ctx *ctx, const void *buffer, size_t bytes);
  *   GPAIR_BATCH_FORWARDS_ONLY): each instance runs its own stage kernels; the
  *   trial forwards of every tensor-core class are grouped launches.
  * Each instance's results are bitwise those of its separate run. Otherwise, or with
- * GPAIR_BATCH_INDEPENDENT, every context's loop is an independent graph branch
- * (gpair_batch_grouped = 0). gpair_batch_run returns GPAIR_ERR_STATE when a
+ * GPAIR_BATCH_INDEPENDENT, every context keeps a loop of its own, one after another
+ * (gpair_batch_grouped = 0). In every layout the graph is a line of nodes: no two
+ * instances' own kernels are in flight together (gpair_batch_branches = 1, the most
+ * nodes of one level that can start together). gpair_batch_run returns GPAIR_ERR_STATE when a
  * context's operand or batch buffers were rebuilt since the batch was created
  * (another precision, tile layout, problem or image size). */
 typedef struct gpair_batch gpair_batch;
@@ -410,6 +411,7 @@ int gpair_batch_create(gpair_batch **batch, gpair_ctx **ctx, int n, int line_sea
 int gpair_batch_create_ex(gpair_batch **batch, gpair_ctx **ctx, int n, int line_search, int flags);
 int gpair_batch_grouped(const gpair_batch *batch);
 int gpair_batch_prep_passes(const gpair_batch *batch);
+int gpair_batch_branches(const gpair_batch *batch);
 /* Stage stamps of a batch created with GPAIR_BATCH_STAGE_STAMPS; returns the
  * number of words (39), or 0 without stamps. Positions 0-18: the device timer
  * (ns) at the pre-phase start, then after the image prep, criterion forwards,
