@@ -327,8 +327,8 @@ int gp_set_problem_core(gpair_ctx *c, int N, float pix, int nuv, const gpair_uv 
         if ((rc = gp_ug_scan(c, uv))) return rc;
     }
     c->have_problem = 1;
-    // the path of the mode, whose kernels run beside the host's sorting of the triangles; with reference
-    // tables (uv == NULL) its tensor operands are built once the tables are on the device
+    // the path of the mode; with reference tables
+    // (uv == NULL) its tensor operands are built once the tables are on the device
     rc = uv ? gp_path_prepare(c) : gp_direct_prepare(c);
     if (!rc) rc = gp_build_incidence(c, uvpnt);
     if (rc) {

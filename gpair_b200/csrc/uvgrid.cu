@@ -344,7 +344,8 @@ static int ug_plan(gpair_ctx *c)
     const long long nt = (long long)nbx * H + (long long)H * (J + 1);
     k_ug_tables<<<gp_cdiv(nt, 256), 256, 0, st>>>(g->invphi, N, H, M, jxf, nbx, J, g->ftab, g->ctab);
     GP_LAUNCH_CHECK(c);
-    return GPAIR_OK;  // the copy has taken the host's arrays, pageable memory, before it returned
+    GP_CUDA(c, cudaStreamSynchronize(st));  // the host's arrays end here
+    return GPAIR_OK;
 }
 
 int gp_ug_choose(gpair_ctx *c)
